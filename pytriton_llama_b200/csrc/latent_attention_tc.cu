@@ -1,0 +1,460 @@
+// Attention over kept rows [latent (R) | rotated key part (n)] that all heads share (parts/latent_attention.py), bfloat16 on
+// the tensor cores, straight from the paged cache: the latent is the key's first R entries and the value.
+//   out[t, h, :] = sum_j softmax_j(scale * q[t, h, :] . row_j) * row_j[:R],   j <= position of t
+// q [T, H * (R + n)], out [T, H * R].  Two kernels share the layout: a row of 16-byte packets in shared memory has one packet
+// more than an even number, so that the eight rows of an ldmatrix start in different banks.
+//
+// latent_prefill: portions of prompts.  The rows of q, (token, head) after (token, head), are one matrix: a block takes 64 of
+// them from a tile of the step's list (128 tokens of one request) and walks the keys up to its last token's position in
+// tiles of 32, a ring of three; eight warps, four row groups by two: for the scores the two split the tile's keys, for the
+// weighted sums the latent's columns, the weights (rounded once to bfloat16, as the softmax over stored scores
+// did) pass through shared memory.  Bound by the warp-level tensor instructions and the fragments read for them, 434 KB per 64 x 32 scores; eight
+// prompts of 65 to 440 tokens (8 heads, R 512, n 64): 68 us a layer.
+//
+// latent_decode: single tokens, all heads of a token (up to 16 per block) against a share of its keys, 64 at a time, two
+// tiles in flight; the float32 weights go to the tensor cores as three bfloat16 terms each (24 bits), so that nothing of
+// them is lost; shares are merged by latent_merge.  Bound by the latency of a tile at eight requests of 1,000 positions: one
+// tile a block, 7.6 us and 7.8 us for the merge.
+//
+// For R of 128, 256 and 512 both replace what was there: per request a gather, two library products around a softmax kernel
+// (260 us of kernels a layer for the eight prompts above, and more launches than the host keeps up with: the whole step of
+// four such layers 5.52 -> 2.61 ms), and for decoding the CUDA-core kernel with a warp per token, head and share (48 + 30 us
+// a layer with dependent launches; a step of eight 731 -> 536 us).
+#include "mma_utils.cuh"
+
+namespace ptl {
+
+constexpr int kLpRows = 64, kLpKeys = 32, kLpStages = 3, kLpThreads = 256;
+constexpr int kLdKeys = 64, kLdStages = 2, kLdThreads = 256, kLdHeads = 16;
+
+__host__ __device__ constexpr int latent_row_bytes(int d) { return d * 2 + 16; }      // d a multiple of 16
+constexpr int kLpWeightBytes = kLpKeys * 2 + 16;
+
+// The packets of `rows` keys from `first` on into shared memory, zeros for keys from `limit` on and for pages not held;
+// eight threads per key.
+template <int KEYS>
+__device__ __forceinline__ void latent_fetch(uint32_t dst, const __nv_bfloat16* __restrict__ cache, const int* __restrict__ bt, int first,
+                                             int limit, int d, int page_size, int num_pages) {
+  constexpr int PASSES = KEYS / 32;      // 256 threads
+  const int sub = threadIdx.x & 7;
+#pragma unroll
+  for (int i = 0; i < PASSES; ++i) {
+    const int row = (threadIdx.x >> 3) + 32 * i, key = first + row;
+    const int page = key < limit ? bt[key / page_size] : -1;
+    const bool ok = page >= 0 && page < num_pages;
+    const __nv_bfloat16* src = ok ? cache + ((size_t)page * page_size + key % page_size) * d : cache;
+    const uint32_t to = dst + row * latent_row_bytes(d);
+    for (int c = sub; c < d / 8; c += 8) cp_async_16(to + 16 * c, src + (ok ? 8 * c : 0), ok);
+  }
+}
+
+template <int R>
+__global__ void __launch_bounds__(kLpThreads, 1)
+latent_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
+                      const int* __restrict__ block_table, const int* __restrict__ tiles, int bt_stride, int H, int d, int page_size,
+                      int num_pages, float scale_log2) {
+  extern __shared__ __align__(128) unsigned char lp_smem[];
+  __shared__ float s_max[2][kLpRows];
+  __shared__ float s_sum[2][kLpRows];
+  const int* tile = tiles + 4 * blockIdx.y;                       // request row, first token row, tokens, first position (inputs of the step)
+  const int req = tile[0], token0 = tile[1], tokens = tile[2], pos0 = tile[3];
+  const int row0 = ((int)gridDim.x - 1 - (int)blockIdx.x) * kLpRows;      // the rows that see most keys first
+  const int rows = tokens * H;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (req < 0 || row0 >= rows) return;
+  const int ld = latent_row_bytes(d);
+  const uint32_t sq = smem_u32(lp_smem), sk = sq + kLpRows * ld, sp = sk + kLpStages * kLpKeys * ld;
+  const int* bt = block_table + (size_t)req * bt_stride;
+  const int last_row = min(row0 + kLpRows, rows) - 1;
+  const int keys = pos0 + last_row / H + 1;                       // keys that the block's last token sees
+  const int n_tiles = (keys + kLpKeys - 1) / kLpKeys;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c2 = (lane & 3) * 2;
+  const int wm = warp & 3, wn = warp >> 2;                        // row group of 16, half of the keys / of the columns
+
+  const __nv_bfloat16* q0 = q + ((size_t)token0 * H + row0) * d;
+  for (int idx = tid; idx < kLpRows * (d / 8); idx += kLpThreads) {
+    const int r = idx / (d / 8), c = idx % (d / 8);
+    const bool ok = row0 + r < rows;
+    cp_async_16(sq + r * ld + 16 * c, q0 + (ok ? (size_t)r * d + 8 * c : 0), ok);
+  }
+  cp_async_commit();
+#pragma unroll
+  for (int s = 0; s < kLpStages - 1; ++s) {
+    if (s < n_tiles) latent_fetch<kLpKeys>(sk + s * kLpKeys * ld, cache, bt, s * kLpKeys, keys, d, page_size, num_pages);
+    cp_async_commit();
+  }
+  // rows of this thread: wm * 16 + g and + 8; a row past the end sees what the last one sees and is not stored
+  int pos[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) pos[i] = pos0 + min(row0 + wm * 16 + g + 8 * i, rows - 1) / H;
+  constexpr int NT = R / 16;                                      // 8-column blocks of a warp's half of the latent
+  float o[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+  const int lm_row = lane & 15, lm_half = lane >> 4;              // rows and packet of an ldmatrix.x4 of 16 x 16
+
+  for (int t = 0; t < n_tiles; ++t) {
+    cp_async_wait<kLpStages - 2>();
+    __syncthreads();
+    if (t + kLpStages - 1 < n_tiles)
+      latent_fetch<kLpKeys>(sk + ((t + kLpStages - 1) % kLpStages) * kLpKeys * ld, cache, bt, (t + kLpStages - 1) * kLpKeys, keys, d,
+                            page_size, num_pages);
+    cp_async_commit();
+    const uint32_t kt = sk + (t % kLpStages) * kLpKeys * ld;
+    // scores of 16 rows and 16 keys
+    float s[2][4];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
+    const uint32_t qa = sq + (wm * 16 + lm_row) * ld + 16 * lm_half;
+    const uint32_t ka = kt + (wn * 16 + (lane & 7) + 8 * lm_half) * ld + 16 * ((lane >> 3) & 1);
+#pragma unroll 4
+    for (int k = 0; k < d / 16; ++k) {
+      uint32_t a[4], b[4];
+      ldmatrix_x4(a, qa + 32 * k);
+      ldmatrix_x4(b, ka + 32 * k);
+      mma_bf16_16816(s[0], a, b[0], b[1]);
+      mma_bf16_16816(s[1], a, b[2], b[3]);
+    }
+    // to base 2, the causal bound, the rows' maxima over both halves of the keys
+    float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int key = t * kLpKeys + wn * 16 + j * 8 + c2 + (e & 1);
+        s[j][e] = key <= pos[e >> 1] ? s[j][e] * scale_log2 : -INFINITY;
+        mx[e >> 1] = fmaxf(mx[e >> 1], s[j][e]);
+      }
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 1));
+      mx[i] = fmaxf(mx[i], __shfl_xor_sync(0xffffffffu, mx[i], 2));
+    }
+    if ((lane & 3) == 0) {
+      s_max[wn][wm * 16 + g] = mx[0];
+      s_max[wn][wm * 16 + g + 8] = mx[1];
+    }
+    __syncthreads();
+    float alpha[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float now = fmaxf(m[i], fmaxf(mx[i], s_max[wn ^ 1][wm * 16 + g + 8 * i]));      // (key 0 is in the first tile: finite)
+      alpha[i] = exp2f(m[i] - now);
+      m[i] = now;
+      l[i] *= alpha[i];
+    }
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      float p[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        p[e] = exp2f(s[j][e] - m[e >> 1]);
+        l[e >> 1] += p[e];
+      }
+      const uint32_t at = sp + (wm * 16 + g) * kLpWeightBytes + (wn * 16 + j * 8 + c2) * 2;
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(pack_bf16(p[0], p[1])) : "memory");
+      asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + 8 * kLpWeightBytes), "r"(pack_bf16(p[2], p[3])) : "memory");
+    }
+    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        o[j][0] *= alpha[0]; o[j][1] *= alpha[0];
+        o[j][2] *= alpha[1]; o[j][3] *= alpha[1];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kLpKeys / 16; ++k) {
+      uint32_t a[4];
+      ldmatrix_x4(a, sp + (wm * 16 + lm_row) * kLpWeightBytes + 32 * k + 16 * lm_half);
+      const uint32_t va = kt + (16 * k + lm_row) * ld + wn * R + 16 * lm_half;       // (R bytes: half of the latent's columns)
+#pragma unroll
+      for (int j = 0; j < NT; j += 2) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, va + 16 * j);
+        mma_bf16_16816(o[j], a, b[0], b[1]);
+        mma_bf16_16816(o[j + 1], a, b[2], b[3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
+    l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
+  }
+  if ((lane & 3) == 0) {
+    s_sum[wn][wm * 16 + g] = l[0];
+    s_sum[wn][wm * 16 + g + 8] = l[1];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int row = wm * 16 + g + 8 * i;
+    if (row0 + row >= rows) continue;
+    const float inv = 1.0f / (s_sum[0][row] + s_sum[1][row]);
+    __nv_bfloat16* dst = out + ((size_t)token0 * H + row0 + row) * R + wn * (R / 2) + c2;
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+      *reinterpret_cast<uint32_t*>(dst + 8 * j) = pack_bf16(o[j][2 * i] * inv, o[j][2 * i + 1] * inv);
+  }
+}
+
+// part [items][splits][H][R] float32 (not yet divided), ml [items][splits][H][2] (maximum to base 2, sum); with one share the
+// result itself.
+template <int R>
+__global__ void __launch_bounds__(kLdThreads, 1)
+latent_decode_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part, float* __restrict__ ml, const __nv_bfloat16* __restrict__ q,
+                     const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table, const int* __restrict__ tok_req,
+                     const int* __restrict__ positions, const int* __restrict__ items, int bt_stride, int H, int d, int page_size,
+                     int num_pages, int splits, float scale_log2) {
+  extern __shared__ __align__(128) unsigned char ld_smem[];
+  __shared__ float s_scores[kLdHeads][kLdKeys + 4];
+  __shared__ __align__(16) __nv_bfloat16 s_w[3][kLdHeads][kLdKeys + 8];
+  __shared__ float s_alpha[kLdHeads], s_m[kLdHeads], s_l[kLdHeads];
+  const int item = blockIdx.y, split = blockIdx.x, h0 = blockIdx.z * kLdHeads;
+  const int token = items ? items[item] : item;                   // inputs of the step
+  const int req = tok_req[token], keys_all = positions[token] + 1;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (req < 0) return;
+  const int heads = min(kLdHeads, H - h0);
+  // whole tiles of 64 keys per share; a share without keys leaves a sum of zero
+  const int n_all = (keys_all + kLdKeys - 1) / kLdKeys;
+  const int each = (n_all + splits - 1) / splits;
+  const int tile0 = split * each, n_tiles = max(0, min(each, n_all - tile0));
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c2 = (lane & 3) * 2;
+  const size_t at = ((size_t)item * splits + split) * H + h0;
+  if (n_tiles == 0) {
+    if (tid < heads) { ml[2 * (at + tid)] = -INFINITY; ml[2 * (at + tid) + 1] = 0.f; }
+    return;
+  }
+  const int ld = latent_row_bytes(d);
+  const uint32_t sq = smem_u32(ld_smem), sk = sq + kLdHeads * ld;
+  const int* bt = block_table + (size_t)req * bt_stride;
+  const __nv_bfloat16* q0 = q + ((size_t)token * H + h0) * d;
+  for (int idx = tid; idx < kLdHeads * (d / 8); idx += kLdThreads) {
+    const int r = idx / (d / 8), c = idx % (d / 8);
+    const bool ok = r < heads;
+    cp_async_16(sq + r * ld + 16 * c, q0 + (ok ? (size_t)r * d + 8 * c : 0), ok);
+  }
+#pragma unroll
+  for (int s = 0; s < kLdStages - 1; ++s) {
+    if (s < n_tiles) latent_fetch<kLdKeys>(sk + s * kLdKeys * ld, cache, bt, (tile0 + s) * kLdKeys, keys_all, d, page_size, num_pages);
+    cp_async_commit();
+  }
+  if (tid < kLdHeads) { s_m[tid] = -INFINITY; s_l[tid] = 0.f; }
+  constexpr int NT = R / 64;                                      // 8-column blocks of a warp's eighth of the latent
+  float o[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+  const int lm_row = lane & 15, lm_half = lane >> 4;
+
+  for (int t = 0; t < n_tiles; ++t) {
+    __syncthreads();                                              // the stage that is filled next has been read
+    if (t + kLdStages - 1 < n_tiles)
+      latent_fetch<kLdKeys>(sk + ((t + kLdStages - 1) % kLdStages) * kLdKeys * ld, cache, bt, (tile0 + t + kLdStages - 1) * kLdKeys,
+                            keys_all, d, page_size, num_pages);
+    cp_async_commit();
+    cp_async_wait<kLdStages - 1>();
+    __syncthreads();
+    const uint32_t kt = sk + (t % kLdStages) * kLdKeys * ld;
+    // scores of all heads and 8 keys per warp; two products at a time, k ranges side by side in one ldmatrix of the keys
+    float s0[4] = {0.f, 0.f, 0.f, 0.f}, s1[4] = {0.f, 0.f, 0.f, 0.f};
+    const uint32_t qa = sq + lm_row * ld + 16 * lm_half;
+    const uint32_t ka = kt + (warp * 8 + (lane & 7)) * ld + 16 * (lane >> 3);
+    int k = 0;
+#pragma unroll 4
+    for (; k + 1 < d / 16; k += 2) {
+      uint32_t a[4], a1[4], b[4];
+      ldmatrix_x4(b, ka + 32 * k);
+      ldmatrix_x4(a, qa + 32 * k);
+      ldmatrix_x4(a1, qa + 32 * k + 32);
+      mma_bf16_16816(s0, a, b[0], b[1]);
+      mma_bf16_16816(s1, a1, b[2], b[3]);
+    }
+    if (k < d / 16) {                                             // an odd number of 16s: the last packet pair alone
+      uint32_t a[4], b[4];
+      ldmatrix_x4(b, kt + (warp * 8 + (lane & 7)) * ld + 32 * k + 16 * ((lane >> 3) & 1));
+      ldmatrix_x4(a, qa + 32 * k);
+      mma_bf16_16816(s0, a, b[0], b[1]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int col = warp * 8 + c2 + (e & 1);
+      const bool seen = (tile0 + t) * kLdKeys + col < keys_all;
+      s_scores[g + 8 * (e >> 1)][col] = seen ? (s0[e] + s1[e]) * scale_log2 : -INFINITY;
+    }
+    __syncthreads();
+    // two heads per warp: maximum, weights (three bfloat16 terms each), sum
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int h = warp * 2 + i;
+      const float a = s_scores[h][lane], b = s_scores[h][lane + 32];
+      const float before = s_m[h];
+      const float now = fmaxf(before, warp_max(fmaxf(a, b)));
+      const float p[2] = {exp2f(a - now), exp2f(b - now)};
+      const float sum = warp_sum(p[0] + p[1]);
+      if (lane == 0) {
+        const float alpha = exp2f(before - now);
+        s_alpha[h] = alpha;
+        s_m[h] = now;
+        s_l[h] = s_l[h] * alpha + sum;
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float rest = p[e];
+#pragma unroll
+        for (int w = 0; w < 3; ++w) {
+          const __nv_bfloat16 term = __float2bfloat16_rn(rest);
+          s_w[w][h][lane + 32 * e] = term;
+          rest -= __bfloat162float(term);
+        }
+      }
+    }
+    __syncthreads();
+    const float al0 = s_alpha[g], al1 = s_alpha[g + 8];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      o[j][0] *= al0; o[j][1] *= al0;
+      o[j][2] *= al1; o[j][3] *= al1;
+    }
+#pragma unroll
+    for (int kk = 0; kk < kLdKeys / 16; ++kk) {
+      uint32_t a[3][4];
+#pragma unroll
+      for (int w = 0; w < 3; ++w) ldmatrix_x4(a[w], smem_u32(&s_w[w][lm_row][16 * kk + 8 * lm_half]));
+      const uint32_t va = kt + (16 * kk + lm_row) * ld + warp * (R / 8) * 2 + 16 * lm_half;
+#pragma unroll
+      for (int j = 0; j < NT; j += 2) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, va + 16 * j);
+#pragma unroll
+        for (int w = 2; w >= 0; --w) {
+          mma_bf16_16816(o[j], a[w], b[0], b[1]);
+          mma_bf16_16816(o[j + 1], a[w], b[2], b[3]);
+        }
+      }
+    }
+  }
+  const int col0 = warp * (R / 8) + c2;
+  if (splits == 1) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int h = g + 8 * i;
+      if (h >= heads) continue;
+      const float inv = 1.0f / s_l[h];
+      __nv_bfloat16* dst = out + ((size_t)token * H + h0 + h) * R + col0;
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+        *reinterpret_cast<uint32_t*>(dst + 8 * j) = pack_bf16(o[j][2 * i] * inv, o[j][2 * i + 1] * inv);
+    }
+    return;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int h = g + 8 * i;
+    if (h >= heads) continue;
+    float* dst = part + (at + h) * R + col0;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) *reinterpret_cast<float2*>(dst + 8 * j) = make_float2(o[j][2 * i], o[j][2 * i + 1]);
+  }
+  if (tid < heads) { ml[2 * (at + tid)] = s_m[tid]; ml[2 * (at + tid) + 1] = s_l[tid]; }
+}
+
+// One block per (item, head): the shares' sums weighted by 2^(their maximum - the largest), R / 4 threads of four columns.
+__global__ void __launch_bounds__(128)
+latent_merge_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ part, const float* __restrict__ ml,
+                    const int* __restrict__ tok_req, const int* __restrict__ items, int H, int R, int splits) {
+  const int item = blockIdx.y, h = blockIdx.x;
+  const int token = items ? items[item] : item;
+  const bool held = tok_req[token] >= 0;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (!held) return;
+  const size_t at = (size_t)item * splits * H + h;
+  float top = -INFINITY;
+  for (int s = 0; s < splits; ++s) top = fmaxf(top, ml[2 * (at + (size_t)s * H)]);
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+  float l = 0.f;
+#pragma unroll 8
+  for (int s = 0; s < splits; ++s) {
+    const float m = ml[2 * (at + (size_t)s * H)];
+    if (m == -INFINITY) continue;                                 // no keys: nothing was written
+    const float w = exp2f(m - top);
+    l = fmaf(w, ml[2 * (at + (size_t)s * H) + 1], l);
+    const float4 v = *reinterpret_cast<const float4*>(part + (at + (size_t)s * H) * R + 4 * threadIdx.x);
+    sum.x = fmaf(w, v.x, sum.x); sum.y = fmaf(w, v.y, sum.y);
+    sum.z = fmaf(w, v.z, sum.z); sum.w = fmaf(w, v.w, sum.w);
+  }
+  const float inv = 1.0f / l;
+  uint2 packed = make_uint2(pack_bf16(sum.x * inv, sum.y * inv), pack_bf16(sum.z * inv, sum.w * inv));
+  *reinterpret_cast<uint2*>(out + ((size_t)token * H + h) * R + 4 * threadIdx.x) = packed;
+}
+
+// What both kernels ask of sizes and addresses; -2: take another path.
+inline bool latent_tc_fits(const void* out, const void* q, const void* cache, int H, int R, int n) {
+  return (R == 128 || R == 256 || R == 512) && n >= 0 && n % 16 == 0 && n <= 64 && H > 0 && H <= 512 && aligned16(out) && aligned16(q) &&
+         aligned16(cache);
+}
+
+template <int R>
+int latent_prefill(void* out, const void* q, const void* cache, const int* bt, const int* tiles, int n_tiles, int bt_stride, int H, int d,
+                   int page_size, int num_pages, float scale, int tile_tokens, void* stream) {
+  const int smem = (kLpRows + kLpStages * kLpKeys) * latent_row_bytes(d) + kLpRows * kLpWeightBytes;
+  static SmemRaised raised;
+  if (int rc = raise_shared_memory("latent_prefill", latent_prefill_kernel<R>, 200 * 1024, raised)) return rc;
+  const dim3 grid((tile_tokens * H + kLpRows - 1) / kLpRows, n_tiles);
+  return launch_kernel("latent_prefill", latent_prefill_kernel<R>, grid, dim3(kLpThreads), smem, as_stream(stream), (__nv_bfloat16*)out,
+                       (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, tiles, bt_stride, H, d, page_size, num_pages,
+                       scale * 1.4426950408889634f);
+}
+
+template <int R>
+int latent_decode(void* out, float* part, float* ml, const void* q, const void* cache, const int* bt, const int* tok_req, const int* positions,
+                  const int* items, int n_items, int bt_stride, int H, int d, int page_size, int num_pages, int splits, float scale,
+                  void* stream) {
+  const int smem = (kLdHeads + kLdStages * kLdKeys) * latent_row_bytes(d);
+  static SmemRaised raised;
+  if (int rc = raise_shared_memory("latent_decode", latent_decode_kernel<R>, 200 * 1024, raised)) return rc;
+  const dim3 grid(splits, n_items, (H + kLdHeads - 1) / kLdHeads);
+  if (int rc = launch_kernel("latent_decode", latent_decode_kernel<R>, grid, dim3(kLdThreads), smem, as_stream(stream), (__nv_bfloat16*)out,
+                             part, ml, (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, tok_req, positions, items, bt_stride, H, d,
+                             page_size, num_pages, splits, scale * 1.4426950408889634f))
+    return rc;
+  if (splits == 1) return 0;
+  return launch_kernel("latent_merge", latent_merge_kernel, dim3(H, n_items), dim3(R / 4), 0, as_stream(stream), (__nv_bfloat16*)out, part,
+                       ml, tok_req, items, H, R, splits);
+}
+
+}  // namespace ptl
+
+PTL_EXPORT int ptl_latent_prefill_bf16(void* out, const void* q, const void* cache, const int* block_table, const int* tiles, int n_tiles,
+                                       int bt_stride, int H, int R, int n, int page_size, int num_pages, float scale, int tile_tokens,
+                                       void* stream) {
+  if (!ptl::latent_tc_fits(out, q, cache, H, R, n)) return -2;
+  PTL_REQUIRE(n_tiles >= 0 && n_tiles <= 65535 && bt_stride > 0 && page_size > 0 && num_pages > 0 && tile_tokens > 0,
+              "latent_prefill: bad sizes");
+  if (n_tiles == 0) return 0;
+  const auto fn = R == 128 ? ptl::latent_prefill<128> : R == 256 ? ptl::latent_prefill<256> : ptl::latent_prefill<512>;
+  return fn(out, q, cache, block_table, tiles, n_tiles, bt_stride, H, R + n, page_size, num_pages, scale, tile_tokens, stream);
+}
+
+PTL_EXPORT int ptl_latent_decode_bf16(void* out, float* part, float* ml, const void* q, const void* cache, const int* block_table,
+                                      const int* tok_req, const int* positions, const int* items, int n_items, int bt_stride, int H, int R,
+                                      int n, int page_size, int num_pages, int splits, float scale, void* stream) {
+  if (!ptl::latent_tc_fits(out, q, cache, H, R, n)) return -2;
+  PTL_REQUIRE(n_items >= 0 && n_items <= 65535 && bt_stride > 0 && page_size > 0 && num_pages > 0 && splits >= 1 &&
+                  (splits == 1 || (part && ml)), "latent_decode: bad sizes");
+  if (n_items == 0) return 0;
+  const auto fn = R == 128 ? ptl::latent_decode<128> : R == 256 ? ptl::latent_decode<256> : ptl::latent_decode<512>;
+  return fn(out, part, ml, q, cache, block_table, tok_req, positions, items, n_items, bt_stride, H, R + n, page_size, num_pages, splits, scale,
+            stream);
+}

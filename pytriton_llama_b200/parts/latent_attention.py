@@ -43,8 +43,10 @@ class LatentAttention(Part):
         self.scale, self.eps = float(p["scale"]), float(p["norm_eps"])
         self.own_kv = bool(p.get("own_kv", True))
         self.position = build_part("position", spec.parts["position"], runtime)
-        # in bfloat16 the operator works prompt portions as matrix products laid out by the step's own lengths
-        self.portions_by_host_lengths = runtime.dtype == torch.bfloat16
+        # in bfloat16 the operator works prompt portions of sizes its tensor-core kernel does not take as matrix
+        # products laid out by the step's own lengths
+        paged = getattr(runtime.ops, "latent_on_tensor_cores", None)
+        self.portions_by_host_lengths = runtime.dtype == torch.bfloat16 and not (paged is not None and paged(self.kv_rank, self.n))
 
     def children(self):
         return {"position": self.position}

@@ -346,6 +346,38 @@ def test_rotation_of_one_part_of_every_head(ops, dtype, H, d, n, R, dims):
     TorchOps().rotate_head_part(x, d + n, d, b, R + n, R, H, n, pos, freq.float(), dims)
     _close(a, b, dtype, "rotated parts")
 
+@pytest.mark.parametrize("H,R,n,page", [(1, 128, 0, 4), (3, 256, 16, 16), (17, 128, 48, 8), (40, 512, 64, 16)])
+def test_latents_on_the_tensor_cores_at_the_edges_of_tiles(ops, H, R, n, page):
+    """Single tokens whose contexts end beside a tile of 64 keys, shared out and not, a row that belongs to no request,
+    portions whose (token, head) rows end beside a block of 64.  Weights are rounded to bfloat16 for portions only:
+    2^-8 of the largest latent, twice over with the result's own rounding; a single token's result is rounded once here and
+    once in the reference, a last place apart at most (2^-7 of it)."""
+    g = torch.Generator().manual_seed(H * R + n)
+    ref, d, dt = TorchOps(), R + n, torch.bfloat16
+    assert ops.latent_on_tensor_cores(R, n)
+    q_lens, starts = [1, 1, 1, 1, 1, 33, 1, 2, 129], [0, 62, 63, 64, 700, 31, 127, 62, 3]
+    cd, cc = _ctx(q_lens, starts, [0] * 9, "cuda:0"), _ctx(q_lens, starts, [0] * 9, "cpu")
+    pages = sum(-(-(s + k) // page) for s, k in zip(starts, q_lens)) + 3
+    bt, _ = _paged(g, q_lens, starts, page, pages, width=-(-701 // page) + 2)
+    q = _rand(g, sum(q_lens), H * d, scale=1.5).to(dt)
+    cache = _rand(g, pages, page * d, scale=0.7).to(dt)
+    want = ref.latent_attention(q, cache, bt, cc, H, R, n, page, d ** -0.5).double()
+    hints = ops.hints_for(q_lens, [s + k for s, k in zip(starts, q_lens)])
+    hints.positions = cd.positions
+    hints.tok_req = cd.tok_req.clone()
+    hints.tok_req[4] = -1                                            # the fifth request's token: a padded row
+    single = torch.tensor([0, 1, 2, 3, 38])
+    for sms in (ops._sm_count, 1):                                   # shares of a token's keys, one share
+        old, ops._sm_count = ops._sm_count, sms
+        try:
+            got = ops.latent_attention(q.cuda(), cache.cuda(), bt.cuda(), hints, H, R, n, page, d ** -0.5).double().cpu()
+        finally:
+            ops._sm_count = old
+        assert ((got - want).abs()[single] <= 2 ** -7 * want.abs()[single] + 1e-4).all()
+        rest = [t for t in range(len(want)) if t != 4 and t not in single]
+        assert (got - want).abs()[rest].max() <= 2 ** -7 * float(cache.abs().max())
+
+
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("T", [1, 7, 13, 40, 150])
