@@ -185,6 +185,8 @@ def load_library() -> ctypes.CDLL:
     lib.ptl_token_logprob.restype = _c_int
     lib.ptl_sample.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_ll, _ptr]
     lib.ptl_sample.restype = _c_int
+    lib.ptl_sample_cluster.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_ll, _ptr]
+    lib.ptl_sample_cluster.restype = _c_int
     lib.ptl_sample_work_words.argtypes = []
     lib.ptl_sample_work_words.restype = _c_int
     lib.ptl_softcap.argtypes = [_ptr, _c_ll, _c_f, _ptr]
@@ -324,7 +326,7 @@ class CudaOps:
         "linear": "product", "linear_add": "product", "gate_up_act": "product", "gemm_tc": "product",
         "_qkv_rope_product": "product", "rope_kv_write": "rope", "_rope_table": "rope",
         "paged_attention": "attention", "_attention_tensor_cores": "attention",
-        "sample": "sampling", "token_logprobs": "sampling",
+        "sample": "sampling", "token_logprobs": "sampling", "sample_tokens": "sampling",
         "stream_mix_norm": "norm", "gelu_tanh": "elementwise", "qk_norm_rotate_store": "rope", "window_attention": "attention",
         "gla_scan": "recurrent", "routed_experts": "experts", "expert_rows": "experts", "combine_experts_add": "experts",
         "add_layernorm": "norm", "xielu": "elementwise", "lowrank_tanh_linear": "recurrent", "general_delta_scan": "recurrent",
@@ -2129,6 +2131,31 @@ class CudaOps:
         self._check(self.lib.ptl_token_logprob(_p(out), _p(logits), _p(tokens), _p(scratch[0]), _p(scratch[1]), rows, vocab, vocab,
                                                self._stream()), kernels=2)
         return out
+
+    def sample_tokens(self, logits: torch.Tensor, temperature: Optional[torch.Tensor], top_p: Optional[torch.Tensor],
+                      u: Optional[torch.Tensor], out: Optional[torch.Tensor] = None, logprobs: bool = False):
+        """(``sample``'s tokens, with ``logprobs`` their ``token_logprobs``, else None) in one launch, for vocabularies of up to
+        131,072 tokens; larger ones by those two.  Greedy rows without log-probabilities have ``sample``'s two short launches."""
+        self._want(logits, "logits", torch.float32)
+        rows, vocab = logits.shape
+        if vocab > self.SAMPLE_CLUSTER_VOCAB or (temperature is None and not logprobs):
+            tokens = self.sample(logits, temperature, top_p, u, out=out)
+            return tokens, self.token_logprobs(logits, tokens) if logprobs else None
+        if out is None:
+            out = self.empty((rows,), torch.int32)
+        else:
+            self._want(out, "out", torch.int32)
+            if out.shape[0] != rows:
+                raise KernelError(f"sample: out has {out.shape[0]} rows, the logits {rows}")
+        if temperature is not None:
+            for name, t in (("temperature", temperature), ("top_p", top_p), ("u", u)):
+                self._want(t, name, torch.float32)
+        lp = self.empty((rows,), torch.float32) if logprobs else None
+        self._check(self.lib.ptl_sample_cluster(_p(out), _p(lp), _p(logits), _p(temperature), _p(top_p) if temperature is not None else None,
+                                                _p(u) if temperature is not None else None, rows, vocab, vocab, self._stream()))
+        return out, lp
+
+    SAMPLE_CLUSTER_VOCAB = 131072
 
     def sample(self, logits: torch.Tensor, temperature: Optional[torch.Tensor], top_p: Optional[torch.Tensor],
                u: Optional[torch.Tensor], out: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -42,15 +42,17 @@ class Sampler:
         """The same without reading anything back: (int32 tokens on the device, written to ``out``
         if given; float32 log-probabilities on the device, or None if no row asks for them)."""
         rows = logits.shape[0]
-        if all(p.temperature <= 0 for p in params):
-            tokens = self.ops.sample(logits, None, None, None, out=out)
-        else:
+        temperature = top_p = u = None
+        if any(p.temperature > 0 for p in params):
             host = torch.empty((3, rows), dtype=torch.float32, pin_memory=self.device.type == "cuda")
             h = host.numpy()
             for i, p in enumerate(params):
                 seed = self.seed if p.seed is None else p.seed
                 h[0, i], h[1, i], h[2, i] = p.temperature, p.top_p, uniform(seed, request_numbers[i], token_indices[i])
             dev = host.to(self.device, non_blocking=True)
-            tokens = self.ops.sample(logits, dev[0], dev[1], dev[2], out=out)
-        lp = self.ops.token_logprobs(logits, tokens) if any(p.logprobs for p in params) else None
-        return tokens, lp
+            temperature, top_p, u = dev[0], dev[1], dev[2]
+        logprobs = any(p.logprobs for p in params)
+        if hasattr(self.ops, "sample_tokens"):       # an operator set that does both at once
+            return self.ops.sample_tokens(logits, temperature, top_p, u, out=out, logprobs=logprobs)
+        tokens = self.ops.sample(logits, temperature, top_p, u, out=out)
+        return tokens, self.ops.token_logprobs(logits, tokens) if logprobs else None

@@ -590,6 +590,28 @@ def test_sampling_is_the_same_every_time_and_leaves_its_histograms_clean(ops):
             assert plain_llama.top_p_keep_mask(p, float(top_p[i]))[first[i]]
 
 
+@pytest.mark.parametrize("rows, vocab", [(1, 37), (9, 1000), (3, 32767), (40, 32769), (12, 128256), (2, 131072), (2, 131073)])
+def test_sampling_in_one_launch_gives_the_tokens_of_the_several(ops, rows, vocab):
+    """Integer masses: the same tokens, also for greedy rows, ties and rows of infinities; log-probabilities to float32 sums
+    (two sums of ``vocab`` exponentials in another order, under 2^-17 of the sum apart)."""
+    g = torch.Generator().manual_seed(rows + vocab)
+    logits = (2.5 * torch.randn(rows, vocab, generator=g)).cuda()
+    logits[0, vocab // 2:] = float("-inf")
+    logits[-1, vocab - 1] = logits[-1, 3] = logits[-1].max() + 1
+    temperature = torch.rand(rows, generator=g).cuda() + 0.3
+    temperature[rows // 2] = 0.0
+    top_p = torch.linspace(0.05, 1.0, rows).cuda()
+    u = torch.rand(rows, generator=g).cuda()
+    want = ops.sample(logits, temperature, top_p, u)
+    for logprobs in (True, False):
+        got, lp = ops.sample_tokens(logits, temperature, top_p, u, logprobs=logprobs)
+        assert torch.equal(got, want)
+        assert (lp is None) == (not logprobs)
+        if logprobs:
+            assert (lp - ops.token_logprobs(logits, want)).abs().max() <= 2e-5
+    assert torch.equal(ops.sample_tokens(logits, None, None, None, logprobs=True)[0], ops.sample(logits, None, None, None))
+
+
 def test_sampling_follows_the_distribution(ops):
     """Many draws with different uniform numbers reproduce the filtered probabilities."""
     vocab, n = 50, 4000
