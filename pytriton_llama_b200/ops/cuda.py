@@ -220,6 +220,12 @@ def load_library() -> ctypes.CDLL:
     lib.ptl_gated_lru_single_bf16.argtypes = [_ptr, _c_int, _c_int, _ptr, _ptr, _c_int, _ptr, _ptr, _ptr, _c_int, _ptr, _ptr, _ptr, _ptr,
                                               _ptr, _c_int, _c_int, _c_f, _ptr]
     lib.ptl_gated_lru_single_bf16.restype = _c_int
+    lib.ptl_latent_prefill_bf16.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f,
+                                            _c_int, _ptr]
+    lib.ptl_latent_prefill_bf16.restype = _c_int
+    lib.ptl_latent_decode_bf16.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
+                                           _c_int, _c_int, _c_int, _c_f, _ptr]
+    lib.ptl_latent_decode_bf16.restype = _c_int
     lib.ptl_last_error.restype = ctypes.c_char_p
     lib.ptl_set_dependent_launch.argtypes = [_c_int]
     lib.ptl_get_dependent_launch.restype = _c_int
@@ -237,12 +243,6 @@ def _suffix(dtype: torch.dtype) -> str:
     if dtype == torch.float32:
         return "_f32"
     if dtype == torch.bfloat16:
-    lib.ptl_latent_prefill_bf16.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f,
-                                            _c_int, _ptr]
-    lib.ptl_latent_prefill_bf16.restype = _c_int
-    lib.ptl_latent_decode_bf16.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
-                                           _c_int, _c_int, _c_int, _c_f, _ptr]
-    lib.ptl_latent_decode_bf16.restype = _c_int
         return "_bf16"
     raise KernelError(f"unsupported element type {dtype}")
 
@@ -1619,6 +1619,9 @@ class CudaOps:
         portion of a step whose context says its host lengths are exact is worked as two tensor-core products
         around a float32 softmax, per request and per ``LATENT_QUERY_CHUNK`` tokens: all heads' queries of the
         chunk against the request's gathered rows, the weights (rounded once) against the gathered latents."""
+        done = self._latent_attention_tensor_cores(q, cache, block_table, ctx, H, R, n, page_size, scale)
+        if done is not None:
+            return done
         d = R + n
         portions = [(r, qn) for r, qn in enumerate(getattr(ctx, "q_lens", []) or []) if qn > 1]
         dec = self._work(ctx, "decode_items")
@@ -1658,6 +1661,43 @@ class CudaOps:
                 weights = self.empty(((b - a) * H, c_pad), q.dtype)
                 self.causal_softmax_rows(weights, scores, ctx.positions, rows.start, H, scale)
                 out[rows] = self.linear(weights, latents_t, fresh_weights=True).view(b - a, H * R)
+        return out
+
+    @staticmethod
+    def latent_on_tensor_cores(R: int, n: int) -> bool:
+        """Sizes of the latent and of the rotated key part that the tensor-core kernels are built for."""
+        return R in (128, 256, 512) and n % 16 == 0 and n <= 64
+
+    def _latent_attention_tensor_cores(self, q, cache, block_table, ctx, H, R, n, page_size, scale) -> Optional[torch.Tensor]:
+        """None where sizes, types or the lack of the step's work lists leave it to the other paths.  A single token's keys
+        are shared out so that all shares together fill the SMs once, 64 keys at least."""
+        dec, tiles = self._work(ctx, "decode_items"), self._work(ctx, "prefill_tiles")
+        if q.dtype != torch.bfloat16 or dec is None or tiles is None or H > 512 or not self.latent_on_tensor_cores(R, n):
+            return None
+        self._want(q, "q")
+        self._want(cache, "cache", q.dtype)
+        for name, t in (("block_table", block_table), ("tok_req", ctx.tok_req), ("positions", ctx.positions)):
+            self._want(t, name, torch.int32)
+        if cache[0].numel() != page_size * (R + n) or q.shape[1] != H * (R + n):
+            raise KernelError("latent_attention: the cache's pages or the queries do not fit the sizes")
+        if q.data_ptr() % 16 or cache.data_ptr() % 16:
+            return None
+        out = self.empty((q.shape[0], H * R), q.dtype)
+        if tiles.items:
+            self._check(self.lib.ptl_latent_prefill_bf16(
+                _p(out), _p(q), _p(cache), _p(block_table), _p(tiles.tensor), tiles.items, block_table.shape[1], H, R, n, page_size,
+                cache.shape[0], float(scale), self.QUERY_TILE, self._stream()))
+        if dec.items:
+            longest = getattr(ctx, "max_ctx_len", 0) or block_table.shape[1] * page_size
+            splits = max(1, min(-(-longest // 64), self._sm_count // (dec.items * -(-H // 16))))
+            part = ml = None
+            if splits > 1:
+                part = self.empty((dec.items, splits, H, R), torch.float32)
+                ml = self.empty((dec.items, splits, H, 2), torch.float32)
+            self._check(self.lib.ptl_latent_decode_bf16(
+                _p(out), _p(part), _p(ml), _p(q), _p(cache), _p(block_table), _p(ctx.tok_req), _p(ctx.positions),
+                None if dec.in_order else _p(dec.tensor), dec.items, block_table.shape[1], H, R, n, page_size, cache.shape[0], splits,
+                float(scale), self._stream()), kernels=2 if splits > 1 else 1)
         return out
 
     def latent_gather(self, keys: torch.Tensor, latents_t: torch.Tensor, cache: torch.Tensor, block_table: torch.Tensor, r: int,
@@ -1720,9 +1760,6 @@ class CudaOps:
                 matmul.allow_bf16_reduced_precision_reduction = before
             if gate is not None:
                 self._check(self.lib.ptl_head_gate_bf16(_p(out), out_ld, out_col, n_out, T, H, gate_ptr, gate.shape[1], self._stream()))
-        done = self._latent_attention_tensor_cores(q, cache, block_table, ctx, H, R, n, page_size, scale)
-        if done is not None:
-            return done
             return
         fn = getattr(self.lib, "ptl_head_linear" + _suffix(x.dtype))
         if (x.dtype == torch.bfloat16 and T <= self.HEAD_FEW_MAX_TOKENS and n_in % 8 == 0 and n_in <= 1536 and x_ld % 8 == 0
@@ -1764,43 +1801,6 @@ class CudaOps:
         rows = self.expert_rows(x, logits, w_gate_up, w_down, top, scale_input, **routing)
         T, width = x.shape
         out = self.empty((T, width), torch.float32)
-    @staticmethod
-    def latent_on_tensor_cores(R: int, n: int) -> bool:
-        """Sizes of the latent and of the rotated key part that the tensor-core kernels are built for."""
-        return R in (128, 256, 512) and n % 16 == 0 and n <= 64
-
-    def _latent_attention_tensor_cores(self, q, cache, block_table, ctx, H, R, n, page_size, scale) -> Optional[torch.Tensor]:
-        """None where sizes, types or the lack of the step's work lists leave it to the other paths.  A single token's keys
-        are shared out so that all shares together fill the SMs once, 64 keys at least."""
-        dec, tiles = self._work(ctx, "decode_items"), self._work(ctx, "prefill_tiles")
-        if q.dtype != torch.bfloat16 or dec is None or tiles is None or H > 512 or not self.latent_on_tensor_cores(R, n):
-            return None
-        self._want(q, "q")
-        self._want(cache, "cache", q.dtype)
-        for name, t in (("block_table", block_table), ("tok_req", ctx.tok_req), ("positions", ctx.positions)):
-            self._want(t, name, torch.int32)
-        if cache[0].numel() != page_size * (R + n) or q.shape[1] != H * (R + n):
-            raise KernelError("latent_attention: the cache's pages or the queries do not fit the sizes")
-        if q.data_ptr() % 16 or cache.data_ptr() % 16:
-            return None
-        out = self.empty((q.shape[0], H * R), q.dtype)
-        if tiles.items:
-            self._check(self.lib.ptl_latent_prefill_bf16(
-                _p(out), _p(q), _p(cache), _p(block_table), _p(tiles.tensor), tiles.items, block_table.shape[1], H, R, n, page_size,
-                cache.shape[0], float(scale), self.QUERY_TILE, self._stream()))
-        if dec.items:
-            longest = getattr(ctx, "max_ctx_len", 0) or block_table.shape[1] * page_size
-            splits = max(1, min(-(-longest // 64), self._sm_count // (dec.items * -(-H // 16))))
-            part = ml = None
-            if splits > 1:
-                part = self.empty((dec.items, splits, H, R), torch.float32)
-                ml = self.empty((dec.items, splits, H, 2), torch.float32)
-            self._check(self.lib.ptl_latent_decode_bf16(
-                _p(out), _p(part), _p(ml), _p(q), _p(cache), _p(block_table), _p(ctx.tok_req), _p(ctx.positions),
-                None if dec.in_order else _p(dec.tensor), dec.items, block_table.shape[1], H, R, n, page_size, cache.shape[0], splits,
-                float(scale), self._stream()), kernels=2 if splits > 1 else 1)
-        return out
-
         self._check(getattr(self.lib, "ptl_moe_combine" + _suffix(x.dtype))(_p(out), _p(rows.y), _p(shared), _p(rows.pos), _p(rows.weights), T,
                                                                             top, width, int(bool(scale_input)), self._stream()))
         return out

@@ -333,19 +333,6 @@ def test_attention_over_the_latents_portions_as_products_and_single_tokens(ops, 
     _close(got, want, dtype, "chunks of 64", tol=2e-5 if dtype == "float32" else 2e-2)
 
 
-@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
-@pytest.mark.parametrize("H,d,n,R,dims", [(3, 16, 8, 20, 8), (4, 64, 32, 64, 32), (1, 8, 24, 12, 24), (5, 6, 4, 6, 2), (2, 128, 64, 512, 64)])
-def test_rotation_of_one_part_of_every_head(ops, dtype, H, d, n, R, dims):
-    g = torch.Generator().manual_seed(H + d + n)
-    dt, T = DTYPES[dtype], 23
-    x = _rand(g, T, H * (d + n)).to(dt)
-    pos = torch.randint(0, 5000, (T,), generator=g, dtype=torch.int32)
-    freq = 1000.0 ** (-torch.arange(dims // 2, dtype=torch.float64) * 2 / dims)
-    a, b = torch.zeros(T, H * (R + n), dtype=dt).cuda(), torch.zeros(T, H * (R + n), dtype=dt)
-    ops.rotate_head_part(x.cuda(), d + n, d, a, R + n, R, H, n, pos.cuda(), freq.float().cuda(), dims)
-    TorchOps().rotate_head_part(x, d + n, d, b, R + n, R, H, n, pos, freq.float(), dims)
-    _close(a, b, dtype, "rotated parts")
-
 @pytest.mark.parametrize("H,R,n,page", [(1, 128, 0, 4), (3, 256, 16, 16), (17, 128, 48, 8), (40, 512, 64, 16)])
 def test_latents_on_the_tensor_cores_at_the_edges_of_tiles(ops, H, R, n, page):
     """Single tokens whose contexts end beside a tile of 64 keys, shared out and not, a row that belongs to no request,
@@ -377,6 +364,19 @@ def test_latents_on_the_tensor_cores_at_the_edges_of_tiles(ops, H, R, n, page):
         rest = [t for t in range(len(want)) if t != 4 and t not in single]
         assert (got - want).abs()[rest].max() <= 2 ** -7 * float(cache.abs().max())
 
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H,d,n,R,dims", [(3, 16, 8, 20, 8), (4, 64, 32, 64, 32), (1, 8, 24, 12, 24), (5, 6, 4, 6, 2), (2, 128, 64, 512, 64)])
+def test_rotation_of_one_part_of_every_head(ops, dtype, H, d, n, R, dims):
+    g = torch.Generator().manual_seed(H + d + n)
+    dt, T = DTYPES[dtype], 23
+    x = _rand(g, T, H * (d + n)).to(dt)
+    pos = torch.randint(0, 5000, (T,), generator=g, dtype=torch.int32)
+    freq = 1000.0 ** (-torch.arange(dims // 2, dtype=torch.float64) * 2 / dims)
+    a, b = torch.zeros(T, H * (R + n), dtype=dt).cuda(), torch.zeros(T, H * (R + n), dtype=dt)
+    ops.rotate_head_part(x.cuda(), d + n, d, a, R + n, R, H, n, pos.cuda(), freq.float().cuda(), dims)
+    TorchOps().rotate_head_part(x, d + n, d, b, R + n, R, H, n, pos, freq.float(), dims)
+    _close(a, b, dtype, "rotated parts")
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
