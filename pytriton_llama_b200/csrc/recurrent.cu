@@ -285,6 +285,127 @@ selective_scan_kernel(T* __restrict__ out, const T* __restrict__ xc, const float
   }
 }
 
+// The same for steps with portions of many tokens and up to kScanStates states: the tokens of every request in segments of
+// kScanSegment.  A segment's walk from zero and the sum of its step sizes (scan_segments, ENDS) say how it moves a state on;
+// scan_carry applies that segment after segment, which leaves the state before each; then every segment is walked once more from
+// its own state with the read-outs.  A thread owns a channel with all its states in registers (no sums over lanes), a block 128
+// channels of one segment.  Bound by the exponentials' instructions, twice those of one walk, but in parallel over the segments: one
+// walk of 2,048 tokens and 2,048 channels took 603 us on 512 warps, 0.3 us a token of latency.
+// Workspace per segment: the states [kScanStates][inner], the sums of step sizes [inner].
+constexpr int kScanSegment = 64, kScanStates = 16, kScanBatch = 8;
+
+// (request, first row, rows, number of the segment in its request); request -1 behind the last segment of the step
+__device__ __forceinline__ int4 scan_locate(const int* __restrict__ q_start, int requests, int segment) {
+  for (int r = 0; r < requests; ++r) {
+    const int lo = q_start[r], n = q_start[r + 1] - lo;
+    const int segments = n > 0 ? (n + kScanSegment - 1) / kScanSegment : 0;
+    if (segment < segments) return make_int4(r, lo + segment * kScanSegment, min(kScanSegment, n - segment * kScanSegment), segment);
+    segment -= segments;
+  }
+  return make_int4(-1, 0, 0, 0);
+}
+
+template <typename T, bool ENDS>
+__global__ void __launch_bounds__(128)
+scan_segments_kernel(T* __restrict__ out, float* __restrict__ work, const T* __restrict__ xc, const float* __restrict__ dt_raw,
+                     const float* __restrict__ dt_bias, const float* __restrict__ A, const T* __restrict__ bc, const float* __restrict__ D,
+                     const T* __restrict__ z, int z_ld, int z_column, int inner, int n_state, const int* __restrict__ q_start,
+                     const int* __restrict__ state_slot, int requests) {
+  __shared__ __align__(16) float s_bc[kScanSegment][2 * kScanStates];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int4 at = scan_locate(q_start, requests, blockIdx.y);
+  if (at.x < 0 || state_slot[at.x] < 0) return;
+  const int n = at.z;
+  for (int i = threadIdx.x; i < kScanSegment * 2 * kScanStates; i += 128) {
+    const int t = i / (2 * kScanStates), e = i % (2 * kScanStates), k = e % kScanStates;
+    const bool there = t < n && k < n_state;
+    s_bc[t][e] = there ? to_f32(bc[(size_t)(at.y + t) * 2 * n_state + (e < kScanStates ? k : n_state + k)]) : 0.f;
+  }
+  __syncthreads();
+  const int c = blockIdx.x * 128 + threadIdx.x;
+  if (c >= inner) return;
+  float* states = work + (size_t)blockIdx.y * (kScanStates + 1) * inner + c;
+  float S[kScanStates], a[kScanStates];
+#pragma unroll
+  for (int k = 0; k < kScanStates; ++k) {
+    a[k] = k < n_state ? A[(size_t)c * n_state + k] : 0.f;
+    S[k] = ENDS ? 0.f : states[(size_t)k * inner];
+  }
+  const float bias = dt_bias[c], skip = ENDS ? 0.f : D[c];
+  float sum = 0.f;
+  for (int t0 = 0; t0 < n; t0 += kScanBatch) {
+    float x[kScanBatch], dt[kScanBatch], gate[kScanBatch];
+#pragma unroll
+    for (int i = 0; i < kScanBatch; ++i) {                 // (eight tokens' loads side by side)
+      const size_t row = at.y + min(t0 + i, n - 1);
+      x[i] = to_f32(xc[row * inner + c]);
+      dt[i] = dt_raw[row * inner + c];
+      gate[i] = ENDS ? 0.f : to_f32(z[row * z_ld + z_column + c]);
+    }
+#pragma unroll
+    for (int i = 0; i < kScanBatch; ++i) {
+      if (t0 + i >= n) break;
+      const float step = softplus_f32(dt[i] + bias), dx = step * x[i];
+      const float4* b = reinterpret_cast<const float4*>(s_bc[t0 + i]);
+      float y[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int k4 = 0; k4 < kScanStates / 4; ++k4) {
+        const float4 bv = b[k4], cv = b[kScanStates / 4 + k4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int k = 4 * k4 + e;
+          S[k] = fmaf(expf(step * a[k]), S[k], dx * (&bv.x)[e]);
+          if (!ENDS) y[e] = fmaf(S[k], (&cv.x)[e], y[e]);
+        }
+      }
+      if (ENDS) sum += step;
+      else out[(size_t)(at.y + t0 + i) * inner + c] = from_f32<T>(((y[0] + y[1]) + (y[2] + y[3]) + skip * x[i]) * silu_f32(gate[i]));
+    }
+  }
+  if (ENDS) {
+#pragma unroll
+    for (int k = 0; k < kScanStates; ++k) states[(size_t)k * inner] = S[k];
+    states[(size_t)kScanStates * inner] = sum;
+  }
+}
+
+// Per channel and state: replaces the ends that the segments of a request reached from zero by the states before them, and
+// moves the request's own state on.
+__global__ void __launch_bounds__(128)
+scan_carry_kernel(float* __restrict__ work, float* __restrict__ state, const float* __restrict__ A, int inner, int n_state,
+                  const int* __restrict__ q_start, const int* __restrict__ positions, const int* __restrict__ state_slot) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int r = blockIdx.z, k = blockIdx.y, c = blockIdx.x * 128 + threadIdx.x;
+  const int lo = q_start[r], n = q_start[r + 1] - lo;
+  if (c >= inner || n <= 0 || state_slot[r] < 0) return;
+  int first = 0;
+  for (int i = 0; i < r; ++i) first += (max(q_start[i + 1] - q_start[i], 0) + kScanSegment - 1) / kScanSegment;
+  const int segments = (n + kScanSegment - 1) / kScanSegment;
+  float* st = state + ((size_t)state_slot[r] * inner + c) * n_state + k;
+  float S = positions[lo] == 0 ? 0.f : *st;
+  const float a = A[(size_t)c * n_state + k];
+  const size_t stride = (size_t)(kScanStates + 1) * inner;
+  float* w = work + first * stride + c;
+  for (int s0 = 0; s0 < segments; s0 += kScanBatch) {
+    float end[kScanBatch], sum[kScanBatch];
+#pragma unroll
+    for (int i = 0; i < kScanBatch; ++i) {
+      const size_t at = (size_t)min(s0 + i, segments - 1) * stride;
+      end[i] = w[at + (size_t)k * inner];
+      sum[i] = w[at + (size_t)kScanStates * inner];
+    }
+#pragma unroll
+    for (int i = 0; i < kScanBatch; ++i) {
+      if (s0 + i >= segments) break;
+      w[(size_t)(s0 + i) * stride + (size_t)k * inner] = S;
+      S = fmaf(expf(a * sum[i]), S, end[i]);
+    }
+  }
+  *st = S;
+}
+
 // ------------------------------------------------------------------ gated delta rule
 // Per value head h (query/key head c = h / (heads / kv_heads)) and token, with k, q scaled to unit length
 // (q also by q_scale), beta = sigmoid(b), g = exp(-rate[h] * softplus(a + dt_bias[h])):
@@ -677,6 +798,25 @@ int selective_scan(void* out, const void* xc, const float* dt_raw, const float* 
 }
 
 template <typename T>
+int scan_segments(void* out, float* work, int segments, const void* xc, const float* dt_raw, const float* dt_bias, const float* A,
+                  const void* bc, const float* D, const void* z, int z_ld, int z_column, int inner, int n_state, float* state,
+                  const int* q_start, const int* positions, const int* state_slot, int requests, void* stream) {
+  PTL_REQUIRE(requests >= 0 && requests <= 65535 && segments >= 0 && segments <= 65535 && inner > 0 && n_state > 0 &&
+                  n_state <= kScanStates && z_column >= 0 && z_column + inner <= z_ld,
+              "selective_scan in segments: bad sizes inner=%d state=%d (at most %d)", inner, n_state, kScanStates);
+  if (requests == 0 || segments == 0) return 0;
+  const dim3 grid((inner + 127) / 128, segments), block(128);
+  if (int rc = launch_kernel("scan_segments", scan_segments_kernel<T, true>, grid, block, 0, as_stream(stream), (T*)out, work, (const T*)xc,
+                             dt_raw, dt_bias, A, (const T*)bc, D, (const T*)z, z_ld, z_column, inner, n_state, q_start, state_slot, requests))
+    return rc;
+  if (int rc = launch_kernel("scan_carry", scan_carry_kernel, dim3((inner + 127) / 128, n_state, requests), block, 0, as_stream(stream), work,
+                             state, A, inner, n_state, q_start, positions, state_slot))
+    return rc;
+  return launch_kernel("scan_segments", scan_segments_kernel<T, false>, grid, block, 0, as_stream(stream), (T*)out, work, (const T*)xc,
+                       dt_raw, dt_bias, A, (const T*)bc, D, (const T*)z, z_ld, z_column, inner, n_state, q_start, state_slot, requests);
+}
+
+template <typename T>
 int gated_delta_rule(float* out, const void* qkv, const float* ba, const float* rate, const float* dt_bias, float* state,
                      const int* q_start, const int* positions, const int* state_slot, int requests, int heads, int kv_heads, int d,
                      int dv, float unit_eps, float q_scale, void* stream) {
@@ -738,6 +878,13 @@ int gated_head_norm(void* out, int out_ld, int column, const float* o, const flo
                                             const int* state_slot, int requests, void* stream) {                                  \
     return ptl::selective_scan<TYPE>(out, xc, dt_raw, dt_bias, A, bc, D, z, z_ld, z_column, inner, n_state, state, q_start,        \
                                      positions, state_slot, requests, stream);                                                    \
+  }                                                                                                                               \
+  PTL_EXPORT int ptl_scan_segments##SUFFIX(void* out, float* work, int segments, const void* xc, const float* dt_raw,              \
+                                           const float* dt_bias, const float* A, const void* bc, const float* D, const void* z,    \
+                                           int z_ld, int z_column, int inner, int n_state, float* state, const int* q_start,      \
+                                           const int* positions, const int* state_slot, int requests, void* stream) {             \
+    return ptl::scan_segments<TYPE>(out, work, segments, xc, dt_raw, dt_bias, A, bc, D, z, z_ld, z_column, inner, n_state, state,  \
+                                    q_start, positions, state_slot, requests, stream);                                            \
   }                                                                                                                               \
   PTL_EXPORT int ptl_gated_delta_rule##SUFFIX(float* out, const void* qkv, const float* ba, const float* rate,                     \
                                               const float* dt_bias, float* state, const int* q_start, const int* positions,       \

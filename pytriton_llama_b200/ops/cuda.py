@@ -38,6 +38,8 @@ _SIGNATURES = {
                         _c_int, _c_int, _ptr, _ptr],
     "ptl_selective_scan": [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr,
                            _c_int, _ptr],
+    "ptl_scan_segments": [_ptr, _ptr, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr,
+                          _ptr, _c_int, _ptr],
     "ptl_gated_delta_rule": [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f,
                              _c_f, _ptr],
     "ptl_gated_head_norm": [_ptr, _c_int, _c_int, _ptr, _ptr, _c_f, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_int,
@@ -1104,6 +1106,11 @@ class CudaOps:
                        single, _p(in_bias), self._stream()), kernels=2 if taps > 1 and not single else 1)
         return out
 
+    # The longest portion of a step that the selective scan walks token by token.  2,048
+    # tokens of 2,048 channels of 16 states: 603 us token by token, 116 in segments (51 their products, 5 the carries, 60 the outputs);
+    # a segment's work is done twice, so that below one segment (64 tokens) the walk is the shorter.
+    SCAN_WALK_MAX_TOKENS = 64
+
     def selective_scan(self, xc: torch.Tensor, dt: torch.Tensor, dt_b: torch.Tensor, A: torch.Tensor, bc: torch.Tensor,
                        D: torch.Tensor, xz: torch.Tensor, z_column: int, state: torch.Tensor, ctx) -> torch.Tensor:
         """The scan of ``parts/scan.py``: xc [T, inner], dt float32 [T, inner] before bias and softplus, A float32
@@ -1117,6 +1124,14 @@ class CudaOps:
         if xc.shape[1] != inner or dt.shape != xc.shape or bc.shape[1] != 2 * n or tuple(state.shape[1:]) != (inner, n):
             raise KernelError("selective_scan: shapes do not fit")
         out = self.empty(xc.shape, xc.dtype)
+        if ctx.max_q_len > self.SCAN_WALK_MAX_TOKENS and n <= 16:
+            segments = xc.shape[0] // 64 + ctx.num_requests      # at least the segments of 64 tokens that the portions make
+            work = self.empty((segments, 17, inner), torch.float32)
+            fn = getattr(self.lib, "ptl_scan_segments" + _suffix(xc.dtype))
+            self._check(fn(_p(out), _p(work), segments, _p(xc), _p(dt), _p(dt_b), _p(A), _p(bc), _p(D), _p(xz), xz.shape[1], int(z_column),
+                           inner, n, _p(state), _p(ctx.q_start), _p(ctx.positions), _p(ctx.state_slot), ctx.num_requests,
+                           self._stream()), kernels=3)
+            return out
         fn = getattr(self.lib, "ptl_selective_scan" + _suffix(xc.dtype))
         self._check(fn(_p(out), _p(xc), _p(dt), _p(dt_b), _p(A), _p(bc), _p(D), _p(xz), xz.shape[1], int(z_column), inner, n,
                        _p(state), _p(ctx.q_start), _p(ctx.positions), _p(ctx.state_slot), ctx.num_requests, self._stream()))

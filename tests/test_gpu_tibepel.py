@@ -109,6 +109,24 @@ def test_gated_delta_rule(ops, dtype, H, G, d, dv):
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("inner,n", [(40, 16), (129, 5), (256, 16)])
+def test_selective_scan_in_segments_of_64_tokens(ops, dtype, inner, n):
+    """Portions that end beside a segment, fresh and running, beside single tokens, to the walk's own bound."""
+    g = torch.Generator().manual_seed(inner + n)
+    step = ([64, 1, 65, 200, 2, 63, 128], [0, 17, 3, 0, 9, 5, 0], [2, 0, 3, 1, 6, 4, 5])
+    T, dt = sum(step[0]), DTYPES[dtype]
+    tensors = {"xc": torch.randn(T, inner, generator=g).to(dt), "dt": torch.randn(T, inner, generator=g) - 2,
+               "dt_b": torch.randn(inner, generator=g), "A": -torch.exp(torch.randn(inner, n, generator=g)),
+               "bc": torch.randn(T, 2 * n, generator=g).to(dt), "D": torch.randn(inner, generator=g),
+               "xz": torch.randn(T, 2 * inner, generator=g).to(dt), "state": torch.randn(7, inner, n, generator=g)}
+    run = lambda o, t, ctx: o.selective_scan(t["xc"], t["dt"], t["dt_b"], t["A"], t["bc"], t["D"], t["xz"], inner, t["state"], ctx)
+    assert max(step[0]) > ops.SCAN_WALK_MAX_TOKENS
+    got, ref, dev, cpu = _both(ops, run, tensors, step, dtype)
+    _close(got, ref, dtype, "outputs")
+    _close(dev["state"], cpu["state"], "float32", "state after the step")
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_row_wise_operators(ops, dtype):
     g = torch.Generator().manual_seed(3)
     dt = DTYPES[dtype]
