@@ -1,0 +1,214 @@
+// The token-indexed side term of a layer (see token_side_kernel in stream_ops.cu) for 16-bit weights, sixteen tokens per cluster of eight
+// blocks: s = residual + x + bias;  z = W_gate s;  g = gelu_tanh(z) * table[token, column + j];  y = W_proj g;
+// residual = s + y * rsqrt(mean(y^2) + eps) * norm.
+// Block b owns an eighth of the width: its columns of s and of W_gate give partial sums of all z, block b adds up and
+// activates its eighth of the dims, and its rows of W_proj give its columns of y.  Partial sums, g and the sums of squares cross
+// the cluster through distributed shared memory.  Both products run on the tensor cores; s and g are float32 and go there as three
+// bfloat16 terms each (24 bits).  The weights' parts (32 KB a block at 1,024 x 64) are fetched before the wait on the
+// predecessor.  Bound by the latency of three cluster barriers at a few tokens.  2,048 tokens of width 1,024: 91 us
+// as one block per token, 36 here; 8 tokens: 22.4 and 7.7.
+#include "mma_utils.cuh"
+
+namespace ptl {
+
+constexpr int kTsBlocks = 8, kTsTokens = 16, kTsThreads = 256, kTsMaxDim = 128;
+
+__device__ __forceinline__ float ts_gelu_tanh(float z) {
+  return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
+}
+__device__ __forceinline__ void ts_split(float x, __nv_bfloat16* at, int stride) {      // three terms, `stride` elements apart
+#pragma unroll
+  for (int w = 0; w < 3; ++w) {
+    const __nv_bfloat16 t = __float2bfloat16_rn(x);
+    at[w * stride] = t;
+    x -= __bfloat162float(t);
+  }
+}
+// bytes: s float32, s in three terms, W_gate part, W_proj part, partial sums, g float32, g in three terms
+__host__ __device__ constexpr size_t ts_smem(int sl, int dim) {
+  return (size_t)4 * kTsTokens * (sl + 4) + 6 * kTsTokens * (sl + 8) + 2 * dim * (sl + 8) + 2 * sl * (dim + 8) + 4 * kTsTokens * dim +
+         4 * kTsTokens * dim + 6 * kTsTokens * (dim + 8);
+}
+
+template <int SL>
+__global__ void __launch_bounds__(kTsThreads)
+token_side_cluster_kernel(float* __restrict__ residual, const __nv_bfloat16* __restrict__ x, const float* __restrict__ bias,
+                          const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ table, int table_ld, int column, int dim,
+                          int vocab, const __nv_bfloat16* __restrict__ w_gate, const __nv_bfloat16* __restrict__ w_proj,
+                          const float* __restrict__ norm_w, float eps, int n_tokens) {
+  constexpr int width = SL * kTsBlocks, LS = SL + 4, LB = SL + 8;
+  extern __shared__ __align__(16) unsigned char ts_raw[];
+  float* s32 = reinterpret_cast<float*>(ts_raw);                                     // [16][LS]
+  __nv_bfloat16* s16 = reinterpret_cast<__nv_bfloat16*>(s32 + kTsTokens * LS);       // [3][16][LB]
+  __nv_bfloat16* wg = s16 + 3 * kTsTokens * LB;                                      // [dim][LB]
+  __nv_bfloat16* wp = wg + dim * LB;                                                 // [SL][dim + 8]
+  const int LD = dim + 8, per = dim / kTsBlocks;
+  float* zrecv = reinterpret_cast<float*>(wp + SL * LD);                             // [8 sources][16][per]
+  float* g32 = zrecv + kTsTokens * dim;                                              // [16][dim]
+  __nv_bfloat16* g16 = reinterpret_cast<__nv_bfloat16*>(g32 + kTsTokens * dim);      // [3][16][LD]
+  __shared__ float s_ss[kTsThreads / 32][kTsTokens];
+  __shared__ float s_recv[kTsBlocks][kTsTokens];
+  cluster_arrive();                                     // every block runs before a peer writes into it
+  const int rank = blockIdx.x % kTsBlocks, t0 = blockIdx.x / kTsBlocks * kTsTokens, c0 = rank * SL;
+  const int nt = min(kTsTokens, n_tokens - t0);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c2 = (lane & 3) * 2;
+  // the weights, and this thread's table entries: written by no kernel of the step
+  for (int i = tid; i < dim * (SL / 8); i += kTsThreads)
+    cp_async_16(smem_u32(wg + (i / (SL / 8)) * LB + i % (SL / 8) * 8), w_gate + (size_t)(i / (SL / 8)) * width + c0 + i % (SL / 8) * 8, true);
+  for (int i = tid; i < SL * (dim / 8); i += kTsThreads)
+    cp_async_16(smem_u32(wp + (i / (dim / 8)) * LD + i % (dim / 8) * 8), w_proj + (size_t)(c0 + i / (dim / 8)) * dim + i % (dim / 8) * 8, true);
+  cp_async_commit();
+  const bool own = tid < kTsTokens * per;
+  float entry = 0.f;
+  if (own && tid / per < nt) {
+    int tok = tokens[t0 + tid / per];
+    if (tok < 0 || tok >= vocab) tok = 0;
+    entry = __bfloat162float(table[(size_t)tok * table_ld + column + rank * per + tid % per]);
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int i = tid; i < kTsTokens * (SL / 4); i += kTsThreads) {
+    const int r = i / (SL / 4), c = i % (SL / 4) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < nt) {
+      v = *reinterpret_cast<const float4*>(residual + (size_t)(t0 + r) * width + c0 + c);
+      if (x) {
+        const uint2 raw = *reinterpret_cast<const uint2*>(x + (size_t)(t0 + r) * width + c0 + c);
+        const float2 lo = unpack_bf16(raw.x), hi = unpack_bf16(raw.y);
+        v.x += lo.x; v.y += lo.y; v.z += hi.x; v.w += hi.y;
+      }
+      if (bias) {
+        const float4 b = *reinterpret_cast<const float4*>(bias + c0 + c);
+        v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+      }
+    }
+    *reinterpret_cast<float4*>(s32 + r * LS + c) = v;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ts_split((&v.x)[e], s16 + r * LB + c + e, kTsTokens * LB);
+  }
+  cp_async_wait<0>();
+  __syncthreads();
+  const int lm_row = lane & 15, lm_half = lane >> 4;
+  // partial z: a warp per eight dims
+  cluster_wait();
+  for (int n = warp; n < dim / 8; n += kTsThreads / 32) {
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int k = 0; k < SL / 16; k += 2) {
+      uint32_t b[4];
+      ldmatrix_x4(b, smem_u32(wg + (8 * n + (lane & 7)) * LB + 16 * k + 8 * (lane >> 3)));
+#pragma unroll
+      for (int w = 2; w >= 0; --w) {
+        uint32_t a[4];
+        ldmatrix_x4(a, smem_u32(s16 + (w * kTsTokens + lm_row) * LB + 16 * k + 8 * lm_half));
+        mma_bf16_16816(acc, a, b[0], b[1]);
+        ldmatrix_x4(a, smem_u32(s16 + (w * kTsTokens + lm_row) * LB + 16 * k + 16 + 8 * lm_half));
+        mma_bf16_16816(acc, a, b[2], b[3]);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int d = 8 * n + c2 + (e & 1), row = g + 8 * (e >> 1);
+      st_peer_f32(map_to_peer(smem_u32(zrecv + (rank * kTsTokens + row) * per + d % per), d / per), acc[e]);
+    }
+  }
+  cluster_arrive();
+  cluster_wait();
+  if (own) {
+    const int row = tid / per, d = tid % per;
+    float z = 0.f;
+#pragma unroll
+    for (int b = 0; b < kTsBlocks; ++b) z += zrecv[(b * kTsTokens + row) * per + d];
+    const float v = ts_gelu_tanh(z) * entry;
+#pragma unroll
+    for (int b = 0; b < kTsBlocks; ++b) st_peer_f32(map_to_peer(smem_u32(g32 + row * dim + rank * per + d), b), v);
+  }
+  cluster_arrive();
+  cluster_wait();
+  for (int i = tid; i < kTsTokens * dim; i += kTsThreads) ts_split(g32[i], g16 + i / dim * LD + i % dim, kTsTokens * LD);
+  __syncthreads();
+  constexpr int NT = SL / 64;                           // blocks of eight columns per warp
+  float y[NT][4];
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y[j][e] = 0.f;
+  for (int k = 0; k < dim / 16; ++k) {
+    uint32_t a[3][4];
+#pragma unroll
+    for (int w = 0; w < 3; ++w) ldmatrix_x4(a[w], smem_u32(g16 + (w * kTsTokens + lm_row) * LD + 16 * k + 8 * lm_half));
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      uint32_t b[4];                                    // (the upper half of the lanes names the same rows again)
+      ldmatrix_x4(b, smem_u32(wp + (8 * (warp * NT + j) + (lane & 7)) * LD + 16 * k + 8 * ((lane >> 3) & 1)));
+#pragma unroll
+      for (int w = 2; w >= 0; --w) mma_bf16_16816(y[j], a[w], b[0], b[1]);
+    }
+  }
+  float ss[2] = {0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ss[e >> 1] = fmaf(y[j][e], y[j][e], ss[e >> 1]);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 1);
+    ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 2);
+    if ((lane & 3) == 0) s_ss[warp][g + 8 * i] = ss[i];
+  }
+  __syncthreads();
+  if (tid < kTsTokens * kTsBlocks) {
+    const int row = tid % kTsTokens, peer = tid / kTsTokens;
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < kTsThreads / 32; ++w) v += s_ss[w][row];
+    st_peer_f32(map_to_peer(smem_u32(&s_recv[rank][row]), peer), v);
+  }
+  cluster_arrive();
+  cluster_wait();
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int row = g + 8 * i;
+    if (row >= nt) continue;
+    float total = 0.f;
+#pragma unroll
+    for (int b = 0; b < kTsBlocks; ++b) total += s_recv[b][row];
+    const float rrms = 1.0f / sqrtf(total / (float)width + eps);
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+      const int c = 8 * (warp * NT + j) + c2;
+      const float2 w = *reinterpret_cast<const float2*>(norm_w + c0 + c);
+      *reinterpret_cast<float2*>(residual + (size_t)(t0 + row) * width + c0 + c) =
+          make_float2(s32[row * LS + c] + y[j][2 * i] * rrms * w.x, s32[row * LS + c + 1] + y[j][2 * i + 1] * rrms * w.y);
+    }
+  }
+}
+
+template <int SL>
+int token_side_cluster(float* residual, const void* x, const float* bias, const int* tokens, const void* table, int table_ld, int column,
+                       int dim, int vocab, const void* w_gate, const void* w_proj, const float* norm_w, int n_tokens, float eps,
+                       void* stream) {
+  static SmemRaised raised;
+  if (int rc = raise_shared_memory("token_side", token_side_cluster_kernel<SL>, (int)ts_smem(SL, kTsMaxDim), raised)) return rc;
+  return launch_kernel_cluster("token_side", token_side_cluster_kernel<SL>, dim3((n_tokens + kTsTokens - 1) / kTsTokens * kTsBlocks),
+                               dim3(kTsThreads), ts_smem(SL, dim), as_stream(stream), kTsBlocks, residual, (const __nv_bfloat16*)x, bias,
+                               tokens, (const __nv_bfloat16*)table, table_ld, column, dim, vocab, (const __nv_bfloat16*)w_gate,
+                               (const __nv_bfloat16*)w_proj, norm_w, eps, n_tokens);
+}
+
+}  // namespace ptl
+
+// -2: widths other than 512, 1,024 and 2,048, dims that are no whole sixteens up to 128, or rows off their boundaries.
+PTL_EXPORT int ptl_token_side_cluster_bf16(float* residual, const void* x, const float* bias, const int* tokens, const void* table,
+                                           int table_ld, int column, int dim, int vocab, const void* w_gate, const void* w_proj,
+                                           const float* norm_w, int n_tokens, int width, float eps, void* stream) {
+  using namespace ptl;
+  if ((width != 512 && width != 1024 && width != 2048) || dim < 16 || dim % 16 || dim > kTsMaxDim || !aligned16(residual) ||
+      (x && !aligned16(x)) || (bias && !aligned16(bias)) || !aligned16(w_gate) || !aligned16(w_proj) || !aligned16(norm_w))
+    return -2;
+  PTL_REQUIRE(n_tokens >= 0 && n_tokens <= (1 << 27) && column >= 0 && column + dim <= table_ld && eps > 0.f && vocab > 0,
+              "token_side: bad sizes width=%d dim=%d column=%d of %d", width, dim, column, table_ld);
+  if (n_tokens == 0) return 0;
+  const auto fn = width == 512 ? token_side_cluster<64> : width == 1024 ? token_side_cluster<128> : token_side_cluster<256>;
+  return fn(residual, x, bias, tokens, table, table_ld, column, dim, vocab, w_gate, w_proj, norm_w, n_tokens, eps, stream);
+}

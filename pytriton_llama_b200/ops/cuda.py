@@ -197,6 +197,8 @@ def load_library() -> ctypes.CDLL:
                                                     _c_int, _c_int, _c_f, _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_f, _c_int,
                                                     _c_int, _ptr, _ptr, _c_int, _c_int, _ptr, _c_f, _c_int, _c_int, _c_f, _ptr]
     lib.ptl_prefill_attention_opts_bf16.restype = _c_int
+    lib.ptl_token_side_cluster_bf16.argtypes = _SIGNATURES["ptl_token_side"]
+    lib.ptl_token_side_cluster_bf16.restype = _c_int
     lib.ptl_moe_tile_rows.argtypes = []
     lib.ptl_moe_tile_rows.restype = _c_int
     lib.ptl_moe_route.argtypes = [_ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _c_f, _ptr, _ptr]
@@ -1079,6 +1081,13 @@ class CudaOps:
             self._want(x, "x", table.dtype)
         if bias is not None:
             self._want(bias, "bias", torch.float32)
+        if table.dtype == torch.bfloat16:
+            rc = self.lib.ptl_token_side_cluster_bf16(_p(residual), _p(x), _p(bias), _p(tokens), _p(table), table.shape[1], int(column), int(dim),
+                                                      table.shape[0], _p(w_gate), _p(w_proj), _p(norm_w), residual.shape[0],
+                                                      residual.shape[1], float(eps), self._stream())
+            if rc != -2:
+                self._check(rc)
+                return
         fn = getattr(self.lib, "ptl_token_side" + _suffix(table.dtype))
         self._check(fn(_p(residual), _p(x), _p(bias), _p(tokens), _p(table), table.shape[1], int(column), int(dim), table.shape[0],
                        _p(w_gate), _p(w_proj), _p(norm_w), residual.shape[0], residual.shape[1], float(eps), self._stream()))

@@ -126,6 +126,24 @@ def test_selective_scan_in_segments_of_64_tokens(ops, dtype, inner, n):
     _close(dev["state"], cpu["state"], "float32", "state after the step")
 
 
+@pytest.mark.parametrize("T,W,dim", [(1, 512, 16), (8, 1024, 64), (17, 1024, 128), (70, 2048, 48)])
+def test_side_term_in_a_cluster(ops, T, W, dim):
+    """Sixteen tokens a cluster, remainders, with and without the pending output: against 64 bits to float32 sums, as the row
+    kernel is (weights N(0, 1/fan_in): results of order one)."""
+    g = torch.Generator().manual_seed(T * W)
+    V = 50
+    ids = torch.randint(0, V, (T,), generator=g, dtype=torch.int32)
+    side = torch.randn(V, 3 * dim, generator=g).bfloat16()
+    wg, wp = (torch.randn(dim, W, generator=g) / W ** 0.5).bfloat16(), (torch.randn(W, dim, generator=g) / dim ** 0.5).bfloat16()
+    res, nw, bias, x = torch.randn(T, W, generator=g), torch.randn(W, generator=g), torch.randn(W, generator=g), torch.randn(T, W, generator=g).bfloat16()
+    for xx, bb in ((x, bias), (None, None)):
+        want, got = res.double(), res.cuda()
+        TorchOps().token_side(want, xx, bb, ids, side, dim, dim, wg, wp, nw, 1e-5)
+        ops.token_side(got, None if xx is None else xx.cuda(), None if bb is None else bb.cuda(), ids.cuda(), side.cuda(), dim, dim,
+                       wg.cuda(), wp.cuda(), nw.cuda(), 1e-5)
+        assert (got.double().cpu() - want).abs().max() <= 2e-5 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_row_wise_operators(ops, dtype):
     g = torch.Generator().manual_seed(3)
