@@ -52,7 +52,7 @@ kv_write_normed_kernel(T* __restrict__ cache, const T* __restrict__ qkv, const f
 
 constexpr int kMaxMixedHeads = 128;     // heads whose weights can be mixed (a thread holds one key's column of them)
 
-// One block per query token.  Keys j = lo .. p of the token's request, lo = p - p % chunk (0 without chunks):
+// One block per query token (`items`: the token rows, else rows 0 .. tokens - 1).  Keys j = lo .. p of the token's request, lo = p - p % chunk (0 without chunks):
 //   score_h(j) = (q_h + bias) . k_j * scale - r1[h] * log1p(r2[h] * (p - j));   w_h = softmax_j;
 //   w'_h = sum_g talk[h, g] w_g;   out_h = out_scale * sum_j w'_h(j) v_j.
 // Shared memory: max_keys page addresses, the query (H * d floats), H * max_keys weights.
@@ -62,14 +62,15 @@ chunk_attention_kernel(T* __restrict__ out, int out_ld, int column, const T* __r
                        const float* __restrict__ q_bias, const T* __restrict__ cache, const int* __restrict__ block_table,
                        int table_width, const int* __restrict__ tok_req, const int* __restrict__ positions, int H, int G, int d,
                        int dv, int page_size, float scale, int chunk, const float* __restrict__ r1, const float* __restrict__ r2,
-                       const float* __restrict__ talk, int max_keys, int num_pages, float out_scale, int vec_ok) {
+                       const float* __restrict__ talk, int max_keys, int num_pages, float out_scale, int vec_ok,
+                       const int* __restrict__ items) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   long long* page_at = reinterpret_cast<long long*>(smem_raw);       // first element of the page that holds key j, -1: none
   float* q = reinterpret_cast<float*>(page_at + max_keys);
   float* w = q + H * d;
   pdl_wait();
   pdl_launch_dependents();
-  const int t = blockIdx.x;
+  const int t = items ? items[blockIdx.x] : blockIdx.x;
   const int r = tok_req[t];
   if (r < 0) return;
   const int p = positions[t];
@@ -207,7 +208,7 @@ template <typename T>
 int chunk_attention(void* out, int out_ld, int column, const void* qkv, int q_ld, const float* q_bias, const void* cache,
                     const int* block_table, int table_width, const int* tok_req, const int* positions, int tokens, int H, int G,
                     int d, int dv, int page_size, float scale, int chunk, const float* r1, const float* r2, const float* talk,
-                    int max_keys, int num_pages, float out_scale, void* stream) {
+                    int max_keys, int num_pages, float out_scale, const int* items, void* stream) {
   PTL_REQUIRE(tokens >= 0 && H > 0 && G > 0 && H % G == 0 && d > 0 && dv > 0 && page_size > 0 && chunk >= 0 && max_keys > 0,
               "chunk_attention: bad sizes tokens=%d H=%d G=%d d=%d dv=%d page=%d chunk=%d keys=%d", tokens, H, G, d, dv, page_size,
               chunk, max_keys);
@@ -225,7 +226,7 @@ int chunk_attention(void* out, int out_ld, int column, const void* qkv, int q_ld
   const int vec_ok = d % Vec16<T>::N == 0 && dv % Vec16<T>::N == 0 && d % 4 == 0 && aligned16(cache);   // every key row starts on a 16-byte boundary
   return launch_kernel("chunk_attention", chunk_attention_kernel<T>, dim3(tokens), dim3(256), smem, as_stream(stream), (T*)out,
                        out_ld, column, (const T*)qkv, q_ld, q_bias, (const T*)cache, block_table, table_width, tok_req, positions,
-                       H, G, d, dv, page_size, scale, chunk, r1, r2, talk, max_keys, num_pages, out_scale, vec_ok);
+                       H, G, d, dv, page_size, scale, chunk, r1, r2, talk, max_keys, num_pages, out_scale, vec_ok, items);
 }
 
 }  // namespace ptl
@@ -239,10 +240,10 @@ int chunk_attention(void* out, int out_ld, int column, const void* qkv, int q_ld
                                              const void* cache, const int* block_table, int table_width, const int* tok_req,      \
                                              const int* positions, int tokens, int H, int G, int d, int dv, int page_size,        \
                                              float scale, int chunk, const float* r1, const float* r2, const float* talk,         \
-                                             int max_keys, int num_pages, float out_scale, void* stream) {                        \
+                                             int max_keys, int num_pages, float out_scale, const int* items, void* stream) { \
     return ptl::chunk_attention<TYPE>(out, out_ld, column, qkv, q_ld, q_bias, cache, block_table, table_width, tok_req, positions, \
                                       tokens, H, G, d, dv, page_size, scale, chunk, r1, r2, talk, max_keys, num_pages, out_scale, \
-                                      stream);                                                                                    \
+                                      items, stream);                                                                                    \
   }
 PTL_CHUNK_ATTENTION(_f32, float)
 PTL_CHUNK_ATTENTION(_bf16, __nv_bfloat16)

@@ -1,0 +1,276 @@
+// The attention inside blocks of positions (see chunk_attention.cu) for bfloat16 caches on the tensor cores, up to eight query
+// heads over up to two kv heads of 64 or 128 entries, blocks of up to 256 positions: sixteen neighbouring positions of one
+// request per block, a warp per query head.
+//
+// Scores: a query is bfloat16 plus a float32 bias; the bfloat16 part goes to the tensor cores, the bias's product with a key is the
+// same for all queries and is worked out once per head and key in float32.  Keys come in tiles of 64 by cp.async.  A head's scores
+// of all its keys stay in shared memory as float32; the softmax runs over whole rows, the mixing between heads takes a key's
+// column of weights per thread, and the mixed float32 weights go to the tensor cores as three bfloat16 terms each (24 bits).
+// Nothing is rounded to 16 bits but the result.  Bound by the warp-level tensor instructions of a block's keys (one block per
+// SM).  Replaces, for the portions of such sizes, a block per token on the CUDA cores that reads a block's keys and values from
+// L2 once per query: 2,048 tokens of 8 heads of 128 in blocks of 256 took 221 us.  Here: 66 us, bound by the chain of
+// products, exponentials and products of one block of eight warps per SM (12 % of the warp slots).
+#include "mma_utils.cuh"
+
+namespace ptl {
+
+constexpr int kCtRows = 16, kCtKeys = 64, kCtThreads = 256, kCtHeads = 8, kCtMaxBlock = 256;
+constexpr int kCtLd = kCtMaxBlock + 8;               // floats of a row of weights: eight rows' pairs in different banks
+__host__ __device__ constexpr int ct_row_bytes(int d) { return 2 * d + 16; }
+constexpr int ct_smem(int d, int G) { return kCtHeads * kCtRows * kCtLd * 4 + 2 * G * kCtKeys * ct_row_bytes(d); }
+
+// x as three bfloat16 terms, two neighbours at a time
+__device__ __forceinline__ void ct_split(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack_bf16(x, y);
+  float2 back = unpack_bf16(hi);
+  x -= back.x; y -= back.y;
+  mid = pack_bf16(x, y);
+  back = unpack_bf16(mid);
+  lo = pack_bf16(x - back.x, y - back.y);
+}
+
+template <int D>
+__global__ void __launch_bounds__(kCtThreads, 1)
+chunk_attention_tc_kernel(__nv_bfloat16* __restrict__ out, int out_ld, int column, const __nv_bfloat16* __restrict__ qkv, int q_ld,
+                          const float* __restrict__ q_bias, const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table,
+                          int table_width, const int* __restrict__ tiles, int H, int G, int page_size, float scale, int chunk, const float* __restrict__ r1,
+                          const float* __restrict__ r2, const float* __restrict__ talk, int num_pages, float out_scale) {
+  extern __shared__ __align__(128) unsigned char ct_raw[];
+  float* s_w = reinterpret_cast<float*>(ct_raw);                                   // [8 heads][16][kCtLd]
+  const uint32_t s_kv = smem_u32(ct_raw) + kCtHeads * kCtRows * kCtLd * 4;         // [2][G][64] rows of a head
+  __shared__ float s_talk[kCtHeads * kCtHeads];
+  __shared__ __align__(16) float s_bias[kCtHeads * D], s_key[kCtHeads][kCtKeys];    // the queries' bias; its product with a tile's keys
+  __shared__ int s_there[kCtMaxBlock];                                              // keys that have a page
+  constexpr int RB = ct_row_bytes(D);
+  // the block's sixteen positions first .. first + 15, of which those from pos0 to end - 1 are tokens of its tile (inputs of
+  // the step: request row, first token row, tokens, first position)
+  const int* tile = tiles + 4 * blockIdx.y;
+  const int req = tile[0], token0 = tile[1], pos0 = tile[3], end = pos0 + tile[2];
+  const int first = pos0 / kCtRows * kCtRows + (int)blockIdx.x * kCtRows;
+  pdl_wait();
+  pdl_launch_dependents();
+  if (req < 0 || first >= end) return;
+  const int lo = first - first % chunk;                           // (a block of positions is a whole number of sixteens)
+  const int n = min(first + kCtRows, end) - lo;                   // keys
+  const int n_tiles = (n + kCtKeys - 1) / kCtKeys;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c2 = (lane & 3) * 2;
+  const int h = warp, group = H / G;
+  const size_t page_stride = (size_t)G * page_size * 2 * D;
+  const int* bt = block_table + (size_t)req * table_width;
+  auto fetch = [&](int tile, int values, int stage) {             // 64 keys (or values) of every kv head
+    const uint32_t dst = s_kv + stage * G * kCtKeys * RB;
+    for (int i = tid; i < G * kCtKeys * (D / 8); i += kCtThreads) {
+      const int p = i % (D / 8), row = i / (D / 8), c = row / kCtKeys, j = tile * kCtKeys + row % kCtKeys, pos = lo + j;
+      const int page = j < n ? bt[pos / page_size] : -1;
+      const bool ok = page >= 0 && page < num_pages;
+      const __nv_bfloat16* src = cache + (ok ? (size_t)page * page_stride + (size_t)values * G * page_size * D +
+                                                   ((size_t)c * page_size + pos % page_size) * D + 8 * p : 0);
+      cp_async_16(dst + row * RB + 16 * p, src, ok);
+    }
+    cp_async_commit();
+  };
+  fetch(0, 0, 0);
+  for (int j = tid; j < n_tiles * kCtKeys; j += kCtThreads) {
+    const int page = j < n ? bt[(lo + j) / page_size] : -1;
+    s_there[j] = page >= 0 && page < num_pages;
+  }
+  // tokens of this thread's rows g and g + 8; a row that is no token of the step reads the nearest one's query
+  int token[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) token[i] = token0 + min(max(first + g + 8 * i, pos0), end - 1) - pos0;
+  if (talk)
+    for (int i = tid; i < H * H; i += kCtThreads) s_talk[i] = talk[i];
+  uint32_t q[D / 16][4];
+  if (h < H) {
+#pragma unroll
+    for (int k = 0; k < D / 16; ++k)
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        q[k][e] = *reinterpret_cast<const uint32_t*>(qkv + (size_t)token[e & 1] * q_ld + h * D + 16 * k + c2 + 8 * (e >> 1));
+  }
+  if (q_bias)
+    for (int i = tid; i < H * D; i += kCtThreads) s_bias[i] = q_bias[i];
+  float* w_h = s_w + h * kCtRows * kCtLd;
+  const float f1 = r1 && h < H ? r1[h] : 0.f, f2 = r1 && h < H ? r2[h] : 0.f;
+  for (int t = 0; t < n_tiles; ++t) {
+    if (t + 1 < n_tiles) fetch(t + 1, 0, (t + 1) & 1);
+    else fetch(0, 1, (t + 1) & 1);                                // behind the last keys the first values
+    cp_async_wait<1>();
+    __syncthreads();
+    if (h < H) {
+      const uint32_t kt = s_kv + ((t & 1) * G + h / group) * kCtKeys * RB;
+      const uint32_t ka = kt + ((lane & 7) + 8 * (lane >> 4)) * RB + 16 * ((lane >> 3) & 1);
+      if (q_bias) {                                               // two keys per lane, float32
+        const unsigned char* rows = ct_raw + kCtHeads * kCtRows * kCtLd * 4 + (((t & 1) * G + h / group) * kCtKeys + lane) * RB;
+        float b0 = 0.f, b1 = 0.f;
+#pragma unroll 4
+        for (int e = 0; e < D; e += 8) {
+          const uint4 k0 = *reinterpret_cast<const uint4*>(rows + 2 * e), k1 = *reinterpret_cast<const uint4*>(rows + 32 * RB + 2 * e);
+          const float4 lo4 = *reinterpret_cast<const float4*>(s_bias + h * D + e), hi4 = *reinterpret_cast<const float4*>(s_bias + h * D + e + 4);
+          const float bias[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            const float2 x0 = unpack_bf16((&k0.x)[w]), x1 = unpack_bf16((&k1.x)[w]);
+            b0 = fmaf(bias[2 * w + 1], x0.y, fmaf(bias[2 * w], x0.x, b0));
+            b1 = fmaf(bias[2 * w + 1], x1.y, fmaf(bias[2 * w], x1.x, b1));
+          }
+        }
+        s_key[h][lane] = b0;
+        s_key[h][lane + 32] = b1;
+        __syncwarp();
+      }
+      float s[8][4];
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
+#pragma unroll
+      for (int k = 0; k < D / 16; ++k)
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+          uint32_t b[4];
+          ldmatrix_x4(b, ka + 8 * j * RB + 32 * k);
+          mma_bf16_16816(s[j], q[k], b[0], b[1]);
+          mma_bf16_16816(s[j + 1], q[k], b[2], b[3]);
+        }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          float2 v;
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int key = t * kCtKeys + 8 * j + c2 + e;
+            const int dist = first + g + 8 * i - lo - key;
+            float x = (s[j][2 * i + e] + (q_bias ? s_key[h][8 * j + c2 + e] : 0.f)) * scale;
+            if (r1) x -= f1 * log1pf(f2 * (float)max(dist, 0));
+            (&v.x)[e] = dist >= 0 && s_there[key] ? x : -INFINITY;
+          }
+          *reinterpret_cast<float2*>(w_h + (g + 8 * i) * kCtLd + t * kCtKeys + 8 * j + c2) = v;
+        }
+    }
+    __syncthreads();                                              // the tile's stage is free
+  }
+  const int width = n_tiles * kCtKeys;
+  if (h < H) {
+    for (int r = 0; r < kCtRows; ++r) {
+      float* row = w_h + r * kCtLd;
+      float x[kCtMaxBlock / 32], m = -INFINITY, sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < kCtMaxBlock / 32; ++i) {
+        x[i] = lane + 32 * i < width ? row[lane + 32 * i] : -INFINITY;
+        m = fmaxf(m, x[i]);
+      }
+      m = warp_max(m);
+#pragma unroll
+      for (int i = 0; i < kCtMaxBlock / 32; ++i) {
+        x[i] = x[i] == -INFINITY ? 0.f : expf(x[i] - m);
+        sum += x[i];
+      }
+      sum = warp_sum(sum);
+      const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+#pragma unroll
+      for (int i = 0; i < kCtMaxBlock / 32; ++i)
+        if (lane + 32 * i < width) row[lane + 32 * i] = x[i] * inv;
+    }
+  }
+  __syncthreads();
+  if (talk) {
+    float mixes[kCtHeads][kCtHeads];
+#pragma unroll
+    for (int b = 0; b < kCtHeads; ++b)
+#pragma unroll
+      for (int a = 0; a < kCtHeads; ++a) mixes[b][a] = a < H && b < H ? s_talk[b * H + a] : 0.f;
+    for (int i = tid; i < kCtRows * width; i += kCtThreads) {
+      float* at = s_w + (i / width) * kCtLd + i % width;
+      float x[kCtHeads];
+#pragma unroll
+      for (int a = 0; a < kCtHeads; ++a) x[a] = a < H ? at[a * kCtRows * kCtLd] : 0.f;
+#pragma unroll
+      for (int b = 0; b < kCtHeads; ++b) {
+        if (b >= H) break;
+        float y = 0.f;
+#pragma unroll
+        for (int a = 0; a < kCtHeads; ++a)
+          y = fmaf(mixes[b][a], x[a], y);
+        at[b * kCtRows * kCtLd] = y;
+      }
+    }
+    __syncthreads();
+  }
+  float o[D / 8][4];
+#pragma unroll
+  for (int j = 0; j < D / 8; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
+  const int turn = n_tiles & 1;                                   // the stage that holds the first values
+  for (int t = 0; t < n_tiles; ++t) {
+    if (t + 1 < n_tiles) fetch(t + 1, 1, (turn + t + 1) & 1); else cp_async_commit();
+    cp_async_wait<1>();
+    __syncthreads();
+    if (h < H) {
+      const uint32_t va = s_kv + (((turn + t) & 1) * G + h / group) * kCtKeys * RB + (lane & 15) * RB + 16 * (lane >> 4);
+#pragma unroll
+      for (int k = 0; k < kCtKeys / 16; ++k) {
+        uint32_t a[3][4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 v = *reinterpret_cast<const float2*>(w_h + (g + 8 * (e & 1)) * kCtLd + t * kCtKeys + 16 * k + c2 + 8 * (e >> 1));
+          ct_split(v.x, v.y, a[0][e], a[1][e], a[2][e]);
+        }
+#pragma unroll
+        for (int j = 0; j < D / 8; j += 2) {
+          uint32_t b[4];
+          ldmatrix_x4_trans(b, va + 16 * k * RB + 16 * j);
+#pragma unroll
+          for (int w = 2; w >= 0; --w) {
+            mma_bf16_16816(o[j], a[w], b[0], b[1]);
+            mma_bf16_16816(o[j + 1], a[w], b[2], b[3]);
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (h >= H) return;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int pos = first + g + 8 * i;
+    if (pos < pos0 || pos >= end) continue;
+    __nv_bfloat16* dst = out + (size_t)(token0 + pos - pos0) * out_ld + column + h * D + c2;
+#pragma unroll
+    for (int j = 0; j < D / 8; ++j)
+      *reinterpret_cast<uint32_t*>(dst + 8 * j) = pack_bf16(o[j][2 * i] * out_scale, o[j][2 * i + 1] * out_scale);
+  }
+}
+
+template <int D>
+int chunk_attention_tc(void* out, int out_ld, int column, const void* qkv, int q_ld, const float* q_bias, const void* cache,
+                       const int* bt, int table_width, const int* tiles, dim3 grid, int H, int G, int page_size, float scale, int chunk, const float* r1, const float* r2, const float* talk,
+                       int num_pages, float out_scale, void* stream) {
+  static SmemRaised raised;
+  if (int rc = raise_shared_memory("chunk_attention_tc", chunk_attention_tc_kernel<D>, ct_smem(D, 2), raised)) return rc;
+  return launch_kernel("chunk_attention_tc", chunk_attention_tc_kernel<D>, grid, dim3(kCtThreads), ct_smem(D, G), as_stream(stream),
+                       (__nv_bfloat16*)out, out_ld, column, (const __nv_bfloat16*)qkv, q_ld, q_bias, (const __nv_bfloat16*)cache, bt,
+                       table_width, tiles, H, G, page_size, scale, chunk, r1, r2, talk, num_pages, out_scale);
+}
+
+}  // namespace ptl
+
+// The step's portions: n_tiles tiles of up to tile_tokens tokens.  -2: sizes or addresses for the other kernel.
+PTL_EXPORT int ptl_chunk_attention_tc_bf16(void* out, int out_ld, int column, const void* qkv, int q_ld, const float* q_bias,
+                                           const void* cache, const int* block_table, int table_width, const int* tiles, int n_tiles,
+                                           int tile_tokens, int H, int G, int d, int page_size, float scale, int chunk, const float* r1,
+                                           const float* r2, const float* talk, int num_pages, float out_scale, void* stream) {
+  if ((d != 64 && d != 128) || H < 1 || H > ptl::kCtHeads || G < 1 || G > 2 || H % G || chunk < ptl::kCtRows || chunk % ptl::kCtRows ||
+      chunk > ptl::kCtMaxBlock || q_ld % 2 || out_ld % 2 || column % 2 || !ptl::aligned16(cache) ||
+      (reinterpret_cast<uintptr_t>(qkv) & 3u) || (reinterpret_cast<uintptr_t>(out) & 3u))
+    return -2;
+  PTL_REQUIRE((r1 == nullptr) == (r2 == nullptr) && page_size > 0 && num_pages > 0 && n_tiles >= 0 && n_tiles <= 65535 && tile_tokens > 0 &&
+                  column >= 0 && column + H * d <= out_ld && q_ld >= H * d, "chunk_attention_tc: bad sizes");
+  const dim3 grid((tile_tokens + ptl::kCtRows - 1) / ptl::kCtRows + 1, n_tiles);
+  if (n_tiles == 0) return 0;
+  const auto fn = d == 64 ? ptl::chunk_attention_tc<64> : ptl::chunk_attention_tc<128>;
+  return fn(out, out_ld, column, qkv, q_ld, q_bias, cache, block_table, table_width, tiles, grid, H, G, page_size, scale, chunk, r1, r2, talk,
+            num_pages, out_scale, stream);
+}

@@ -46,7 +46,7 @@ _SIGNATURES = {
                             _ptr],
     "ptl_kv_write_normed": [_ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_f, _ptr],
     "ptl_chunk_attention": [_ptr, _c_int, _c_int, _ptr, _c_int, _ptr, _ptr, _ptr, _c_int, _ptr, _ptr, _c_int, _c_int, _c_int,
-                            _c_int, _c_int, _c_int, _c_f, _c_int, _ptr, _ptr, _ptr, _c_int, _c_int, _c_f, _ptr],
+                            _c_int, _c_int, _c_int, _c_f, _c_int, _ptr, _ptr, _ptr, _c_int, _c_int, _c_f, _ptr, _ptr],
     "ptl_stream_mix_norm": [_ptr, _ptr, _ptr, _ptr, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_f, _ptr],
     "ptl_gelu_tanh": [_ptr, _ptr, _c_ll, _ptr],
     "ptl_qk_norm_rotate_store": [_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _c_f, _ptr, _ptr, _c_int, _c_f, _ptr,
@@ -197,6 +197,9 @@ def load_library() -> ctypes.CDLL:
                                                     _c_int, _c_int, _c_f, _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_f, _c_int,
                                                     _c_int, _ptr, _ptr, _c_int, _c_int, _ptr, _c_f, _c_int, _c_int, _c_f, _ptr]
     lib.ptl_prefill_attention_opts_bf16.restype = _c_int
+    lib.ptl_chunk_attention_tc_bf16.argtypes = [_ptr, _c_int, _c_int, _ptr, _c_int, _ptr, _ptr, _ptr, _c_int, _ptr, _c_int, _c_int, _c_int,
+                                                _c_int, _c_int, _c_int, _c_f, _c_int, _ptr, _ptr, _ptr, _c_int, _c_f, _ptr]
+    lib.ptl_chunk_attention_tc_bf16.restype = _c_int
     lib.ptl_token_side_cluster_bf16.argtypes = _SIGNATURES["ptl_token_side"]
     lib.ptl_token_side_cluster_bf16.restype = _c_int
     lib.ptl_moe_tile_rows.argtypes = []
@@ -326,7 +329,7 @@ class CudaOps:
         "embed_bigram": "elementwise", "_pair_angles": "rope", "pair_rotate_store": "rope",
         "embed_scaled": "elementwise", "softcap": "elementwise", "clamped_glu": "elementwise", "token_side": "token_input",
         "causal_conv": "recurrent", "selective_scan": "recurrent", "gated_delta_rule": "recurrent", "gated_head_norm": "norm",
-        "kv_write_normed": "attention", "chunk_attention": "attention",
+        "kv_write_normed": "attention", "chunk_attention": "attention", "chunk_attention_of_step": "attention",
         "linear": "product", "linear_add": "product", "gate_up_act": "product", "gemm_tc": "product",
         "_qkv_rope_product": "product", "rope_kv_write": "rope", "_rope_table": "rope",
         "paged_attention": "attention", "_attention_tensor_cores": "attention",
@@ -1194,9 +1197,10 @@ class CudaOps:
     def chunk_attention(self, qkv: torch.Tensor, bias: Optional[torch.Tensor], cache: torch.Tensor, block_table: torch.Tensor,
                         tok_req: torch.Tensor, positions: torch.Tensor, H: int, G: int, d: int, dv: int, page_size: int,
                         scale: float, chunk: int, r1: Optional[torch.Tensor], r2: Optional[torch.Tensor],
-                        talk: Optional[torch.Tensor], out: torch.Tensor, column: int, out_scale: float, max_keys: int = 0) -> None:
-        """The attention of ``parts/chunk_attention.py`` for every token of the step; the heads' outputs times
-        ``out_scale`` go to columns ``column``.. of ``out``.  ``max_keys``: the most keys a query sees (default: the
+                        talk: Optional[torch.Tensor], out: torch.Tensor, column: int, out_scale: float, max_keys: int = 0,
+                        rows=None) -> None:
+        """The attention of ``parts/chunk_attention.py`` for every token of the step, or for ``rows`` (int32 row indices or None
+        for 0..n-1, n); the heads' outputs times ``out_scale`` go to columns ``column``.. of ``out``.  ``max_keys``: the most keys a query sees (default: the
         chunk, or every position the block table can name)."""
         self._want(qkv, "qkv")
         self._want(cache, "cache", qkv.dtype)
@@ -1208,10 +1212,43 @@ class CudaOps:
                 self._want(t, name, torch.float32)
         reach = block_table.shape[1] * page_size
         max_keys = int(max_keys) or (min(chunk, reach) if chunk else reach)
+        items, n_rows = (None, qkv.shape[0]) if rows is None else rows
         fn = getattr(self.lib, "ptl_chunk_attention" + _suffix(qkv.dtype))
         self._check(fn(_p(out), out.shape[1], int(column), _p(qkv), qkv.shape[1], _p(bias), _p(cache), _p(block_table),
-                       block_table.shape[1], _p(tok_req), _p(positions), qkv.shape[0], H, G, d, dv, page_size, float(scale),
-                       int(chunk), _p(r1), _p(r2), _p(talk), max_keys, cache.shape[0], float(out_scale), self._stream()))
+                       block_table.shape[1], _p(tok_req), _p(positions), n_rows, H, G, d, dv, page_size, float(scale),
+                       int(chunk), _p(r1), _p(r2), _p(talk), max_keys, cache.shape[0], float(out_scale), _p(items), self._stream()))
+
+    def chunk_attention_of_step(self, ctx, qkv: torch.Tensor, bias: Optional[torch.Tensor], cache: torch.Tensor,
+                                block_table: torch.Tensor, H: int, G: int, d: int, dv: int, page_size: int, scale: float, chunk: int,
+                                r1: Optional[torch.Tensor], r2: Optional[torch.Tensor], talk: Optional[torch.Tensor],
+                                out: torch.Tensor, column: int, out_scale: float) -> None:
+        """``chunk_attention`` for a step whose context carries the work lists: in bfloat16, with heads of 64 or 128 and blocks
+        of whole sixteens up to 256 positions, its portions on the tensor cores."""
+        dec, tiles, rows = self._work(ctx, "decode_items"), self._work(ctx, "prefill_tiles"), None
+        if qkv.dtype == torch.bfloat16 and d == dv and dec is not None and tiles is not None:
+            self._want(qkv, "qkv")
+            self._want(cache, "cache", qkv.dtype)
+            self._want(out, "out", qkv.dtype)
+            for name, t in (("block_table", block_table), ("tok_req", ctx.tok_req), ("positions", ctx.positions)):
+                self._want(t, name, torch.int32)
+            for name, t in (("bias", bias), ("r1", r1), ("r2", r2), ("talk", talk)):
+                if t is not None:
+                    self._want(t, name, torch.float32)
+            if cache[0].numel() != G * page_size * 2 * d:
+                raise KernelError("chunk_attention: the cache's pages do not fit the heads")
+            rc = -2
+            if tiles.items:
+                rc = self.lib.ptl_chunk_attention_tc_bf16(
+                    _p(out), out.shape[1], int(column), _p(qkv), qkv.shape[1], _p(bias), _p(cache), _p(block_table), block_table.shape[1],
+                    _p(tiles.tensor), tiles.items, self.QUERY_TILE, H, G, d, page_size, float(scale), int(chunk), _p(r1), _p(r2), _p(talk),
+                    cache.shape[0], float(out_scale), self._stream())
+            if rc != -2:
+                self._check(rc)
+                if not dec.items:
+                    return
+                rows = (None if dec.in_order else dec.tensor, dec.items)       # the single tokens, a block each
+        self.chunk_attention(qkv, bias, cache, block_table, ctx.tok_req, ctx.positions, H, G, d, dv, page_size, scale, chunk, r1, r2, talk,
+                             out, column, out_scale, rows=rows)
 
     # ------------------------------------------------------------------ copies of the stream, windowed attention, gated linear attention, experts
     def stream_mix_norm(self, streams: Optional[torch.Tensor], init: Optional[torch.Tensor], y: Optional[torch.Tensor],

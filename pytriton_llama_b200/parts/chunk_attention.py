@@ -76,8 +76,12 @@ class ChunkAttention(Part):
         if cache.write:
             ops.kv_write_normed(qkv, self.b_qkv, g.slots, cache.kv, self.heads, self.kv_heads, self.d, self.dv, g.page_size,
                                 self.value_norm_eps)
-        ops.chunk_attention(qkv, self.b_qkv, cache.kv, g.block_table, ctx.tok_req, ctx.positions, self.heads, self.kv_heads,
-                            self.d, self.dv, g.page_size, self.scale, self.chunk, self.r1, self.r2, self.talk, out, column, scale)
+        sizes = (self.heads, self.kv_heads, self.d, self.dv, g.page_size, self.scale, self.chunk, self.r1, self.r2, self.talk)
+        whole_step = getattr(ops, "chunk_attention_of_step", None)       # an operator set that looks at the step's work lists
+        if whole_step is not None:
+            whole_step(ctx, qkv, self.b_qkv, cache.kv, g.block_table, *sizes, out, column, scale)
+        else:
+            ops.chunk_attention(qkv, self.b_qkv, cache.kv, g.block_table, ctx.tok_req, ctx.positions, *sizes, out, column, scale)
 
     def forward(self, x, ctx, cache):
         out = self.rt.ops.empty((x.shape[0], self.inner_width), self.rt.dtype)

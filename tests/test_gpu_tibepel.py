@@ -144,6 +144,38 @@ def test_side_term_in_a_cluster(ops, T, W, dim):
         assert (got.double().cpu() - want).abs().max() <= 2e-5 * float(want.abs().max())
 
 
+@pytest.mark.parametrize("H,G,d,page,chunk,options", [(8, 2, 128, 16, 256, True), (4, 2, 64, 8, 48, True), (1, 1, 128, 4, 16, False),
+                                                      (6, 2, 64, 16, 240, True)])
+def test_chunk_attention_on_the_tensor_cores(ops, H, G, d, page, chunk, options):
+    """Against the general kernel on the same inputs: scores, weights and sums are float32 in both, so that only the result's
+    rounding (2^-8 of it) and float32 sums differ.  Portions begin and end inside sixteens and cross blocks of positions."""
+    g = torch.Generator().manual_seed(H * 10 + d)
+    q_lens, starts = [9, 1, 300, 1, 130, 2, 16], [0, 40, 5, 0, 250, 255, 256]
+    ctx = [s + n for s, n in zip(starts, q_lens)]
+    T, width = sum(q_lens), H * d + 2 * G * d
+    pages = [-(-c // page) for c in ctx]
+    order, table, at = torch.randperm(sum(pages) + 2, generator=g).tolist(), torch.full((7, max(pages) + 1), -1, dtype=torch.int32), 0
+    for r, k in enumerate(pages):
+        table[r, :k] = torch.tensor(order[at:at + k], dtype=torch.int32)
+        at += k
+    cache = torch.randn(sum(pages) + 2, G * page * 2 * d, generator=g).bfloat16().cuda()
+    qkv = torch.randn(T, width, generator=g).bfloat16().cuda()
+    opt = [t.cuda() if options else None for t in (torch.randn(width, generator=g) * 0.3, torch.rand(H, generator=g),
+                                                   torch.rand(H, generator=g) + 0.1, torch.randn(H, H, generator=g))]
+    c, table = _ctx(q_lens, starts, list(range(7)), "cuda:0"), table.cuda()
+    c.work = ops.hints_for(q_lens, ctx).work
+    outs = []
+    for whole in (True, False):
+        out = torch.zeros(T, H * d + 6, dtype=torch.bfloat16, device="cuda")
+        if whole:
+            ops.chunk_attention_of_step(c, qkv, opt[0], cache, table, H, G, d, d, page, 0.2, chunk, *opt[1:], out, 4, 0.7)
+        else:
+            ops.chunk_attention(qkv, opt[0], cache, table, c.tok_req, c.positions, H, G, d, d, page, 0.2, chunk, *opt[1:], out, 4, 0.7)
+        outs.append(out.double().cpu())
+    assert not outs[0][:, :4].any() and not outs[0][:, -2:].any()
+    assert ((outs[0] - outs[1]).abs() <= 2 ** -7 * outs[1].abs() + 2e-5 * float(outs[1].abs().max())).all()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_row_wise_operators(ops, dtype):
     g = torch.Generator().manual_seed(3)
