@@ -1,0 +1,370 @@
+// The gated delta rule (see recurrent.cu) for portions of many tokens, 64 tokens at a time.  Inside a chunk, with L_t the
+// running sum of log decays, k and q scaled to unit length and S the state before the chunk:
+//     u_t = beta_t (v_t - e^(L_t) S^T k_t - sum_{i<t} e^(L_t - L_i) (k_t . k_i) u_i)        a triangular system
+//     o_t = e^(L_t) S^T q_t + sum_{i<=t} e^(L_t - L_i) (q_t . k_i) u_i
+//     S  <- e^(L_end) S + sum_i e^(L_end - L_i) k_i u_i^T
+// Everything that does not know S is worked out for all chunks side by side (delta_chunk_prepare: the system solved for its
+// two right sides, U = WV - WK S, and the factors of the other two lines); what is left of the serial walk is three small
+// products a chunk (delta_chunk_walk).  All of it float32 multiply-adds; the running sums are kept in 64 bits, because a
+// difference of two of them is the exponent of a decay.  (An input that is no number reaches the results of its whole chunk,
+// where the walk kept it from the tokens before it.)
+//
+// The token-by-token walk is bound by the latency of its chain, 0.36 us a token at heads of 128 x 128: 738 us for
+// 2,048 tokens, whatever the number of SMs.  Here 16 heads of that size take 88 us (prepare: the chains of the 64 x 64 systems,
+// two blocks an SM) and 118 us (walk: 32 dependent chunks of three products).  The error against 64 bits is the walk's or less.
+#include "mma_utils.cuh"
+
+namespace ptl {
+
+constexpr int kDcTokens = 64, kDcThreads = 256, kDcCols = 8;
+constexpr int kDcSysLd = kDcTokens + 4;
+
+__device__ __forceinline__ float dc_softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
+
+// Which request a chunk of the step belongs to: (request, first row, rows), request -1 behind the last one; chunks of a
+// request are numbered one after the other, requests in order.
+__device__ __forceinline__ int3 dc_locate(const int* __restrict__ q_start, int requests, int chunk) {
+  for (int r = 0; r < requests; ++r) {
+    const int lo = q_start[r], n = q_start[r + 1] - lo;
+    const int chunks = n > 0 ? (n + kDcTokens - 1) / kDcTokens : 0;
+    if (chunk < chunks) return make_int3(r, lo + chunk * kDcTokens, min(kDcTokens, n - chunk * kDcTokens));
+    chunk -= chunks;
+  }
+  return make_int3(-1, 0, 0);
+}
+
+// Floats of a (chunk, head) in the workspace: WK and the decayed queries [64][D], the decayed keys [D][64], the read-out's
+// weights [64][64], WV [64][dv], the chunk's decay (padded to 16 bytes).
+__host__ __device__ __forceinline__ size_t dc_floats(int D, int dv) { return (size_t)kDcTokens * (3 * D + kDcTokens + dv) + 4; }
+constexpr size_t dc_prepare_smem(int D) { return sizeof(float) * (2 * kDcTokens * (D + 4) + kDcTokens * kDcSysLd); }
+constexpr size_t dc_walk_smem(int D) {
+  return sizeof(float) * (2 * 2 * kDcTokens * (D + 4) + (kDcTokens + D) * kDcSysLd + kDcCols * (D + 4) + kDcCols * kDcSysLd);
+}
+
+// Bound by its multiply-adds (2.1 M a chunk and head of 128 x 128) and the 64 steps of the substitution, a column per thread
+// held in registers, which update all later rows at once.
+template <typename T, int D>
+__global__ void __launch_bounds__(kDcThreads, 2)
+delta_chunk_prepare_kernel(float* __restrict__ work, const T* __restrict__ qkv, const float* __restrict__ ba, const float* __restrict__ rate,
+                           const float* __restrict__ dt_bias, const int* __restrict__ q_start, const int* __restrict__ state_slot,
+                           int requests, int heads, int kv_heads, int dv, float unit_eps, float q_scale) {
+  constexpr int LD = D + 4;
+  extern __shared__ __align__(16) float dp_smem[];
+  float* s_k = dp_smem;                            // [64][LD], as projected: the lengths are applied to what is made of them,
+  float* s_q = s_k + kDcTokens * LD;               // [64][LD]  which is then rounded once
+  float* s_sys = s_q + kDcTokens * LD;             // [i][t]: what u_i takes off row t > i
+  __shared__ double s_log[kDcTokens];
+  __shared__ float s_beta[kDcTokens], s_decay[kDcTokens], s_kn[kDcTokens], s_qn[kDcTokens];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int3 at = dc_locate(q_start, requests, blockIdx.x);
+  if (at.x < 0 || state_slot[at.x] < 0) return;
+  const int h = blockIdx.y, c = h / (heads / kv_heads), n = at.z;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int ld = 2 * kv_heads * D + heads * dv;
+  const T* rows = qkv + (size_t)at.y * ld;
+  float* wk = work + ((size_t)blockIdx.x * heads + h) * dc_floats(D, dv);
+  float* qg = wk + kDcTokens * D;
+  float* kdt = qg + kDcTokens * D;
+  float* mix = kdt + kDcTokens * D;
+  float* wv = mix + kDcTokens * kDcTokens;
+  // q and k of a token per warp and turn; rows past the portion are zero throughout
+  for (int t = warp; t < kDcTokens; t += kDcThreads / 32) {
+    float q[D / 32], k[D / 32], qq = 0.f, kk = 0.f;
+#pragma unroll
+    for (int i = 0; i < D / 32; ++i) {
+      q[i] = t < n ? to_f32(rows[(size_t)t * ld + c * D + lane + 32 * i]) : 0.f;
+      k[i] = t < n ? to_f32(rows[(size_t)t * ld + (kv_heads + c) * D + lane + 32 * i]) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < D / 32; ++i) { qq = fmaf(q[i], q[i], qq); kk = fmaf(k[i], k[i], kk); }
+    qq = warp_sum(qq);
+    kk = warp_sum(kk);
+    if (lane == 0) {
+      s_qn[t] = q_scale / sqrtf(qq + unit_eps);
+      s_kn[t] = 1.0f / sqrtf(kk + unit_eps);
+    }
+#pragma unroll
+    for (int i = 0; i < D / 32; ++i) {
+      s_q[t * LD + lane + 32 * i] = q[i];
+      s_k[t * LD + lane + 32 * i] = k[i];
+    }
+  }
+  if (warp == 0) {
+    double run = 0.0;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int t = lane + 32 * half;
+      double x = 0.0;
+      float beta = 0.f;
+      if (t < n) {
+        const float* g = ba + (size_t)(at.y + t) * 2 * heads;
+        beta = 1.0f / (1.0f + expf(-g[h]));
+        x = (double)(-rate[h] * dc_softplus(g[heads + h] + dt_bias[h]));
+        if (x < -1e4) x = -1e4;                    // a decay of zero either way; differences of the sums stay numbers
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double before = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += before;
+      }
+      x += run;
+      run = __shfl_sync(0xffffffffu, x, 31);
+      s_log[t] = x;
+      s_beta[t] = beta;
+      s_decay[t] = expf((float)x);
+    }
+  }
+  __syncthreads();
+  {
+    // k_t . k_i and q_t . k_i, four by four per thread
+    const int tx = tid & 15, ty = tid >> 4;
+    float kk[4][4], qk[4][4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) { kk[a][b] = 0.f; qk[a][b] = 0.f; }
+#pragma unroll 1
+    for (int e0 = 0; e0 < D; e0 += 16) {       // sixteen products a chain, the chains' sums added up: shorter chains round less
+      float k16[4][4], q16[4][4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) { k16[a][b] = 0.f; q16[a][b] = 0.f; }
+#pragma unroll 2
+      for (int e = e0; e < e0 + 16; e += 4) {
+        float4 col[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) col[b] = *reinterpret_cast<const float4*>(s_k + (tx + 16 * b) * LD + e);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+          const float4 kt = *reinterpret_cast<const float4*>(s_k + (ty + 16 * a) * LD + e);
+          const float4 qt = *reinterpret_cast<const float4*>(s_q + (ty + 16 * a) * LD + e);
+#pragma unroll
+          for (int b = 0; b < 4; ++b) {
+            k16[a][b] = fmaf(kt.x, col[b].x, fmaf(kt.y, col[b].y, fmaf(kt.z, col[b].z, fmaf(kt.w, col[b].w, k16[a][b]))));
+            q16[a][b] = fmaf(qt.x, col[b].x, fmaf(qt.y, col[b].y, fmaf(qt.z, col[b].z, fmaf(qt.w, col[b].w, q16[a][b]))));
+          }
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) { kk[a][b] += k16[a][b]; qk[a][b] += q16[a][b]; }
+    }
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int t = ty + 16 * a, i = tx + 16 * b;
+        const float decay = i <= t ? expf((float)(s_log[t] - s_log[i])) : 0.f;
+        s_sys[i * kDcSysLd + t] = i < t ? s_beta[t] * decay * (s_kn[t] * s_kn[i]) * kk[a][b] : 0.f;
+        mix[t * kDcTokens + i] = i <= t ? decay * (s_qn[t] * s_kn[i]) * qk[a][b] : 0.f;
+      }
+  }
+  const double end = s_log[kDcTokens - 1];
+  for (int i = tid; i < kDcTokens * D; i += kDcThreads) {
+    const int t = i / D, e = i % D;
+    qg[i] = s_decay[t] * s_qn[t] * s_q[t * LD + e];
+    const int t2 = i % kDcTokens, e2 = i / kDcTokens;
+    kdt[i] = expf((float)(end - s_log[t2])) * s_kn[t2] * s_k[t2 * LD + e2];
+  }
+  if (tid == 0) wv[kDcTokens * dv] = s_decay[kDcTokens - 1];
+  __syncthreads();
+  for (int col = tid; col < D + dv; col += kDcThreads) {
+    float u[kDcTokens];
+    if (col < D) {
+#pragma unroll
+      for (int t = 0; t < kDcTokens; ++t) u[t] = s_beta[t] * s_decay[t] * s_kn[t] * s_k[t * LD + col];
+    } else {
+      const T* v = rows + 2 * kv_heads * D + (size_t)h * dv + (col - D);
+#pragma unroll
+      for (int t = 0; t < kDcTokens; ++t) u[t] = t < n ? s_beta[t] * to_f32(v[(size_t)t * ld]) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < kDcTokens - 1; ++i) {
+      asm volatile("" ::: "memory");               // (a row's loads are not all moved ahead: two blocks per SM need the registers)
+#pragma unroll
+      for (int t4 = (i + 1) & ~3; t4 < kDcTokens; t4 += 4) {      // (rows up to i have a zero there)
+        const float4 a = *reinterpret_cast<const float4*>(s_sys + i * kDcSysLd + t4);
+        u[t4] = t4 > i ? fmaf(-a.x, u[i], u[t4]) : u[t4];
+        u[t4 + 1] = t4 + 1 > i ? fmaf(-a.y, u[i], u[t4 + 1]) : u[t4 + 1];
+        u[t4 + 2] = t4 + 2 > i ? fmaf(-a.z, u[i], u[t4 + 2]) : u[t4 + 2];
+        u[t4 + 3] = fmaf(-a.w, u[i], u[t4 + 3]);
+      }
+    }
+    float* dst = col < D ? wk + col : wv + (col - D);
+    const int step = col < D ? D : dv;
+#pragma unroll
+    for (int t = 0; t < kDcTokens; ++t) dst[(size_t)t * step] = u[t];
+  }
+}
+
+// Eight columns of one head's state per block.  Eight lanes share a row of a product: lane s takes the entries 4 s .. 4 s + 3 of
+// every 32 (a quarter warp reads 128 bytes of one row, the state's column packets are the same for the whole warp) against
+// all eight columns, and the lanes' sums meet by halves, so that lane s ends up with column s.  WK and the queries of the
+// next chunk are on their way while a chunk is worked; its decayed keys and read-out weights while the next one's first
+// product runs.  Bound by these multiply-adds and by L2: 120 KB a chunk and block.
+template <int ROWS>
+__device__ __forceinline__ void dc_meet(float (&acc)[ROWS][kDcCols], int s, float (&sum)[ROWS]) {
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j) {
+    float h4[4], h2[2];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float mine = s & 4 ? acc[j][c + 4] : acc[j][c], theirs = s & 4 ? acc[j][c] : acc[j][c + 4];
+      h4[c] = mine + __shfl_xor_sync(0xffffffffu, theirs, 4);
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const float mine = s & 2 ? h4[c + 2] : h4[c], theirs = s & 2 ? h4[c] : h4[c + 2];
+      h2[c] = mine + __shfl_xor_sync(0xffffffffu, theirs, 2);
+    }
+    const float mine = s & 1 ? h2[1] : h2[0], theirs = s & 1 ? h2[0] : h2[1];
+    sum[j] = mine + __shfl_xor_sync(0xffffffffu, theirs, 1);
+  }
+}
+
+template <int ROWS, int K, int LDA, int LDB>
+__device__ __forceinline__ void dc_product(const float* __restrict__ a, const float* __restrict__ b, int s, float (&sum)[ROWS]) {
+  float acc[ROWS][kDcCols];
+#pragma unroll
+  for (int j = 0; j < ROWS; ++j)
+#pragma unroll
+    for (int c = 0; c < kDcCols; ++c) acc[j][c] = 0.f;
+#pragma unroll
+  for (int k = 0; k < K; k += 32) {
+    float4 x[ROWS];
+#pragma unroll
+    for (int j = 0; j < ROWS; ++j) x[j] = *reinterpret_cast<const float4*>(a + 32 * j * LDA + k + 4 * s);
+#pragma unroll
+    for (int c = 0; c < kDcCols; ++c) {
+      const float4 y = *reinterpret_cast<const float4*>(b + c * LDB + k + 4 * s);
+#pragma unroll
+      for (int j = 0; j < ROWS; ++j)
+        acc[j][c] = fmaf(x[j].x, y.x, fmaf(x[j].y, y.y, fmaf(x[j].z, y.z, fmaf(x[j].w, y.w, acc[j][c]))));
+    }
+  }
+  dc_meet<ROWS>(acc, s, sum);
+}
+
+template <int D>
+__global__ void __launch_bounds__(kDcThreads, 1)
+delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, const float* __restrict__ work, const int* __restrict__ q_start,
+                        const int* __restrict__ positions, const int* __restrict__ state_slot, int heads, int dv) {
+  constexpr int LD = D + 4, RB = 2 + D / 32;
+  extern __shared__ __align__(16) float dw_smem[];
+  float* s_a = dw_smem;                                  // [2][WK 64 | q 64][LD]
+  float* s_b = s_a + 2 * 2 * kDcTokens * LD;             // [read-out weights 64 | keys D][68]
+  float* s_s = s_b + (kDcTokens + D) * kDcSysLd;         // [8][LD]: the state's columns
+  float* s_u = s_s + kDcCols * LD;                       // [8][68]
+  pdl_wait();
+  pdl_launch_dependents();
+  const int r = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * kDcCols;
+  const int lo = q_start[r], n = q_start[r + 1] - lo;
+  if (n <= 0 || state_slot[r] < 0) return;
+  int chunk0 = 0;
+  for (int i = 0; i < r; ++i) chunk0 += (max(q_start[i + 1] - q_start[i], 0) + kDcTokens - 1) / kDcTokens;
+  const int chunks = (n + kDcTokens - 1) / kDcTokens;
+  const int tid = threadIdx.x, lane = tid & 31, s = lane & 7, rg = (tid >> 5) * 4 + (lane >> 3);
+  const size_t stride = (size_t)heads * dc_floats(D, dv);
+  const float* base = work + ((size_t)chunk0 * heads + h) * dc_floats(D, dv);
+  float* st = state + (((size_t)state_slot[r] * heads + h) * D) * dv + j0;
+  const bool from_zero = positions[lo] == 0;
+  for (int i = tid; i < D * kDcCols; i += kDcThreads) {
+    const int e = i / kDcCols, c = i % kDcCols;
+    s_s[c * LD + e] = from_zero ? 0.f : st[(size_t)e * dv + c];
+  }
+  auto fetch_a = [&](int chunk) {
+    const float* src = base + chunk * stride;
+    const uint32_t dst = smem_u32(s_a + (chunk & 1) * 2 * kDcTokens * LD);
+    for (int i = tid; i < 2 * kDcTokens * (D / 4); i += kDcThreads)
+      cp_async_16(dst + ((i / (D / 4)) * LD + (i % (D / 4)) * 4) * 4, src + 4 * i, true);      // (the queries follow WK)
+    cp_async_commit();
+  };
+  auto fetch_b = [&](int chunk) {
+    const float* src = base + chunk * stride + 2 * kDcTokens * D;
+    const uint32_t dst = smem_u32(s_b);
+    for (int i = tid; i < (D + kDcTokens) * (kDcTokens / 4); i += kDcThreads) {
+      const int row = i / (kDcTokens / 4), p = i % (kDcTokens / 4);
+      const int to = row < D ? kDcTokens + row : row - D;                                      // keys come first, go last
+      cp_async_16(dst + (to * kDcSysLd + p * 4) * 4, src + 4 * i, true);
+    }
+    cp_async_commit();
+  };
+  fetch_a(0);
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    const int rows = min(kDcTokens, n - chunk * kDcTokens);
+    const float* wv = base + chunk * stride + (size_t)kDcTokens * (3 * D + kDcTokens);
+    const float v0 = wv[(size_t)rg * dv + j0 + s], v1 = wv[(size_t)(rg + 32) * dv + j0 + s], decay = wv[(size_t)kDcTokens * dv];
+    cp_async_wait<0>();
+    __syncthreads();                       // WK and q are here; the chunk before has been read and its state written
+    fetch_b(chunk);
+    if (chunk + 1 < chunks) fetch_a(chunk + 1); else cp_async_commit();
+    float first[4];
+    dc_product<4, D, LD, LD>(s_a + (chunk & 1) * 2 * kDcTokens * LD + rg * LD, s_s, s, first);
+    s_u[s * kDcSysLd + rg] = v0 - first[0];
+    s_u[s * kDcSysLd + rg + 32] = v1 - first[1];
+    cp_async_wait<1>();
+    __syncthreads();                       // U is whole, keys and read-out weights are here
+    float second[RB];
+    dc_product<RB, kDcTokens, kDcSysLd, kDcSysLd>(s_b + rg * kDcSysLd, s_u, s, second);
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      if (rg + 32 * j < rows)
+        out[((size_t)(lo + chunk * kDcTokens + rg + 32 * j) * heads + h) * dv + j0 + s] = first[2 + j] + second[j];
+#pragma unroll
+    for (int j = 2; j < RB; ++j) {
+      float* e = s_s + s * LD + rg + 32 * (j - 2);
+      *e = fmaf(decay, *e, second[j]);
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < D * kDcCols; i += kDcThreads) {
+    const int e = i / kDcCols, c = i % kDcCols;
+    st[(size_t)e * dv + c] = s_s[c * LD + e];
+  }
+}
+
+template <typename T, int D>
+int delta_chunks(float* out, float* work, int chunks, const void* qkv, const float* ba, const float* rate, const float* dt_bias, float* state,
+                 const int* q_start, const int* positions, const int* state_slot, int requests, int heads, int kv_heads, int dv,
+                 float unit_eps, float q_scale, void* stream) {
+  static SmemRaised raised_p, raised_w;
+  if (int rc = raise_shared_memory("delta_chunk_prepare", delta_chunk_prepare_kernel<T, D>, (int)dc_prepare_smem(D), raised_p)) return rc;
+  if (int rc = raise_shared_memory("delta_chunk_walk", delta_chunk_walk_kernel<D>, (int)dc_walk_smem(D), raised_w)) return rc;
+  if (int rc = launch_kernel("delta_chunk_prepare", delta_chunk_prepare_kernel<T, D>, dim3(chunks, heads), dim3(kDcThreads), dc_prepare_smem(D),
+                             as_stream(stream), work, (const T*)qkv, ba, rate, dt_bias, q_start, state_slot, requests, heads, kv_heads, dv,
+                             unit_eps, q_scale))
+    return rc;
+  return launch_kernel("delta_chunk_walk", delta_chunk_walk_kernel<D>, dim3(dv / kDcCols, heads, requests), dim3(kDcThreads), dc_walk_smem(D),
+                       as_stream(stream), out, state, work, q_start, positions, state_slot, heads, dv);
+}
+
+template <typename T>
+int delta_chunks_any(float* out, float* work, int chunks, const void* qkv, const float* ba, const float* rate, const float* dt_bias,
+                     float* state, const int* q_start, const int* positions, const int* state_slot, int requests, int heads, int kv_heads,
+                     int d, int dv, float unit_eps, float q_scale, void* stream) {
+  PTL_REQUIRE(requests >= 0 && requests <= 65535 && heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0 && chunks >= 0 &&
+                  (d == 64 || d == 128) && dv > 0 && dv % kDcCols == 0 && aligned16(work),
+              "gated_delta_rule in chunks: bad sizes heads=%d kv_heads=%d d=%d (64 or 128) dv=%d", heads, kv_heads, d, dv);
+  if (requests == 0 || chunks == 0) return 0;
+  const auto fn = d == 64 ? delta_chunks<T, 64> : delta_chunks<T, 128>;
+  return fn(out, work, chunks, qkv, ba, rate, dt_bias, state, q_start, positions, state_slot, requests, heads, kv_heads, dv, unit_eps,
+            q_scale, stream);
+}
+
+}  // namespace ptl
+
+PTL_EXPORT long long ptl_delta_chunk_floats(int d, int dv) { return (long long)ptl::dc_floats(d, dv); }
+
+#define PTL_DELTA_CHUNKS(SUFFIX, TYPE)                                                                                                \
+  PTL_EXPORT int ptl_gated_delta_chunks##SUFFIX(float* out, float* work, int chunks, const void* qkv, const float* ba, const float* rate, \
+                                                const float* dt_bias, float* state, const int* q_start, const int* positions,         \
+                                                const int* state_slot, int requests, int heads, int kv_heads, int d, int dv,          \
+                                                float unit_eps, float q_scale, void* stream) {                                        \
+    return ptl::delta_chunks_any<TYPE>(out, work, chunks, qkv, ba, rate, dt_bias, state, q_start, positions, state_slot, requests,    \
+                                       heads, kv_heads, d, dv, unit_eps, q_scale, stream);                                            \
+  }
+PTL_DELTA_CHUNKS(_f32, float)
+PTL_DELTA_CHUNKS(_bf16, __nv_bfloat16)

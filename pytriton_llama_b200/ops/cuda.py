@@ -42,6 +42,8 @@ _SIGNATURES = {
                           _ptr, _c_int, _ptr],
     "ptl_gated_delta_rule": [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f,
                              _c_f, _ptr],
+    "ptl_gated_delta_chunks": [_ptr, _ptr, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
+                               _c_f, _c_f, _ptr],
     "ptl_gated_head_norm": [_ptr, _c_int, _c_int, _ptr, _ptr, _c_f, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_int,
                             _ptr],
     "ptl_kv_write_normed": [_ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_f, _ptr],
@@ -202,6 +204,8 @@ def load_library() -> ctypes.CDLL:
     lib.ptl_chunk_attention_tc_bf16.restype = _c_int
     lib.ptl_token_side_cluster_bf16.argtypes = _SIGNATURES["ptl_token_side"]
     lib.ptl_token_side_cluster_bf16.restype = _c_int
+    lib.ptl_delta_chunk_floats.argtypes = [_c_int, _c_int]
+    lib.ptl_delta_chunk_floats.restype = _c_ll
     lib.ptl_moe_tile_rows.argtypes = []
     lib.ptl_moe_tile_rows.restype = _c_int
     lib.ptl_moe_route.argtypes = [_ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _c_f, _ptr, _ptr]
@@ -1149,6 +1153,10 @@ class CudaOps:
                        _p(state), _p(ctx.q_start), _p(ctx.positions), _p(ctx.state_slot), ctx.num_requests, self._stream()))
         return out
 
+    # The longest portion of a step for which the gated delta rule walks token by token: up to
+    # one chunk (2,048 tokens of heads of 128: 738 us by the walk, 206 in chunks; 64: 23 by the walk, one chunk costs as much).
+    DELTA_WALK_MAX_TOKENS = 64
+
     def gated_delta_rule(self, qkv: torch.Tensor, ba: torch.Tensor, rate: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor,
                          ctx, H: int, G: int, d: int, dv: int, unit_eps: float, q_scale: float) -> torch.Tensor:
         """The recurrence of ``parts/delta_rule.py``: qkv [T, q | k | v] after convolution, ba float32 [T, 2H]; returns the
@@ -1158,7 +1166,15 @@ class CudaOps:
             self._want(t, name, torch.float32)
         if qkv.shape[1] != 2 * G * d + H * dv or ba.shape[1] != 2 * H or tuple(state.shape[1:]) != (H, d, dv):
             raise KernelError("gated_delta_rule: shapes do not fit")
-        out = self.empty((qkv.shape[0], H * dv), torch.float32)
+        T = qkv.shape[0]
+        out = self.empty((T, H * dv), torch.float32)
+        if ctx.max_q_len > self.DELTA_WALK_MAX_TOKENS and d in (64, 128) and dv % 8 == 0:
+            chunks = T // 64 + ctx.num_requests          # at least the chunks of 64 tokens that the requests' portions make
+            work = self.empty((chunks * H, self.lib.ptl_delta_chunk_floats(d, dv)), torch.float32)
+            fn = getattr(self.lib, "ptl_gated_delta_chunks" + _suffix(qkv.dtype))
+            self._check(fn(_p(out), _p(work), chunks, _p(qkv), _p(ba), _p(rate), _p(dt_bias), _p(state), _p(ctx.q_start), _p(ctx.positions),
+                           _p(ctx.state_slot), ctx.num_requests, H, G, d, dv, float(unit_eps), float(q_scale), self._stream()), kernels=2)
+            return out
         fn = getattr(self.lib, "ptl_gated_delta_rule" + _suffix(qkv.dtype))
         self._check(fn(_p(out), _p(qkv), _p(ba), _p(rate), _p(dt_bias), _p(state), _p(ctx.q_start), _p(ctx.positions),
                        _p(ctx.state_slot), ctx.num_requests, H, G, d, dv, float(unit_eps), float(q_scale), self._stream()))

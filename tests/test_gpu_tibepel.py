@@ -126,6 +126,31 @@ def test_selective_scan_in_segments_of_64_tokens(ops, dtype, inner, n):
     _close(dev["state"], cpu["state"], "float32", "state after the step")
 
 
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("H,G,d,dv", [(2, 1, 64, 8), (3, 3, 128, 40), (4, 2, 128, 128)])
+def test_gated_delta_rule_in_chunks_of_64_tokens(ops, dtype, H, G, d, dv):
+    """Portions that end beside a chunk, fresh and running, beside single tokens; the error against 64 bits is held to the
+    walk's own bound (the test above) and to half as much again as the token-by-token walk has on the same inputs."""
+    g = torch.Generator().manual_seed(H * 1000 + d)
+    step = ([64, 1, 65, 200, 2, 63, 128], [0, 17, 3, 0, 9, 5, 0], [2, 0, 3, 1, 6, 4, 5])
+    T = sum(step[0])
+    tensors = {"qkv": torch.randn(T, 2 * G * d + H * dv, generator=g).to(DTYPES[dtype]), "ba": torch.randn(T, 2 * H, generator=g),
+               "rate": torch.exp(torch.randn(H, generator=g)), "dt_bias": torch.randn(H, generator=g),
+               "S": torch.randn(7, H, d, dv, generator=g)}
+    run = lambda o, t, ctx: o.gated_delta_rule(t["qkv"], t["ba"], t["rate"], t["dt_bias"], t["S"], ctx, H, G, d, dv, 1e-6, d ** -0.5)
+    assert max(step[0]) > ops.DELTA_WALK_MAX_TOKENS
+    got, ref, dev, cpu = _both(ops, run, tensors, step, dtype)
+    _close(got, ref, "float32", "read-outs", scale=max(1.0, float(ref.abs().max())) * 5)
+    _close(dev["S"], cpu["S"], "float32", "state after the step", scale=max(1.0, float(cpu["S"].abs().max())) * 5)
+    old, ops.DELTA_WALK_MAX_TOKENS = ops.DELTA_WALK_MAX_TOKENS, 10 ** 6
+    try:
+        walked, _, wdev, _ = _both(ops, run, tensors, step, dtype)
+    finally:
+        ops.DELTA_WALK_MAX_TOKENS = old
+    off = lambda a, b: float((a.double().cpu() - b.double()).norm())
+    assert off(got, ref) <= 1.5 * off(walked, ref) and off(dev["S"], cpu["S"]) <= 1.5 * off(wdev["S"], cpu["S"])
+
+
 @pytest.mark.parametrize("T,W,dim", [(1, 512, 16), (8, 1024, 64), (17, 1024, 128), (70, 2048, 48)])
 def test_side_term_in_a_cluster(ops, T, W, dim):
     """Sixteen tokens a cluster, remainders, with and without the pending output: against 64 bits to float32 sums, as the row
