@@ -84,7 +84,7 @@ static int gemm_tc_impl(void* out, const void* X, const void* W, int M, int N, i
                         int sumsq_ld, int* slots_out, const float* scale_sumsq, int scale_slots,
                         int scale_ld, float scale_eps, const ptl::GemmParams* rope, void* stream,
                         unsigned poll_limit = ptl::kPollLimit, int withhold_first_load = 0,
-                        const ptl::GemmParams* tail = nullptr) {
+                        const ptl::GemmParams* tail = nullptr, const ptl::GemmParams* glu = nullptr) {
   using namespace ptl;
   PTL_REQUIRE(M >= 0 && N > 0 && K > 0 && ld_out > 0, "gemm_tc: bad sizes M=%d N=%d K=%d", M, N, K);
   if (K % 8 != 0 || K < kTileK) return -2;
@@ -104,7 +104,10 @@ static int gemm_tc_impl(void* out, const void* X, const void* W, int M, int N, i
     if (epi != 2 || M > 64) return -2;
     p.tail_scale = tail->tail_scale; p.tail_w = tail->tail_w; p.tail_b = tail->tail_b; p.tail_alpha = tail->tail_alpha; p.tail_y = tail->tail_y;
   }
-  PTL_REQUIRE(epi != 3 || N % 2 == 0, "gemm_tc: the gate*up epilogue needs an even number of weight rows");
+  if (epi == 7) {
+    p.gate_a = glu->gate_a; p.glu_bias = glu->glu_bias; p.glu_limit = glu->glu_limit; p.glu_shift = glu->glu_shift;
+  }
+  PTL_REQUIRE(!is_gated(epi) || N % 2 == 0, "gemm_tc: the gate*up epilogue needs an even number of weight rows");
   if (M == 0) return 0;
   p.out = out; p.status = status;
   p.K = K; p.ld_out = ld_out;
@@ -250,4 +253,16 @@ PTL_EXPORT int ptl_gemm_tc_wait_selftest(void* out, const void* X, const void* W
   PTL_REQUIRE(poll_limit >= 1 && poll_limit <= (1u << 16), "gemm_tc_wait_selftest: between 1 and 65536 polls");
   return gemm_tc_impl(out, X, W, M, N, K, N, 0, status, M <= 64 ? 1 : 0, nullptr, nullptr, nullptr, 0, nullptr, nullptr, 0, 0, 0.f,
                       nullptr, stream, poll_limit, 1);
+}
+
+// The product of weight rows that alternate gate_j, up_j with clamped branches: out bf16 [M, N/2],
+//   g sigmoid(alpha g) (u + shift),  g = min(gate + bias, limit),  u = clamp(up + bias, -limit, limit);
+// bias float32 [N], alternating like the rows, or null.  -2: sizes for another product.
+PTL_EXPORT int ptl_gemm_tc_bf16_clamped_glu(void* out, const void* X, const void* W, int M, int N, int K, const float* bias, float limit,
+                                            float alpha, float shift, int* status, void* stream) {
+  PTL_REQUIRE(limit > 0.f && (reinterpret_cast<uintptr_t>(bias) & 7u) == 0, "gemm_tc: the clamped epilogue needs a positive bound and biases in pairs");
+  ptl::GemmParams glu{};
+  glu.gate_a = alpha; glu.glu_bias = bias; glu.glu_limit = limit; glu.glu_shift = shift;
+  return gemm_tc_impl(out, X, W, M, N, K, N / 2, 7, status, 0, nullptr, nullptr, nullptr, 0, nullptr, nullptr, 0, 0, 0.f, nullptr, stream,
+                      ptl::kPollLimit, 0, nullptr, &glu);
 }

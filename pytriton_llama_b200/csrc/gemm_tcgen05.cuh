@@ -87,7 +87,11 @@ struct GemmParams {
   float tail_alpha;
   __nv_bfloat16* tail_y;
   int relu2;                      // epilogue 0: the square of max(result, 0) is stored
-  float gate_a, gate_b;           // epilogue 3: the gate's activation (gate_act)
+  float gate_a, gate_b;           // epilogues 3 and 7: the gate's activation (gate_act)
+  // Epilogue 7: biases of the weight rows (alternating like them, or null), bounds of gate (above) and up (both sides), and
+  // what is added to up afterwards.
+  const float* glu_bias;
+  float glu_limit, glu_shift;
   unsigned long long* timeline;   // measurements: where the first and the last block stamp %globaltimer (null: nowhere)
   int timeline_kind;
 };
@@ -139,6 +143,24 @@ __device__ __forceinline__ float gate_act(const GemmParams& p, float g) {
   return __fdividef(g, 1.0f + __expf(-g * fmaf(p.gate_b, g * g, p.gate_a)));
 }
 
+// Epilogues whose weight rows alternate gate_j, up_j; 7 adds biases and bounds.  (An instance of its own: the few-token form of 3
+// has no registers to spare.)  2,048 tokens of width 1,024 to 2 x 4,096: 46 us with 7, 34 as a plain product with a pass of 36 behind it.
+__host__ __device__ constexpr bool is_gated(int epi) { return epi == 3 || epi == 7; }
+// The result of weight rows n (gate) and n + 1 (up).
+template <int EPI>
+__device__ __forceinline__ float gate_pair(const GemmParams& p, int n, float g, float u) {
+  if constexpr (EPI == 7) {
+    if (p.glu_bias) {
+      const float2 b = __ldg(reinterpret_cast<const float2*>(p.glu_bias + n));
+      g += b.x;
+      u += b.y;
+    }
+    g = fminf(g, p.glu_limit);
+    u = fminf(fmaxf(u, -p.glu_limit), p.glu_limit) + p.glu_shift;
+  }
+  return gate_act(p, g) * u;
+}
+
 __device__ __forceinline__ float plain_act(const GemmParams& p, float v) {
   if (!p.relu2) return v;
   v = fmaxf(v, 0.f);
@@ -156,21 +178,22 @@ template <int EPI>
 __device__ __forceinline__ void store_normal(const GemmParams& p, int row, int c0, const float (&v)[16], size_t out_row) {
   if (row >= p.rows) return;
   const int n_total = p.cols;
-  if (EPI == 3) {
+  if (is_gated(EPI)) {
     __nv_bfloat16* o = (__nv_bfloat16*)p.out + out_row * p.ld_out + c0 / 2;
     if (c0 + 16 <= n_total && (p.ld_out % 8 == 0)) {
       uint4 pk;
       uint32_t* w = reinterpret_cast<uint32_t*>(&pk);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        __nv_bfloat162 t = __floats2bfloat162_rn(gate_act(p, v[4 * j]) * v[4 * j + 1], gate_act(p, v[4 * j + 2]) * v[4 * j + 3]);
+        __nv_bfloat162 t = __floats2bfloat162_rn(gate_pair<EPI>(p, c0 + 4 * j, v[4 * j], v[4 * j + 1]),
+                                                   gate_pair<EPI>(p, c0 + 4 * j + 2, v[4 * j + 2], v[4 * j + 3]));
         w[j] = *reinterpret_cast<uint32_t*>(&t);
       }
       *reinterpret_cast<uint4*>(o) = pk;
     } else {
 #pragma unroll
       for (int j = 0; j < 8; ++j)
-        if (c0 + 2 * j + 1 < n_total) o[j] = __float2bfloat16_rn(gate_act(p, v[2 * j]) * v[2 * j + 1]);
+        if (c0 + 2 * j + 1 < n_total) o[j] = __float2bfloat16_rn(gate_pair<EPI>(p, c0 + 2 * j, v[2 * j], v[2 * j + 1]));
     }
     return;
   }
@@ -251,10 +274,10 @@ __device__ __forceinline__ void store_swapped(const GemmParams& p, int row, int 
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
     const int tok = c0 + j;
-    if (EPI == 3) {
+    if (is_gated(EPI)) {
       const float up = __shfl_down_sync(0xffffffffu, v[j], 1);   // odd rows hold up_j; all lanes take part
       if (n_ok && tok < p.cols && (n & 1) == 0)
-        ((__nv_bfloat16*)p.out)[(size_t)tok * p.ld_out + n / 2] = __float2bfloat16_rn(gate_act(p, v[j]) * up);
+        ((__nv_bfloat16*)p.out)[(size_t)tok * p.ld_out + n / 2] = __float2bfloat16_rn(gate_pair<EPI>(p, n, v[j], up));
     } else if (EPI == 2) {
       add_and_emit(p, n, tok, v[j], false, 0.f, threadIdx.x & 31);
     } else if (n_ok && tok < p.cols) {
@@ -271,7 +294,7 @@ __device__ __forceinline__ void store_swapped_one(const GemmParams& p, int n, in
   if (EPI == 0) ((__nv_bfloat16*)p.out)[(size_t)tok * p.ld_out + n] = __float2bfloat16_rn(plain_act(p, v));
   else if (EPI == 1) ((float*)p.out)[(size_t)tok * p.ld_out + n] = v;
   else if (EPI == 2) ((float*)p.out)[(size_t)tok * p.ld_out + n] += v;
-  else ((__nv_bfloat16*)p.out)[(size_t)tok * p.ld_out + n / 2] = __float2bfloat16_rn(gate_act(p, v) * up);
+  else ((__nv_bfloat16*)p.out)[(size_t)tok * p.ld_out + n / 2] = __float2bfloat16_rn(gate_pair<EPI>(p, n, v, up));
 }
 
 // 16 columns of this thread's TMEM lane, added over the issuers' accumulators; an issuer that had
@@ -823,15 +846,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_row, const __grid_constan
               sq += __shfl_xor_sync(0xffffffffu, sq, 2);
               if ((lane & 3) == 0 && live) p.sumsq[(size_t)col * p.sumsq_ld + n / 16] = sq;
             }
-          } else if (EPI == 3) {
+          } else if (is_gated(EPI)) {
             // rows alternate gate_j, up_j: two results
             if (col < p.cols) {
               __nv_bfloat16* o = (__nv_bfloat16*)p.out + (size_t)col * p.ld_out + n / 2;
               if (n + 3 < p.rows && p.ld_out % 2 == 0) {
-                *reinterpret_cast<uint32_t*>(o) = pack_bf16x2(gate_act(p, v[0]) * v[1], gate_act(p, v[2]) * v[3]);
+                *reinterpret_cast<uint32_t*>(o) = pack_bf16x2(gate_pair<EPI>(p, n, v[0], v[1]), gate_pair<EPI>(p, n + 2, v[2], v[3]));
               } else {
-                if (n + 1 < p.rows) o[0] = __float2bfloat16_rn(gate_act(p, v[0]) * v[1]);
-                if (n + 3 < p.rows) o[1] = __float2bfloat16_rn(gate_act(p, v[2]) * v[3]);
+                if (n + 1 < p.rows) o[0] = __float2bfloat16_rn(gate_pair<EPI>(p, n, v[0], v[1]));
+                if (n + 3 < p.rows) o[1] = __float2bfloat16_rn(gate_pair<EPI>(p, n + 2, v[2], v[3]));
               }
             }
           } else if (col < p.cols) {
@@ -859,13 +882,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_row, const __grid_constan
         }
       }
     } else {
-      const int group = EPI == 3 ? rows_per / 2 : rows_per;  // items per column: rows, or gate/up pairs
+      const int group = is_gated(EPI) ? rows_per / 2 : rows_per;  // items per column: rows, or gate/up pairs
       const int items = group * BN;
       const int t = threadIdx.x - 64;                        // 0..255 in the epilogue warps
       const bool worker = warp >= 2;
       auto item_pos = [&](int idx, int& r, int& col) {
         col = idx / group;
-        r = EPI == 3 ? 2 * (idx % group) : idx % group;
+        r = is_gated(EPI) ? 2 * (idx % group) : idx % group;
       };
       cluster_arrive();
       // what the add epilogue adds to and multiplies by, fetched under the barrier: this thread's first
@@ -912,7 +935,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_row, const __grid_constan
             for (int j = 0; j < kAheadItems; ++j) if (j == i) { have = res0[j]; nwv = nw0[j]; }
             add_and_emit(p, n, col, v, i < kAheadItems, have, lane, nwv);     // (every lane: the sums of squares are added over half warps)
           } else {
-            store_swapped_one<EPI>(p, n, col, v, EPI == 3 ? sum_sources(r + 1, col) * sc : 0.f);
+            store_swapped_one<EPI>(p, n, col, v, is_gated(EPI) ? sum_sources(r + 1, col) * sc : 0.f);
           }
         }
       }
@@ -970,6 +993,7 @@ static int launch_epi(int epi, const CUtensorMap& mr, const CUtensorMap& mc, con
     case 1: return launch_tc<BN, 1, PAIR>(mr, mc, mo, p, grid, s);
     case 2: return launch_tc<BN, 2, PAIR>(mr, mc, mo, p, grid, s);
     case 3: return launch_tc<BN, 3, PAIR>(mr, mc, mo, p, grid, s);
+    case 7: return launch_tc<BN, 7, PAIR>(mr, mc, mo, p, grid, s);
     case 4:
       if constexpr (BN >= 128) return launch_tc<BN, 4, PAIR>(mr, mc, mo, p, grid, s);
       else break;

@@ -202,6 +202,8 @@ def load_library() -> ctypes.CDLL:
     lib.ptl_chunk_attention_tc_bf16.argtypes = [_ptr, _c_int, _c_int, _ptr, _c_int, _ptr, _ptr, _ptr, _c_int, _ptr, _c_int, _c_int, _c_int,
                                                 _c_int, _c_int, _c_int, _c_f, _c_int, _ptr, _ptr, _ptr, _c_int, _c_f, _ptr]
     lib.ptl_chunk_attention_tc_bf16.restype = _c_int
+    lib.ptl_gemm_tc_bf16_clamped_glu.argtypes = [_ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _ptr, _c_f, _c_f, _c_f, _ptr, _ptr]
+    lib.ptl_gemm_tc_bf16_clamped_glu.restype = _c_int
     lib.ptl_token_side_cluster_bf16.argtypes = _SIGNATURES["ptl_token_side"]
     lib.ptl_token_side_cluster_bf16.restype = _c_int
     lib.ptl_delta_chunk_floats.argtypes = [_c_int, _c_int]
@@ -334,7 +336,7 @@ class CudaOps:
         "embed_scaled": "elementwise", "softcap": "elementwise", "clamped_glu": "elementwise", "token_side": "token_input",
         "causal_conv": "recurrent", "selective_scan": "recurrent", "gated_delta_rule": "recurrent", "gated_head_norm": "norm",
         "kv_write_normed": "attention", "chunk_attention": "attention", "chunk_attention_of_step": "attention",
-        "linear": "product", "linear_add": "product", "gate_up_act": "product", "gemm_tc": "product",
+        "linear": "product", "linear_add": "product", "gate_up_act": "product", "clamped_gate_up": "product", "gemm_tc": "product",
         "_qkv_rope_product": "product", "rope_kv_write": "rope", "_rope_table": "rope",
         "paged_attention": "attention", "_attention_tensor_cores": "attention",
         "sample": "sampling", "token_logprobs": "sampling", "sample_tokens": "sampling",
@@ -585,6 +587,25 @@ class CudaOps:
         if y is None:
             raise KernelError("gate_up_act: sizes not taken; load the weights in the plain layout instead")
         return y
+
+    def clamped_gate_up(self, x: torch.Tensor, w_alternating: torch.Tensor, bias: Optional[torch.Tensor], limit: float, alpha: float,
+                        up_shift: float) -> torch.Tensor:
+        """``clamped_glu`` in the epilogue of the product whose weight rows (and biases, float32) alternate gate_j, up_j: [T, inter]."""
+        self._want(x, "x", torch.bfloat16)
+        self._want(w_alternating, "w", torch.bfloat16)
+        if bias is not None:
+            self._want(bias, "bias", torch.float32)
+        M, K = x.shape
+        N = w_alternating.shape[0]
+        if w_alternating.shape[1] != K or (bias is not None and bias.numel() != N):
+            raise KernelError("clamped_gate_up: shapes do not fit")
+        out = self.empty((M, N // 2), torch.bfloat16)
+        rc = self.lib.ptl_gemm_tc_bf16_clamped_glu(_p(out), _p(x), _p(w_alternating), M, N, K, _p(bias), float(limit), float(alpha),
+                                                   float(up_shift), _p(self._tc_status_word()), self._stream())
+        if rc == -2:
+            raise KernelError("clamped_gate_up: sizes not taken; load the weights in the plain layout instead")
+        self._check(rc)
+        return out
 
     # epilogues of the tensor-core product
     EPI_BF16, EPI_F32, EPI_ADD_F32, EPI_SILU_MUL, EPI_GELU_MUL, EPI_RELU2 = 0, 1, 2, 3, 5, 6

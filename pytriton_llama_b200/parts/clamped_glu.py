@@ -30,12 +30,18 @@ class ClampedGLU(Part):
                 "up.b": TensorSpec((self.inter,), "zeros_jitter"), "down.b": TensorSpec((self.hidden,), "zeros_jitter")}
 
     def load(self, t) -> None:
-        self.w_gate_up = self._to_compute(torch.cat([t["gate"], t["up"]], dim=0))
-        self.b_gate_up = self._to_f32(torch.cat([t["gate.b"], t["up.b"]], dim=0))
+        # an operator set that applies the activation in the product's epilogue wants rows gate_0, up_0, gate_1, up_1, ...
+        ops = self.rt.ops
+        self.alternating = hasattr(ops, "clamped_gate_up") and ops.fused_ffn_layout(self.rt.dtype, self.hidden, self.inter)
+        join = (lambda a, b: torch.stack([a, b], dim=1).flatten(0, 1)) if self.alternating else (lambda a, b: torch.cat([a, b], dim=0))
+        self.w_gate_up = self._to_compute(join(t["gate"], t["up"]))
+        self.b_gate_up = self._to_f32(join(t["gate.b"], t["up.b"]))
         self.w_down = self._to_compute(t["down"])
         self.output_bias = self._to_f32(t["down.b"])
 
     def forward(self, x):
         ops = self.rt.ops
+        if self.alternating:
+            return ops.linear(ops.clamped_gate_up(x, self.w_gate_up, self.b_gate_up, self.limit, self.alpha, self.up_shift), self.w_down)
         y = ops.clamped_glu(ops.linear(x, self.w_gate_up), self.b_gate_up, self.limit, self.alpha, self.up_shift)
         return ops.linear(y, self.w_down)

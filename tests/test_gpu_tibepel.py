@@ -151,6 +151,21 @@ def test_gated_delta_rule_in_chunks_of_64_tokens(ops, dtype, H, G, d, dv):
     assert off(got, ref) <= 1.5 * off(walked, ref) and off(dev["S"], cpu["S"]) <= 1.5 * off(wdev["S"], cpu["S"])
 
 
+@pytest.mark.parametrize("M,inter,K,bias", [(1, 52, 64, True), (8, 300, 1024, True), (20, 2048, 512, False), (64, 96, 2048, True),
+                                            (65, 260, 64, True), (300, 1024, 512, True), (700, 130, 200, False)])
+def test_clamped_activation_in_the_product(ops, M, inter, K, bias):
+    """Every form of the product (few tokens, K split over a cluster, many tokens, edges of tiles) against 64 bits: one rounding
+    to bfloat16 (2^-8 of the result) over float32 sums of K products of order 1 / sqrt(K)."""
+    g = torch.Generator().manual_seed(M + inter)
+    x, w = torch.randn(M, K, generator=g).bfloat16(), (torch.randn(2 * inter, K, generator=g) * 3 / K ** 0.5).bfloat16()
+    b = torch.randn(2 * inter, generator=g) if bias else None
+    got = ops.clamped_gate_up(x.cuda(), w.cuda(), None if b is None else b.cuda(), 2.5, 1.702, 1.0).double().cpu()
+    y = x.double() @ w.double().T + (0 if b is None else b.double())
+    gate, up = y[:, 0::2].clamp(max=2.5), y[:, 1::2].clamp(-2.5, 2.5)
+    want = gate * torch.sigmoid(1.702 * gate) * (up + 1)
+    assert ((got - want).abs() <= 2 ** -8 * want.abs() + 1e-4).all()
+
+
 @pytest.mark.parametrize("T,W,dim", [(1, 512, 16), (8, 1024, 64), (17, 1024, 128), (70, 2048, 48)])
 def test_side_term_in_a_cluster(ops, T, W, dim):
     """Sixteen tokens a cluster, remainders, with and without the pending output: against 64 bits to float32 sums, as the row
