@@ -41,7 +41,14 @@ __device__ __forceinline__ void two_scale(float& hi, float& lo, float c) {
   hi = h;
 }
 
-template <typename T>
+// (Sums in one order; what is fetched ahead of them is not part of it: kPacketsAhead packets of a key, the
+// values of values_ahead keys.
+// Fetched one by one, every value waited for L2: 103 us a launch for four tokens of 32 heads at contexts of 33 to 143,
+// 39 us so.)
+constexpr int kPacketsAhead = 16;     // packets of a key per lane: the whole key up to 64 floats
+__host__ __device__ constexpr int values_ahead(int dpl) { return dpl <= 2 ? 16 : dpl <= 4 ? 8 : 4; }
+
+template <typename T, int DPL>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 paged_attention_simt_kernel(T* __restrict__ out, float* __restrict__ part_acc, float* __restrict__ part_ml,
                             const T* __restrict__ q, const T* __restrict__ cache,
@@ -77,9 +84,9 @@ paged_attention_simt_kernel(T* __restrict__ out, float* __restrict__ part_acc, f
   constexpr int VN = Vec16<T>::N;
 
   float m = -INFINITY, l = 0.f, l_lo = 0.f;
-  float acc[kMaxDimPerLane], acc_lo[kMaxDimPerLane];
+  float acc[DPL], acc_lo[DPL];
 #pragma unroll
-  for (int i = 0; i < kMaxDimPerLane; ++i) { acc[i] = 0.f; acc_lo[i] = 0.f; }
+  for (int i = 0; i < DPL; ++i) { acc[i] = 0.f; acc_lo[i] = 0.f; }
 
   for (int k0 = k_begin; k0 < k_end; k0 += 32) {
     const int key = k0 + lane;
@@ -92,12 +99,19 @@ paged_attention_simt_kernel(T* __restrict__ out, float* __restrict__ part_acc, f
       base = ((size_t)page * 2) * plane + ((size_t)kvh * page_size + key % page_size) * d;
       const T* kp = cache + base;
       float dot = 0.f, dot_lo = 0.f;
-      for (int i = 0; i < d; i += VN) {
-        Vec16<T> kv = load16(kp + i);
+      for (int i0 = 0; i0 < d; i0 += kPacketsAhead * VN) {
+        Vec16<T> kv[kPacketsAhead];
 #pragma unroll
-        for (int e = 0; e < VN; ++e) {
-          if constexpr (kCompensated) two_fma(dot, dot_lo, qs[i + e], kv.get(e));
-          else dot = fmaf(qs[i + e], kv.get(e), dot);
+        for (int j = 0; j < kPacketsAhead; ++j) kv[j] = load16(kp + min(i0 + j * VN, d - VN));
+#pragma unroll
+        for (int j = 0; j < kPacketsAhead; ++j) {
+          const int i = i0 + j * VN;
+          if (i >= d) break;
+#pragma unroll
+          for (int e = 0; e < VN; ++e) {
+            if constexpr (kCompensated) two_fma(dot, dot_lo, qs[i + e], kv[j].get(e));
+            else dot = fmaf(qs[i + e], kv[j].get(e), dot);
+          }
         }
       }
       s = kCompensated ? __fadd_rn(dot, dot_lo) * scale : dot;
@@ -109,27 +123,38 @@ paged_attention_simt_kernel(T* __restrict__ out, float* __restrict__ part_acc, f
       if (alpha != 1.f) {                 // (uniform over the warp) the maximum grew: everything so far shrinks
         two_scale(l, l_lo, alpha);
 #pragma unroll
-        for (int i = 0; i < kMaxDimPerLane; ++i) two_scale(acc[i], acc_lo[i], alpha);
+        for (int i = 0; i < DPL; ++i) two_scale(acc[i], acc_lo[i], alpha);
       }
       two_fma(l, l_lo, warp_sum(pr), 1.f);
     } else {
       l = l * alpha + warp_sum(pr);
 #pragma unroll
-      for (int i = 0; i < kMaxDimPerLane; ++i) acc[i] *= alpha;
+      for (int i = 0; i < DPL; ++i) acc[i] *= alpha;
     }
     m = m_new;
     const int nvalid = min(32, k_end - k0);
-    for (int j = 0; j < nvalid; ++j) {
-      const float pj = __shfl_sync(0xffffffffu, pr, j);
-      const unsigned long long bj = __shfl_sync(0xffffffffu, (unsigned long long)base, j);
-      if (pj == 0.f) continue;   // uniform over the warp: a skipped key has no valid address
-      const T* vp = cache + (size_t)bj + plane;
+    constexpr int kValuesAhead = values_ahead(DPL);
+    for (int j0 = 0; j0 < nvalid; j0 += kValuesAhead) {
+      float pj[kValuesAhead];
+      T v[kValuesAhead][DPL];
 #pragma unroll
-      for (int i = 0; i < kMaxDimPerLane; ++i) {
-        const int dd = lane + 32 * i;
-        if (dd < d) {
-          if constexpr (kCompensated) two_fma(acc[i], acc_lo[i], pj, to_f32(vp[dd]));
-          else acc[i] = fmaf(pj, to_f32(vp[dd]), acc[i]);
+      for (int u = 0; u < kValuesAhead; ++u) {
+        pj[u] = __shfl_sync(0xffffffffu, pr, j0 + u);         // 0 behind the last key, and for a key without a page
+        const unsigned long long bj = __shfl_sync(0xffffffffu, (unsigned long long)base, j0 + u);
+        const T* vp = cache + (size_t)bj + plane;
+#pragma unroll
+        for (int i = 0; i < DPL; ++i)
+          if (pj[u] != 0.f && lane + 32 * i < d) v[u][i] = vp[lane + 32 * i];
+      }
+#pragma unroll
+      for (int u = 0; u < kValuesAhead; ++u) {
+        if (pj[u] == 0.f) continue;                           // (uniform over the warp)
+#pragma unroll
+        for (int i = 0; i < DPL; ++i) {
+          if (lane + 32 * i < d) {
+            if constexpr (kCompensated) two_fma(acc[i], acc_lo[i], pj[u], to_f32(v[u][i]));
+            else acc[i] = fmaf(pj[u], to_f32(v[u][i]), acc[i]);
+          }
         }
       }
     }
@@ -137,14 +162,14 @@ paged_attention_simt_kernel(T* __restrict__ out, float* __restrict__ part_acc, f
   if constexpr (kCompensated) {
     l = __fadd_rn(l, l_lo);
 #pragma unroll
-    for (int i = 0; i < kMaxDimPerLane; ++i) acc[i] = __fadd_rn(acc[i], acc_lo[i]);
+    for (int i = 0; i < DPL; ++i) acc[i] = __fadd_rn(acc[i], acc_lo[i]);
   }
 
   if (splits == 1) {
     const float inv = l > 0.f ? 1.0f / l : 0.f;
     T* o = out + (size_t)t * out_stride + (size_t)h * d;
 #pragma unroll
-    for (int i = 0; i < kMaxDimPerLane; ++i) {
+    for (int i = 0; i < DPL; ++i) {
       const int dd = lane + 32 * i;
       if (dd < d) o[dd] = from_f32<T>(acc[i] * inv);
     }
@@ -152,7 +177,7 @@ paged_attention_simt_kernel(T* __restrict__ out, float* __restrict__ part_acc, f
     const size_t idx = ((size_t)t * nq + h) * splits + split;
     float* pa = part_acc + idx * d;
 #pragma unroll
-    for (int i = 0; i < kMaxDimPerLane; ++i) {
+    for (int i = 0; i < DPL; ++i) {
       const int dd = lane + 32 * i;
       if (dd < d) pa[dd] = acc[i];
     }
@@ -233,7 +258,9 @@ int paged_attention_simt(void* out, const void* q, const void* cache, const int*
   if (tokens == 0) return 0;
   dim3 grid(tokens, (nq + kWarpsPerBlock - 1) / kWarpsPerBlock, splits);
   const size_t smem = (size_t)kWarpsPerBlock * d * sizeof(float);
-  int rc = launch_kernel("paged_attention", paged_attention_simt_kernel<T>, grid, dim3(kWarpsPerBlock * 32), smem,
+  const auto kernel = d <= 64 ? paged_attention_simt_kernel<T, 2> : d <= 128 ? paged_attention_simt_kernel<T, 4> :
+                                                                             paged_attention_simt_kernel<T, kMaxDimPerLane>;
+  int rc = launch_kernel("paged_attention", kernel, grid, dim3(kWarpsPerBlock * 32), smem,
                          as_stream(stream), (T*)out, part_acc, part_ml, (const T*)q, (const T*)cache, block_table, tok_req,
                          positions, q_stride, out_stride, bt_stride, nq, nkv, d, page_size, scale, window, splits, num_pages);
   if (rc) return rc;
