@@ -49,12 +49,81 @@ add_layernorm_kernel(TY* __restrict__ y, float* __restrict__ residual_out, const
     yo[i] = from_f32<TY>(fmaf((ln_row[i] - mean) * rstd, w[i], b[i]));
 }
 
+// The same with the row in registers, PER entries a thread, and the same sums in the same order, so that a row has the same bits from
+// both; few weights are fetched before the wait on the predecessor.  2,020 rows of 1,024: 10.8 us with the row in shared memory
+// and loops of unknown length, 7.7 so (25 MB, 3.2 TB/s); 8 rows 4.65 and 3.0, the latency of two sums over a block.
+template <typename TX, typename TY, int PER>
+__global__ void __launch_bounds__(256)
+add_layernorm_registers_kernel(TY* __restrict__ y, float* __restrict__ residual_out, const float* __restrict__ residual_in,
+                               const TX* __restrict__ x, const float* __restrict__ add_bias, const float* __restrict__ w,
+                               const float* __restrict__ b, const int* __restrict__ rows, int hidden, float eps) {
+  __shared__ float red[33];
+  constexpr bool EARLY = PER <= 8;
+  const int first = threadIdx.x, m = blockIdx.x;
+  float wv[EARLY ? PER : 1], bv[EARLY ? PER : 1];
+  if constexpr (EARLY) {
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+      const int i = min(k * 256 + first, hidden - 1);
+      wv[k] = w[i];
+      bv[k] = b[i];
+    }
+  }
+  pdl_wait();
+  pdl_launch_dependents();
+  const int r = rows ? rows[m] : m;
+  const float* rin = residual_in ? residual_in + (size_t)r * hidden : nullptr;
+  const TX* xin = x ? x + (size_t)r * hidden : nullptr;
+  float* rout = residual_out ? residual_out + (size_t)m * hidden : nullptr;
+  const bool write_back = rout && (xin || add_bias || rout != rin);      // unchanged rows are not rewritten
+  float s[PER], sum = 0.f, sq = 0.f;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int i = k * 256 + first;
+    s[k] = rin && i < hidden ? __ldcg(rin + i) : 0.f;
+    if (xin && i < hidden) s[k] += to_f32(xin[i]);
+    if (add_bias && i < hidden) s[k] += add_bias[i];
+  }
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int i = k * 256 + first;
+    if (i >= hidden) continue;
+    if (write_back) rout[i] = s[k];
+    sum += s[k];
+  }
+  const float mean = block_sum(sum, red) / (float)hidden;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    s[k] -= mean;
+    if (k * 256 + first < hidden) sq = fmaf(s[k], s[k], sq);
+  }
+  const float rstd = 1.0f / sqrtf(block_sum(sq, red) / (float)hidden + eps);
+  TY* yo = y + (size_t)m * hidden;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int i = k * 256 + first;
+    if (i >= hidden) continue;
+    float g, c;
+    if constexpr (EARLY) { g = wv[k]; c = bv[k]; }
+    else { g = __ldg(w + i); c = __ldg(b + i); }
+    yo[i] = from_f32<TY>(fmaf(s[k] * rstd, g, c));
+  }
+}
+
 template <typename TX, typename TY>
 int add_layernorm(void* y, float* residual_out, const float* residual_in, const void* x, const float* add_bias, const float* w,
                   const float* b, const int* rows, int out_rows, int hidden, float eps, void* stream) {
   PTL_REQUIRE(out_rows >= 0 && hidden > 0 && eps > 0.f && w && b && (x || residual_in), "add_layernorm: bad arguments");
   PTL_REQUIRE((size_t)hidden * sizeof(float) <= 200 * 1024, "add_layernorm: rows of %d do not fit shared memory", hidden);
   if (out_rows == 0) return 0;
+#define PTL_LN(PER)                                                                                                              \
+  if (hidden <= 256 * PER)                                                                                                        \
+    return launch_kernel("add_layernorm", add_layernorm_registers_kernel<TX, TY, PER>, dim3(out_rows), dim3(256), 0,             \
+                         as_stream(stream), (TY*)y, residual_out, residual_in, (const TX*)x, add_bias, w, b, rows, hidden, eps)
+  PTL_LN(4);
+  PTL_LN(8);
+  PTL_LN(16);
+#undef PTL_LN
   const size_t smem = (size_t)hidden * sizeof(float);
   static SmemRaised raised;
   if (smem > 48 * 1024)

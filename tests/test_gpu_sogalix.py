@@ -65,6 +65,19 @@ def _paged(gen, q_lens, starts, page, pages, width):
 
 # ---------------------------------------------------------------------------- layer norm and activation
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("T,width", [(300, 1024), (2, 1025), (301, 1000), (5, 1), (3, 2048), (3, 2049), (299, 4096), (2, 4097)])
+def test_layer_norm_with_the_row_in_registers(ops, dtype, T, width):
+    g = torch.Generator().manual_seed(width + T)
+    dt, ref = DTYPES[dtype], TorchOps()
+    x, res, extra = _rand(g, T, width).to(dt), _rand(g, T, width, scale=3.0) + 50.0, _rand(g, width)
+    w, b = 1 + 0.2 * _rand(g, width), 0.3 * _rand(g, width)
+    ya, ra = ops.add_layernorm(x.cuda(), res.clone().cuda(), w.cuda(), b.cuda(), 1e-5, add_bias=extra.cuda())
+    yb, rb = ref.add_layernorm(x, res.clone(), w, b, 1e-5, add_bias=extra)
+    _close(ya, yb, dtype, "normed sum")
+    _close(ra, rb, "float32", "sum")
+
+
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("width", [32, 48, 257, 1024, 5000])
 def test_layer_norm_with_the_residual_add(ops, dtype, width):
     g = torch.Generator().manual_seed(width)
