@@ -29,7 +29,7 @@ __device__ __forceinline__ void kahan_add(float& sum, float& comp, float chunk) 
 template <typename TI, typename TO, int BM, int BN, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_simt_kernel(TO* __restrict__ out, const TI* __restrict__ A, const TI* __restrict__ W,
-                 int M, int N, int K, int lda, int ldw, int ldo, int accumulate, int vec_ok,
+                 int M, int N, int K, int lda, int ldw, int ldo, int accumulate,
                  long long batch_a, long long batch_w, long long batch_o, const TI* __restrict__ gate, int gate_ld) {
   constexpr int BK = kSimtChunk;
   constexpr int THREADS = (BM / TM) * (BN / TN);
@@ -52,36 +52,16 @@ gemm_simt_kernel(TO* __restrict__ out, const TI* __restrict__ A, const TI* __res
     for (int j = 0; j < TN; ++j) { sum[i][j] = 0.f; comp[i][j] = 0.f; }
 
   for (int k0 = 0; k0 < K; k0 += BK) {
-    if (vec_ok) {
-      // float32 operands whose rows start on 16-byte boundaries: four k values per load
-      if constexpr (sizeof(TI) == 4) {
-        for (int e = tid; e < BM * (BK / 4); e += THREADS) {
-          const int r = e / (BK / 4), c4 = e % (BK / 4);
-          const int gm = m0 + r, gk = k0 + c4 * 4;
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (gm < M && gk < K) v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(A) + (size_t)gm * lda + gk);
-          As[c4 * 4 + 0][r] = v.x; As[c4 * 4 + 1][r] = v.y; As[c4 * 4 + 2][r] = v.z; As[c4 * 4 + 3][r] = v.w;
-        }
-        for (int e = tid; e < BN * (BK / 4); e += THREADS) {
-          const int r = e / (BK / 4), c4 = e % (BK / 4);
-          const int gn = n0 + r, gk = k0 + c4 * 4;
-          float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (gn < N && gk < K) v = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(W) + (size_t)gn * ldw + gk);
-          Ws[c4 * 4 + 0][r] = v.x; Ws[c4 * 4 + 1][r] = v.y; Ws[c4 * 4 + 2][r] = v.z; Ws[c4 * 4 + 3][r] = v.w;
-        }
-      }
-    } else {
-      // any element type and alignment: consecutive threads walk along K so that global reads coalesce
-      for (int e = tid; e < BM * BK; e += THREADS) {
-        const int r = e / BK, c = e % BK;
-        const int gm = m0 + r, gk = k0 + c;
-        As[c][r] = (gm < M && gk < K) ? to_f32(A[(size_t)gm * lda + gk]) : 0.f;
-      }
-      for (int e = tid; e < BN * BK; e += THREADS) {
-        const int r = e / BK, c = e % BK;
-        const int gn = n0 + r, gk = k0 + c;
-        Ws[c][r] = (gn < N && gk < K) ? to_f32(W[(size_t)gn * ldw + gk]) : 0.f;
-      }
+    // any element type and alignment: consecutive threads walk along K so that global reads coalesce
+    for (int e = tid; e < BM * BK; e += THREADS) {
+      const int r = e / BK, c = e % BK;
+      const int gm = m0 + r, gk = k0 + c;
+      As[c][r] = (gm < M && gk < K) ? to_f32(A[(size_t)gm * lda + gk]) : 0.f;
+    }
+    for (int e = tid; e < BN * BK; e += THREADS) {
+      const int r = e / BK, c = e % BK;
+      const int gn = n0 + r, gk = k0 + c;
+      Ws[c][r] = (gn < N && gk < K) ? to_f32(W[(size_t)gn * ldw + gk]) : 0.f;
     }
     __syncthreads();
 #pragma unroll
@@ -123,6 +103,261 @@ gemm_simt_kernel(TO* __restrict__ out, const TI* __restrict__ A, const TI* __res
   }
 }
 
+// ---------------------------------------------------------------- float32, rows in packets of 16 bytes
+__device__ __forceinline__ void copy16_async(float* dst, const float* src, bool valid) {
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  const int bytes = valid ? 16 : 0;           // 0: the sixteen bytes become zeros, nothing is read
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+__device__ __forceinline__ void store_result(float* __restrict__ out, size_t at, float v, int accumulate) {
+  out[at] = accumulate ? v + out[at] : v;
+}
+
+// Up to 32 rows (a decode step): bound by the weights' bytes.  A block owns 8 or 16 weight rows; its warps take the K range in
+// turns of 256 values (8 chunks).  A lane owns one chunk of 32 values for a quarter of the weight rows and all MT token rows, so
+// a chunk's sum is the same chain of FMAs as anywhere else; the chunk sums of a round of turns meet in shared memory, where a
+// warp of its own adds them in order while the others are at the next round.  Weights and tokens come by cp.async into rows of 36 floats per chunk (a
+// quarter warp reads 8 chunks' packets from 32 different banks); the first turn's weights are asked for before the wait
+// on the predecessor, and a warp asks for its next turn as soon as it has multiplied the last.  What a warp cannot do is
+// multiply one turn while it waits for the next, so the blocks are small and many warps share an SM: 8 rows and four warps (three blocks an
+// SM) against 16 rows and two warps 35 us and 47 (4 rows of 2,048 to 16,384 features), 16 rows and four warps from 9 rows on, where
+// the tokens' share of the copies counts (16 rows: 87 us against 101).  The tile kernel with 32 x 16 tiles that stood here
+// before read a K range of 32 between two barriers: 4 rows against the 16 layers and the head of the 1B shape 16.2 ms a step, here 1.6.
+// From 17 rows on wide weights go to the tiles below (32 rows to 16,384 features: 229 us here, 152 there), narrow ones stay
+// (to 2,048 features 49 us here, 62 there).
+constexpr int kFewTurn = 8 * kSimtChunk, kFewLd = 8 * 36;
+// floats of a chunk's sums: 8 behind every quarter of the rows, 1 behind a chunk, for the banks
+__host__ __device__ constexpr int few_sums_ld(int mt, int rows) { return rows * mt + 33; }
+constexpr size_t few_smem_bytes(int mt, int rows, int warps) {
+  return sizeof(float) * ((size_t)warps * (rows + mt) * kFewLd + (size_t)2 * warps * 8 * few_sums_ld(mt, rows));
+}
+
+template <int MT, int ROWS, int WARPS>
+__global__ void __launch_bounds__((WARPS + 1) * 32)
+gemm_simt_few_kernel(float* __restrict__ out, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K, int lda,
+                     int ldw, int ldo, int accumulate, long long batch_a, long long batch_w, long long batch_o,
+                     const float* __restrict__ gate, int gate_ld) {
+  extern __shared__ __align__(16) float few_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float* ws = few_smem + (size_t)warp * (ROWS + MT) * kFewLd;       // [ROWS][8 chunks][36]
+  float* xs = ws + ROWS * kFewLd;                                    // [MT][8 chunks][36]
+  float* sums = few_smem + (size_t)WARPS * (ROWS + MT) * kFewLd;    // [2][warp][8 chunks][4 groups][RL rows][MT]
+  A += (size_t)blockIdx.z * batch_a;
+  W += (size_t)blockIdx.z * batch_w;
+  out += (size_t)blockIdx.z * batch_o;
+  const int n0 = blockIdx.x * ROWS;
+  const int turns = (K + kFewTurn - 1) / kFewTurn;
+
+  // a row of a turn is 64 packets
+  auto copy_rows = [&](float* dst, const float* src, int ld, int rows, int valid_rows, int k0) {
+#pragma unroll 4
+    for (int e = lane; e < rows * 64; e += 32) {
+      const int r = e >> 6, p = e & 63, k = k0 + 4 * p;
+      const bool ok = r < valid_rows && k < K;
+      copy16_async(dst + r * kFewLd + (p >> 3) * 36 + (p & 7) * 4, ok ? src + (size_t)r * ld + k : src, ok);
+    }
+  };
+  const float* w_rows = W + (size_t)n0 * ldw;
+  const int valid_n = min(ROWS, N - n0);
+  const bool works = warp < WARPS;                                       // the last warp adds up
+  if (works && warp < turns) copy_rows(ws, w_rows, ldw, ROWS, valid_n, warp * kFewTurn);
+  pdl_wait();
+  pdl_launch_dependents();
+  if (works && warp < turns) copy_rows(xs, A, lda, MT, M, warp * kFewTurn);
+  copy_commit();
+
+  const int chunk = lane & 7, group = lane >> 3;
+  constexpr int RL = ROWS / 4;                                           // weight rows of a lane
+  constexpr int SUMS_LD = few_sums_ld(MT, ROWS);
+  constexpr int RESULTS = ROWS * MT, PER = (RESULTS + 31) / 32;          // of the last warp's lanes
+  float sum[PER], comp[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) { sum[i] = 0.f; comp[i] = 0.f; }
+
+  const int rounds = (turns + WARPS - 1) / WARPS;
+  for (int round = 0; round <= rounds; ++round) {
+    float* round_sums = sums + (size_t)(round & 1) * WARPS * 8 * SUMS_LD;
+    const int turn = round * WARPS + warp;
+    if (works && turn < turns) {
+      copy_wait<0>();
+      __syncwarp();
+      float acc[RL][MT];
+#pragma unroll
+      for (int r = 0; r < RL; ++r)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) acc[r][m] = 0.f;
+      const float* wp = ws + group * RL * kFewLd + chunk * 36;
+      const float* xp = xs + chunk * 36;
+#pragma unroll 2
+      for (int k = 0; k < kSimtChunk; k += 4) {
+        float4 w[RL];
+#pragma unroll
+        for (int r = 0; r < RL; ++r) w[r] = *reinterpret_cast<const float4*>(wp + r * kFewLd + k);
+#pragma unroll
+        for (int m = 0; m < MT; ++m) {
+          const float4 x = *reinterpret_cast<const float4*>(xp + m * kFewLd + k);
+#pragma unroll
+          for (int r = 0; r < RL; ++r) {
+            float a = acc[r][m];
+            a = fmaf(x.x, w[r].x, a);
+            a = fmaf(x.y, w[r].y, a);
+            a = fmaf(x.z, w[r].z, a);
+            a = fmaf(x.w, w[r].w, a);
+            acc[r][m] = a;
+          }
+        }
+      }
+      __syncwarp();
+      if (turn + WARPS < turns) {
+        copy_rows(ws, w_rows, ldw, ROWS, valid_n, (turn + WARPS) * kFewTurn);
+        copy_rows(xs, A, lda, MT, M, (turn + WARPS) * kFewTurn);
+        copy_commit();
+      }
+      float* dst = round_sums + (warp * 8 + chunk) * SUMS_LD + group * (RL * MT + 8);
+#pragma unroll
+      for (int r = 0; r < RL; ++r)
+#pragma unroll
+        for (int m = 0; m < MT; ++m) dst[r * MT + m] = acc[r][m];
+    }
+    if (!works && round > 0) {                                           // the round before, while this one is multiplied
+      const float* done = sums + (size_t)((round - 1) & 1) * WARPS * 8 * SUMS_LD;
+      const int chunks = min(WARPS * 8, (K - (round - 1) * WARPS * kFewTurn + kSimtChunk - 1) / kSimtChunk);
+#pragma unroll 4
+      for (int c = 0; c < chunks; ++c)
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+          const int at = min(lane + 32 * i, RESULTS - 1);
+          kahan_add(sum[i], comp[i], done[c * SUMS_LD + at + at / (RL * MT) * 8]);
+        }
+    }
+    __syncthreads();
+  }
+  if (works) return;
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int at = lane + 32 * i;
+    const int n = n0 + at / MT, m = at % MT;
+    if (at >= RESULTS || n >= N || m >= M) continue;
+    const float row_gate = gate ? 1.0f / (1.0f + expf(-gate[(size_t)m * gate_ld + blockIdx.z])) : 1.0f;
+    store_result(out, (size_t)m * ldo + n, sum[i] * row_gate, accumulate);
+  }
+}
+
+// More rows (prompts): bound by the FMAs.  128 threads, TM x TN results each (rows 8 apart, columns 16 apart) with sum, compensation
+// and chunk accumulator in registers; a chunk of 32 k values per stage, rows kept along K as they come (cp.async, a ring of
+// three stages) with 36 floats a row: a thread reads four k values of a row in one packet, and the eight rows of a quarter
+// warp's packets start in different banks.  8 x 8 results read a packet per 16 FMAs; smaller ones are for weights of few rows,
+// whose 64 x 128 tiles leave SMs without work (simt_tile below).  320 rows to 16,384 features of 2,048: 596 us, 36 TFLOP/s, three
+// quarters of what shared memory's bandwidth allows at a packet per 16 FMAs; the 32 x 16 tiles that were here: 12.5 TFLOP/s.
+constexpr int kTileLd = kSimtChunk + 4, kTileStages = 3, kTileThreads = 128;
+
+template <int TM, int TN>
+__global__ void __launch_bounds__(kTileThreads, TM * TN >= 64 ? 2 : TM * TN >= 32 ? 3 : 4)
+gemm_simt_tile_kernel(float* __restrict__ out, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K, int lda,
+                      int ldw, int ldo, int accumulate, long long batch_a, long long batch_w, long long batch_o,
+                      const float* __restrict__ gate, int gate_ld) {
+  constexpr int BM = 8 * TM, BN = 16 * TN, ROWS = BM + BN;
+  extern __shared__ __align__(16) float tile_smem[];                     // [stage][x BM rows | w BN rows][36]
+  A += (size_t)blockIdx.z * batch_a;
+  W += (size_t)blockIdx.z * batch_w;
+  out += (size_t)blockIdx.z * batch_o;
+  const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;                  // the tiles of one set of weight rows run side by side
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int chunks = (K + kSimtChunk - 1) / kSimtChunk;
+  pdl_wait();
+  pdl_launch_dependents();
+  auto fetch = [&](int c) {
+    float* stage = tile_smem + (size_t)(c % kTileStages) * ROWS * kTileLd;
+    const int p = tid & 7, k = c * kSimtChunk + 4 * p;
+#pragma unroll
+    for (int i = 0; i < (ROWS + 15) / 16; ++i) {
+      const int r = (tid >> 3) + 16 * i;
+      if (ROWS % 16 && r >= ROWS) break;
+      const bool is_x = r < BM;
+      const int row = is_x ? m0 + r : n0 + r - BM;
+      const bool ok = k < K && row < (is_x ? M : N);
+      const float* src = is_x ? A + (size_t)row * lda + k : W + (size_t)row * ldw + k;
+      copy16_async(stage + r * kTileLd + 4 * p, ok ? src : A, ok);
+    }
+  };
+  float sum[TM][TN], comp[TM][TN];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < TN; ++j) { sum[i][j] = 0.f; comp[i][j] = 0.f; }
+#pragma unroll
+  for (int c = 0; c < kTileStages - 1; ++c) {
+    if (c < chunks) fetch(c);
+    copy_commit();
+  }
+  for (int c = 0; c < chunks; ++c) {
+    copy_wait<kTileStages - 2>();
+    __syncthreads();
+    if (c + kTileStages - 1 < chunks) fetch(c + kTileStages - 1);
+    copy_commit();
+    const float* xs = tile_smem + (size_t)(c % kTileStages) * ROWS * kTileLd + ty * kTileLd;
+    const float* ws = tile_smem + ((size_t)(c % kTileStages) * ROWS + BM + tx) * kTileLd;
+    float acc[TM][TN];
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+#pragma unroll 2
+    for (int k = 0; k < kSimtChunk; k += 4) {
+      float4 w[TN];
+#pragma unroll
+      for (int j = 0; j < TN; ++j) w[j] = *reinterpret_cast<const float4*>(ws + 16 * j * kTileLd + k);
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(xs + 8 * i * kTileLd + k);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(x.x, w[j].x, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(x.y, w[j].y, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(x.z, w[j].z, acc[i][j]);
+#pragma unroll
+        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(x.w, w[j].w, acc[i][j]);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j) kahan_add(sum[i][j], comp[i][j], acc[i][j]);
+  }
+#pragma unroll
+  for (int i = 0; i < TM; ++i) {
+    const int m = m0 + ty + 8 * i;
+    if (m >= M) continue;
+    const float row_gate = gate ? 1.0f / (1.0f + expf(-gate[(size_t)m * gate_ld + blockIdx.z])) : 1.0f;
+#pragma unroll
+    for (int j = 0; j < TN; ++j) {
+      const int n = n0 + tx + 16 * j;
+      if (n < N) store_result(out, (size_t)m * ldo + n, sum[i][j] * row_gate, accumulate);
+    }
+  }
+}
+
+// Results per thread (10 TM + TN) of a product.  An SM holds `held` blocks of a shape, which take about as long together as
+// fewer do (`us`, for 2,048 k values on a B200), so the busiest SM's blocks count in whole sets; measured for 64, 320 and
+// 1,024 rows against weights of 2,048 to 16,384 rows: 320 rows 152 / 108 / 595 / 425 us (q|k|v, output, gate and up, down
+// projection of the 1B shape) with the shapes this picks, 163 / 161 / 726 / 635 with 8 x 8 everywhere.
+inline int simt_tile(int M, int N, int batch) {
+  constexpr struct { int tm, tn, held; float us; } shapes[] = {{8, 8, 2, 246.f}, {8, 4, 3, 201.f}, {5, 4, 2, 105.f}, {4, 4, 4, 152.f}};
+  int best = 88;
+  float least = 0.f;
+  for (const auto& s : shapes) {
+    const long long blocks = (long long)batch * ((M + 8 * s.tm - 1) / (8 * s.tm)) * ((N + 16 * s.tn - 1) / (16 * s.tn));
+    const long long busiest = (blocks + 147) / 148;
+    const float cost = s.tn == 8 && busiest == 1 ? 163.f : (float)((busiest + s.held - 1) / s.held) * s.us;
+    if (least == 0.f || cost < least) { least = cost; best = 10 * s.tm + s.tn; }
+  }
+  return best;
+}
+
 template <typename TI, typename TO>
 int gemm_simt(void* out, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldo,
               int accumulate, void* stream, int batch = 1, long long batch_a = 0, long long batch_w = 0, long long batch_o = 0,
@@ -134,19 +369,60 @@ int gemm_simt(void* out, const void* A, const void* W, int M, int N, int K, int 
   const TI* gate = (const TI*)gate_v;
   const int vec_ok = sizeof(TI) == 4 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && aligned16(A) && aligned16(W) &&
                      batch_a % 4 == 0 && batch_w % 4 == 0;
+  if constexpr (sizeof(TI) == 4 && sizeof(TO) == 4) {
+    if (vec_ok && N >= 16) {
+      const auto few = [&](auto kernel, int mt, int rows, int warps, SmemRaised& raised) {
+        const size_t smem = few_smem_bytes(mt, rows, warps);
+        if (int rc = raise_shared_memory("gemm_simt_few", kernel, (int)smem, raised)) return rc;
+        return launch_kernel("gemm_simt_few", kernel, dim3((N + rows - 1) / rows, 1, batch), dim3(warps * 32 + 32), smem,
+                             as_stream(stream), (float*)out, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldo, accumulate,
+                             batch_a, batch_w, batch_o, (const float*)gate_v, gate_ld);
+      };
+#define PTL_FEW(MT, ROWS, WARPS)                                                              \
+      {                                                                                       \
+        static SmemRaised raised;                                                             \
+        return few(gemm_simt_few_kernel<MT, ROWS, WARPS>, MT, ROWS, WARPS, raised);           \
+      }
+      const bool narrow = (long long)N * batch < 4736;       // fewer than four blocks of eight rows per SM
+      if (M <= 1) PTL_FEW(1, 8, 4)
+      if (M <= 2) PTL_FEW(2, 8, 4)
+      if (M <= 4) PTL_FEW(4, 8, 4)
+      if (M <= 8 && narrow) PTL_FEW(8, 8, 4)
+      if (M <= 8) PTL_FEW(8, 8, 3)
+      if (M <= 16) PTL_FEW(16, 16, 4)
+      if (M <= 32 && narrow) PTL_FEW(32, 8, 2)
+#undef PTL_FEW
+      const auto tiled = [&](auto kernel, int tm, int tn, SmemRaised& raised) {
+        const int smem = kTileStages * (8 * tm + 16 * tn) * kTileLd * (int)sizeof(float);
+        if (int rc = raise_shared_memory("gemm_simt_tile", kernel, smem, raised)) return rc;
+        const dim3 grid((M + 8 * tm - 1) / (8 * tm), (N + 16 * tn - 1) / (16 * tn), batch);
+        PTL_REQUIRE(grid.y <= 65535, "gemm_simt: N=%d too large", N);
+        return launch_kernel("gemm_simt_tile", kernel, grid, dim3(kTileThreads), smem, as_stream(stream), (float*)out, (const float*)A,
+                             (const float*)W, M, N, K, lda, ldw, ldo, accumulate, batch_a, batch_w, batch_o, (const float*)gate_v, gate_ld);
+      };
+      static SmemRaised r88, r84, r54, r44;
+      switch (simt_tile(M, N, batch)) {
+        case 88: return tiled(gemm_simt_tile_kernel<8, 8>, 8, 8, r88);
+        case 84: return tiled(gemm_simt_tile_kernel<8, 4>, 8, 4, r84);
+        case 54: return tiled(gemm_simt_tile_kernel<5, 4>, 5, 4, r54);
+        default: return tiled(gemm_simt_tile_kernel<4, 4>, 4, 4, r44);
+      }
+    }
+  }
+  // narrow tiles: the rows the kernels above cannot read in packets of 16 bytes, and the library-free check of the
+  // bfloat16 products
   if (M > 32) {
     constexpr int BM = 128, BN = 64, TM = 8, TN = 4;
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
     PTL_REQUIRE(grid.y <= 65535, "gemm_simt: M=%d too large", M);
     return launch_kernel("gemm_simt", gemm_simt_kernel<TI, TO, BM, BN, TM, TN>, grid, dim3((BM / TM) * (BN / TN)), 0,
-                         as_stream(stream), (TO*)out, (const TI*)A, (const TI*)W, M, N, K, lda, ldw, ldo, accumulate, vec_ok,
+                         as_stream(stream), (TO*)out, (const TI*)A, (const TI*)W, M, N, K, lda, ldw, ldo, accumulate,
                          batch_a, batch_w, batch_o, gate, gate_ld);
   } else {
-    // few rows: narrow tiles so that the weight matrix is spread over many blocks
     constexpr int BM = 32, BN = 16, TM = 4, TN = 1;
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
     return launch_kernel("gemm_simt", gemm_simt_kernel<TI, TO, BM, BN, TM, TN>, grid, dim3((BM / TM) * (BN / TN)), 0,
-                         as_stream(stream), (TO*)out, (const TI*)A, (const TI*)W, M, N, K, lda, ldw, ldo, accumulate, vec_ok,
+                         as_stream(stream), (TO*)out, (const TI*)A, (const TI*)W, M, N, K, lda, ldw, ldo, accumulate,
                          batch_a, batch_w, batch_o, gate, gate_ld);
   }
 }

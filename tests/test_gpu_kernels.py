@@ -94,6 +94,19 @@ def test_linear_float32_is_true_32_bit(ops, M, N, K):
     assert (out.double().cpu() - ref).abs().max() < 3e-6 * math.sqrt(K) * 4
 
 
+@pytest.mark.parametrize("N, K", [(16, 4), (17, 36), (250, 252), (64, 1028), (130, 2048), (48, 8196)])
+def test_linear_float32_gives_a_row_the_same_bits_whatever_its_company(ops, N, K):
+    """Every kernel of the float32 product (1, 2, 4, 8, 16, 32 rows, tiles of 64) adds in one order: chunks of 32, then the
+    chunks with compensation, so its error is that of one chunk (32 roundings of a partial sum)."""
+    x, w = rnd((200, K), torch.float32, 7).cuda(), rnd((N, K), torch.float32, 8).cuda()
+    whole = ops.linear(x, w)
+    ref = x.double() @ w.double().T
+    bound = 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) * min(K, 32) + 1e-30
+    assert ((whole.double() - ref).abs() <= bound).all()
+    for rows in (1, 2, 3, 5, 8, 9, 16, 17, 32, 33, 65):
+        assert torch.equal(ops.linear(x[:rows].contiguous(), w), whole[:rows]), rows
+
+
 @pytest.mark.parametrize("M, N, K", [(1, 304, 80), (7, 64, 200), (130, 264, 96), (64, 1000, 512)])
 def test_linear_bfloat16(ops, M, N, K):
     x, w = rnd((M, K), torch.bfloat16, 5), rnd((N, K), torch.bfloat16, 6)
