@@ -462,12 +462,12 @@ class Engine:
                 return c
         return self.config.max_seq_len
 
-    GRAPH_MAX_TOKENS = 1024      # larger steps keep the GPU busy for longer than the host needs to launch them
+    GRAPH_MAX_TOKENS = 2048      # larger steps keep the GPU busy for longer than the host needs to launch them (2,020 tokens of eight layers with latent attention: 2.61 ms launched, 1.82 captured)
     GRAPH_MAX_SHAPES = 24
     GRAPH_MAX_CAPTURES = 96      # a workload that keeps cycling through more shapes than are kept stops capturing new ones
 
     def _shape_bucket(self, batch: "_HostBatch"):
-        """Steps with prompt portions of up to 1,024 tokens are bound by the host's launches (about
+        """Steps with prompt portions of up to 2,048 tokens are bound by the host's launches (about
         11 us each, twice the GPU's time at 300 tokens), so they run from captured graphs too: the
         step's shape is padded to (tokens, requests, wants logits, items of each of the operator
         set's work lists) with few values each, and a shape that comes a second time is captured.
