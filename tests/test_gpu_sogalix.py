@@ -134,6 +134,16 @@ def test_decay_argument_tiles_and_single_rows(ops, T, n, rank, extra):
     assert torch.equal(alone[0], za[t])
 
 
+@pytest.mark.parametrize("T,rank,n", [(2369, 70, 100), (300, 33, 1025), (17, 64, 31), (5, 65, 1)])
+def test_decay_argument_in_wide_and_narrow_blocks(ops, T, rank, n):
+    """Blocks of 128 columns and of 32, at and beside their edges: a token's row has the same bits from both."""
+    g = torch.Generator().manual_seed(T + rank)
+    x, w2 = _rand(g, T, rank, scale=1.5), _rand(g, n, rank)
+    z = ops.lowrank_tanh_linear(x.cuda(), 0, w2.cuda())
+    _close(z, TorchOps().lowrank_tanh_linear(x, 0, w2), "float32", "decay argument")
+    assert torch.equal(ops.lowrank_tanh_linear(x[:3].cuda(), 0, w2.cuda()), z[:3])
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("H,d", [(3, 32), (2, 20), (1, 128), (2, 200), (4, 4), (1, 64), (5, 8), (1, 40)])
 def test_delta_walk_and_its_state(ops, dtype, H, d):
