@@ -171,6 +171,183 @@ general_delta_kernel(float* __restrict__ out, const T* __restrict__ proj, int ld
   }
 }
 
+// The same for heads of 17 to 64 channels, with two columns per group of lanes and the staging by warps of its own: warps 0 to 3
+// walk batch i while warps 4 to 7 put batch i + 1 into the other half of shared memory and fetch batch i + 2.  The walk is
+// bound by the latency of its chain (two sums over eight lanes a token); in the kernel above every warp also works
+// exponentials and quotients out between two batches and meets the others three times a batch, and the four blocks of a
+// head do so four times.  A column's sums are the same, in the same order.
+// Eight prompts of 65 to 440 tokens, 16 heads of 64: 154 us, the kernel above 235 (with two columns a group alone 219, four 240);
+// eight single tokens 6.0 us and 9.8.
+template <typename T, int RPL>
+__global__ void __launch_bounds__(256, 2)
+general_delta_pairs_kernel(float* __restrict__ out, const T* __restrict__ proj, int ld, const float* __restrict__ a_pre, int a_ld,
+                           const float* __restrict__ a_bias, const float* __restrict__ z, const float* __restrict__ w_bias,
+                           float decay_limit, float* __restrict__ state, const int* __restrict__ q_start,
+                           const int* __restrict__ positions, const int* __restrict__ state_slot, int heads, int d, float unit_eps) {
+  constexpr int DS = 8 * RPL, HP = RPL / 2, COLS = 32;
+  constexpr int kBatchFloats = kGdBatch * (4 * DS + COLS + 1);
+  __shared__ __align__(16) float smem[2 * kBatchFloats];
+  // floats of a batch: r, k, decay, rate times key [batch][DS]; values [batch][COLS]; 1 / (|k|^2 + unit_eps) [batch]
+  constexpr int kKey = kGdBatch * DS, kDecay = 2 * kKey, kRate = 3 * kKey, kValue = 4 * kKey, kNorm = kValue + kGdBatch * COLS;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int r = blockIdx.z, h = blockIdx.y;
+  const int lo = q_start[r], hi = q_start[r + 1];
+  if (hi <= lo || state_slot[r] < 0) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int j0 = blockIdx.x * COLS;
+  const int n = heads * d;
+  const int batches = (hi - lo + kGdBatch - 1) / kGdBatch;
+  for (int i = threadIdx.x; i < 2 * kBatchFloats; i += 256) smem[i] = 0.f;       // zero beyond d for good
+  __syncthreads();
+  if (warp >= 4) {
+    // element i of a thread's share of a batch: flat index tid + 128 i over [batch][d]
+    const int tid = threadIdx.x - 128;
+    T pr[RPL], pk[RPL], pv[4];
+    float pz[RPL], pa[RPL];
+    const int tok_first = tid / d, e_first = tid % d, tok_step = 128 / d, e_step = 128 % d;
+    auto fetch = [&](int t0) {
+      const int nb = min(kGdBatch, hi - t0);
+      int tok = tok_first, e = e_first;
+#pragma unroll
+      for (int i = 0; i < RPL; ++i) {
+        if (tok < nb) {
+          const size_t t = (size_t)(t0 + tok);
+          pr[i] = proj[t * ld + h * d + e];
+          pk[i] = proj[t * ld + n + h * d + e];
+          pz[i] = z[t * n + h * d + e];
+          pa[i] = a_pre[t * a_ld + h * d + e];
+        }
+        tok += tok_step;
+        e += e_step;
+        if (e >= d) { e -= d; ++tok; }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int idx = tid + 128 * i;
+        if (idx / COLS < nb) pv[i] = proj[(size_t)(t0 + idx / COLS) * ld + 2 * n + h * d + min(j0 + idx % COLS, d - 1)];
+      }
+    };
+    auto stage = [&](int t0, float* dst) {
+      const int nb = min(kGdBatch, hi - t0);
+      int tok = tok_first, e = e_first;
+#pragma unroll
+      for (int i = 0; i < RPL; ++i) {
+        if (tok < nb) {
+          const float kf = to_f32(pk[i]);
+          dst[tok * DS + e] = to_f32(pr[i]);
+          dst[kKey + tok * DS + e] = kf;
+          dst[kDecay + tok * DS + e] = expf(-decay_limit * sigmoid_f32(pz[i] + w_bias[h * d + e]));
+          dst[kRate + tok * DS + e] = sigmoid_f32(pa[i] + a_bias[h * d + e]) * kf;
+        }
+        tok += tok_step;
+        e += e_step;
+        if (e >= d) { e -= d; ++tok; }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int idx = tid + 128 * i;
+        if (idx / COLS < nb) dst[kValue + idx] = to_f32(pv[i]);
+      }
+      if (t0 + kGdBatch < hi) fetch(t0 + kGdBatch);
+      asm volatile("bar.sync 1, 128;" ::: "memory");           // the staging warps: the keys are in place
+#pragma unroll
+      for (int m = 0; m < 4; ++m) {                             // warp w takes tokens w, w + 4, w + 8, w + 12
+        const int tk = warp - 4 + 4 * m;
+        if (tk < nb) {
+          float kk = 0.f;
+          for (int e2 = lane; e2 < d; e2 += 32) kk = fmaf(dst[kKey + tk * DS + e2], dst[kKey + tk * DS + e2], kk);
+          kk = warp_sum(kk);
+          if (lane == 0) dst[kNorm + tk] = 1.0f / (kk + unit_eps);
+        }
+      }
+    };
+    fetch(lo);
+    stage(lo, smem);
+    __syncthreads();
+    for (int b = 0; b < batches; ++b) {
+      if (b + 1 < batches) stage(lo + (b + 1) * kGdBatch, smem + ((b + 1) & 1) * kBatchFloats);
+      __syncthreads();
+    }
+    return;
+  }
+  const int sub = threadIdx.x & 7, grp = threadIdx.x >> 3;     // columns j0 + grp and j0 + grp + 16
+  float* st = state + (((size_t)state_slot[r] * heads + h) * d) * d + j0 + grp;
+  const bool from_zero = positions[lo] == 0;
+  float2 S[2][HP];
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+#pragma unroll
+    for (int m = 0; m < HP; ++m) {
+      const int row = 16 * m + 2 * sub;
+      const bool live = !from_zero && j0 + grp + 16 * c < d;
+      S[c][m].x = row < d && live ? st[(size_t)row * d + 16 * c] : 0.f;
+      S[c][m].y = row + 1 < d && live ? st[(size_t)(row + 1) * d + 16 * c] : 0.f;
+    }
+  __syncthreads();
+  for (int b = 0; b < batches; ++b) {
+    const int t0 = lo + b * kGdBatch, nb = min(kGdBatch, hi - t0);
+    const float* src = smem + (b & 1) * kBatchFloats;
+#pragma unroll 2
+    for (int tok = 0; tok < nb; ++tok) {
+      const float2* rp = reinterpret_cast<const float2*>(src + tok * DS) + sub;                // pair m of this lane: rp[8 * m]
+      float2 k[HP], w[HP], ak[HP], rv[HP];
+#pragma unroll
+      for (int m = 0; m < HP; ++m) {
+        k[m] = rp[kKey / 2 + 8 * m];
+        w[m] = rp[kDecay / 2 + 8 * m];
+        ak[m] = rp[kRate / 2 + 8 * m];
+        rv[m] = rp[8 * m];
+      }
+      float dot[2], acc[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        float2 dot0 = make_float2(0.f, 0.f), dot1 = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int m = 0; m < HP; ++m) {
+          if (m & 1) dot1 = __ffma2_rn(S[c][m], k[m], dot1); else dot0 = __ffma2_rn(S[c][m], k[m], dot0);
+        }
+        dot[c] = (dot0.x + dot0.y) + (dot1.x + dot1.y);
+      }
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        dot[0] += __shfl_xor_sync(0xffffffffu, dot[0], o);
+        dot[1] += __shfl_xor_sync(0xffffffffu, dot[1], o);
+      }
+      const float kn = src[kNorm + tok];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const float cc = -dot[c] * kn, v = src[kValue + tok * COLS + grp + 16 * c];
+        const float2 c2 = make_float2(cc, cc), v2 = make_float2(v, v);
+        float2 acc0 = make_float2(0.f, 0.f), acc1 = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int m = 0; m < HP; ++m) {
+          S[c][m] = __ffma2_rn(w[m], S[c][m], __ffma2_rn(ak[m], c2, __fmul2_rn(k[m], v2)));
+          if (m & 1) acc1 = __ffma2_rn(S[c][m], rv[m], acc1); else acc0 = __ffma2_rn(S[c][m], rv[m], acc0);
+        }
+        acc[c] = (acc0.x + acc0.y) + (acc1.x + acc1.y);
+      }
+      // both sums at once: even lanes of a group end with column 0's, odd lanes with column 1's
+      const bool odd = sub & 1;
+      float sum = (odd ? acc[1] : acc[0]) + __shfl_xor_sync(0xffffffffu, odd ? acc[0] : acc[1], 1);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+      sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+      if (sub < 2 && j0 + grp + 16 * sub < d) out[(size_t)(t0 + tok) * n + h * d + j0 + grp + 16 * sub] = sum;
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int c = 0; c < 2; ++c)
+    if (j0 + grp + 16 * c < d) {
+#pragma unroll
+      for (int m = 0; m < HP; ++m) {
+        const int row = 16 * m + 2 * sub;
+        if (row < d) st[(size_t)row * d + 16 * c] = S[c][m].x;
+        if (row + 1 < d) st[(size_t)(row + 1) * d + 16 * c] = S[c][m].y;
+      }
+    }
+}
+
 template <typename T>
 int general_delta_scan(float* out, const void* proj, int ld, const float* a_pre, int a_ld, const float* a_bias, const float* z,
                        const float* w_bias, float decay_limit, float* state, const int* q_start, const int* positions,
@@ -180,7 +357,11 @@ int general_delta_scan(float* out, const void* proj, int ld, const float* a_pre,
   PTL_REQUIRE(requests <= 65535 && heads <= 65535, "general_delta_scan: at most 65535 requests and heads");
   if (requests == 0) return 0;
   const dim3 grid((d + 15) / 16, heads, requests), block(128);
-  static SmemRaised raised[6];
+  if (d > 16 && d <= 64)
+    return launch_kernel("general_delta_scan", d <= 32 ? general_delta_pairs_kernel<T, 4> : general_delta_pairs_kernel<T, 8>,
+                         dim3((d + 31) / 32, heads, requests), dim3(256), 0, as_stream(stream), out, (const T*)proj, ld, a_pre, a_ld, a_bias,
+                         z, w_bias, decay_limit, state, q_start, positions, state_slot, heads, d, unit_eps);
+  static SmemRaised raised[4];
 #define PTL_GD(RPL, SLOT)                                                                                                      \
   {                                                                                                                            \
     const size_t smem = (size_t)kGdBatch * (4 * 8 * RPL + 16 + 1) * sizeof(float);                                             \
@@ -192,11 +373,9 @@ int general_delta_scan(float* out, const void* proj, int ld, const float* a_pre,
   }
   const int per_lane = (d + 7) / 8;
   if (per_lane <= 2) PTL_GD(2, 0)
-  if (per_lane <= 4) PTL_GD(4, 1)
-  if (per_lane <= 8) PTL_GD(8, 2)
-  if (per_lane <= 12) PTL_GD(12, 3)
-  if (per_lane <= 16) PTL_GD(16, 4)
-  PTL_GD(32, 5)
+  if (per_lane <= 12) PTL_GD(12, 1)
+  if (per_lane <= 16) PTL_GD(16, 2)
+  PTL_GD(32, 3)
 #undef PTL_GD
 }
 

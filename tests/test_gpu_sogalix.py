@@ -176,6 +176,13 @@ def test_delta_walk_and_its_state(ops, dtype, H, d):
     assert torch.equal(Sd[[0, 2, 3]].cpu(), S0[[0, 2, 3]]) and not torch.equal(Sd[1].cpu(), S0[1])
 
 
+@pytest.mark.parametrize("H,d", [(1, 17), (2, 31), (2, 33), (1, 48), (1, 49), (2, 63)])
+def test_delta_walk_at_the_edges_of_a_group_of_columns(ops, H, d):
+    """Eight lanes walk two or four columns of the state, sixteen apart: heads that end inside such a group, to the same bounds."""
+    for dtype in DTYPES:
+        test_delta_walk_and_its_state(ops, dtype, H, d)
+
+
 def test_a_far_token_survives_hundreds_of_decays_and_a_removed_one_is_gone(ops):
     """Decay close to one and no removal: the value written at token 0 is read 600 tokens later, smaller by the decays
     alone.  Then a second key along the same direction with removal rate one wipes it: only the new value is read."""
