@@ -189,6 +189,7 @@ class Engine:
         if self.config.timing and hasattr(self.ops, "enable_timing"):
             self.ops.enable_timing()
         self._portions_by_host_lengths = self.model.any_part(lambda part: getattr(part, "portions_by_host_lengths", False))
+        self._many_launches = self.model.any_part(lambda part: getattr(part, "many_launches", False))
         self._graphs = {}          # captured steps: padded batch size or _DecodeShape (single tokens only), or a shape tuple
         self._shape_seen: Dict[tuple, int] = {}
         self._shape_captures = 0
@@ -462,19 +463,22 @@ class Engine:
                 return c
         return self.config.max_seq_len
 
-    GRAPH_MAX_TOKENS = 2048      # larger steps keep the GPU busy for longer than the host needs to launch them (2,020 tokens of eight layers with latent attention: 2.61 ms launched, 1.82 captured)
+    GRAPH_MAX_TOKENS = 1024      # larger steps keep the GPU busy for longer than the host needs to launch them ...
+    # ... in layers of five launches; in those with a part that says ``many_launches`` (12 to 16 a layer) they do not yet (2,020 tokens of
+    # eight layers with latent attention: 2.61 ms launched, 1.82 captured)
+    GRAPH_MAX_TOKENS_MANY_LAUNCHES = 2048
     GRAPH_MAX_SHAPES = 24
     GRAPH_MAX_CAPTURES = 96      # a workload that keeps cycling through more shapes than are kept stops capturing new ones
 
     def _shape_bucket(self, batch: "_HostBatch"):
-        """Steps with prompt portions of up to 2,048 tokens are bound by the host's launches (about
+        """Steps with prompt portions of up to 1,024 tokens (2,048 in models of many launches) are bound by the host's launches (about
         11 us each, twice the GPU's time at 300 tokens), so they run from captured graphs too: the
         step's shape is padded to (tokens, requests, wants logits, items of each of the operator
         set's work lists) with few values each, and a shape that comes a second time is captured.
         Padded token rows have request -1 and slot -1, padded list items are what the operator set
         says they must be: every kernel skips them."""
         T, R, M = batch.T, batch.R, len(batch.logit_rows)
-        if T > self.GRAPH_MAX_TOKENS:
+        if T > (self.GRAPH_MAX_TOKENS_MANY_LAUNCHES if self._many_launches else self.GRAPH_MAX_TOKENS):
             return 0
         pow2 = lambda n: 0 if n == 0 else 1 << (n - 1).bit_length()
         step = 64 if T <= 256 else 128

@@ -34,6 +34,8 @@ Contracts (``T`` = tokens of the step, all tensors on the runtime's device):
   result, and returns what the tail returns;
 * a mixer or ffn with the class attribute ``fuses_residual = True`` is called with
   ``residual=<float32 [T, H]>`` as well and may add its output into it and return None;
+* a part with the class attribute ``many_launches = True`` puts its layer's launches at a dozen or more: larger steps of
+  such a model run from captured graphs;
 * embedding: ``cache_need() -> CacheNeed`` of kind "none" (its per-request states);
   ``start_stream(token_ids, table, scale, ctx, cache) -> float32 [T, H]``;
 * block: ``forward(x, residual, ctx, cache) -> (x, residual)``.

@@ -27,6 +27,8 @@ class GatedDeltaRule(Part):
     ``v.conv`` [channels, taps], ``b``, ``a`` [heads, hidden], ``A_log``, ``dt_bias`` [heads], ``norm`` [value_dim],
     ``o`` [hidden, heads*value_dim]."""
 
+    many_launches = True
+
     def __init__(self, spec: PartSpec, runtime: Runtime):
         super().__init__(spec, runtime)
         p = spec.params

@@ -32,6 +32,8 @@ class GeneralDeltaRule(Part):
     Tensors: ``r``, ``k``, ``v``, ``g``, ``a`` [heads*head_dim, hidden], ``a.b``, ``w0``, ``norm`` [heads*head_dim],
     ``w1`` [rank, hidden], ``w2`` [heads*head_dim, rank], ``o`` [hidden, heads*head_dim]."""
 
+    many_launches = True
+
     def __init__(self, spec: PartSpec, runtime: Runtime):
         super().__init__(spec, runtime)
         p = spec.params

@@ -34,6 +34,8 @@ class LatentAttention(Part):
     kv_rank], ``uv`` [heads*value_dim, kv_rank], ``g`` [heads, hidden], ``o`` [hidden, heads*value_dim]; with ``own_kv``
     ``dkv`` [kv_rank+rot_dim, hidden], ``dkv.norm`` [kv_rank]."""
 
+    many_launches = True
+
     def __init__(self, spec: PartSpec, runtime: Runtime):
         super().__init__(spec, runtime)
         p = spec.params

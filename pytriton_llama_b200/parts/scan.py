@@ -24,6 +24,8 @@ class SelectiveScan(Part):
     ``conv`` [inner, taps], ``conv.b`` [inner], ``x`` [dt_rank + 2*state, inner], ``dt`` [inner, dt_rank],
     ``dt.b`` [inner], ``A_log`` [inner, state], ``D`` [inner], ``o`` [hidden, inner]."""
 
+    many_launches = True
+
     def __init__(self, spec: PartSpec, runtime: Runtime):
         super().__init__(spec, runtime)
         p = spec.params
