@@ -1,20 +1,28 @@
 // Decode attention over the paged cache in bfloat16: one block per (single-token request, kv
-// head, split of the key range).  All query heads of the group ride in the 16 rows of one
+// head, part of the key range).  All query heads of the group ride in the 16 rows of one
 // m16n8k16 tile, so each key and value is fetched from HBM once for the whole group; the kernel
-// is a streaming read of the cache.  Four warps share 64-key tiles brought in by a ring of
-// cp.async stages (16 keys per warp and tile), keep their own running max / sum / accumulator in
-// float32 and are merged through shared memory at the end.  With splits > 1 the partial results of
-// a (token, kv head) are combined in one of three ways: up to 8 splits with 128-key tiles form a
+// is a streaming read of the cache.  Four warps share tiles of 64 or 128 keys (16 or 32 keys per warp
+// and tile), keep their own running max / sum / accumulator in float32 and are merged through shared
+// memory at the end.  Pages of whole sixteens come by TMA, every warp's keys into a ring of its own;
+// other pages by a ring of cp.async stages for the block.  The parts of a (token, kv head) are combined in
+// one of three ways: up to 8 equal splits of few (token, kv head) pairs form a
 // thread-block cluster, every warp sends its partial rows into the shared memory of the block
 // that owns the row (distributed shared memory), and after one cluster barrier the owners
 // finish them; otherwise the block writes an unnormalised partial result to global memory and
 // the block that finishes last combines them (or, without counters, the kernel `attention_merge`
 // of attention_simt.cu does).
 //
+// By cp.async the kernel reached 40 to 60 % of the copy bandwidth with few warps per SM (32 requests of 128 to 2,304 tokens, 8
+// heads of 128: 60 us against a floor of 24): its warps waited on the fixed latencies of their own instructions, the copies'
+// addresses, the products and the softmax of a tile one behind the other between two block barriers (DRAM 25 % busy, 0.18
+// instructions issued per scheduler and cycle).  By TMA a warp's copies are a few instructions of one lane, warps run free of one
+// another, and the ring takes less shared memory for the same bytes in flight: 32 us.
+//
 // The token list `items` names the tokens of the step that take this path (nullptr: tokens
 // 0..n-1).  Token t of request r = tok_req[t] at position p sees keys max(0, p-window+1)..p;
 // r < 0 marks a padding row, which yields zeros.
 #include "mma_utils.cuh"
+#include "tcgen05_utils.cuh"
 
 namespace ptl {
 
@@ -29,31 +37,120 @@ constexpr int kDecStagedPages = 512;    // block-table entries of a block's key 
 
 // KP = groups of 16 keys per warp and tile: 1 (64-key tiles, four blocks per SM) for large batches,
 // 2 (128-key tiles, two blocks per SM, fewer barriers per key) when few blocks are in flight.
-template <int D, int KP> struct DecodeCfg {
-  static constexpr int kKeys = 64 * KP;
+// RING > 0: pages of whole sixteens of keys, fetched by TMA: every warp fetches its own 16 * KP keys of a tile, RING tiles ahead,
+// into slots of its own with barriers of their own, and no warp waits for another inside the loop.  RING 0: any page size, the
+// block's tiles by cp.async with a block barrier per tile.
+template <int D, int KP, int RING> struct DecodeCfg {
+  static constexpr int kKeys = 16 * KP * kDecWarps;
   // 64-key tiles: three stages (48 KB for D = 64, four blocks per SM).  128-key tiles: two stages, so that
   // two blocks leave room for a block of the product that follows to move in and fetch its weights
   // early (alone the kernel is 2 us slower with two stages, a decode step 2 % faster)
-  static constexpr int kStages = KP == 2 ? 2 : 3;
+  static constexpr int kStages = RING ? RING : KP == 2 ? 2 : 3;
   static constexpr int kChunks = D / 8;                       // 16-byte chunks per row
   static constexpr int kTileBytes = kKeys * D * 2;             // one of K / V
   static constexpr int kSmem = kStages * 2 * kTileBytes;
+  static constexpr int kSlotBytes = 2 * kTileBytes / kDecWarps;  // a warp's keys and values of a tile
+  static constexpr int kAlign = RING ? 1024 : 0;                 // the slots are swizzled by address
+  static constexpr int kMaxSums = (kSmem - 80 - kDecWarps * 512) / 8;  // (head of the group, split) pairs the merge at the end has room for
 };
 
-template <int D, int KP>
+// Many (token, kv head) pairs of contexts of any lengths (`per_head` > 0): the step's tiles are dealt out in units of at most c
+// tiles, c the smallest with at most `per_head` units per kv head, so that a request of 2,500 tokens is not one block's work beside
+// one of 250 and all units are in flight at once.  A token of n tiles gets ceil(n / c) units per kv head (one, if it has none);
+// they are numbered token by token, kv head by kv head, so that the partial results of a (token, kv head) lie side by side.
+// Every warp works its block's unit out by itself from the step's integers, before the wait.  Above 256 tokens c comes from
+// a bound instead of a search.
+struct DecodeUnit { int item, kvh, split, splits; };
+constexpr int kDecHeld = 8;                                   // tokens per lane whose lengths stay in registers
+
+__device__ __forceinline__ int decode_tiles(const int* items, const int* tok_req, const int* positions, int i, int window, int tile_keys) {
+  const int t = items ? __ldcg(items + i) : i;
+  const int p = __ldcg(positions + t);
+  const int keys = window > 0 && p + 1 > window ? window : p + 1;
+  return __ldcg(tok_req + t) < 0 ? 0 : (keys + tile_keys - 1) / tile_keys;
+}
+
+template <int KEYS>
+__device__ __forceinline__ DecodeUnit decode_unit(const int* items, const int* tok_req, const int* positions, int n_items, int nkv,
+                                                  int window, int per_head, int max_splits, int unit) {
+  const int lane = threadIdx.x & 31;
+  const bool few = n_items <= 32 * kDecHeld;
+  int held[kDecHeld], total = 0, longest = 1;
+#pragma unroll
+  for (int j = 0; j < kDecHeld; ++j) {
+    const int i = lane + 32 * j;
+    held[j] = few && i < n_items ? decode_tiles(items, tok_req, positions, i, window, KEYS) : 0;
+    total += held[j];
+    longest = max(longest, held[j]);
+  }
+  if (!few)
+    for (int i = lane; i < n_items; i += 32) {
+      const int tiles = decode_tiles(items, tok_req, positions, i, window, KEYS);
+      total += tiles;
+      longest = max(longest, tiles);
+    }
+  total = __reduce_add_sync(0xffffffffu, total);
+  longest = __reduce_max_sync(0xffffffffu, longest);
+  int c = max((total + per_head - 1) / per_head, max(1, (longest + max_splits - 1) / max_splits));
+  if (few) {
+    int hi = longest;
+    while (c < hi) {                                          // (the same in every lane)
+      const int mid = (c + hi) / 2;
+      int units = 0;
+#pragma unroll
+      for (int j = 0; j < kDecHeld; ++j)
+        if (32 * j < n_items) units += lane + 32 * j < n_items ? max(1, (held[j] + mid - 1) / mid) : 0;
+      if ((int)__reduce_add_sync(0xffffffffu, units) <= per_head) hi = mid; else c = mid + 1;
+    }
+  } else {
+    c = per_head > n_items ? max(c, (total + per_head - n_items - 1) / (per_head - n_items)) : longest;
+  }
+  int before = 0;                                             // units of the tokens before, per kv head
+  for (int i0 = 0; i0 < n_items; i0 += 32) {
+    const int i = i0 + lane;
+    int tiles = 0;
+    if (few) {
+#pragma unroll
+      for (int j = 0; j < kDecHeld; ++j)
+        if (i0 == 32 * j) tiles = held[j];
+    } else if (i < n_items) {
+      tiles = decode_tiles(items, tok_req, positions, i, window, KEYS);
+    }
+    const int mine = i < n_items ? max(1, (tiles + c - 1) / c) : 0;
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int below = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += below;
+    }
+    const unsigned past = __ballot_sync(0xffffffffu, unit < (before + incl) * nkv);
+    if (past) {
+      const int who = __ffs(past) - 1;
+      const int n = __shfl_sync(0xffffffffu, mine, who), first = before + __shfl_sync(0xffffffffu, incl - mine, who);
+      const int at = unit - first * nkv;
+      return DecodeUnit{i0 + who, at / n, at % n, n};
+    }
+    before += __shfl_sync(0xffffffffu, incl, 31);
+  }
+  return DecodeUnit{-1, 0, 0, 1};
+}
+
+template <int D, int KP, int RING>
 __global__ void __launch_bounds__(kDecWarps * 32)
-decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ part_acc, float* __restrict__ part_ml,
+decode_attention_kernel(const __grid_constant__ CUtensorMap map_kv, __nv_bfloat16* __restrict__ out, float* __restrict__ part_acc, float* __restrict__ part_ml,
                         const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
                         const int* __restrict__ block_table, const int* __restrict__ items,
                         const int* __restrict__ tok_req, const int* __restrict__ positions, int q_stride,
                         int out_stride, int bt_stride, int nq, int nkv, int page_size, float scale_log2,
                         int window, int splits, int num_pages, int page_shift, int* __restrict__ counters,
                         int cluster_merge, int fused, const float* __restrict__ inv_freq,
-                        const int* __restrict__ slots, unsigned long long* timeline) {
-  using Cfg = DecodeCfg<D, KP>;
+                        const int* __restrict__ slots, unsigned long long* timeline, int n_items, int per_head, int* status) {
+  using Cfg = DecodeCfg<D, KP, RING>;
   constexpr int kDecKeys = Cfg::kKeys;
   constexpr int kDecKP = KP;
-  extern __shared__ __align__(128) unsigned char smem[];
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  unsigned char* smem = smem_raw;
+  if (RING) smem += (1024u - (smem_u32(smem_raw) & 1023u)) & 1023u;
   if (threadIdx.x == 0 && timeline) { timeline_stamp(timeline, 0); if (blockIdx.x == 0) timeline[0] = 1; }
   // with a cluster, peers write into this block's shared memory later on: none may do so before
   // every block runs, which the wait that matches this arrival establishes
@@ -63,9 +160,17 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
   // predecessor writes q and the slot of position p).  So it runs under the predecessor's tail.
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, c = lane & 3;
-  const int split = blockIdx.x % splits;
-  const int kvh = (blockIdx.x / splits) % nkv;
-  const int ti = blockIdx.x / (splits * nkv);
+  int split = blockIdx.x % splits;
+  int kvh = (blockIdx.x / splits) % nkv;
+  int ti = blockIdx.x / (splits * nkv);
+  if (per_head) {
+    const DecodeUnit unit = decode_unit<kDecKeys>(items, tok_req, positions, n_items, nkv, window, per_head, Cfg::kMaxSums / (nq / nkv), blockIdx.x);
+    if (unit.item < 0) return;                                // (no cluster in this form: nobody waits for this block)
+    split = unit.split;
+    splits = unit.splits;
+    kvh = unit.kvh;
+    ti = unit.item;
+  }
   const int t = items ? __ldcg(items + ti) : ti;
   const int G = nq / nkv;
   const int r = __ldcg(tok_req + t);
@@ -76,7 +181,8 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
   chunk_keys = (chunk_keys + kDecKeys - 1) / kDecKeys * kDecKeys;
   const int k_begin = lo + split * chunk_keys;
   const int k_end = r < 0 ? k_begin : min(k_begin + chunk_keys, p + 1);
-  const int ntiles = k_end > k_begin ? (k_end - k_begin + kDecKeys - 1) / kDecKeys : 0;
+  const int k_first = RING ? k_begin & ~15 : k_begin;         // TMA fetches whole groups of sixteen keys of a page
+  const int ntiles = k_end > k_begin ? (k_end - k_first + kDecKeys - 1) / kDecKeys : 0;
   const int* bt_global = block_table + (size_t)(r < 0 ? 0 : r) * bt_stride;
   const size_t plane = (size_t)nkv * page_size * D;
   const uint32_t smem_base = smem_u32(smem);
@@ -84,13 +190,23 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
   // ---- the block-table entries of this block's key range go to shared memory once (when they
   // fit), so that the copies of a tile never wait on a global load for their page
   __shared__ int s_pages[kDecStagedPages];
-  const int first_block = ntiles > 0 ? k_begin / page_size : 0;
+  const int first_block = ntiles > 0 ? k_first / page_size : 0;
   const int n_blocks = ntiles > 0 ? (k_end - 1) / page_size - first_block + 1 : 0;
   const bool staged = n_blocks <= kDecStagedPages;
-  if (staged) {
-    for (int i = tid; i < n_blocks; i += kDecWarps * 32) s_pages[i] = __ldcg(bt_global + first_block + i);
-    __syncthreads();
+  __shared__ __align__(8) uint64_t s_full[RING ? kDecWarps * RING : 1];
+  __shared__ int s_abort;
+  const uint32_t full0 = smem_u32(s_full) + 8u * (warp * RING);
+  if (RING) {
+    if (tid == 0) s_abort = 0;
+    if (lane == 0) {
+#pragma unroll
+      for (int i = 0; i < RING; ++i) mbar_init(full0 + 8 * i, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
   }
+  if (staged)
+    for (int i = tid; i < n_blocks; i += kDecWarps * 32) s_pages[i] = __ldcg(bt_global + first_block + i);
+  if (staged || RING) __syncthreads();
   const int* bt = staged ? s_pages - first_block : bt_global;
 
   // ---- with `fused` the kernel does the work of rope_kv_write for its single tokens itself: q is
@@ -138,6 +254,34 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
     }
   };
 
+  // ---- the same by TMA, by one lane of every warp for the warp's own keys: 64 values of sixteen keys and of their values, which lie
+  // in the next plane, at a time.  Keys of a page number outside the cache come from behind the cache's last plane, where
+  // TMA reads zeros.
+  const int row0 = warp * 16 * kDecKP;                        // this warp's keys of a tile
+  const uint32_t slot0 = smem_base + warp * (RING * Cfg::kSlotBytes);
+  auto load_keys = [&](int tile) {
+    const int k0 = k_first + tile * kDecKeys + row0;
+    const int groups = min(kDecKP, (k_end - k0 + 15) / 16);
+    if (groups <= 0) return;
+    const uint32_t bar = full0 + 8u * (tile % Cfg::kStages), dst = slot0 + (tile % Cfg::kStages) * Cfg::kSlotBytes;
+    mbar_expect_tx(bar, groups * (16 * D * 4));
+#pragma unroll
+    for (int kp = 0; kp < kDecKP; ++kp) {
+      if (kp >= groups) break;
+      const int key = k0 + 16 * kp;
+      const int block = page_shift >= 0 ? key >> page_shift : key / page_size;
+      const int page = bt[block];
+      const int plane0 = page >= 0 && page < num_pages ? 2 * page : 2 * num_pages;
+#pragma unroll
+      for (int ch = 0; ch < D / 64; ++ch)
+        tma_load_3d(dst + (kp * (D / 64) + ch) * 4096, &map_kv, bar, ch * 64, kvh * page_size + key - block * page_size, plane0);
+    }
+  };
+  // byte offset of a 16-byte chunk of a row of this warp's keys (values: 2,048 further) inside its slot, as TMA's swizzle puts it
+  auto slot_offset = [&](int row, int chunk) {
+    return (uint32_t)(((row >> 4) * (D / 64) + (chunk >> 3)) * 4096 + (row & 15) * 128 + (((chunk & 7) ^ (row & 7)) << 4));
+  };
+
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
   float o[D / 8][4];
 #pragma unroll
@@ -146,7 +290,12 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
   // the first tiles are requested before the wait when none of them holds position p
   const int first_tiles = min(ntiles, Cfg::kStages - 1);
   const bool early = first_tiles > 0 && k_begin + first_tiles * kDecKeys <= p;
-  if (early) {
+  // (by TMA: as many whole tiles before position p as there are slots)
+  const int early_tiles = ntiles > 0 ? min(min(ntiles, Cfg::kStages), (p - k_first) / kDecKeys) : 0;
+  if (RING) {
+    if (lane == 0)
+      for (int s = 0; s < early_tiles; ++s) load_keys(s);
+  } else if (early) {
 #pragma unroll
     for (int s = 0; s < Cfg::kStages - 1; ++s) {
       if (s < ntiles) load_tile(s, s);
@@ -167,23 +316,25 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
     const int slot = __ldcg(slots + t);                       // the same for every thread of the block
     owner = slot >= 0 && slot < (long long)num_pages * page_size;   // a layer that does not write reads the cache as it is
     if (owner) {
-    const bool store = true;
     const __nv_bfloat16* ksrc = q + (size_t)t * q_stride + (size_t)(nq + kvh) * D;
     __nv_bfloat16* kdst = const_cast<__nv_bfloat16*>(cache) + ((size_t)(slot / page_size) * 2) * plane +
                           ((size_t)kvh * page_size + slot % page_size) * D;
-    if (tid < D / 2) {
-      const float x1 = __bfloat162float(ksrc[tid]), x2 = __bfloat162float(ksrc[tid + D / 2]);
-      float o1 = x1, o2 = x2;
-      if (inv_freq) rope_rotate(x1, x2, s_cs[tid], s_cs[D / 2 + tid], o1, o2);
-      const __nv_bfloat16 b1 = __float2bfloat16_rn(o1), b2 = __float2bfloat16_rn(o2);
-      s_new[tid] = b1;
-      s_new[tid + D / 2] = b2;
-      if (store) { kdst[tid] = b1; kdst[tid + D / 2] = b2; }
-    } else if (tid - D / 2 < D / 8) {
-      const int ch = tid - D / 2;
-      const uint4 v = *reinterpret_cast<const uint4*>(ksrc + (size_t)nkv * D + ch * 8);
-      *reinterpret_cast<uint4*>(s_new + D + ch * 8) = v;
-      if (store) *reinterpret_cast<uint4*>(kdst + plane + ch * 8) = v;
+    for (int e = tid; e < D / 2 + D / 8; e += kDecWarps * 32) {
+      if (e < D / 2) {
+        const float x1 = __bfloat162float(ksrc[e]), x2 = __bfloat162float(ksrc[e + D / 2]);
+        float o1 = x1, o2 = x2;
+        if (inv_freq) rope_rotate(x1, x2, s_cs[e], s_cs[D / 2 + e], o1, o2);
+        const __nv_bfloat16 b1 = __float2bfloat16_rn(o1), b2 = __float2bfloat16_rn(o2);
+        s_new[e] = b1;
+        s_new[e + D / 2] = b2;
+        kdst[e] = b1;
+        kdst[e + D / 2] = b2;
+      } else {
+        const int ch = e - D / 2;
+        const uint4 v = *reinterpret_cast<const uint4*>(ksrc + (size_t)nkv * D + ch * 8);
+        *reinterpret_cast<uint4*>(s_new + D + ch * 8) = v;
+        *reinterpret_cast<uint4*>(kdst + plane + ch * 8) = v;
+      }
     }
     }
   }
@@ -218,26 +369,53 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
     }
   }
 
-  if (!early) {
+  if (RING) {
+    if (lane == 0)
+      for (int s = early_tiles; s < min(ntiles, Cfg::kStages); ++s) load_keys(s);
+    if (fused) __syncthreads();                               // the token's own key and value are in place
+  } else if (!early) {
 #pragma unroll
     for (int s = 0; s < Cfg::kStages - 1; ++s) {
       if (s < ntiles) load_tile(s, s);
       cp_async_commit();
     }
   }
+  int gave_up = -1;                                           // the tile whose wait ran out (the status says so)
   for (int tile = 0; tile < ntiles; ++tile) {
-    cp_async_wait<Cfg::kStages - 2>();
-    __syncthreads();
-    if (tile == 0 && tid == 0) timeline_stamp(timeline, 2);
-    {
+    const int stage = tile % Cfg::kStages;
+    const uint32_t kbase = RING ? slot0 + stage * Cfg::kSlotBytes : smem_base + stage * 2 * Cfg::kTileBytes;
+    const uint32_t vbase = kbase + (RING ? 2048 : Cfg::kTileBytes);
+    if (RING) {
+      const int k0 = k_first + tile * kDecKeys + row0;
+      if (k0 >= k_end) break;                                 // (only the last tile ends before this warp's keys)
+      if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8u * stage, (tile / Cfg::kStages) & 1, &s_abort, status, 9))) { gave_up = tile; break; }
+      // Values of keys outside the range have weight 0, but 0 times what lies there need not be 0: zeros in their place.
+      const bool new_here = owner && p >= k0 && p < k0 + 16 * kDecKP;
+      if (new_here || k0 < k_begin || k0 + 16 * kDecKP > k_end) {
+        for (int i = lane; i < 16 * kDecKP * Cfg::kChunks; i += 32) {
+          const int row = i / Cfg::kChunks;
+          if (k0 + row < k_begin || k0 + row >= k_end) st_shared_16(vbase + slot_offset(row, i % Cfg::kChunks), make_uint4(0u, 0u, 0u, 0u));
+        }
+        if (new_here) {
+          // the token's own key and value take their place
+          for (int i = lane; i < 2 * Cfg::kChunks; i += 32) {
+            const int ch = i % Cfg::kChunks;
+            const uint4 v = *reinterpret_cast<const uint4*>(s_new + (i / Cfg::kChunks) * D + ch * 8);
+            st_shared_16((i < Cfg::kChunks ? kbase : vbase) + slot_offset(p - k0, ch), v);
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // before the slot's next copy
+        __syncwarp();
+      }
+    } else {
+      cp_async_wait<Cfg::kStages - 2>();
+      __syncthreads();
       const int nxt = tile + Cfg::kStages - 1;
       if (nxt < ntiles) load_tile(nxt, nxt % Cfg::kStages);
       cp_async_commit();
     }
-    const int stage = tile % Cfg::kStages;
-    const uint32_t kbase = smem_base + stage * 2 * Cfg::kTileBytes;
-    const uint32_t vbase = kbase + Cfg::kTileBytes;
-    if (owner && tile == ntiles - 1) {
+    if (tile == 0 && tid == 0) timeline_stamp(timeline, 2);
+    if (!RING && owner && tile == ntiles - 1) {
       // the token's own key and value take their place in the tile (row p of the range)
       const int prow = p - (k_begin + tile * kDecKeys);
       if (tid < 2 * Cfg::kChunks) {
@@ -247,7 +425,6 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
       }
       __syncthreads();
     }
-    const int row0 = warp * 16 * kDecKP;                      // this warp's keys of the tile
     // S = Q K^T: two n-tiles of 8 keys per group of 16
     float sc[kDecKP][2][4];
 #pragma unroll
@@ -260,21 +437,21 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
       for (int kp = 0; kp < kDecKP; ++kp) {
         uint32_t kb[4];
         const int id = lane >> 3;
-        const int krow = row0 + kp * 16 + (id >> 1) * 8 + (lane & 7);
-        ldmatrix_x4(kb, kbase + tile_offset<D>(krow, 2 * ks + (id & 1)));
+        const int krow = kp * 16 + (id >> 1) * 8 + (lane & 7);
+        ldmatrix_x4(kb, kbase + (RING ? slot_offset(krow, 2 * ks + (id & 1)) : tile_offset<D>(row0 + krow, 2 * ks + (id & 1))));
         mma_bf16_16816(sc[kp][0], qa[ks], kb[0], kb[1]);
         mma_bf16_16816(sc[kp][1], qa[ks], kb[2], kb[3]);
       }
     }
     // mask keys past the range, scale into log2 units
-    const int key0 = k_begin + tile * kDecKeys + row0 + 2 * c;
+    const int key0 = k_first + tile * kDecKeys + row0 + 2 * c;
 #pragma unroll
     for (int kp = 0; kp < kDecKP; ++kp)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         const int kk0 = key0 + kp * 16 + (e & 1), kk1 = kk0 + 8;
-        sc[kp][0][e] = kk0 < k_end ? sc[kp][0][e] * scale_log2 : -INFINITY;
-        sc[kp][1][e] = kk1 < k_end ? sc[kp][1][e] * scale_log2 : -INFINITY;
+        sc[kp][0][e] = kk0 < k_end && (!RING || kk0 >= k_begin) ? sc[kp][0][e] * scale_log2 : -INFINITY;
+        sc[kp][1][e] = kk1 < k_end && (!RING || kk1 >= k_begin) ? sc[kp][1][e] * scale_log2 : -INFINITY;
       }
     // online softmax for rows g (e = 0,1) and g+8 (e = 2,3)
     uint32_t pa[kDecKP][4];
@@ -315,14 +492,26 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
       for (int nt = 0; nt < D / 8; nt += 2) {
         uint32_t vb[4];
         const int id = lane >> 3;
-        const int vrow = row0 + kp * 16 + (id & 1) * 8 + (lane & 7);
-        ldmatrix_x4_trans(vb, vbase + tile_offset<D>(vrow, nt + (id >> 1)));
+        const int vrow = kp * 16 + (id & 1) * 8 + (lane & 7);
+        ldmatrix_x4_trans(vb, vbase + (RING ? slot_offset(vrow, nt + (id >> 1)) : tile_offset<D>(row0 + vrow, nt + (id >> 1))));
         mma_bf16_16816(o[nt], pa[kp], vb[0], vb[1]);
         mma_bf16_16816(o[nt + 1], pa[kp], vb[2], vb[3]);
       }
     }
+    if (RING) {
+      __syncwarp();                                           // the slot is read: its next tile
+      if (lane == 0 && tile + Cfg::kStages < ntiles) load_keys(tile + Cfg::kStages);
+    }
   }
-  cp_async_wait<0>();
+  if (RING) {
+    // after a wait that gave up: this warp's copies still under way end before the memory is used for something else
+    if (gave_up >= 0)
+      for (int t2 = gave_up; t2 < min(gave_up + Cfg::kStages, ntiles); ++t2)
+        if (k_first + t2 * kDecKeys + row0 < k_end)
+          for (uint32_t n = 0; n < (1u << 16) && !mbar_test_wait(full0 + 8u * (t2 % Cfg::kStages), (t2 / Cfg::kStages) & 1); ++n) __nanosleep(40);
+  } else {
+    cp_async_wait<0>();
+  }
   __syncthreads();
   if (tid == 0) timeline_stamp(timeline, 3);
 
@@ -413,7 +602,7 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
     if (splits == 1) {
       out[(size_t)t * out_stride + (size_t)h * D + col] = __float2bfloat16_rn(L > 0.f ? acc / L : 0.f);
     } else {
-      const size_t idx = ((size_t)t * nq + h) * splits + split;
+      const size_t idx = per_head ? (size_t)blockIdx.x * G + row : ((size_t)t * nq + h) * splits + split;
       part_acc[idx * D + col] = acc;
       if (col == 0) {
         part_ml[idx * 2] = M == -INFINITY ? -INFINITY : M * 0.6931471805599453f;   // natural-log units for the merge
@@ -436,8 +625,10 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  // partial results of the group's heads are contiguous: [G][splits][D] and [G][splits][2]
-  const size_t idx0 = ((size_t)t * nq + (size_t)kvh * G) * splits;
+  // partial results of the group's heads are contiguous: [G][splits][D] and [G][splits][2], or, dealt out in units,
+  // [splits][G][D] from the first unit of this (token, kv head) on
+  const size_t idx0 = per_head ? (size_t)(blockIdx.x - split) * G : ((size_t)t * nq + (size_t)kvh * G) * splits;
+  const size_t of_head = per_head ? 1 : splits, of_split = per_head ? G : 1;
   float* w = reinterpret_cast<float*>(smem);                   // [G][splits] maxima m, then weights e^{m - M}
   float* lz = w + G * splits;                                  // [G][splits] sums l
   float* inv_l = lz + G * splits;                              // [G]
@@ -453,15 +644,15 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
   float4 ahead[kAhead];
   {
     const int gh = ul / kD4, d4 = ul % kD4;
-    const float4* src = reinterpret_cast<const float4*>(part_acc + (idx0 + (size_t)gh * splits) * D) + d4;
+    const float4* src = reinterpret_cast<const float4*>(part_acc + (idx0 + gh * of_head) * D) + d4;
 #pragma unroll
     for (int i = 0; i < kAhead; ++i) {
       const int z = zl + i * zlanes;
-      ahead[i] = (ul < units && zl < zlanes && z < splits) ? __ldcg(src + (size_t)z * kD4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      ahead[i] = (ul < units && zl < zlanes && z < splits) ? __ldcg(src + z * of_split * kD4) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   }
   for (int e = tid; e < G * splits; e += kDecWarps * 32) {
-    const float2 ml = __ldcg(reinterpret_cast<const float2*>(part_ml + (idx0 + e) * 2));
+    const float2 ml = __ldcg(reinterpret_cast<const float2*>(part_ml + (idx0 + e / splits * of_head + e % splits * of_split) * 2));
     w[e] = ml.x;
     lz[e] = ml.y;
   }
@@ -484,7 +675,7 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
     float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
     if (u < units && zl < zlanes) {
       const int gh = u / kD4, d4 = u % kD4;
-      const float4* src = reinterpret_cast<const float4*>(part_acc + (idx0 + (size_t)gh * splits) * D) + d4;
+      const float4* src = reinterpret_cast<const float4*>(part_acc + (idx0 + gh * of_head) * D) + d4;
       int z = zl;
       if (u0 == 0) {
 #pragma unroll
@@ -497,7 +688,7 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
 #pragma unroll 8
       for (; z < splits; z += zlanes) {
         const float wz = w[gh * splits + z];
-        const float4 v = __ldcg(src + (size_t)z * kD4);
+        const float4 v = __ldcg(src + z * of_split * kD4);
         a.x = fmaf(wz, v.x, a.x); a.y = fmaf(wz, v.y, a.y); a.z = fmaf(wz, v.z, a.z); a.w = fmaf(wz, v.w, a.w);
       }
     }
@@ -524,33 +715,35 @@ decode_attention_kernel(__nv_bfloat16* __restrict__ out, float* __restrict__ par
 int attention_merge_bf16(void* out, const float* part_acc, const float* part_ml, int tokens, int out_stride,
                          int nq, int d, int splits, const int* items, void* stream);
 
-template <int D, int KP>
-int launch_decode(void* out, float* part_acc, float* part_ml, const void* q, const void* cache,
+template <int D, int KP, int RING>
+int launch_decode(const CUtensorMap& map_kv, int* status, void* out, float* part_acc, float* part_ml, const void* q, const void* cache,
                   const int* block_table, const int* items, const int* tok_req, const int* positions, int n_items,
                   int q_stride, int out_stride, int bt_stride, int nq, int nkv, int page_size, float scale,
                   int window, int splits, int num_pages, int* counters, void* stream, int fused,
-                  const float* inv_freq, const int* slots) {
-  using Cfg = DecodeCfg<D, KP>;
+                  const float* inv_freq, const int* slots, int per_head) {
+  using Cfg = DecodeCfg<D, KP, RING>;
+  constexpr int kSmem = Cfg::kSmem + Cfg::kAlign;
   static SmemRaised raised = {};                         // level 1: the ring; 2: the ring and the rows a cluster exchanges
-  if (int rc = raise_shared_memory("decode_attention", decode_attention_kernel<D, KP>, Cfg::kSmem, raised, 1)) return rc;
+  if (int rc = raise_shared_memory("decode_attention", decode_attention_kernel<D, KP, RING>, kSmem, raised, 1)) return rc;
   int page_shift = -1;                                   // log2(page_size) when it is a power of two
   for (int b = 0; b < 20; ++b) if ((1 << b) == page_size) page_shift = b;
-  const long long blocks = (long long)n_items * nkv * splits;
+  const long long blocks = per_head ? (long long)nkv * per_head : (long long)n_items * nkv * splits;
   PTL_REQUIRE(blocks <= 0x7fffffffLL, "decode_attention: too many blocks");
   // a cluster per (token, kv head) when its splits fit one and the rows they exchange are small
   const int G = nq / nkv;
+  if ((long long)G * splits > Cfg::kMaxSums) counters = nullptr;
   const size_t recv_bytes = (size_t)splits * kDecWarps * ((G + splits - 1) / splits) * (D + 2) * sizeof(float);
-  const bool cluster = KP == 2 && splits >= 2 && splits <= 8 && recv_bytes <= 16 * 1024;
+  const bool cluster = (RING || KP == 2) && !per_head && splits >= 2 && splits <= 8 && n_items * nkv * splits <= 296 && recv_bytes <= 16 * 1024;
   if (cluster)
-    if (int rc = raise_shared_memory("decode_attention", decode_attention_kernel<D, KP>, Cfg::kSmem + 16 * 1024, raised, 2)) return rc;
-  int rc = launch_kernel_cluster("decode_attention", decode_attention_kernel<D, KP>, dim3((unsigned)blocks), dim3(kDecWarps * 32),
-                                 Cfg::kSmem + (cluster ? recv_bytes : 0), as_stream(stream), cluster ? splits : 1,
+    if (int rc = raise_shared_memory("decode_attention", decode_attention_kernel<D, KP, RING>, kSmem + 16 * 1024, raised, 2)) return rc;
+  int rc = launch_kernel_cluster("decode_attention", decode_attention_kernel<D, KP, RING>, dim3((unsigned)blocks), dim3(kDecWarps * 32),
+                                 kSmem + (cluster ? recv_bytes : 0), as_stream(stream), cluster ? splits : 1, map_kv,
                                  (__nv_bfloat16*)out, part_acc, part_ml, (const __nv_bfloat16*)q,
                                  (const __nv_bfloat16*)cache, block_table, items, tok_req, positions, q_stride, out_stride, bt_stride,
                                  nq, nkv, page_size, scale * 1.4426950408889634f, window, splits, num_pages, page_shift, counters,
-                                 cluster ? 1 : 0, fused, inv_freq, slots, timeline_slot());
+                                 cluster ? 1 : 0, fused, inv_freq, slots, timeline_slot(), n_items, per_head, status);
   if (rc) return rc;
-  if (cluster) return 0;
+  if (cluster || per_head) return 0;
   if (splits > 1 && counters == nullptr)
     rc = attention_merge_bf16(out, part_acc, part_ml, n_items, out_stride, nq, D, splits, items, stream);
   return rc;
@@ -564,7 +757,8 @@ static int decode_attention_entry(void* out, float* part_acc, float* part_ml, co
                                   const int* block_table, const int* items, const int* tok_req, const int* positions,
                                   int n_items, int q_stride, int out_stride, int bt_stride, int nq, int nkv, int d,
                                   int page_size, float scale, int window, int splits, int num_pages, int* counters,
-                                  void* stream, int fused, const float* inv_freq, const int* slots) {
+                                  void* stream, int fused, const float* inv_freq, const int* slots, int per_head = 0,
+                                  int* status = nullptr) {
   PTL_REQUIRE(n_items >= 0 && nq > 0 && nkv > 0 && page_size > 0 && num_pages > 0, "decode_attention: bad sizes");
   PTL_REQUIRE(nq % nkv == 0, "decode_attention: %d query heads are no multiple of %d kv heads", nq, nkv);
   if ((d != 64 && d != 128) || nq / nkv > 16) return -2;
@@ -572,16 +766,36 @@ static int decode_attention_entry(void* out, float* part_acc, float* part_ml, co
   PTL_REQUIRE(counters == nullptr || splits <= 512, "decode_attention: at most 512 splits with in-kernel merging");
   PTL_REQUIRE(aligned16(q) && aligned16(cache) && q_stride % 8 == 0, "decode_attention: q and cache must be 16-byte aligned");
   PTL_REQUIRE(!fused || q_stride >= (nq + 2 * nkv) * d, "decode_attention: the fused form needs the whole q|k|v row, %d < %d", q_stride, (nq + 2 * nkv) * d);
+  PTL_REQUIRE(per_head == 0 || (per_head >= n_items && counters && part_acc && part_ml && splits == 1),
+              "decode_attention: units of equal length need scratch buffers and counters");
   if (n_items == 0) return 0;
   // the in-kernel merge keeps a maximum and a sum per (head of the group, split) in shared memory
   if ((long long)(nq / nkv) * splits > 4096) counters = nullptr;
+#define PTL_DECODE_ARGS map, status, out, part_acc, part_ml, q, cache, block_table, items, tok_req, positions, n_items, q_stride, \
+                        out_stride, bt_stride, nq, nkv, page_size, scale, window, splits, num_pages, counters, stream, \
+                        fused, inv_freq, slots, per_head
+  CUtensorMap map{};
+  if (status) {
+    if (page_size % 16 || num_pages > 0x3ffffff0 || (long long)nkv * page_size > 0x7ffffff0LL) return -2;
+    if (int rc = make_map(&map, cache, 2 * num_pages, d, 16, -nkv * page_size)) return rc;
+    // Head size 64 (alone, us): in clusters 32 keys per warp, three tiles ahead (two blocks per SM; 8 x 4,096 tokens 13.6, two tiles ahead
+    // 14.8, 16 keys 16); two ahead (three per SM) where clusters of more than two would need more than 256 of the 296 places, which
+    // the GPCs do not all offer to them (12 x 1,000 in clusters of three: 7.6 against 11.6).  Otherwise 16 keys, three ahead (four per
+    // SM; 64 x 256..2,560 in units 36.3, two ahead 38.8).  Head size 128: 16 keys, two ahead (three per SM; 32 x 128..2,304 in units 32.0, three
+    // ahead, two per SM, 38.9; clusters 8 x 4,096 23.8 and 24.2, 12 x 1,000 11.3 and 17.4); pairs that go whole three ahead (64 x 1,408: 57.9, two
+    // ahead 68.3).
+    const long long blocks = (long long)n_items * nkv * splits;
+    const bool clustered = splits > 1 && splits <= 8 && blocks <= 296;
+    if (d == 64) {
+      if (!clustered) return launch_decode<64, 1, 3>(PTL_DECODE_ARGS);
+      return splits <= 2 || blocks <= 256 ? launch_decode<64, 2, 3>(PTL_DECODE_ARGS) : launch_decode<64, 2, 2>(PTL_DECODE_ARGS);
+    }
+    return clustered || per_head ? launch_decode<128, 1, 2>(PTL_DECODE_ARGS) : launch_decode<128, 1, 3>(PTL_DECODE_ARGS);
+  }
   // few blocks in flight: 128-key tiles; many: 64-key tiles and twice the blocks per SM
   const bool wide = (long long)n_items * nkv * splits <= 296;
-#define PTL_DECODE_ARGS out, part_acc, part_ml, q, cache, block_table, items, tok_req, positions, n_items, q_stride, \
-                        out_stride, bt_stride, nq, nkv, page_size, scale, window, splits, num_pages, counters, stream, \
-                        fused, inv_freq, slots
-  if (d == 64) return wide ? launch_decode<64, 2>(PTL_DECODE_ARGS) : launch_decode<64, 1>(PTL_DECODE_ARGS);
-  return wide ? launch_decode<128, 2>(PTL_DECODE_ARGS) : launch_decode<128, 1>(PTL_DECODE_ARGS);
+  if (d == 64) return wide ? launch_decode<64, 2, 0>(PTL_DECODE_ARGS) : launch_decode<64, 1, 0>(PTL_DECODE_ARGS);
+  return wide ? launch_decode<128, 2, 0>(PTL_DECODE_ARGS) : launch_decode<128, 1, 0>(PTL_DECODE_ARGS);
 #undef PTL_DECODE_ARGS
 }
 
@@ -615,4 +829,19 @@ PTL_EXPORT int ptl_decode_attention_rope_bf16(void* out, float* part_acc, float*
   return ptl::decode_attention_entry(out, part_acc, part_ml, qkv, cache, block_table, items, tok_req, positions, n_items,
                                      q_stride, out_stride, bt_stride, nq, nkv, d, page_size, scale, window, splits,
                                      num_pages, counters, stream, 1, inv_freq, slots);
+}
+
+// Either form (fused != 0: as ptl_decode_attention_rope_bf16) for pages of whole sixteens of positions, fetched by TMA; -2 for
+// others.  per_head > 0, at least n_items: the step's keys dealt out in at most that many units per kv head (splits is 1,
+// part_acc [nkv * per_head][nq / nkv][d], part_ml [...][2]).  *status: raised when a wait for a copy gave up.
+PTL_EXPORT int ptl_decode_attention_pages_bf16(void* out, float* part_acc, float* part_ml, const void* q, void* cache,
+                                               const int* block_table, const int* items, const int* tok_req,
+                                               const int* positions, int n_items, int q_stride, int out_stride, int bt_stride,
+                                               int nq, int nkv, int d, int page_size, float scale, int window, int splits, int per_head,
+                                               int num_pages, int* counters, int fused, const float* inv_freq, const int* slots,
+                                               int* status, void* stream) {
+  PTL_REQUIRE(status != nullptr, "decode_attention: needs a status word");
+  return ptl::decode_attention_entry(out, part_acc, part_ml, q, cache, block_table, items, tok_req, positions, n_items,
+                                     q_stride, out_stride, bt_stride, nq, nkv, d, page_size, scale, window, splits, num_pages, counters,
+                                     stream, fused, inv_freq, slots, per_head, status);
 }

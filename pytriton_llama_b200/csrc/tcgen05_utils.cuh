@@ -53,6 +53,10 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");
 }
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
+               ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z) : "memory");
+}
 // Adds a tile of float32 in shared memory (rows of 128 bytes, 128-byte swizzle) into global memory:
 // the sum is formed in L2, the block reads nothing.  Issue, commit, and the two waits of the
 // issuing thread: for the tile to have been read out of shared memory, and for everything to be done.
@@ -193,7 +197,7 @@ inline EncodeTiledFn encode_fn() {
 
 // Tensor maps already encoded by this process: weights are asked for again every step.
 struct MapKey {
-  const void* base; int rows, K, box, ld;      // ld: 0 for bfloat16 matrices (rows are K apart), else the float32 row distance
+  const void* base; int rows, K, box, ld;      // ld: 0 for bfloat16 matrices (rows are K apart), the float32 row distance, or planes (below)
   bool operator==(const MapKey& o) const { return base == o.base && rows == o.rows && K == o.K && box == o.box && ld == o.ld; }
 };
 struct MapKeyHash {
@@ -206,9 +210,11 @@ struct MapKeyHash {
 };
 
 inline int encode_map_f32(CUtensorMap* map, const void* base, int rows, int cols, int ld, int box_rows);
+inline int encode_map_planes(CUtensorMap* map, const void* base, int planes, int rows, int K, int box_rows);
 
 // A [rows, K] bfloat16 matrix, K contiguous, fetched in boxes of 64 (K) x box_rows with the 128-byte
-// swizzle; with ld > 0 a [rows, K] float32 matrix whose rows are ld apart, in boxes of 32 x box_rows.
+// swizzle; with ld > 0 a [rows, K] float32 matrix whose rows are ld apart, in boxes of 32 x box_rows; with ld < 0 `rows` planes
+// of [-ld, K] bfloat16, in boxes of 64 x box_rows x 2 planes.
 // (A map says where a matrix lies and how it is cut, nothing about its contents: one that was
 // encoded for an address and shape serves every later matrix there.)
 inline int make_map(CUtensorMap* map, const void* base, int rows, int K, int box_rows, int ld = 0) {
@@ -220,7 +226,8 @@ inline int make_map(CUtensorMap* map, const void* base, int rows, int K, int box
     auto it = cache.find(key);
     if (it != cache.end()) { *map = it->second; return 0; }
   }
-  int rc = ld > 0 ? encode_map_f32(map, base, rows, K, ld, box_rows) : encode_map(map, base, rows, K, box_rows);
+  int rc = ld > 0 ? encode_map_f32(map, base, rows, K, ld, box_rows)
+           : ld < 0 ? encode_map_planes(map, base, rows, -ld, K, box_rows) : encode_map(map, base, rows, K, box_rows);
   if (rc) return rc;
   std::lock_guard<std::mutex> g(lock);
   if (cache.size() > 8192) cache.clear();
@@ -258,5 +265,19 @@ inline int encode_map(CUtensorMap* map, const void* base, int rows, int K, int b
   return 0;
 }
 
+// Planes [planes][rows][K] of bfloat16, fetched in boxes of 64 (K) x box_rows of two neighbouring planes.
+inline int encode_map_planes(CUtensorMap* map, const void* base, int planes, int rows, int K, int box_rows) {
+  EncodeTiledFn fn = encode_fn();
+  PTL_REQUIRE(fn != nullptr, "tensor map: the driver has no cuTensorMapEncodeTiled");
+  cuuint64_t dims[3] = {(cuuint64_t)K, (cuuint64_t)rows, (cuuint64_t)planes};
+  cuuint64_t strides[2] = {(cuuint64_t)K * 2, (cuuint64_t)rows * K * 2};
+  cuuint32_t box[3] = {64u, (cuuint32_t)box_rows, 2u};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  PTL_REQUIRE(r == CUDA_SUCCESS, "tensor map: cuTensorMapEncodeTiled (planes) failed with %d (planes=%d rows=%d K=%d box=%d)", (int)r, planes, rows, K, box_rows);
+  return 0;
+}
 
 }  // namespace ptl

@@ -156,6 +156,10 @@ def load_library() -> ctypes.CDLL:
                                                    _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_int, _c_int, _ptr,
                                                    _ptr, _ptr, _ptr]
     lib.ptl_decode_attention_rope_bf16.restype = _c_int
+    lib.ptl_decode_attention_pages_bf16.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int,
+                                                    _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_int, _c_int, _c_int, _ptr, _c_int,
+                                                    _ptr, _ptr, _ptr, _ptr]
+    lib.ptl_decode_attention_pages_bf16.restype = _c_int
     lib.ptl_prefill_attention_bf16.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                                _c_int, _c_int, _c_f, _c_int, _c_int, _ptr]
     lib.ptl_prefill_attention_bf16.restype = _c_int
@@ -969,7 +973,15 @@ class CudaOps:
     DECODE_BLOCKS = int(os.environ.get("PTL_DECODE_BLOCKS", "592"))    # blocks the decode attention aims for: the four per SM that fit at once
     DECODE_KEYS_PER_WIDE_BLOCK = int(os.environ.get("PTL_DECODE_KEYS_PER_WIDE_BLOCK", "1024"))   # keys a block of the two-per-SM form walks at most
 
+    DECODE_UNITS = {64: 592, 128: 444}      # the blocks of the decode attention by TMA that fit at once, by head size
+
     _DECODE_COUNTERS = 1 << 16
+
+    def _decode_tickets(self) -> torch.Tensor:
+        """One int per (token row, kv head), zero between calls."""
+        if getattr(self, "_decode_counters", None) is None:
+            self._decode_counters = torch.zeros(self._DECODE_COUNTERS, dtype=torch.int32, device=self.device)
+        return self._decode_counters
 
     def _attention_tensor_cores(self, out, q, cache, block_table, tok_req, positions, nq, nkv, d, page_size, scale,
                                 window, hints, rope=None) -> None:
@@ -997,16 +1009,48 @@ class CudaOps:
             # holds (``attn_splits`` of the step context is the CUDA-core kernel's).  A caller may fix
             # it (``decode_splits``) and leave the counters out (``decode_counters`` False) to pin one
             # of the three ways of merging.
-            splits = int(getattr(hints, "decode_splits", 0) or splits)
+            forced = int(getattr(hints, "decode_splits", 0))
+            group = nq // nkv
+            tickets = q.shape[0] * nkv <= self._DECODE_COUNTERS and getattr(hints, "decode_counters", True)
+            # Pages of whole sixteens are fetched by TMA.  Up to 148 pairs go in clusters where those fill three quarters of their 296
+            # blocks or the contexts are short; more pairs in units of equal length, as many as fit at once (a batch of unequal
+            # contexts otherwise ends with the long ones' blocks alone: 64 requests of 256 to 2,560 tokens, heads of 64, 45 us whole by
+            # cp.async, 36 in units; all of 1,408: 30.5 and 31.8); pairs beyond 7/8 of what fits at once go whole.  Few pairs of long
+            # contexts go in units too with heads of 128 (one of 131,072 tokens: 92 us, 104 by splits); with heads of 64 the
+            # splits below stay (51 us against 55).
+            parts = max(1, min(8, 296 // pairs, -(-longest // 128)))
+            few_and_long = longest > self.DECODE_KEYS_PER_WIDE_BLOCK * parts and pairs * parts < 222 and pairs <= 148
+            if not forced and tickets and page_size % 16 == 0 and not (d == 64 and few_and_long):
+                per_head = 0
+                if pairs > 148 or few_and_long:
+                    parts = 1
+                    if few_and_long or pairs <= self.DECODE_UNITS[d] * 7 // 8:
+                        per_head = max(self.DECODE_UNITS[d] // nkv, n_decode)
+                part_acc = part_ml = None
+                if per_head:
+                    part_acc = self.empty((nkv * per_head, group, d), torch.float32)
+                    part_ml = self.empty((nkv * per_head, group, 2), torch.float32)
+                elif parts > 1:
+                    part_acc = self.empty((q.shape[0], nq, parts, d), torch.float32)
+                    part_ml = self.empty((q.shape[0], nq, parts, 2), torch.float32)
+                rc = self.lib.ptl_decode_attention_pages_bf16(
+                    _p(out), _p(part_acc), _p(part_ml), _p(q), _p(cache), _p(block_table), None if dec.in_order else _p(dec.tensor),
+                    _p(tok_req), _p(positions), n_decode, q.shape[1], nq * d, block_table.shape[1], nq, nkv, d, page_size, float(scale),
+                    int(window), parts, per_head, num_pages, _p(self._decode_tickets()), int(rope is not None),
+                    _p(rope[0]) if rope is not None else None, _p(rope[1]) if rope is not None else None, _p(self._tc_status_word()),
+                    stream)
+                if rc != -2:
+                    self._check(rc)
+                    n_decode = 0
+        if n_decode:
+            splits = forced or splits
             part_acc = part_ml = counters = None
             if splits > 1:
                 splits = min(splits, 512)
                 part_acc = self.empty((q.shape[0], nq, splits, d), torch.float32)
                 part_ml = self.empty((q.shape[0], nq, splits, 2), torch.float32)
                 if q.shape[0] * nkv <= self._DECODE_COUNTERS and getattr(hints, "decode_counters", True):
-                    if getattr(self, "_decode_counters", None) is None:
-                        self._decode_counters = torch.zeros(self._DECODE_COUNTERS, dtype=torch.int32, device=self.device)
-                    counters = self._decode_counters        # the last block of a token's splits merges them in the kernel
+                    counters = self._decode_tickets()        # the last block of a token's splits merges them in the kernel
             items = None if dec.in_order else _p(dec.tensor)
             if rope is not None:
                 rc = self.lib.ptl_decode_attention_rope_bf16(
@@ -1018,7 +1062,6 @@ class CudaOps:
                     _p(out), _p(part_acc), _p(part_ml), _p(q), _p(cache), _p(block_table), items, _p(tok_req),
                     _p(positions), n_decode, q.shape[1], nq * d, block_table.shape[1], nq, nkv, d, page_size,
                     float(scale), int(window), splits, num_pages, _p(counters), stream)
-            group = nq // nkv
             in_cluster = (n_decode * nkv * splits <= 296 and 2 <= splits <= 8
                           and splits * 4 * -(-group // splits) * (d + 2) * 4 <= 16 * 1024)     # as launch_decode decides
             self._check(rc, kernels=2 if splits > 1 and counters is None and not in_cluster else 1)

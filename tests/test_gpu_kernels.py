@@ -441,6 +441,39 @@ def test_decode_attention_padding_rows_named_several_times_leave_the_counters_cl
     close(out, ref, "bfloat16", "row 20 as a real token", scale=4.0)
 
 
+@pytest.mark.parametrize("nq, nkv, d, page, window, n, contexts", [
+    (32, 8, 64, 16, 0, 30, [1, 64, 65, 4000, 63, 128, 2, 700]), (24, 8, 128, 16, 0, 24, [2300, 1, 129, 64]),       # units
+    (20, 20, 64, 8, 100, 12, [50, 900, 101, 100]), (16, 4, 128, 32, 0, 44, [5, 5, 5, 3000]), (16, 1, 64, 16, 0, 300, [20, 33, 700]),
+    (4, 1, 128, 16, 0, 4, [30000, 9000, 17, 1]),                                                                   # few and long: units
+    (32, 8, 64, 16, 0, 6, [1, 127, 128, 129, 900, 16]), (24, 8, 128, 48, 70, 4, [15, 1000, 69, 71]),               # clusters
+    (8, 8, 64, 16, 0, 66, [1, 17, 64, 300]), (24, 8, 128, 16, 33, 60, [16, 32, 33, 400])])                         # whole pairs
+def test_decode_attention_by_pages_of_sixteen(ops, nq, nkv, d, page, window, n, contexts):
+    """Contexts of very different lengths in units of equal length, in clusters and whole, rows that belong to no request, one of
+    them named by several items, no numbers in the slots behind every context: against the plain operator as the other ways of
+    splitting are, twice (the tickets come back)."""
+    ctx = [contexts[i % len(contexts)] for i in range(n)]
+    pages = sum(-(-c // page) for c in ctx) + 3
+    bt = _random_paging(n, ctx, page, pages, seed=d + page)
+    cache = rnd((pages, 2, nkv, page, d), torch.bfloat16, 61)
+    q = rnd((n, nq * d), torch.bfloat16, 62, 2.0)
+    positions, req, scale = torch.tensor([c - 1 for c in ctx]).int(), torch.arange(n).int(), 1 / math.sqrt(d)
+    ref = REF.paged_attention(q, cache, bt, req, positions, nq, nkv, d, page, scale, window=window)
+    req[2], req[n - 1] = -1, -1
+    hints = _hints([1] * n, ctx)
+    hints.work["decode_items"] = _work(torch.tensor(list(range(n)) + [n - 1] * 5, dtype=torch.int32).cuda(), n + 5)
+    real = req >= 0
+    for r, c in enumerate(ctx):
+        if c % page:
+            cache[bt[r, (c - 1) // page], :, :, c % page:] = float("nan")
+    for _ in range(2):
+        launches = ops.launches
+        out = ops.paged_attention(q.cuda(), cache.cuda(), bt.cuda(), req.cuda(), positions.cuda(), nq, nkv, d, page, scale, window=window,
+                                  hints=hints)
+        assert ops.launches - launches == 1
+        close(out[real], ref[real], "bfloat16", "equal units", scale=4.0)
+        assert not out[~real].any() and int(ops._decode_counters.abs().sum()) == 0
+
+
 @pytest.mark.parametrize("d, page, window", [(64, 16, 0), (128, 16, 0), (128, 32, 600), (64, 64, 600), (128, 8, 0)])
 def test_tensor_core_attention_over_a_long_prompt(ops, d, page, window):
     """A 1,300-token portion after 700 cached tokens: dozens of key tiles per query tile, so that the
