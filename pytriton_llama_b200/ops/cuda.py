@@ -1014,17 +1014,19 @@ class CudaOps:
             tickets = q.shape[0] * nkv <= self._DECODE_COUNTERS and getattr(hints, "decode_counters", True)
             # Pages of whole sixteens are fetched by TMA.  Up to 148 pairs go in clusters where those fill three quarters of their 296
             # blocks or the contexts are short; more pairs in units of equal length, as many as fit at once (a batch of unequal
-            # contexts otherwise ends with the long ones' blocks alone: 64 requests of 256 to 2,560 tokens, heads of 64, 45 us whole by
-            # cp.async, 36 in units; all of 1,408: 30.5 and 31.8); pairs beyond 7/8 of what fits at once go whole.  Few pairs of long
-            # contexts go in units too with heads of 128 (one of 131,072 tokens: 92 us, 104 by splits); with heads of 64 the
-            # splits below stay (51 us against 55).
+            # contexts otherwise ends with the long ones' blocks alone: a step of 64 requests of 256 to 2,560 tokens, heads of 64,
+            # 1,742 us whole by cp.async, 1,625 in units; all of 1,408: 1,516 and 1,550); pairs beyond 7/8 of what fits at once go
+            # whole with heads of 128 (200 requests of 64 to 1,024: 72 us, 98 by cp.async).  Few pairs of long contexts go in units
+            # too with heads of 128 (one of 131,072 tokens: 92 us, 104 by splits).  With heads of 64 these two keep the
+            # cp.async form (a step of 100 requests of 500: 2,855 us and 2,881; one context of 131,072: 51 us and 55).
             parts = max(1, min(8, 296 // pairs, -(-longest // 128)))
             few_and_long = longest > self.DECODE_KEYS_PER_WIDE_BLOCK * parts and pairs * parts < 222 and pairs <= 148
-            if not forced and tickets and page_size % 16 == 0 and not (d == 64 and few_and_long):
+            whole = pairs > 148 and pairs > self.DECODE_UNITS[d] * 7 // 8
+            if not forced and tickets and page_size % 16 == 0 and not (d == 64 and (few_and_long or whole)):
                 per_head = 0
                 if pairs > 148 or few_and_long:
                     parts = 1
-                    if few_and_long or pairs <= self.DECODE_UNITS[d] * 7 // 8:
+                    if not whole:
                         per_head = max(self.DECODE_UNITS[d] // nkv, n_decode)
                 part_acc = part_ml = None
                 if per_head:
