@@ -450,7 +450,8 @@ sample_draw_kernel(int* __restrict__ tokens, const SampleLevelArgs a, const int*
 // cluster through distributed shared memory (a block adds up 128 buckets of all eight histograms and hands the sums to all).
 // The masses, their integer sums and with them the tokens are those of the launches above, one by one.  With `logprob` the
 // log softmax of the unscaled logits at the chosen token as well, the sum of exponentials taken against the row's maximum.
-// Bound by its nine cluster barriers and the scans between them.  Eight rows of 128,256 at temperature 0.6 and top-p 0.9, with
+// Bound by its nine cluster barriers (the start, the maxima, two a level, the kept masses; three in a greedy row) and the scans
+// between them.  Eight rows of 128,256 at temperature 0.6 and top-p 0.9, with
 // the host's part of the call: 79 us as several launches, 44 us as this one (the kernel alone 30).
 constexpr int kScBlocks = 8, kScThreads = 1024, kScMaxPerThread = 16;
 
@@ -482,6 +483,7 @@ sample_cluster_kernel(int* __restrict__ tokens, float* __restrict__ logprob, con
   __shared__ int redi[33];
   __shared__ int s_bucket;
   __shared__ unsigned long long s_left;
+  cluster_arrive();                                          // every block runs before a peer writes into it
   pdl_wait();
   pdl_launch_dependents();
   const int row = blockIdx.x / kScBlocks, rank = blockIdx.x % kScBlocks, tid = threadIdx.x, lane = tid & 31;
@@ -505,6 +507,7 @@ sample_cluster_kernel(int* __restrict__ tokens, float* __restrict__ logprob, con
   for (int j = 0; j < VPT; ++j)
     if (first + j < vocab && (e[j] > mx || (e[j] == mx && first + j < at))) { mx = e[j]; at = first + j; }
   block_argmax(mx, at, red, redi);
+  cluster_wait();
   if (tid < kScBlocks) {
     st_peer_u32(map_to_peer((uint32_t)__cvta_generic_to_shared(s_max + rank), tid), __float_as_uint(mx));
     st_peer_u32(map_to_peer((uint32_t)__cvta_generic_to_shared(s_idx + rank), tid), (unsigned)at);

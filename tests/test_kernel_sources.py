@@ -1,0 +1,37 @@
+"""Orders inside kernels that a run cannot show (a missing wait mostly goes unpunished): read from the sources."""
+import re
+
+import pytest
+
+from conftest import ROOT
+
+SOURCES = sorted((ROOT / "pytriton_llama_b200" / "csrc").glob("*.cu*"))
+
+
+def _kernels(path):
+    """(name, body) of every __global__ function of a source, comments left out."""
+    text = re.sub(r"//[^\n]*", "", path.read_text())
+    for m in re.finditer(r"__global__", text):
+        open_at = text.index("{", m.end())
+        depth, at = 1, open_at + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[at], 0)
+            at += 1
+        names = [n for n in re.findall(r"(\w+)\s*\(", text[m.end():open_at]) if n != "__launch_bounds__"]
+        yield names[0], text[open_at:at]
+
+
+KERNELS = [(path.name, name, body) for path in SOURCES for name, body in _kernels(path)]
+PEER_ACCESS = re.compile(r"\b(?:st_peer_\w+|ld_peer_\w+|mbar_arrive_cluster|tma_load_2d_pair)\s*\(")
+
+
+@pytest.mark.parametrize("source,name,body", [k for k in KERNELS if PEER_ACCESS.search(k[2])], ids=lambda v: v if len(v) < 60 else "")
+def test_peers_run_before_their_shared_memory_is_touched(source, name, body):
+    """The shared memory of another block of a cluster may be used only once that block is known to run: a cluster barrier comes first."""
+    waits = [m.start() for m in re.finditer(r"\bcluster_(?:wait|meet)\s*\(", body)]
+    assert waits and waits[0] < PEER_ACCESS.search(body).start(), f"{source}: {name}"
+
+
+def test_the_kernels_with_clusters_are_found():
+    found = {name for _, name, body in KERNELS if PEER_ACCESS.search(body)}
+    assert {"decode_attention_kernel", "gemm_tc_kernel", "sample_cluster_kernel", "token_side_cluster_kernel"} <= found
