@@ -153,7 +153,8 @@ constexpr int kSampleBatch = 8;                          // loads a thread has i
 constexpr int kSampleWorkPerRow = 3 * kSampleBuckets + 64;   // 64-bit words of `work` per row: three histograms, 32 kept masses, the cut
 constexpr float kSampleFixedPoint = 1099511627776.f;     // 2^40
 
-__device__ __forceinline__ unsigned long long mass_of(float e) { return __float2ull_rz(e * kSampleFixedPoint); }
+// (A NaN has no mass: converted, it would be 2^63, and the sums of a row with two of them would wrap.)
+__device__ __forceinline__ unsigned long long mass_of(float e) { return __float2ull_rz(fmaxf(e, 0.f) * kSampleFixedPoint); }
 
 __device__ __forceinline__ unsigned long long warp_scan_u64(unsigned long long v, int lane) {     // inclusive
 #pragma unroll

@@ -658,6 +658,23 @@ def test_sampling_in_one_launch_gives_the_tokens_of_the_several(ops, rows, vocab
     assert torch.equal(ops.sample_tokens(logits, None, None, None, logprobs=True)[0], ops.sample(logits, None, None, None))
 
 
+@pytest.mark.parametrize("vocab", [37, 32769, 131073])
+def test_sampling_gives_no_mass_to_logits_that_are_no_numbers(ops, vocab):
+    """Rows with several NaNs, far apart and side by side, and rows with infinities: one token, the same from both kernels, and
+    never a NaN's; an infinite logit is the only token with mass, the first of several."""
+    g = torch.Generator().manual_seed(vocab)
+    logits = torch.randn(12, vocab, generator=g)
+    logits[:8, ::5] = float("nan")
+    logits[:4, 1:4] = float("nan")
+    logits[8:, vocab // 2] = logits[10:, vocab - 2] = float("inf")
+    t, p, u = (x.cuda() for x in (torch.full((12,), 0.8), torch.linspace(0.3, 1.0, 12), torch.rand(12, generator=g)))
+    want = ops.sample(logits.cuda(), t, p, u)
+    for _ in range(3):
+        assert torch.equal(ops.sample_tokens(logits.cuda(), t, p, u, logprobs=True)[0], want)
+    chosen = logits.gather(1, want.cpu().long()[:, None])[:, 0]
+    assert not chosen.isnan().any() and want[8:].tolist() == [vocab // 2] * 4
+
+
 def test_sampling_follows_the_distribution(ops):
     """Many draws with different uniform numbers reproduce the filtered probabilities."""
     vocab, n = 50, 4000
