@@ -21,16 +21,40 @@ constexpr int kDcSysLd = kDcTokens + 4;
 
 __device__ __forceinline__ float dc_softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
-// Which request a chunk of the step belongs to: (request, first row, rows), request -1 behind the last one; chunks of a
-// request are numbered one after the other, requests in order.
-__device__ __forceinline__ int3 dc_locate(const int* __restrict__ q_start, int requests, int chunk) {
-  for (int r = 0; r < requests; ++r) {
-    const int lo = q_start[r], n = q_start[r + 1] - lo;
-    const int chunks = n > 0 ? (n + kDcTokens - 1) / kDcTokens : 0;
-    if (chunk < chunks) return make_int3(r, lo + chunk * kDcTokens, min(kDcTokens, n - chunk * kDcTokens));
-    chunk -= chunks;
+// Chunks of a request that brings n tokens: none up to `walk_max` tokens, which gated_delta_rule_kernel walks.  The lengths
+// are read on the device, so a captured step decides by those that it is replayed with, and a request's path by its own alone.
+__device__ __forceinline__ int dc_chunks(int n, int walk_max) { return n > walk_max ? (n + kDcTokens - 1) / kDcTokens : 0; }
+
+// A portion in chunks: its request, first row, tokens, and the number of its first chunk among the step's; request -1: there is none.
+struct DcPortion { int r, lo, n, chunk0; };
+
+// The portion that chunk `index` of the step belongs to or, BY_PORTION, the portion of that number (requests in order, chunks
+// of a request one after the other).  Every warp works it out, 32 requests at a time.
+template <bool BY_PORTION>
+__device__ __forceinline__ DcPortion dc_locate(const int* __restrict__ q_start, int requests, int walk_max, int index) {
+  const int lane = threadIdx.x & 31;
+  int chunks_before = 0, portions_before = 0;
+  for (int r0 = 0; r0 < requests; r0 += 32) {
+    const int r = r0 + lane;
+    const int lo = r < requests ? q_start[r] : 0, n = r < requests ? q_start[r + 1] - lo : 0;
+    const int chunks = dc_chunks(n, walk_max);
+    int incl = chunks;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int below = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += below;
+    }
+    const unsigned with = __ballot_sync(0xffffffffu, chunks > 0);
+    const int portion = portions_before + __popc(with & ((1u << lane) - 1u)), chunk0 = chunks_before + incl - chunks;
+    const unsigned here = __ballot_sync(0xffffffffu, chunks > 0 && (BY_PORTION ? portion == index : index >= chunk0 && index < chunk0 + chunks));
+    if (here) {
+      const int who = __ffs(here) - 1;
+      return DcPortion{r0 + who, __shfl_sync(0xffffffffu, lo, who), __shfl_sync(0xffffffffu, n, who), __shfl_sync(0xffffffffu, chunk0, who)};
+    }
+    chunks_before += __shfl_sync(0xffffffffu, incl, 31);
+    portions_before += __popc(with);
   }
-  return make_int3(-1, 0, 0);
+  return DcPortion{-1, 0, 0, 0};
 }
 
 // Floats of a (chunk, head) in the workspace: WK and the decayed queries [64][D], the decayed keys [D][64], the read-out's
@@ -47,7 +71,7 @@ template <typename T, int D>
 __global__ void __launch_bounds__(kDcThreads, 2)
 delta_chunk_prepare_kernel(float* __restrict__ work, const T* __restrict__ qkv, const float* __restrict__ ba, const float* __restrict__ rate,
                            const float* __restrict__ dt_bias, const int* __restrict__ q_start, const int* __restrict__ state_slot,
-                           int requests, int heads, int kv_heads, int dv, float unit_eps, float q_scale) {
+                           int requests, int heads, int kv_heads, int dv, float unit_eps, float q_scale, int walk_max) {
   constexpr int LD = D + 4;
   extern __shared__ __align__(16) float dp_smem[];
   float* s_k = dp_smem;                            // [64][LD], as projected: the lengths are applied to what is made of them,
@@ -55,14 +79,17 @@ delta_chunk_prepare_kernel(float* __restrict__ work, const T* __restrict__ qkv, 
   float* s_sys = s_q + kDcTokens * LD;             // [i][t]: what u_i takes off row t > i
   __shared__ double s_log[kDcTokens];
   __shared__ float s_beta[kDcTokens], s_decay[kDcTokens], s_kn[kDcTokens], s_qn[kDcTokens];
+  __shared__ int s_at[2];
   pdl_wait();
   pdl_launch_dependents();
-  const int3 at = dc_locate(q_start, requests, blockIdx.x);
-  if (at.x < 0 || state_slot[at.x] < 0) return;
-  const int h = blockIdx.y, c = h / (heads / kv_heads), n = at.z;
+  const DcPortion at = dc_locate<false>(q_start, requests, walk_max, blockIdx.x);
+  if (at.r < 0 || state_slot[at.r] < 0) return;
+  const int first = ((int)blockIdx.x - at.chunk0) * kDcTokens, row0 = at.lo + first;
+  const int h = blockIdx.y, c = h / (heads / kv_heads), n = min(kDcTokens, at.n - first);
+  if (threadIdx.x == 0) { s_at[0] = row0; s_at[1] = n; }       // (for the values' turn, which has no register to spare)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ld = 2 * kv_heads * D + heads * dv;
-  const T* rows = qkv + (size_t)at.y * ld;
+  const T* rows = qkv + (size_t)row0 * ld;
   float* wk = work + ((size_t)blockIdx.x * heads + h) * dc_floats(D, dv);
   float* qg = wk + kDcTokens * D;
   float* kdt = qg + kDcTokens * D;
@@ -98,7 +125,7 @@ delta_chunk_prepare_kernel(float* __restrict__ work, const T* __restrict__ qkv, 
       double x = 0.0;
       float beta = 0.f;
       if (t < n) {
-        const float* g = ba + (size_t)(at.y + t) * 2 * heads;
+        const float* g = ba + (size_t)(row0 + t) * 2 * heads;
         beta = 1.0f / (1.0f + expf(-g[h]));
         x = (double)(-rate[h] * dc_softplus(g[heads + h] + dt_bias[h]));
         if (x < -1e4) x = -1e4;                    // a decay of zero either way; differences of the sums stay numbers
@@ -177,9 +204,10 @@ delta_chunk_prepare_kernel(float* __restrict__ work, const T* __restrict__ qkv, 
 #pragma unroll
       for (int t = 0; t < kDcTokens; ++t) u[t] = s_beta[t] * s_decay[t] * s_kn[t] * s_k[t * LD + col];
     } else {
-      const T* v = rows + 2 * kv_heads * D + (size_t)h * dv + (col - D);
+      const T* v = qkv + (size_t)s_at[0] * ld + 2 * kv_heads * D + (size_t)h * dv + (col - D);
+      const int tokens = s_at[1];
 #pragma unroll
-      for (int t = 0; t < kDcTokens; ++t) u[t] = t < n ? s_beta[t] * to_f32(v[(size_t)t * ld]) : 0.f;
+      for (int t = 0; t < kDcTokens; ++t) u[t] = t < tokens ? s_beta[t] * to_f32(v[(size_t)t * ld]) : 0.f;
     }
 #pragma unroll
     for (int i = 0; i < kDcTokens - 1; ++i) {
@@ -251,7 +279,8 @@ __device__ __forceinline__ void dc_product(const float* __restrict__ a, const fl
 template <int D>
 __global__ void __launch_bounds__(kDcThreads, 1)
 delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, const float* __restrict__ work, const int* __restrict__ q_start,
-                        const int* __restrict__ positions, const int* __restrict__ state_slot, int heads, int dv) {
+                        const int* __restrict__ positions, const int* __restrict__ state_slot, int requests, int heads, int dv,
+                        int walk_max) {
   constexpr int LD = D + 4, RB = 2 + D / 32;
   extern __shared__ __align__(16) float dw_smem[];
   float* s_a = dw_smem;                                  // [2][WK 64 | q 64][LD]
@@ -260,11 +289,9 @@ delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, cons
   float* s_u = s_s + kDcCols * LD;                       // [8][68]
   pdl_wait();
   pdl_launch_dependents();
-  const int r = blockIdx.z, h = blockIdx.y, j0 = blockIdx.x * kDcCols;
-  const int lo = q_start[r], n = q_start[r + 1] - lo;
-  if (n <= 0 || state_slot[r] < 0) return;
-  int chunk0 = 0;
-  for (int i = 0; i < r; ++i) chunk0 += (max(q_start[i + 1] - q_start[i], 0) + kDcTokens - 1) / kDcTokens;
+  const DcPortion at = dc_locate<true>(q_start, requests, walk_max, blockIdx.z);
+  if (at.r < 0 || state_slot[at.r] < 0) return;
+  const int r = at.r, lo = at.lo, n = at.n, chunk0 = at.chunk0, h = blockIdx.y, j0 = blockIdx.x * kDcCols;
   const int chunks = (n + kDcTokens - 1) / kDcTokens;
   const int tid = threadIdx.x, lane = tid & 31, s = lane & 7, rg = (tid >> 5) * 4 + (lane >> 3);
   const size_t stride = (size_t)heads * dc_floats(D, dv);
@@ -327,31 +354,31 @@ delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, cons
 }
 
 template <typename T, int D>
-int delta_chunks(float* out, float* work, int chunks, const void* qkv, const float* ba, const float* rate, const float* dt_bias, float* state,
+int delta_chunks(float* out, float* work, int chunks, int portions, const void* qkv, const float* ba, const float* rate, const float* dt_bias, float* state,
                  const int* q_start, const int* positions, const int* state_slot, int requests, int heads, int kv_heads, int dv,
-                 float unit_eps, float q_scale, void* stream) {
+                 float unit_eps, float q_scale, int walk_max, void* stream) {
   static SmemRaised raised_p, raised_w;
   if (int rc = raise_shared_memory("delta_chunk_prepare", delta_chunk_prepare_kernel<T, D>, (int)dc_prepare_smem(D), raised_p)) return rc;
   if (int rc = raise_shared_memory("delta_chunk_walk", delta_chunk_walk_kernel<D>, (int)dc_walk_smem(D), raised_w)) return rc;
   if (int rc = launch_kernel("delta_chunk_prepare", delta_chunk_prepare_kernel<T, D>, dim3(chunks, heads), dim3(kDcThreads), dc_prepare_smem(D),
                              as_stream(stream), work, (const T*)qkv, ba, rate, dt_bias, q_start, state_slot, requests, heads, kv_heads, dv,
-                             unit_eps, q_scale))
+                             unit_eps, q_scale, walk_max))
     return rc;
-  return launch_kernel("delta_chunk_walk", delta_chunk_walk_kernel<D>, dim3(dv / kDcCols, heads, requests), dim3(kDcThreads), dc_walk_smem(D),
-                       as_stream(stream), out, state, work, q_start, positions, state_slot, heads, dv);
+  return launch_kernel("delta_chunk_walk", delta_chunk_walk_kernel<D>, dim3(dv / kDcCols, heads, portions), dim3(kDcThreads), dc_walk_smem(D),
+                       as_stream(stream), out, state, work, q_start, positions, state_slot, requests, heads, dv, walk_max);
 }
 
 template <typename T>
-int delta_chunks_any(float* out, float* work, int chunks, const void* qkv, const float* ba, const float* rate, const float* dt_bias,
+int delta_chunks_any(float* out, float* work, int chunks, int portions, const void* qkv, const float* ba, const float* rate, const float* dt_bias,
                      float* state, const int* q_start, const int* positions, const int* state_slot, int requests, int heads, int kv_heads,
-                     int d, int dv, float unit_eps, float q_scale, void* stream) {
-  PTL_REQUIRE(requests >= 0 && requests <= 65535 && heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0 && chunks >= 0 &&
+                     int d, int dv, float unit_eps, float q_scale, int walk_max, void* stream) {
+  PTL_REQUIRE(requests >= 0 && requests <= 65535 && portions >= 0 && portions <= requests && heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0 && chunks >= 0 && walk_max >= 0 &&
                   (d == 64 || d == 128) && dv > 0 && dv % kDcCols == 0 && aligned16(work),
               "gated_delta_rule in chunks: bad sizes heads=%d kv_heads=%d d=%d (64 or 128) dv=%d", heads, kv_heads, d, dv);
-  if (requests == 0 || chunks == 0) return 0;
+  if (requests == 0 || chunks == 0 || portions == 0) return 0;
   const auto fn = d == 64 ? delta_chunks<T, 64> : delta_chunks<T, 128>;
-  return fn(out, work, chunks, qkv, ba, rate, dt_bias, state, q_start, positions, state_slot, requests, heads, kv_heads, dv, unit_eps,
-            q_scale, stream);
+  return fn(out, work, chunks, portions, qkv, ba, rate, dt_bias, state, q_start, positions, state_slot, requests, heads, kv_heads, dv, unit_eps,
+            q_scale, walk_max, stream);
 }
 
 }  // namespace ptl
@@ -359,12 +386,12 @@ int delta_chunks_any(float* out, float* work, int chunks, const void* qkv, const
 PTL_EXPORT long long ptl_delta_chunk_floats(int d, int dv) { return (long long)ptl::dc_floats(d, dv); }
 
 #define PTL_DELTA_CHUNKS(SUFFIX, TYPE)                                                                                                \
-  PTL_EXPORT int ptl_gated_delta_chunks##SUFFIX(float* out, float* work, int chunks, const void* qkv, const float* ba, const float* rate, \
+  PTL_EXPORT int ptl_gated_delta_chunks##SUFFIX(float* out, float* work, int chunks, int portions, const void* qkv, const float* ba, const float* rate, \
                                                 const float* dt_bias, float* state, const int* q_start, const int* positions,         \
                                                 const int* state_slot, int requests, int heads, int kv_heads, int d, int dv,          \
-                                                float unit_eps, float q_scale, void* stream) {                                        \
-    return ptl::delta_chunks_any<TYPE>(out, work, chunks, qkv, ba, rate, dt_bias, state, q_start, positions, state_slot, requests,    \
-                                       heads, kv_heads, d, dv, unit_eps, q_scale, stream);                                            \
+                                                float unit_eps, float q_scale, int walk_max, void* stream) {                          \
+    return ptl::delta_chunks_any<TYPE>(out, work, chunks, portions, qkv, ba, rate, dt_bias, state, q_start, positions, state_slot, requests,    \
+                                       heads, kv_heads, d, dv, unit_eps, q_scale, walk_max, stream);                                  \
   }
 PTL_DELTA_CHUNKS(_f32, float)
 PTL_DELTA_CHUNKS(_bf16, __nv_bfloat16)

@@ -421,6 +421,7 @@ scan_carry_kernel(float* __restrict__ work, float* __restrict__ state, const flo
 // scaling is folded into the walk: with kn = 1 / |k| and qn = q_scale / |q|,
 //     dot = kn * (S^T k);  u = beta (v - dot);  S <- S + k (kn u);  o = qn * (S^T q).
 // qkv rows: [q: kv_heads * d | k: kv_heads * d | v: heads * dv];  ba rows: [b: heads | a: heads] float32.
+// Requests that bring more than `walk_max` tokens are left to the kernels of delta_chunks.cu.
 // Shared memory: kDeltaBatch * (2 * 8 * RPL + 16 + 4) floats; rows of q and k are 8 * RPL floats apart, zero beyond d.
 constexpr int kDeltaBatch = 16;
 
@@ -429,7 +430,7 @@ __global__ void __launch_bounds__(128)
 gated_delta_rule_kernel(float* __restrict__ out, const T* __restrict__ qkv, const float* __restrict__ ba,
                         const float* __restrict__ rate, const float* __restrict__ dt_bias, float* __restrict__ state,
                         const int* __restrict__ q_start, const int* __restrict__ positions, const int* __restrict__ state_slot,
-                        int heads, int kv_heads, int d, int dv, float unit_eps, float q_scale) {
+                        int heads, int kv_heads, int d, int dv, float unit_eps, float q_scale, int walk_max) {
   static_assert(RPL % 2 == 0, "a lane holds pairs of rows");
   constexpr int DS = 8 * RPL;                       // floats between rows of q and k in shared memory
   constexpr int HP = RPL / 2;                       // row pairs of a lane
@@ -445,7 +446,7 @@ gated_delta_rule_kernel(float* __restrict__ out, const T* __restrict__ qkv, cons
   pdl_launch_dependents();
   const int r = blockIdx.z, h = blockIdx.y;
   const int lo = q_start[r], hi = q_start[r + 1];
-  if (hi <= lo || state_slot[r] < 0) return;
+  if (hi <= lo || hi - lo > walk_max || state_slot[r] < 0) return;      // (longer portions: delta_chunks.cu)
   const int sub = threadIdx.x & 7, grp = threadIdx.x >> 3;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j0 = blockIdx.x * 16;
@@ -819,7 +820,7 @@ int scan_segments(void* out, float* work, int segments, const void* xc, const fl
 template <typename T>
 int gated_delta_rule(float* out, const void* qkv, const float* ba, const float* rate, const float* dt_bias, float* state,
                      const int* q_start, const int* positions, const int* state_slot, int requests, int heads, int kv_heads, int d,
-                     int dv, float unit_eps, float q_scale, void* stream) {
+                     int dv, float unit_eps, float q_scale, int walk_max, void* stream) {
   PTL_REQUIRE(requests >= 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && d > 0 && d <= 256 && dv > 0,
               "gated_delta_rule: bad sizes heads=%d kv_heads=%d d=%d (at most 256) dv=%d", heads, kv_heads, d, dv);
   PTL_REQUIRE(requests <= 65535 && heads <= 65535, "gated_delta_rule: at most 65535 requests and heads");
@@ -827,7 +828,7 @@ int gated_delta_rule(float* out, const void* qkv, const float* ba, const float* 
   const dim3 grid((dv + 15) / 16, heads, requests), block(128);
 #define PTL_DELTA(RPL) return launch_kernel("gated_delta_rule", gated_delta_rule_kernel<T, RPL>, grid, block, \
     (size_t)kDeltaBatch * (2 * 8 * RPL + 16 + 4) * sizeof(float) /* at most 34 KB */, as_stream(stream), \
-    out, (const T*)qkv, ba, rate, dt_bias, state, q_start, positions, state_slot, heads, kv_heads, d, dv, unit_eps, q_scale)
+    out, (const T*)qkv, ba, rate, dt_bias, state, q_start, positions, state_slot, heads, kv_heads, d, dv, unit_eps, q_scale, walk_max)
   const int per_lane = (d + 7) / 8;
   if (per_lane <= 2) PTL_DELTA(2);
   if (per_lane <= 4) PTL_DELTA(4);
@@ -889,9 +890,9 @@ int gated_head_norm(void* out, int out_ld, int column, const float* o, const flo
   PTL_EXPORT int ptl_gated_delta_rule##SUFFIX(float* out, const void* qkv, const float* ba, const float* rate,                     \
                                               const float* dt_bias, float* state, const int* q_start, const int* positions,       \
                                               const int* state_slot, int requests, int heads, int kv_heads, int d, int dv,        \
-                                              float unit_eps, float q_scale, void* stream) {                                      \
+                                              float unit_eps, float q_scale, int walk_max, void* stream) {                        \
     return ptl::gated_delta_rule<TYPE>(out, qkv, ba, rate, dt_bias, state, q_start, positions, state_slot, requests, heads,        \
-                                       kv_heads, d, dv, unit_eps, q_scale, stream);                                               \
+                                       kv_heads, d, dv, unit_eps, q_scale, walk_max, stream);                                               \
   }                                                                                                                               \
   PTL_EXPORT int ptl_gated_head_norm##SUFFIX(void* out, int out_ld, int column, const float* o, const float* w, float eps,         \
                                              const void* gate, int gate_ld, int gate_column, int tokens, int heads, int dv,        \

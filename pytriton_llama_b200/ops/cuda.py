@@ -41,9 +41,9 @@ _SIGNATURES = {
     "ptl_scan_segments": [_ptr, _ptr, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr,
                           _ptr, _c_int, _ptr],
     "ptl_gated_delta_rule": [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f,
-                             _c_f, _ptr],
-    "ptl_gated_delta_chunks": [_ptr, _ptr, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
-                               _c_f, _c_f, _ptr],
+                             _c_f, _c_int, _ptr],
+    "ptl_gated_delta_chunks": [_ptr, _ptr, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
+                               _c_f, _c_f, _c_int, _ptr],
     "ptl_gated_head_norm": [_ptr, _c_int, _c_int, _ptr, _ptr, _c_f, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_int,
                             _ptr],
     "ptl_kv_write_normed": [_ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_f, _ptr],
@@ -1219,9 +1219,20 @@ class CudaOps:
                        _p(state), _p(ctx.q_start), _p(ctx.positions), _p(ctx.state_slot), ctx.num_requests, self._stream()))
         return out
 
-    # The longest portion of a step for which the gated delta rule walks token by token: up to
-    # one chunk (2,048 tokens of heads of 128: 738 us by the walk, 206 in chunks; 64: 23 by the walk, one chunk costs as much).
+    # The longest portion that the gated delta rule walks token by token: up to one chunk (2,048 tokens of 8 heads of 128:
+    # 738 us by the walk, 206 in chunks; 64: 23 by the walk, one chunk costs as much).  Every request goes by its own length.
     DELTA_WALK_MAX_TOKENS = 64
+
+    @staticmethod
+    def _portion_paths(ctx, walk_max: int) -> Tuple[bool, int, int]:
+        """(whether portions of up to ``walk_max`` tokens may come, the most longer ones, the most pieces of 64 tokens that these
+        make).  The kernels tell portions apart by the lengths on the device; the host's say which kernels there is no use for,
+        where they are the step's own: a captured step meets others, of as many tokens as it was padded to."""
+        tokens = int(ctx.positions.shape[0])
+        if ctx.max_q_len <= walk_max:
+            return True, 0, 0
+        long = min(ctx.num_requests, tokens // (walk_max + 1))
+        return not (getattr(ctx, "host_lengths_exact", False) and min(ctx.q_lens) > walk_max), long, tokens // 64 + long
 
     def gated_delta_rule(self, qkv: torch.Tensor, ba: torch.Tensor, rate: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor,
                          ctx, H: int, G: int, d: int, dv: int, unit_eps: float, q_scale: float) -> torch.Tensor:
@@ -1234,16 +1245,18 @@ class CudaOps:
             raise KernelError("gated_delta_rule: shapes do not fit")
         T = qkv.shape[0]
         out = self.empty((T, H * dv), torch.float32)
-        if ctx.max_q_len > self.DELTA_WALK_MAX_TOKENS and d in (64, 128) and dv % 8 == 0:
-            chunks = T // 64 + ctx.num_requests          # at least the chunks of 64 tokens that the requests' portions make
+        walk_max = self.DELTA_WALK_MAX_TOKENS if d in (64, 128) and dv % 8 == 0 else 1 << 30
+        short, long, chunks = self._portion_paths(ctx, walk_max)
+        if short:
+            fn = getattr(self.lib, "ptl_gated_delta_rule" + _suffix(qkv.dtype))
+            self._check(fn(_p(out), _p(qkv), _p(ba), _p(rate), _p(dt_bias), _p(state), _p(ctx.q_start), _p(ctx.positions),
+                           _p(ctx.state_slot), ctx.num_requests, H, G, d, dv, float(unit_eps), float(q_scale), walk_max, self._stream()))
+        if long:
             work = self.empty((chunks * H, self.lib.ptl_delta_chunk_floats(d, dv)), torch.float32)
             fn = getattr(self.lib, "ptl_gated_delta_chunks" + _suffix(qkv.dtype))
-            self._check(fn(_p(out), _p(work), chunks, _p(qkv), _p(ba), _p(rate), _p(dt_bias), _p(state), _p(ctx.q_start), _p(ctx.positions),
-                           _p(ctx.state_slot), ctx.num_requests, H, G, d, dv, float(unit_eps), float(q_scale), self._stream()), kernels=2)
-            return out
-        fn = getattr(self.lib, "ptl_gated_delta_rule" + _suffix(qkv.dtype))
-        self._check(fn(_p(out), _p(qkv), _p(ba), _p(rate), _p(dt_bias), _p(state), _p(ctx.q_start), _p(ctx.positions),
-                       _p(ctx.state_slot), ctx.num_requests, H, G, d, dv, float(unit_eps), float(q_scale), self._stream()))
+            self._check(fn(_p(out), _p(work), chunks, long, _p(qkv), _p(ba), _p(rate), _p(dt_bias), _p(state), _p(ctx.q_start), _p(ctx.positions),
+                           _p(ctx.state_slot), ctx.num_requests, H, G, d, dv, float(unit_eps), float(q_scale), walk_max, self._stream()),
+                        kernels=2)
         return out
 
     def gated_head_norm(self, o: torch.Tensor, weight: torch.Tensor, eps: float, gate: torch.Tensor, gate_column: int, H: int,

@@ -151,6 +151,40 @@ def test_gated_delta_rule_in_chunks_of_64_tokens(ops, dtype, H, G, d, dv):
     assert off(got, ref) <= 1.5 * off(walked, ref) and off(dev["S"], cpu["S"]) <= 1.5 * off(wdev["S"], cpu["S"])
 
 
+def _alone_and_together(run, tensors, per_token, lens):
+    """A step of many requests, as a launched step sees it and as one captured for more tokens does, against every request's
+    own step: the same bits of results and states, since the path goes by the request's own length."""
+    starts, slots = [(7 * r) % 3 * 5 for r in range(len(lens))], list(range(len(lens)))
+    first = [sum(lens[:r]) for r in range(len(lens))]
+    for captured in (False, True):
+        dev = {k: v.cuda() for k, v in tensors.items()}
+        ctx = _ctx(lens, starts, slots, "cuda:0")
+        if captured:
+            ctx.max_q_len = sum(lens)
+        else:
+            ctx.q_lens, ctx.host_lengths_exact = lens, True
+        together = run(dev, ctx)
+        for r, n in enumerate(lens):
+            one = {k: (v[first[r]:first[r] + n] if k in per_token else v).contiguous().cuda() for k, v in tensors.items()}
+            alone = run(one, _ctx([n], [starts[r]], [r], "cuda:0"))
+            assert torch.equal(alone, together[first[r]:first[r] + n]), (captured, r, n)
+            assert torch.equal(one["state"][r], dev["state"][r]), (captured, r, n)
+
+
+COMPANY = [1] * 20 + [10, 200, 1, 64, 65, 2] + [1] * 20      # more requests than a warp has lanes, long portions among them
+
+
+@pytest.mark.parametrize("H,G,d,dv", [(2, 1, 64, 16), (3, 3, 128, 40)])
+def test_gated_delta_rule_of_a_request_does_not_depend_on_its_company(ops, H, G, d, dv):
+    g = torch.Generator().manual_seed(d)
+    T, R = sum(COMPANY), len(COMPANY)
+    tensors = {"qkv": torch.randn(T, 2 * G * d + H * dv, generator=g).bfloat16(), "ba": torch.randn(T, 2 * H, generator=g),
+               "rate": torch.exp(torch.randn(H, generator=g)), "dt_bias": torch.randn(H, generator=g),
+               "state": torch.randn(R, H, d, dv, generator=g)}
+    run = lambda t, ctx: ops.gated_delta_rule(t["qkv"], t["ba"], t["rate"], t["dt_bias"], t["state"], ctx, H, G, d, dv, 1e-6, d ** -0.5)
+    _alone_and_together(run, tensors, ("qkv", "ba"), COMPANY)
+
+
 @pytest.mark.parametrize("M,inter,K,bias", [(1, 52, 64, True), (8, 300, 1024, True), (20, 2048, 512, False), (64, 96, 2048, True),
                                             (65, 260, 64, True), (300, 1024, 512, True), (700, 130, 200, False)])
 def test_clamped_activation_in_the_product(ops, M, inter, K, bias):

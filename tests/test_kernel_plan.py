@@ -1,8 +1,11 @@
 """Host-side decisions of the kernel library that need no device: into how many parts the many-token
 product cuts its K range (the launcher's plan runs with 148 SMs when it finds no GPU)."""
 import ctypes
+import random
+from types import SimpleNamespace
 
 import pytest
+import torch
 
 
 @pytest.fixture(scope="module")
@@ -29,3 +32,23 @@ def test_parts_of_the_k_range(lib):
         assert 2 <= p <= 8, (m, n, k, p)
         assert -(-k // 64) // p >= 8 or p == 1, (m, n, k, p)      # at least 8 blocks of 64 values per part
     assert parts(300, 2048, 256) == 1                  # too short a K range to cut
+
+
+def test_pieces_of_long_portions_fit_what_a_step_provides_for():
+    """However a step's tokens are shared out, its portions beyond the walk's longest make no more portions and pieces of 64
+    tokens than the launch and its workspace are laid out for, in a captured step of more token rows too; where there can be
+    none, nothing is provided for."""
+    from pytriton_llama_b200.ops.cuda import CudaOps
+    rng = random.Random(3)
+    for _ in range(2000):
+        walk = rng.choice([64, 64, 1, 100])
+        lens = [rng.choice([1, 1, rng.randint(1, 70), 64, 65, rng.randint(1, 700)]) for _ in range(rng.randint(1, 40))]
+        rows = sum(lens) + rng.choice([0, 3, 128])
+        long = [n for n in lens if n > walk]
+        for exact in (True, False):
+            ctx = SimpleNamespace(positions=torch.empty(sum(lens) if exact else rows), num_requests=len(lens), q_lens=lens,
+                                  max_q_len=max(lens) if exact else rows, host_lengths_exact=exact)
+            short, portions, pieces = CudaOps._portion_paths(ctx, walk)
+            assert len(long) <= portions <= len(lens) and sum(-(-n // 64) for n in long) <= pieces
+            assert short or len(long) == len(lens)
+            assert not exact or ((portions > 0) == bool(long) and short == (len(long) < len(lens)))
