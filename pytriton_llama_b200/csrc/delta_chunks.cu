@@ -12,6 +12,7 @@
 // The token-by-token walk is bound by the latency of its chain, 0.36 us a token at heads of 128 x 128: 738 us for
 // 2,048 tokens, whatever the number of SMs.  Here 16 heads of that size take 88 us (prepare: the chains of the 64 x 64 systems,
 // two blocks an SM) and 118 us (walk: 32 dependent chunks of three products).  The error against 64 bits is the walk's or less.
+#include "long_portions.cuh"
 #include "mma_utils.cuh"
 
 namespace ptl {
@@ -20,42 +21,6 @@ constexpr int kDcTokens = 64, kDcThreads = 256, kDcCols = 8;
 constexpr int kDcSysLd = kDcTokens + 4;
 
 __device__ __forceinline__ float dc_softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
-
-// Chunks of a request that brings n tokens: none up to `walk_max` tokens, which gated_delta_rule_kernel walks.  The lengths
-// are read on the device, so a captured step decides by those that it is replayed with, and a request's path by its own alone.
-__device__ __forceinline__ int dc_chunks(int n, int walk_max) { return n > walk_max ? (n + kDcTokens - 1) / kDcTokens : 0; }
-
-// A portion in chunks: its request, first row, tokens, and the number of its first chunk among the step's; request -1: there is none.
-struct DcPortion { int r, lo, n, chunk0; };
-
-// The portion that chunk `index` of the step belongs to or, BY_PORTION, the portion of that number (requests in order, chunks
-// of a request one after the other).  Every warp works it out, 32 requests at a time.
-template <bool BY_PORTION>
-__device__ __forceinline__ DcPortion dc_locate(const int* __restrict__ q_start, int requests, int walk_max, int index) {
-  const int lane = threadIdx.x & 31;
-  int chunks_before = 0, portions_before = 0;
-  for (int r0 = 0; r0 < requests; r0 += 32) {
-    const int r = r0 + lane;
-    const int lo = r < requests ? q_start[r] : 0, n = r < requests ? q_start[r + 1] - lo : 0;
-    const int chunks = dc_chunks(n, walk_max);
-    int incl = chunks;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int below = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += below;
-    }
-    const unsigned with = __ballot_sync(0xffffffffu, chunks > 0);
-    const int portion = portions_before + __popc(with & ((1u << lane) - 1u)), chunk0 = chunks_before + incl - chunks;
-    const unsigned here = __ballot_sync(0xffffffffu, chunks > 0 && (BY_PORTION ? portion == index : index >= chunk0 && index < chunk0 + chunks));
-    if (here) {
-      const int who = __ffs(here) - 1;
-      return DcPortion{r0 + who, __shfl_sync(0xffffffffu, lo, who), __shfl_sync(0xffffffffu, n, who), __shfl_sync(0xffffffffu, chunk0, who)};
-    }
-    chunks_before += __shfl_sync(0xffffffffu, incl, 31);
-    portions_before += __popc(with);
-  }
-  return DcPortion{-1, 0, 0, 0};
-}
 
 // Floats of a (chunk, head) in the workspace: WK and the decayed queries [64][D], the decayed keys [D][64], the read-out's
 // weights [64][64], WV [64][dv], the chunk's decay (padded to 16 bytes).
@@ -82,9 +47,9 @@ delta_chunk_prepare_kernel(float* __restrict__ work, const T* __restrict__ qkv, 
   __shared__ int s_at[2];
   pdl_wait();
   pdl_launch_dependents();
-  const DcPortion at = dc_locate<false>(q_start, requests, walk_max, blockIdx.x);
+  const LongPortion at = locate_portion<false, kDcTokens>(q_start, requests, walk_max, blockIdx.x);
   if (at.r < 0 || state_slot[at.r] < 0) return;
-  const int first = ((int)blockIdx.x - at.chunk0) * kDcTokens, row0 = at.lo + first;
+  const int first = ((int)blockIdx.x - at.piece0) * kDcTokens, row0 = at.lo + first;
   const int h = blockIdx.y, c = h / (heads / kv_heads), n = min(kDcTokens, at.n - first);
   if (threadIdx.x == 0) { s_at[0] = row0; s_at[1] = n; }       // (for the values' turn, which has no register to spare)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -289,9 +254,9 @@ delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, cons
   float* s_u = s_s + kDcCols * LD;                       // [8][68]
   pdl_wait();
   pdl_launch_dependents();
-  const DcPortion at = dc_locate<true>(q_start, requests, walk_max, blockIdx.z);
+  const LongPortion at = locate_portion<true, kDcTokens>(q_start, requests, walk_max, blockIdx.z);
   if (at.r < 0 || state_slot[at.r] < 0) return;
-  const int r = at.r, lo = at.lo, n = at.n, chunk0 = at.chunk0, h = blockIdx.y, j0 = blockIdx.x * kDcCols;
+  const int r = at.r, lo = at.lo, n = at.n, chunk0 = at.piece0, h = blockIdx.y, j0 = blockIdx.x * kDcCols;
   const int chunks = (n + kDcTokens - 1) / kDcTokens;
   const int tid = threadIdx.x, lane = tid & 31, s = lane & 7, rg = (tid >> 5) * 4 + (lane >> 3);
   const size_t stride = (size_t)heads * dc_floats(D, dv);

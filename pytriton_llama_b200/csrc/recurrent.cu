@@ -6,6 +6,7 @@
 // tokens lie request after request: request r owns rows q_start[r] .. q_start[r + 1] - 1.
 // T is the element type of the projections' results; everything inside is float32.
 #include "common.cuh"
+#include "long_portions.cuh"
 
 namespace ptl {
 
@@ -202,6 +203,7 @@ __global__ void conv_state_kernel(float* __restrict__ state, const T* __restrict
 // The tokens come in batches of `tb`: the block first brings a batch's B | C rows, its 16 channels' x, step sizes
 // (softplus applied) and gates (silu applied) into shared memory with all threads, so that the walk, whose steps
 // depend on one another, waits for shared memory only; the batch's results leave the same way.
+// Requests that bring more than `walk_max` tokens are left to the kernels in segments below.
 // Shared memory: tb * (2 * n_state + 64) floats.
 template <typename T, int NPL>
 __global__ void __launch_bounds__(128)
@@ -209,7 +211,7 @@ selective_scan_kernel(T* __restrict__ out, const T* __restrict__ xc, const float
                       const float* __restrict__ dt_bias, const float* __restrict__ A, const T* __restrict__ bc,
                       const float* __restrict__ D, const T* __restrict__ z, int z_ld, int z_column, int inner, int n_state,
                       float* __restrict__ state, const int* __restrict__ q_start, const int* __restrict__ positions,
-                      const int* __restrict__ state_slot, int tb) {
+                      const int* __restrict__ state_slot, int tb, int walk_max) {
   extern __shared__ __align__(16) float scan_smem[];
   float* s_bc = scan_smem;                        // [tb][2 * n_state]
   float* s_x = s_bc + (size_t)tb * 2 * n_state;   // [tb][16]
@@ -220,7 +222,7 @@ selective_scan_kernel(T* __restrict__ out, const T* __restrict__ xc, const float
   pdl_launch_dependents();
   const int r = blockIdx.y;
   const int lo = q_start[r], hi = q_start[r + 1];
-  if (hi <= lo || state_slot[r] < 0) return;
+  if (hi <= lo || hi - lo > walk_max || state_slot[r] < 0) return;      // (longer portions: the segments below)
   const int sub = threadIdx.x & 7, grp = threadIdx.x >> 3;
   const int c0 = blockIdx.x * 16;
   const bool live = c0 + grp < inner;
@@ -285,7 +287,7 @@ selective_scan_kernel(T* __restrict__ out, const T* __restrict__ xc, const float
   }
 }
 
-// The same for steps with portions of many tokens and up to kScanStates states: the tokens of every request in segments of
+// The same for portions of more than `walk_max` tokens and up to kScanStates states: the tokens of such a request in segments of
 // kScanSegment.  A segment's walk from zero and the sum of its step sizes (scan_segments, ENDS) say how it moves a state on;
 // scan_carry applies that segment after segment, which leaves the state before each; then every segment is walked once more from
 // its own state with the read-outs.  A thread owns a channel with all its states in registers (no sums over lanes), a block 128
@@ -294,38 +296,27 @@ selective_scan_kernel(T* __restrict__ out, const T* __restrict__ xc, const float
 // Workspace per segment: the states [kScanStates][inner], the sums of step sizes [inner].
 constexpr int kScanSegment = 64, kScanStates = 16, kScanBatch = 8;
 
-// (request, first row, rows, number of the segment in its request); request -1 behind the last segment of the step
-__device__ __forceinline__ int4 scan_locate(const int* __restrict__ q_start, int requests, int segment) {
-  for (int r = 0; r < requests; ++r) {
-    const int lo = q_start[r], n = q_start[r + 1] - lo;
-    const int segments = n > 0 ? (n + kScanSegment - 1) / kScanSegment : 0;
-    if (segment < segments) return make_int4(r, lo + segment * kScanSegment, min(kScanSegment, n - segment * kScanSegment), segment);
-    segment -= segments;
-  }
-  return make_int4(-1, 0, 0, 0);
-}
-
 template <typename T, bool ENDS>
 __global__ void __launch_bounds__(128)
 scan_segments_kernel(T* __restrict__ out, float* __restrict__ work, const T* __restrict__ xc, const float* __restrict__ dt_raw,
                      const float* __restrict__ dt_bias, const float* __restrict__ A, const T* __restrict__ bc, const float* __restrict__ D,
                      const T* __restrict__ z, int z_ld, int z_column, int inner, int n_state, const int* __restrict__ q_start,
-                     const int* __restrict__ state_slot, int requests) {
+                     const int* __restrict__ state_slot, int requests, int walk_max) {
   __shared__ __align__(16) float s_bc[kScanSegment][2 * kScanStates];
   pdl_wait();
   pdl_launch_dependents();
-  const int4 at = scan_locate(q_start, requests, blockIdx.y);
-  if (at.x < 0 || state_slot[at.x] < 0) return;
-  const int n = at.z;
+  const LongPortion at = locate_portion<false, kScanSegment>(q_start, requests, walk_max, blockIdx.x);
+  if (at.r < 0 || state_slot[at.r] < 0) return;
+  const int first = ((int)blockIdx.x - at.piece0) * kScanSegment, row0 = at.lo + first, n = min(kScanSegment, at.n - first);
   for (int i = threadIdx.x; i < kScanSegment * 2 * kScanStates; i += 128) {
     const int t = i / (2 * kScanStates), e = i % (2 * kScanStates), k = e % kScanStates;
     const bool there = t < n && k < n_state;
-    s_bc[t][e] = there ? to_f32(bc[(size_t)(at.y + t) * 2 * n_state + (e < kScanStates ? k : n_state + k)]) : 0.f;
+    s_bc[t][e] = there ? to_f32(bc[(size_t)(row0 + t) * 2 * n_state + (e < kScanStates ? k : n_state + k)]) : 0.f;
   }
   __syncthreads();
-  const int c = blockIdx.x * 128 + threadIdx.x;
+  const int c = blockIdx.y * 128 + threadIdx.x;
   if (c >= inner) return;
-  float* states = work + (size_t)blockIdx.y * (kScanStates + 1) * inner + c;
+  float* states = work + (size_t)blockIdx.x * (kScanStates + 1) * inner + c;
   float S[kScanStates], a[kScanStates];
 #pragma unroll
   for (int k = 0; k < kScanStates; ++k) {
@@ -338,7 +329,7 @@ scan_segments_kernel(T* __restrict__ out, float* __restrict__ work, const T* __r
     float x[kScanBatch], dt[kScanBatch], gate[kScanBatch];
 #pragma unroll
     for (int i = 0; i < kScanBatch; ++i) {                 // (eight tokens' loads side by side)
-      const size_t row = at.y + min(t0 + i, n - 1);
+      const size_t row = row0 + min(t0 + i, n - 1);
       x[i] = to_f32(xc[row * inner + c]);
       dt[i] = dt_raw[row * inner + c];
       gate[i] = ENDS ? 0.f : to_f32(z[row * z_ld + z_column + c]);
@@ -360,7 +351,7 @@ scan_segments_kernel(T* __restrict__ out, float* __restrict__ work, const T* __r
         }
       }
       if (ENDS) sum += step;
-      else out[(size_t)(at.y + t0 + i) * inner + c] = from_f32<T>(((y[0] + y[1]) + (y[2] + y[3]) + skip * x[i]) * silu_f32(gate[i]));
+      else out[(size_t)(row0 + t0 + i) * inner + c] = from_f32<T>(((y[0] + y[1]) + (y[2] + y[3]) + skip * x[i]) * silu_f32(gate[i]));
     }
   }
   if (ENDS) {
@@ -374,14 +365,13 @@ scan_segments_kernel(T* __restrict__ out, float* __restrict__ work, const T* __r
 // moves the request's own state on.
 __global__ void __launch_bounds__(128)
 scan_carry_kernel(float* __restrict__ work, float* __restrict__ state, const float* __restrict__ A, int inner, int n_state,
-                  const int* __restrict__ q_start, const int* __restrict__ positions, const int* __restrict__ state_slot) {
+                  const int* __restrict__ q_start, const int* __restrict__ positions, const int* __restrict__ state_slot, int requests,
+                  int walk_max) {
   pdl_wait();
   pdl_launch_dependents();
-  const int r = blockIdx.z, k = blockIdx.y, c = blockIdx.x * 128 + threadIdx.x;
-  const int lo = q_start[r], n = q_start[r + 1] - lo;
-  if (c >= inner || n <= 0 || state_slot[r] < 0) return;
-  int first = 0;
-  for (int i = 0; i < r; ++i) first += (max(q_start[i + 1] - q_start[i], 0) + kScanSegment - 1) / kScanSegment;
+  const LongPortion at = locate_portion<true, kScanSegment>(q_start, requests, walk_max, blockIdx.z);
+  const int r = at.r, lo = at.lo, n = at.n, first = at.piece0, k = blockIdx.y, c = blockIdx.x * 128 + threadIdx.x;
+  if (r < 0 || c >= inner || state_slot[r] < 0) return;
   const int segments = (n + kScanSegment - 1) / kScanSegment;
   float* st = state + ((size_t)state_slot[r] * inner + c) * n_state + k;
   float S = positions[lo] == 0 ? 0.f : *st;
@@ -776,7 +766,7 @@ int causal_conv(void* out, const void* x, int ld, int column, int channels, cons
 template <typename T>
 int selective_scan(void* out, const void* xc, const float* dt_raw, const float* dt_bias, const float* A, const void* bc,
                    const float* D, const void* z, int z_ld, int z_column, int inner, int n_state, float* state, const int* q_start,
-                   const int* positions, const int* state_slot, int requests, void* stream) {
+                   const int* positions, const int* state_slot, int requests, int walk_max, void* stream) {
   PTL_REQUIRE(requests >= 0 && inner > 0 && n_state > 0 && n_state <= 256 && z_column >= 0 && z_column + inner <= z_ld,
               "selective_scan: bad sizes inner=%d state=%d (at most 256)", inner, n_state);
   PTL_REQUIRE(requests <= 65535, "selective_scan: at most 65535 requests per step, got %d", requests);
@@ -786,7 +776,7 @@ int selective_scan(void* out, const void* xc, const float* dt_raw, const float* 
   const size_t smem = (size_t)tb * (2 * n_state + 64) * sizeof(float);
 #define PTL_SCAN(NPL) return launch_kernel("selective_scan", selective_scan_kernel<T, NPL>, grid, block, smem, as_stream(stream), \
     (T*)out, (const T*)xc, dt_raw, dt_bias, A, (const T*)bc, D, (const T*)z, z_ld, z_column, inner, n_state, state, q_start, \
-    positions, state_slot, tb)
+    positions, state_slot, tb, walk_max)
   const int per_lane = (n_state + 7) / 8;
   if (per_lane <= 1) PTL_SCAN(1);
   if (per_lane <= 2) PTL_SCAN(2);
@@ -799,22 +789,24 @@ int selective_scan(void* out, const void* xc, const float* dt_raw, const float* 
 }
 
 template <typename T>
-int scan_segments(void* out, float* work, int segments, const void* xc, const float* dt_raw, const float* dt_bias, const float* A,
-                  const void* bc, const float* D, const void* z, int z_ld, int z_column, int inner, int n_state, float* state,
-                  const int* q_start, const int* positions, const int* state_slot, int requests, void* stream) {
-  PTL_REQUIRE(requests >= 0 && requests <= 65535 && segments >= 0 && segments <= 65535 && inner > 0 && n_state > 0 &&
-                  n_state <= kScanStates && z_column >= 0 && z_column + inner <= z_ld,
+int scan_segments(void* out, float* work, int segments, int portions, const void* xc, const float* dt_raw, const float* dt_bias,
+                  const float* A, const void* bc, const float* D, const void* z, int z_ld, int z_column, int inner, int n_state,
+                  float* state, const int* q_start, const int* positions, const int* state_slot, int requests, int walk_max, void* stream) {
+  PTL_REQUIRE(requests >= 0 && portions >= 0 && portions <= 65535 && portions <= requests && segments >= 0 && inner > 0 &&
+                  (inner + 127) / 128 <= 65535 && n_state > 0 && n_state <= kScanStates && walk_max >= 0 && z_column >= 0 &&
+                  z_column + inner <= z_ld,
               "selective_scan in segments: bad sizes inner=%d state=%d (at most %d)", inner, n_state, kScanStates);
-  if (requests == 0 || segments == 0) return 0;
-  const dim3 grid((inner + 127) / 128, segments), block(128);
+  if (segments == 0 || portions == 0) return 0;
+  const dim3 grid(segments, (inner + 127) / 128), block(128);
   if (int rc = launch_kernel("scan_segments", scan_segments_kernel<T, true>, grid, block, 0, as_stream(stream), (T*)out, work, (const T*)xc,
-                             dt_raw, dt_bias, A, (const T*)bc, D, (const T*)z, z_ld, z_column, inner, n_state, q_start, state_slot, requests))
+                             dt_raw, dt_bias, A, (const T*)bc, D, (const T*)z, z_ld, z_column, inner, n_state, q_start, state_slot, requests,
+                             walk_max))
     return rc;
-  if (int rc = launch_kernel("scan_carry", scan_carry_kernel, dim3((inner + 127) / 128, n_state, requests), block, 0, as_stream(stream), work,
-                             state, A, inner, n_state, q_start, positions, state_slot))
+  if (int rc = launch_kernel("scan_carry", scan_carry_kernel, dim3((inner + 127) / 128, n_state, portions), block, 0, as_stream(stream), work,
+                             state, A, inner, n_state, q_start, positions, state_slot, requests, walk_max))
     return rc;
   return launch_kernel("scan_segments", scan_segments_kernel<T, false>, grid, block, 0, as_stream(stream), (T*)out, work, (const T*)xc,
-                       dt_raw, dt_bias, A, (const T*)bc, D, (const T*)z, z_ld, z_column, inner, n_state, q_start, state_slot, requests);
+                       dt_raw, dt_bias, A, (const T*)bc, D, (const T*)z, z_ld, z_column, inner, n_state, q_start, state_slot, requests, walk_max);
 }
 
 template <typename T>
@@ -876,16 +868,16 @@ int gated_head_norm(void* out, int out_ld, int column, const float* o, const flo
   PTL_EXPORT int ptl_selective_scan##SUFFIX(void* out, const void* xc, const float* dt_raw, const float* dt_bias, const float* A,  \
                                             const void* bc, const float* D, const void* z, int z_ld, int z_column, int inner,      \
                                             int n_state, float* state, const int* q_start, const int* positions,                  \
-                                            const int* state_slot, int requests, void* stream) {                                  \
+                                            const int* state_slot, int requests, int walk_max, void* stream) {                    \
     return ptl::selective_scan<TYPE>(out, xc, dt_raw, dt_bias, A, bc, D, z, z_ld, z_column, inner, n_state, state, q_start,        \
-                                     positions, state_slot, requests, stream);                                                    \
+                                     positions, state_slot, requests, walk_max, stream);                                          \
   }                                                                                                                               \
-  PTL_EXPORT int ptl_scan_segments##SUFFIX(void* out, float* work, int segments, const void* xc, const float* dt_raw,              \
+  PTL_EXPORT int ptl_scan_segments##SUFFIX(void* out, float* work, int segments, int portions, const void* xc, const float* dt_raw, \
                                            const float* dt_bias, const float* A, const void* bc, const float* D, const void* z,    \
                                            int z_ld, int z_column, int inner, int n_state, float* state, const int* q_start,      \
-                                           const int* positions, const int* state_slot, int requests, void* stream) {             \
-    return ptl::scan_segments<TYPE>(out, work, segments, xc, dt_raw, dt_bias, A, bc, D, z, z_ld, z_column, inner, n_state, state,  \
-                                    q_start, positions, state_slot, requests, stream);                                            \
+                                           const int* positions, const int* state_slot, int requests, int walk_max, void* stream) { \
+    return ptl::scan_segments<TYPE>(out, work, segments, portions, xc, dt_raw, dt_bias, A, bc, D, z, z_ld, z_column, inner, n_state, \
+                                    state, q_start, positions, state_slot, requests, walk_max, stream);                           \
   }                                                                                                                               \
   PTL_EXPORT int ptl_gated_delta_rule##SUFFIX(float* out, const void* qkv, const float* ba, const float* rate,                     \
                                               const float* dt_bias, float* state, const int* q_start, const int* positions,       \

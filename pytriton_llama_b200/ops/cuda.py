@@ -37,9 +37,9 @@ _SIGNATURES = {
     "ptl_causal_conv": [_ptr, _ptr, _c_int, _c_int, _c_int, _ptr, _ptr, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int,
                         _c_int, _c_int, _ptr, _ptr],
     "ptl_selective_scan": [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr,
-                           _c_int, _ptr],
-    "ptl_scan_segments": [_ptr, _ptr, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr, _ptr,
-                          _ptr, _c_int, _ptr],
+                           _c_int, _c_int, _ptr],
+    "ptl_scan_segments": [_ptr, _ptr, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr,
+                          _ptr, _ptr, _c_int, _c_int, _ptr],
     "ptl_gated_delta_rule": [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f,
                              _c_f, _c_int, _ptr],
     "ptl_gated_delta_chunks": [_ptr, _ptr, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
@@ -1188,9 +1188,20 @@ class CudaOps:
                        single, _p(in_bias), self._stream()), kernels=2 if taps > 1 and not single else 1)
         return out
 
-    # The longest portion of a step that the selective scan walks token by token.  2,048
+    @staticmethod
+    def _portion_paths(ctx, walk_max: int) -> Tuple[bool, int, int]:
+        """(whether portions of up to ``walk_max`` tokens may come, the most longer ones, the most pieces of 64 tokens that these
+        make).  The kernels tell portions apart by the lengths on the device; the host's say which kernels there is no use for,
+        where they are the step's own: a captured step meets others, of as many tokens as it was padded to."""
+        tokens = int(ctx.positions.shape[0])
+        if ctx.max_q_len <= walk_max:
+            return True, 0, 0
+        long = min(ctx.num_requests, tokens // (walk_max + 1))
+        return not (getattr(ctx, "host_lengths_exact", False) and min(ctx.q_lens) > walk_max), long, tokens // 64 + long
+
+    # The longest portion that the selective scan walks token by token.  2,048
     # tokens of 2,048 channels of 16 states: 603 us token by token, 116 in segments (51 their products, 5 the carries, 60 the outputs);
-    # a segment's work is done twice, so that below one segment (64 tokens) the walk is the shorter.
+    # a segment's work is done twice, so that below one segment (64 tokens) the walk is the shorter.  Every request goes by its own length.
     SCAN_WALK_MAX_TOKENS = 64
 
     def selective_scan(self, xc: torch.Tensor, dt: torch.Tensor, dt_b: torch.Tensor, A: torch.Tensor, bc: torch.Tensor,
@@ -1206,33 +1217,23 @@ class CudaOps:
         if xc.shape[1] != inner or dt.shape != xc.shape or bc.shape[1] != 2 * n or tuple(state.shape[1:]) != (inner, n):
             raise KernelError("selective_scan: shapes do not fit")
         out = self.empty(xc.shape, xc.dtype)
-        if ctx.max_q_len > self.SCAN_WALK_MAX_TOKENS and n <= 16:
-            segments = xc.shape[0] // 64 + ctx.num_requests      # at least the segments of 64 tokens that the portions make
+        walk_max = self.SCAN_WALK_MAX_TOKENS if n <= 16 else 1 << 30
+        short, long, segments = self._portion_paths(ctx, walk_max)
+        if short:
+            fn = getattr(self.lib, "ptl_selective_scan" + _suffix(xc.dtype))
+            self._check(fn(_p(out), _p(xc), _p(dt), _p(dt_b), _p(A), _p(bc), _p(D), _p(xz), xz.shape[1], int(z_column), inner, n, _p(state),
+                           _p(ctx.q_start), _p(ctx.positions), _p(ctx.state_slot), ctx.num_requests, walk_max, self._stream()))
+        if long:
             work = self.empty((segments, 17, inner), torch.float32)
             fn = getattr(self.lib, "ptl_scan_segments" + _suffix(xc.dtype))
-            self._check(fn(_p(out), _p(work), segments, _p(xc), _p(dt), _p(dt_b), _p(A), _p(bc), _p(D), _p(xz), xz.shape[1], int(z_column),
-                           inner, n, _p(state), _p(ctx.q_start), _p(ctx.positions), _p(ctx.state_slot), ctx.num_requests,
-                           self._stream()), kernels=3)
-            return out
-        fn = getattr(self.lib, "ptl_selective_scan" + _suffix(xc.dtype))
-        self._check(fn(_p(out), _p(xc), _p(dt), _p(dt_b), _p(A), _p(bc), _p(D), _p(xz), xz.shape[1], int(z_column), inner, n,
-                       _p(state), _p(ctx.q_start), _p(ctx.positions), _p(ctx.state_slot), ctx.num_requests, self._stream()))
+            self._check(fn(_p(out), _p(work), segments, long, _p(xc), _p(dt), _p(dt_b), _p(A), _p(bc), _p(D), _p(xz), xz.shape[1],
+                           int(z_column), inner, n, _p(state), _p(ctx.q_start), _p(ctx.positions), _p(ctx.state_slot), ctx.num_requests,
+                           walk_max, self._stream()), kernels=3)
         return out
 
     # The longest portion that the gated delta rule walks token by token: up to one chunk (2,048 tokens of 8 heads of 128:
     # 738 us by the walk, 206 in chunks; 64: 23 by the walk, one chunk costs as much).  Every request goes by its own length.
     DELTA_WALK_MAX_TOKENS = 64
-
-    @staticmethod
-    def _portion_paths(ctx, walk_max: int) -> Tuple[bool, int, int]:
-        """(whether portions of up to ``walk_max`` tokens may come, the most longer ones, the most pieces of 64 tokens that these
-        make).  The kernels tell portions apart by the lengths on the device; the host's say which kernels there is no use for,
-        where they are the step's own: a captured step meets others, of as many tokens as it was padded to."""
-        tokens = int(ctx.positions.shape[0])
-        if ctx.max_q_len <= walk_max:
-            return True, 0, 0
-        long = min(ctx.num_requests, tokens // (walk_max + 1))
-        return not (getattr(ctx, "host_lengths_exact", False) and min(ctx.q_lens) > walk_max), long, tokens // 64 + long
 
     def gated_delta_rule(self, qkv: torch.Tensor, ba: torch.Tensor, rate: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor,
                          ctx, H: int, G: int, d: int, dv: int, unit_eps: float, q_scale: float) -> torch.Tensor:

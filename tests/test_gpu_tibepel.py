@@ -185,6 +185,18 @@ def test_gated_delta_rule_of_a_request_does_not_depend_on_its_company(ops, H, G,
     _alone_and_together(run, tensors, ("qkv", "ba"), COMPANY)
 
 
+@pytest.mark.parametrize("inner,n", [(40, 16), (129, 5)])
+def test_selective_scan_of_a_request_does_not_depend_on_its_company(ops, inner, n):
+    g = torch.Generator().manual_seed(inner)
+    T, R = sum(COMPANY), len(COMPANY)
+    tensors = {"xc": torch.randn(T, inner, generator=g).bfloat16(), "dt": torch.randn(T, inner, generator=g) - 2,
+               "dt_b": torch.randn(inner, generator=g), "A": -torch.exp(torch.randn(inner, n, generator=g)),
+               "bc": torch.randn(T, 2 * n, generator=g).bfloat16(), "D": torch.randn(inner, generator=g),
+               "xz": torch.randn(T, 2 * inner, generator=g).bfloat16(), "state": torch.randn(R, inner, n, generator=g)}
+    run = lambda t, ctx: ops.selective_scan(t["xc"], t["dt"], t["dt_b"], t["A"], t["bc"], t["D"], t["xz"], inner, t["state"], ctx)
+    _alone_and_together(run, tensors, ("xc", "dt", "bc", "xz"), COMPANY)
+
+
 @pytest.mark.parametrize("M,inter,K,bias", [(1, 52, 64, True), (8, 300, 1024, True), (20, 2048, 512, False), (64, 96, 2048, True),
                                             (65, 260, 64, True), (300, 1024, 512, True), (700, 130, 200, False)])
 def test_clamped_activation_in_the_product(ops, M, inter, K, bias):
