@@ -1199,10 +1199,10 @@ class CudaOps:
         long = min(ctx.num_requests, tokens // (walk_max + 1))
         return not (getattr(ctx, "host_lengths_exact", False) and min(ctx.q_lens) > walk_max), long, tokens // 64 + long
 
-    # The longest portion that the selective scan walks token by token.  2,048
-    # tokens of 2,048 channels of 16 states: 603 us token by token, 116 in segments (51 their products, 5 the carries, 60 the outputs);
-    # a segment's work is done twice, so that below one segment (64 tokens) the walk is the shorter.  Every request goes by its own length.
-    SCAN_WALK_MAX_TOKENS = 64
+    # The longest portion that the selective scan walks token by token; every request goes by its own length.  The walk costs 0.26 us a
+    # token and runs beside others' walks, the segments 60 us and up (2,048 channels of 16 states: 192 tokens 51 us walked, 65 in
+    # segments; four of them 59 and 111; one of 320: 84 and 71; of 2,048: 521 and 135).
+    SCAN_WALK_MAX_TOKENS = 192
 
     def selective_scan(self, xc: torch.Tensor, dt: torch.Tensor, dt_b: torch.Tensor, A: torch.Tensor, bc: torch.Tensor,
                        D: torch.Tensor, xz: torch.Tensor, z_column: int, state: torch.Tensor, ctx) -> torch.Tensor:
@@ -1231,9 +1231,10 @@ class CudaOps:
                            walk_max, self._stream()), kernels=3)
         return out
 
-    # The longest portion that the gated delta rule walks token by token: up to one chunk (2,048 tokens of 8 heads of 128:
-    # 738 us by the walk, 206 in chunks; 64: 23 by the walk, one chunk costs as much).  Every request goes by its own length.
-    DELTA_WALK_MAX_TOKENS = 64
+    # The longest portion that the gated delta rule walks token by token; every request goes by its own length.  The walk costs
+    # 0.35 us a token and runs beside others' walks (8 heads of 128: 128 tokens 49 us walked, 49 in chunks; four of them 57 and 77, 16 of
+    # them 220 and 178; one of 160 tokens 60 and 53; of 2,048: 718 and 166).
+    DELTA_WALK_MAX_TOKENS = 128
 
     def gated_delta_rule(self, qkv: torch.Tensor, ba: torch.Tensor, rate: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor,
                          ctx, H: int, G: int, d: int, dv: int, unit_eps: float, q_scale: float) -> torch.Tensor:

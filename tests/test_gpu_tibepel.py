@@ -174,8 +174,9 @@ def _alone_and_together(run, tensors, per_token, lens):
 COMPANY = [1] * 20 + [10, 200, 1, 64, 65, 2] + [1] * 20      # more requests than a warp has lanes, long portions among them
 
 
-@pytest.mark.parametrize("H,G,d,dv", [(2, 1, 64, 16), (3, 3, 128, 40)])
-def test_gated_delta_rule_of_a_request_does_not_depend_on_its_company(ops, H, G, d, dv):
+@pytest.mark.parametrize("H,G,d,dv,walk", [(2, 1, 64, 16, 64), (3, 3, 128, 40, None)])
+def test_gated_delta_rule_of_a_request_does_not_depend_on_its_company(ops, monkeypatch, H, G, d, dv, walk):
+    monkeypatch.setattr(ops, "DELTA_WALK_MAX_TOKENS", walk or ops.DELTA_WALK_MAX_TOKENS)
     g = torch.Generator().manual_seed(d)
     T, R = sum(COMPANY), len(COMPANY)
     tensors = {"qkv": torch.randn(T, 2 * G * d + H * dv, generator=g).bfloat16(), "ba": torch.randn(T, 2 * H, generator=g),
@@ -185,8 +186,9 @@ def test_gated_delta_rule_of_a_request_does_not_depend_on_its_company(ops, H, G,
     _alone_and_together(run, tensors, ("qkv", "ba"), COMPANY)
 
 
-@pytest.mark.parametrize("inner,n", [(40, 16), (129, 5)])
-def test_selective_scan_of_a_request_does_not_depend_on_its_company(ops, inner, n):
+@pytest.mark.parametrize("inner,n,walk", [(40, 16, 64), (129, 5, None)])
+def test_selective_scan_of_a_request_does_not_depend_on_its_company(ops, monkeypatch, inner, n, walk):
+    monkeypatch.setattr(ops, "SCAN_WALK_MAX_TOKENS", walk or ops.SCAN_WALK_MAX_TOKENS)
     g = torch.Generator().manual_seed(inner)
     T, R = sum(COMPANY), len(COMPANY)
     tensors = {"xc": torch.randn(T, inner, generator=g).bfloat16(), "dt": torch.randn(T, inner, generator=g) - 2,
@@ -195,6 +197,15 @@ def test_selective_scan_of_a_request_does_not_depend_on_its_company(ops, inner, 
                "xz": torch.randn(T, 2 * inner, generator=g).bfloat16(), "state": torch.randn(R, inner, n, generator=g)}
     run = lambda t, ctx: ops.selective_scan(t["xc"], t["dt"], t["dt_b"], t["A"], t["bc"], t["D"], t["xz"], inner, t["state"], ctx)
     _alone_and_together(run, tensors, ("xc", "dt", "bc", "xz"), COMPANY)
+
+
+@pytest.mark.parametrize("walk", [1, 64])
+def test_pieces_of_64_tokens_whatever_the_longest_walk(ops, monkeypatch, walk):
+    """The two tests above with their portions of 63 to 128 tokens (and at 1 all but the single tokens) in pieces as well."""
+    monkeypatch.setattr(ops, "SCAN_WALK_MAX_TOKENS", walk)
+    monkeypatch.setattr(ops, "DELTA_WALK_MAX_TOKENS", walk)
+    test_selective_scan_in_segments_of_64_tokens(ops, "float32", 129, 5)
+    test_gated_delta_rule_in_chunks_of_64_tokens(ops, "bfloat16", 3, 3, 128, 40)
 
 
 @pytest.mark.parametrize("M,inter,K,bias", [(1, 52, 64, True), (8, 300, 1024, True), (20, 2048, 512, False), (64, 96, 2048, True),
