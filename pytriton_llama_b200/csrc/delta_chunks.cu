@@ -6,8 +6,8 @@
 // Everything that does not know S is worked out for all chunks side by side (delta_chunk_prepare: the system solved for its
 // two right sides, U = WV - WK S, and the factors of the other two lines); what is left of the serial walk is three small
 // products a chunk (delta_chunk_walk).  All of it float32 multiply-adds; the running sums are kept in 64 bits, because a
-// difference of two of them is the exponent of a decay.  (An input that is no number reaches the results of its whole chunk,
-// where the walk kept it from the tokens before it.)
+// difference of two of them is the exponent of a decay.  A portion with an input that is no finite number (or whose length
+// squared is none) is walked token by token instead: in the products it would reach its chunk's earlier tokens, as 0 times it.
 //
 // The token-by-token walk is bound by the latency of its chain, 0.36 us a token at heads of 128 x 128: 738 us for
 // 2,048 tokens, whatever the number of SMs.  Here 16 heads of that size take 88 us (prepare: the chains of the 64 x 64 systems,
@@ -23,7 +23,7 @@ constexpr int kDcSysLd = kDcTokens + 4;
 __device__ __forceinline__ float dc_softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 
 // Floats of a (chunk, head) in the workspace: WK and the decayed queries [64][D], the decayed keys [D][64], the read-out's
-// weights [64][64], WV [64][dv], the chunk's decay (padded to 16 bytes).
+// weights [64][64], WV [64][dv], the chunk's decay, and 1 where an input is not finite (padded to 16 bytes).
 __host__ __device__ __forceinline__ size_t dc_floats(int D, int dv) { return (size_t)kDcTokens * (3 * D + kDcTokens + dv) + 4; }
 constexpr size_t dc_prepare_smem(int D) { return sizeof(float) * (2 * kDcTokens * (D + 4) + kDcTokens * kDcSysLd); }
 constexpr size_t dc_walk_smem(int D) {
@@ -73,8 +73,9 @@ delta_chunk_prepare_kernel(float* __restrict__ work, const T* __restrict__ qkv, 
     qq = warp_sum(qq);
     kk = warp_sum(kk);
     if (lane == 0) {
-      s_qn[t] = q_scale / sqrtf(qq + unit_eps);
-      s_kn[t] = 1.0f / sqrtf(kk + unit_eps);
+      s_qn[t] = t < n ? q_scale / sqrtf(qq + unit_eps) : 0.f;
+      s_kn[t] = t < n ? 1.0f / sqrtf(kk + unit_eps) : 0.f;
+      if (!isfinite(qq + kk)) s_kn[t] = NAN;       // (a length of infinity would pass as a factor of zero)
     }
 #pragma unroll
     for (int i = 0; i < D / 32; ++i) {
@@ -161,8 +162,8 @@ delta_chunk_prepare_kernel(float* __restrict__ work, const T* __restrict__ qkv, 
     const int t2 = i % kDcTokens, e2 = i / kDcTokens;
     kdt[i] = expf((float)(end - s_log[t2])) * s_kn[t2] * s_k[t2 * LD + e2];
   }
-  if (tid == 0) wv[kDcTokens * dv] = s_decay[kDcTokens - 1];
   __syncthreads();
+  bool finite = tid >= kDcTokens || (isfinite(s_kn[tid] + s_qn[tid] + s_beta[tid]) && !isnan(s_log[tid]));
   for (int col = tid; col < D + dv; col += kDcThreads) {
     float u[kDcTokens];
     if (col < D) {
@@ -172,7 +173,11 @@ delta_chunk_prepare_kernel(float* __restrict__ work, const T* __restrict__ qkv, 
       const T* v = qkv + (size_t)s_at[0] * ld + 2 * kv_heads * D + (size_t)h * dv + (col - D);
       const int tokens = s_at[1];
 #pragma unroll
-      for (int t = 0; t < kDcTokens; ++t) u[t] = t < tokens ? s_beta[t] * to_f32(v[(size_t)t * ld]) : 0.f;
+      for (int t = 0; t < kDcTokens; ++t) {
+        const float x = t < tokens ? to_f32(v[(size_t)t * ld]) : 0.f;
+        finite = finite && isfinite(x);
+        u[t] = s_beta[t] * x;
+      }
     }
 #pragma unroll
     for (int i = 0; i < kDcTokens - 1; ++i) {
@@ -190,6 +195,11 @@ delta_chunk_prepare_kernel(float* __restrict__ work, const T* __restrict__ qkv, 
     const int step = col < D ? D : dv;
 #pragma unroll
     for (int t = 0; t < kDcTokens; ++t) dst[(size_t)t * step] = u[t];
+  }
+  const int bad = __syncthreads_or(!finite);
+  if (tid == 0) {
+    wv[kDcTokens * dv] = s_decay[kDcTokens - 1];
+    wv[kDcTokens * dv + 1] = bad ? 1.f : 0.f;
   }
 }
 
@@ -241,11 +251,57 @@ __device__ __forceinline__ void dc_product(const float* __restrict__ a, const fl
   dc_meet<ROWS>(acc, s, sum);
 }
 
-template <int D>
+// The tokens of a portion one by one, for the eight columns of the state in shared memory (`scratch`: 2 D + 128 floats): the
+// walk's own steps (recurrent.cu).  Rare, so that its speed does not matter.
+template <typename T, int D>
+__device__ __noinline__ void dc_walk_tokens(float* __restrict__ out, const T* __restrict__ rows, const float* __restrict__ ba, int tokens,
+                                            float rate, float dt_bias, int heads, int kv_heads, int dv, int h, int j0, float unit_eps,
+                                            float q_scale, float* s_s, float* scratch) {
+  constexpr int LD = D + 4;
+  float *s_q = scratch, *s_k = scratch + D, *s_part = scratch + 2 * D;      // [2][8 warps][8 columns]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, c = tid & 7, e0 = tid >> 3;       // column, first entry of every 32nd
+  const int ld = 2 * kv_heads * D + heads * dv, head = h / (heads / kv_heads);
+  for (int t = 0; t < tokens; ++t) {
+    const T* row = rows + (size_t)t * ld;
+    __syncthreads();
+    for (int e = tid; e < 2 * D; e += kDcThreads) scratch[e] = to_f32(e < D ? row[head * D + e] : row[(kv_heads + head) * D + e - D]);
+    __syncthreads();
+    float qq = 0.f, kk = 0.f;
+    for (int e = lane; e < D; e += 32) { qq = fmaf(s_q[e], s_q[e], qq); kk = fmaf(s_k[e], s_k[e], kk); }
+    const float qn = q_scale / sqrtf(warp_sum(qq) + unit_eps), kn = 1.0f / sqrtf(warp_sum(kk) + unit_eps);
+    const float* gates = ba + (size_t)t * 2 * heads;
+    const float beta = 1.0f / (1.0f + expf(-gates[h])), g = expf(-rate * dc_softplus(gates[heads + h] + dt_bias));
+    auto over_entries = [&](float v, int which) {                 // a column's sum over the block
+      v += __shfl_xor_sync(0xffffffffu, v, 8);
+      v += __shfl_xor_sync(0xffffffffu, v, 16);
+      if (lane < 8) s_part[which * 64 + warp * 8 + c] = v;
+      __syncthreads();
+      float sum = 0.f;
+      for (int w = 0; w < 8; ++w) sum += s_part[which * 64 + w * 8 + c];
+      return sum;
+    };
+    float part = 0.f;
+    for (int e = e0; e < D; e += 32) {
+      s_s[c * LD + e] *= g;
+      part = fmaf(s_s[c * LD + e], s_k[e], part);
+    }
+    const float u = beta * (to_f32(row[2 * kv_heads * D + h * dv + j0 + c]) - kn * over_entries(part, 0)) * kn;
+    part = 0.f;
+    for (int e = e0; e < D; e += 32) {
+      s_s[c * LD + e] = fmaf(s_k[e], u, s_s[c * LD + e]);
+      part = fmaf(s_s[c * LD + e], s_q[e], part);
+    }
+    const float o = over_entries(part, 1) * qn;
+    if (tid < 8) out[((size_t)t * heads + h) * dv + j0 + c] = o;
+  }
+}
+
+template <typename T, int D>
 __global__ void __launch_bounds__(kDcThreads, 1)
-delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, const float* __restrict__ work, const int* __restrict__ q_start,
-                        const int* __restrict__ positions, const int* __restrict__ state_slot, int requests, int heads, int dv,
-                        int walk_max) {
+delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, const float* __restrict__ work, const T* __restrict__ qkv,
+                        const float* __restrict__ ba, const float* __restrict__ rate, const float* __restrict__ dt_bias, int kv_heads,
+                        float unit_eps, float q_scale, const int* __restrict__ q_start, const int* __restrict__ positions,
+                        const int* __restrict__ state_slot, int requests, int heads, int dv, int walk_max) {
   constexpr int LD = D + 4, RB = 2 + D / 32;
   extern __shared__ __align__(16) float dw_smem[];
   float* s_a = dw_smem;                                  // [2][WK 64 | q 64][LD]
@@ -285,7 +341,13 @@ delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, cons
     cp_async_commit();
   };
   fetch_a(0);
-  for (int chunk = 0; chunk < chunks; ++chunk) {
+  bool bad = false;
+  for (int i = tid; i < chunks; i += kDcThreads) bad = bad || base[i * stride + (size_t)kDcTokens * (3 * D + kDcTokens + dv) + 1] != 0.f;
+  const bool walk = __syncthreads_or(bad);
+  if (walk)
+    dc_walk_tokens<T, D>(out + (size_t)lo * heads * dv, qkv + (size_t)lo * (2 * kv_heads * D + heads * dv), ba + (size_t)lo * 2 * heads, n,
+                         rate[h], dt_bias[h], heads, kv_heads, dv, h, j0, unit_eps, q_scale, s_s, s_b);
+  for (int chunk = walk ? chunks : 0; chunk < chunks; ++chunk) {
     const int rows = min(kDcTokens, n - chunk * kDcTokens);
     const float* wv = base + chunk * stride + (size_t)kDcTokens * (3 * D + kDcTokens);
     const float v0 = wv[(size_t)rg * dv + j0 + s], v1 = wv[(size_t)(rg + 32) * dv + j0 + s], decay = wv[(size_t)kDcTokens * dv];
@@ -311,6 +373,7 @@ delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, cons
       *e = fmaf(decay, *e, second[j]);
     }
   }
+  cp_async_wait<0>();
   __syncthreads();
   for (int i = tid; i < D * kDcCols; i += kDcThreads) {
     const int e = i / kDcCols, c = i % kDcCols;
@@ -324,13 +387,14 @@ int delta_chunks(float* out, float* work, int chunks, int portions, const void* 
                  float unit_eps, float q_scale, int walk_max, void* stream) {
   static SmemRaised raised_p, raised_w;
   if (int rc = raise_shared_memory("delta_chunk_prepare", delta_chunk_prepare_kernel<T, D>, (int)dc_prepare_smem(D), raised_p)) return rc;
-  if (int rc = raise_shared_memory("delta_chunk_walk", delta_chunk_walk_kernel<D>, (int)dc_walk_smem(D), raised_w)) return rc;
+  if (int rc = raise_shared_memory("delta_chunk_walk", delta_chunk_walk_kernel<T, D>, (int)dc_walk_smem(D), raised_w)) return rc;
   if (int rc = launch_kernel("delta_chunk_prepare", delta_chunk_prepare_kernel<T, D>, dim3(chunks, heads), dim3(kDcThreads), dc_prepare_smem(D),
                              as_stream(stream), work, (const T*)qkv, ba, rate, dt_bias, q_start, state_slot, requests, heads, kv_heads, dv,
                              unit_eps, q_scale, walk_max))
     return rc;
-  return launch_kernel("delta_chunk_walk", delta_chunk_walk_kernel<D>, dim3(dv / kDcCols, heads, portions), dim3(kDcThreads), dc_walk_smem(D),
-                       as_stream(stream), out, state, work, q_start, positions, state_slot, requests, heads, dv, walk_max);
+  return launch_kernel("delta_chunk_walk", delta_chunk_walk_kernel<T, D>, dim3(dv / kDcCols, heads, portions), dim3(kDcThreads), dc_walk_smem(D),
+                       as_stream(stream), out, state, work, (const T*)qkv, ba, rate, dt_bias, kv_heads, unit_eps, q_scale, q_start,
+                       positions, state_slot, requests, heads, dv, walk_max);
 }
 
 template <typename T>

@@ -208,6 +208,37 @@ def test_pieces_of_64_tokens_whatever_the_longest_walk(ops, monkeypatch, walk):
     test_gated_delta_rule_in_chunks_of_64_tokens(ops, "bfloat16", 3, 3, 128, 40)
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -1e30])
+@pytest.mark.parametrize("where", ["q", "k", "v", "beta", "decay"])
+def test_delta_rule_keeps_a_bad_input_from_earlier_tokens(ops, where, bad):
+    """A value that is no finite number (or whose square is none) in the middle of a chunk: the results, finite or not, are those
+    of the token-by-token walk, so every token before it is as it would be without it, and so is every column that a value of v
+    does not belong to."""
+    H, G, d, dv, T, at = 2, 1, 64, 16, 300, 165
+    g = torch.Generator().manual_seed(5)
+    tensors = {"qkv": torch.randn(T, 2 * G * d + H * dv, generator=g), "ba": torch.randn(T, 2 * H, generator=g),
+               "rate": torch.exp(torch.randn(H, generator=g)), "dt_bias": torch.randn(H, generator=g), "S": torch.randn(1, H, d, dv, generator=g)}
+    tensors[{"beta": "ba", "decay": "ba"}.get(where, "qkv")][at, {"q": 3, "k": d + 5, "v": 2 * d + 7, "beta": 0, "decay": H}[where]] = bad
+    old, results = ops.DELTA_WALK_MAX_TOKENS, []
+    try:
+        for walk in (10 ** 6, 64):
+            ops.DELTA_WALK_MAX_TOKENS = walk
+            dev = {k: v.cuda() for k, v in tensors.items()}
+            o = ops.gated_delta_rule(dev["qkv"], dev["ba"], dev["rate"], dev["dt_bias"], dev["S"], _ctx([T], [7], [0], "cuda:0"), H, G, d, dv,
+                                     1e-6, d ** -0.5)
+            results.append((o.double().cpu(), dev["S"].double().cpu()))
+    finally:
+        ops.DELTA_WALK_MAX_TOKENS = old
+    for want, got in zip(*results):
+        assert torch.equal(want.isfinite(), got.isfinite())
+        fine = want.isfinite()
+        if where == "v" and abs(bad) == 1e30:                       # (the column itself is of that size)
+            fine &= want.abs() < 1e6
+        off, size = ((want - got)[fine].abs(), want[fine].abs()) if fine.any() else (torch.zeros(1), torch.zeros(1))
+        assert off.max() <= 2e-5 * 5 * max(1.0, float(size.max()))
+    assert results[1][0][:at].isfinite().all()
+
+
 @pytest.mark.parametrize("M,inter,K,bias", [(1, 52, 64, True), (8, 300, 1024, True), (20, 2048, 512, False), (64, 96, 2048, True),
                                             (65, 260, 64, True), (300, 1024, 512, True), (700, 130, 200, False)])
 def test_clamped_activation_in_the_product(ops, M, inter, K, bias):
