@@ -61,6 +61,7 @@ class StepContext:
     ctx_lens: List[int] = field(default_factory=list)
     host_lengths_exact: bool = False    # q_lens and ctx_lens are this step's own (not those a captured step was laid out for)
     max_q_len: int = 0
+    min_q_len: int = 1                  # no request of the step, or of any step that a captured one stands for, brings fewer tokens
     max_ctx_len: int = 0
     attn_splits: int = 1
     tokens: Optional[torch.Tensor] = None   # int32 [T] the step's token ids (set by the model's forward pass)

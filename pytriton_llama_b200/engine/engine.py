@@ -309,6 +309,7 @@ class Engine:
                                             work_items=self._work_items(batch.work),
                                             in_order=self._work_in_order(batch.work, batch.T))
             ctx.host_lengths_exact = True
+            ctx.min_q_len = min(batch.q_lens)
             logits = self.model.forward(layout.view(dev, "tokens"), ctx, cache_view,
                                         layout.view(dev, "logit_rows") if logit_rows else None)
         out = StepOutput(logits, rows, batch.T, batch.R)
@@ -467,6 +468,7 @@ class Engine:
     # ... in layers of five launches; in those with a part that says ``many_launches`` (12 to 16 a layer) they do not yet (2,020 tokens of
     # eight layers with latent attention: 2.61 ms launched, 1.82 captured)
     GRAPH_MAX_TOKENS_MANY_LAUNCHES = 2048
+    SHAPE_PADDING = 128          # token rows that a padded shape has too many, at most
     GRAPH_MAX_SHAPES = 24
     GRAPH_MAX_CAPTURES = 96      # a workload that keeps cycling through more shapes than are kept stops capturing new ones
 
@@ -482,7 +484,7 @@ class Engine:
             return 0
         pow2 = lambda n: 0 if n == 0 else 1 << (n - 1).bit_length()
         step = 64 if T <= 256 else 128
-        t_pad = -(-T // step) * step
+        t_pad = -(-T // step) * step                        # (with the row below, at most SHAPE_PADDING more than T)
         lists, needs_free_row = [], False
         for name, info in sorted(self._work_lists().items()):
             items = len(batch.work.get(name, ())) // info.width
@@ -569,6 +571,8 @@ class Engine:
         splits = self._choose_splits(layout.T, longest)
         ctx, cache_view = self._context(dev, layout, q_lens, [longest] * layout.R, splits,
                                         work_items=work_items, in_order=in_order)
+        if len(q_lens) == 1:
+            ctx.min_q_len = max(1, q_lens[0] - self.SHAPE_PADDING)      # one request brings all the tokens
 
         def run():
             self.ops.take_tokens(layout.view(dev, "tokens"), layout.view(dev, "token_src"), self.sampled)

@@ -1191,13 +1191,13 @@ class CudaOps:
     @staticmethod
     def _portion_paths(ctx, walk_max: int) -> Tuple[bool, int, int]:
         """(whether portions of up to ``walk_max`` tokens may come, the most longer ones, the most pieces of 64 tokens that these
-        make).  The kernels tell portions apart by the lengths on the device; the host's say which kernels there is no use for,
-        where they are the step's own: a captured step meets others, of as many tokens as it was padded to."""
+        make).  The kernels tell portions apart by the lengths on the device; this says which kernels the step, or those that a
+        captured one stands for, can have no use for."""
         tokens = int(ctx.positions.shape[0])
         if ctx.max_q_len <= walk_max:
             return True, 0, 0
         long = min(ctx.num_requests, tokens // (walk_max + 1))
-        return not (getattr(ctx, "host_lengths_exact", False) and min(ctx.q_lens) > walk_max), long, tokens // 64 + long
+        return getattr(ctx, "min_q_len", 1) <= walk_max, long, tokens // 64 + long
 
     # The longest portion that the selective scan walks token by token; every request goes by its own length.  The walk costs 0.26 us a
     # token and runs beside others' walks, the segments 60 us and up (2,048 channels of 16 states: 192 tokens 51 us walked, 65 in

@@ -174,6 +174,23 @@ def test_padded_shapes_of_captured_steps(model_folders):
     assert eng._shape_bucket(plain) == 0 and eng._shape_bucket(plain) == (64, 1, 1, ())
 
 
+def test_a_padded_shape_says_how_short_its_only_portion_can_be(model_folders):
+    """A captured step of one request tells its kernels the fewest tokens that a replay can bring: shapes are padded by at most
+    ``SHAPE_PADDING`` token rows, the row that a padded single-token item needs among them."""
+    from types import SimpleNamespace
+    from pytriton_llama_b200.engine.engine import _HostBatch
+    from pytriton_llama_b200.ops.cuda import CudaOps
+    eng = _engine(model_folders("A"), "A", 16)
+    plan = lambda q_lens, starts: CudaOps.plan_step(SimpleNamespace(QUERY_TILE=CudaOps.QUERY_TILE), q_lens, starts)
+    eng.ops.WORK_LISTS, eng.ops.plan_step = CudaOps.WORK_LISTS, plan
+    for lens in [[n] for n in range(2, 1025)] + [[n, 1, 1, 1][:k] for n in range(2, 700) for k in (2, 4)]:
+        b = _HostBatch([StepEntry(f"r{i}", [0] * n, []) for i, n in enumerate(lens)], lens, [0] * len(lens), [1] * len(lens),
+                       list(range(len(lens))), {}, [0], work=plan(lens, [0] * len(lens)))
+        eng._shape_seen.clear()
+        t_pad = (eng._shape_bucket(b) or eng._shape_bucket(b))[0]
+        assert b.T <= t_pad <= b.T + eng.SHAPE_PADDING
+
+
 def test_rope_parts_with_equal_parameters_share_their_table():
     """An operator set tells frequency tables apart by address when it works a step's angles out
     once for all layers; layers with the same parameters must therefore hold the same tensor."""

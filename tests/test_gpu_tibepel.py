@@ -162,7 +162,7 @@ def _alone_and_together(run, tensors, per_token, lens):
         if captured:
             ctx.max_q_len = sum(lens)
         else:
-            ctx.q_lens, ctx.host_lengths_exact = lens, True
+            ctx.min_q_len = min(lens)
         together = run(dev, ctx)
         for r, n in enumerate(lens):
             one = {k: (v[first[r]:first[r] + n] if k in per_token else v).contiguous().cuda() for k, v in tensors.items()}

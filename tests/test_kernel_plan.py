@@ -47,7 +47,7 @@ def test_pieces_of_long_portions_fit_what_a_step_provides_for():
         long = [n for n in lens if n > walk]
         for exact in (True, False):
             ctx = SimpleNamespace(positions=torch.empty(sum(lens) if exact else rows), num_requests=len(lens), q_lens=lens,
-                                  max_q_len=max(lens) if exact else rows, host_lengths_exact=exact)
+                                  max_q_len=max(lens) if exact else rows, min_q_len=min(lens) if exact else 1)
             short, portions, pieces = CudaOps._portion_paths(ctx, walk)
             assert len(long) <= portions <= len(lens) and sum(-(-n // 64) for n in long) <= pieces
             assert short or len(long) == len(lens)
