@@ -304,6 +304,30 @@ def test_chunk_attention_on_the_tensor_cores(ops, H, G, d, page, chunk, options)
     assert ((outs[0] - outs[1]).abs() <= 2 ** -7 * outs[1].abs() + 2e-5 * float(outs[1].abs().max())).all()
 
 
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("G,d,talk", [(2, 64, True), (1, 128, False)])
+def test_chunk_attention_keeps_a_bad_value_from_earlier_tokens(ops, G, d, talk, bad):
+    """A value in the middle of a portion that is no finite number: the tensor-core kernel's results, finite or not, are those of
+    the general kernel, so that tokens before it, and other elements, do not see it."""
+    H, page, chunk, T, at = 4, 8, 48, 90, 53
+    g = torch.Generator().manual_seed(d)
+    pages = -(-T // page)
+    cache = torch.randn(pages, G * page * 2 * d, generator=g).bfloat16()
+    cache[at // page, G * page * d + (at % page) * d + 5] = bad             # value of kv head 0, element 5
+    cache[(at + 3) // page, ((at + 3) % page) * d + 7] = bad                # a later token's key: its score alone is not finite
+    cache, qkv = cache.cuda(), torch.randn(T, H * d + 2 * G * d, generator=g).bfloat16().cuda()
+    mix = torch.rand(H, H, generator=g).cuda() if talk else None
+    c, table = _ctx([T], [0], [0], "cuda:0"), torch.arange(pages, dtype=torch.int32)[None].cuda()
+    c.work = ops.hints_for([T], [T]).work
+    got, want = (torch.zeros(T, H * d, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    ops.chunk_attention_of_step(c, qkv, None, cache, table, H, G, d, d, page, 0.2, chunk, None, None, mix, got, 0, 1.0)
+    ops.chunk_attention(qkv, None, cache, table, c.tok_req, c.positions, H, G, d, d, page, 0.2, chunk, None, None, mix, want, 0, 1.0)
+    got, want = got.double().cpu(), want.double().cpu()
+    assert torch.equal(got.isfinite(), want.isfinite()) and got[:at].isfinite().all() and not got[at:at + 3].isfinite().all()
+    fine = want.isfinite()
+    assert ((got - want)[fine].abs() <= 2 ** -7 * want[fine].abs() + 2e-5 * float(want[fine].abs().max())).all()
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 def test_row_wise_operators(ops, dtype):
     g = torch.Generator().manual_seed(3)
