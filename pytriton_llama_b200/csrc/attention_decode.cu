@@ -56,83 +56,81 @@ template <int D, int KP, int RING> struct DecodeCfg {
 
 // Many (token, kv head) pairs of contexts of any lengths (`per_head` > 0): the step's tiles are dealt out in units of at most c
 // tiles, c the smallest with at most `per_head` units per kv head, so that a request of 2,500 tokens is not one block's work beside
-// one of 250 and all units are in flight at once.  A token of n tiles gets ceil(n / c) units per kv head (one, if it has none);
-// they are numbered token by token, kv head by kv head, so that the partial results of a (token, kv head) lie side by side.
-// Every warp works its block's unit out by itself from the step's integers, before the wait.  Above 256 tokens c comes from
-// a bound instead of a search.
-struct DecodeUnit { int item, kvh, split, splits; };
-constexpr int kDecHeld = 8;                                   // tokens per lane whose lengths stay in registers
+// one of 250 and all units are in flight at once.  A token of n tiles gets ceil(n / c) units per kv head, a padding row none; units
+// are numbered token by token, kv head by kv head, so that the partial results of a (token, kv head) lie side by side.
+// decode_units_kernel works them out once for all layers of a step from the step's integers; worked out by every block of every
+// layer they cost 2 to 4 us a layer (16 layers, 64 requests of 1,408 tokens 1,576 us a step, 1,510 so; of 256 to 2,560
+// tokens 1,637 and 1,586).  Padding rows took a unit each there: 33 requests captured as 64 1,417 us, 1,333 so.  One block.
+struct DecodeUnit { int t, r, p, kvh, split, splits, pad, pad_kvh; };      // t -1: nothing; pad: a padding row whose zeros the block stores, or -1
+constexpr int kDecPlanItems = 1024;
 
-__device__ __forceinline__ int decode_tiles(const int* items, const int* tok_req, const int* positions, int i, int window, int tile_keys) {
-  const int t = items ? __ldcg(items + i) : i;
-  const int p = __ldcg(positions + t);
-  const int keys = window > 0 && p + 1 > window ? window : p + 1;
-  return __ldcg(tok_req + t) < 0 ? 0 : (keys + tile_keys - 1) / tile_keys;
-}
-
-template <int KEYS>
-__device__ __forceinline__ DecodeUnit decode_unit(const int* items, const int* tok_req, const int* positions, int n_items, int nkv,
-                                                  int window, int per_head, int max_splits, int unit) {
-  const int lane = threadIdx.x & 31;
-  const bool few = n_items <= 32 * kDecHeld;
-  int held[kDecHeld], total = 0, longest = 1;
-#pragma unroll
-  for (int j = 0; j < kDecHeld; ++j) {
-    const int i = lane + 32 * j;
-    held[j] = few && i < n_items ? decode_tiles(items, tok_req, positions, i, window, KEYS) : 0;
-    total += held[j];
-    longest = max(longest, held[j]);
+__global__ void __launch_bounds__(kDecPlanItems)
+decode_units_kernel(int4* __restrict__ units, const int* __restrict__ items, const int* __restrict__ tok_req,
+                    const int* __restrict__ positions, int n_items, int nkv, int window, int per_head, int tile_keys, int max_splits) {
+  __shared__ int s_t[kDecPlanItems], s_r[kDecPlanItems], s_p[kDecPlanItems], s_tiles[kDecPlanItems], s_first[kDecPlanItems + 1];
+  __shared__ int s_sum[32], s_max[32], s_fits[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  pdl_wait();
+  pdl_launch_dependents();
+  int t = -1, r = -1, p = -1, tiles = 0;
+  if (tid < n_items) {
+    t = items ? items[tid] : tid;
+    r = tok_req[t];
+    p = positions[t];
+    const int keys = window > 0 && p + 1 > window ? window : p + 1;
+    tiles = r < 0 ? 0 : max(1, (keys + tile_keys - 1) / tile_keys);
   }
-  if (!few)
-    for (int i = lane; i < n_items; i += 32) {
-      const int tiles = decode_tiles(items, tok_req, positions, i, window, KEYS);
-      total += tiles;
-      longest = max(longest, tiles);
-    }
-  total = __reduce_add_sync(0xffffffffu, total);
-  longest = __reduce_max_sync(0xffffffffu, longest);
-  int c = max((total + per_head - 1) / per_head, max(1, (longest + max_splits - 1) / max_splits));
-  if (few) {
-    int hi = longest;
-    while (c < hi) {                                          // (the same in every lane)
-      const int mid = (c + hi) / 2;
-      int units = 0;
-#pragma unroll
-      for (int j = 0; j < kDecHeld; ++j)
-        if (32 * j < n_items) units += lane + 32 * j < n_items ? max(1, (held[j] + mid - 1) / mid) : 0;
-      if ((int)__reduce_add_sync(0xffffffffu, units) <= per_head) hi = mid; else c = mid + 1;
-    }
-  } else {
-    c = per_head > n_items ? max(c, (total + per_head - n_items - 1) / (per_head - n_items)) : longest;
+  s_t[tid] = t; s_r[tid] = r; s_p[tid] = p; s_tiles[tid] = tiles;
+  const int warp_total = __reduce_add_sync(0xffffffffu, tiles), warp_longest = __reduce_max_sync(0xffffffffu, tiles);
+  if (lane == 0) { s_sum[warp] = warp_total; s_max[warp] = warp_longest; }
+  __syncthreads();
+  const int total = __reduce_add_sync(0xffffffffu, s_sum[lane]), longest = max(1, __reduce_max_sync(0xffffffffu, s_max[lane]));
+  // 32 lengths are tried at once, one per warp; `hi` always fits, since there are no more tokens than units
+  int lo = max(max(1, (total + per_head - 1) / per_head), (longest + max_splits - 1) / max_splits), hi = max(lo, longest);
+  while (lo < hi) {
+    const int step = (hi - lo + 30) / 31, mine = min(hi, lo + warp * step);
+    int sum = 0;
+    for (int i = lane; i < n_items; i += 32) sum += (s_tiles[i] + mine - 1) / mine;
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    __syncthreads();
+    if (lane == 0) s_fits[warp] = sum <= per_head;
+    __syncthreads();
+    const unsigned fits = __ballot_sync(0xffffffffu, s_fits[lane]);
+    const int first = fits ? __ffs(fits) - 1 : 31;
+    hi = min(hi, lo + first * step);
+    lo = first ? min(hi, lo + (first - 1) * step + 1) : hi;
   }
-  int before = 0;                                             // units of the tokens before, per kv head
-  for (int i0 = 0; i0 < n_items; i0 += 32) {
-    const int i = i0 + lane;
-    int tiles = 0;
-    if (few) {
+  const int c = hi, mine = (tiles + c - 1) / c;
+  int incl = mine;
 #pragma unroll
-      for (int j = 0; j < kDecHeld; ++j)
-        if (i0 == 32 * j) tiles = held[j];
-    } else if (i < n_items) {
-      tiles = decode_tiles(items, tok_req, positions, i, window, KEYS);
-    }
-    const int mine = i < n_items ? max(1, (tiles + c - 1) / c) : 0;
-    int incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int below = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += below;
-    }
-    const unsigned past = __ballot_sync(0xffffffffu, unit < (before + incl) * nkv);
-    if (past) {
-      const int who = __ffs(past) - 1;
-      const int n = __shfl_sync(0xffffffffu, mine, who), first = before + __shfl_sync(0xffffffffu, incl - mine, who);
-      const int at = unit - first * nkv;
-      return DecodeUnit{i0 + who, at / n, at % n, n};
-    }
-    before += __shfl_sync(0xffffffffu, incl, 31);
+  for (int o = 1; o < 32; o <<= 1) {
+    const int below = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += below;
   }
-  return DecodeUnit{-1, 0, 0, 1};
+  __syncthreads();
+  if (lane == 31) s_sum[warp] = incl;
+  __syncthreads();
+  int before = 0;
+  for (int w = 0; w < warp; ++w) before += s_sum[w];
+  s_first[tid] = before + incl - mine;                        // units of the tokens before, per kv head
+  if (tid == kDecPlanItems - 1) s_first[kDecPlanItems] = before + incl;
+  __syncthreads();
+  const int units_per_head = s_first[kDecPlanItems];
+  for (int u = tid; u < nkv * per_head; u += kDecPlanItems) {
+    DecodeUnit unit{-1, -1, -1, 0, 0, 1, -1, 0};
+    if (u / nkv < units_per_head) {
+      int i = 0;                                              // the last token that begins at or before this unit
+#pragma unroll
+      for (int half = kDecPlanItems / 2; half; half >>= 1)
+        if (s_first[i + half] <= u / nkv) i += half;
+      const int n = s_first[i + 1] - s_first[i], at = u - s_first[i] * nkv;
+      unit.t = s_t[i]; unit.r = s_r[i]; unit.p = s_p[i];
+      unit.kvh = at / n; unit.split = at % n; unit.splits = n;
+    }
+    if (u < n_items * nkv && s_r[u / nkv] < 0) { unit.pad = s_t[u / nkv]; unit.pad_kvh = u % nkv; }
+    units[2 * u] = make_int4(unit.t, unit.r, unit.p, unit.kvh);
+    units[2 * u + 1] = make_int4(unit.split, unit.splits, unit.pad, unit.pad_kvh);
+  }
 }
 
 template <int D, int KP, int RING>
@@ -144,7 +142,8 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap map_kv, __nv_bfloat1
                         int out_stride, int bt_stride, int nq, int nkv, int page_size, float scale_log2,
                         int window, int splits, int num_pages, int page_shift, int* __restrict__ counters,
                         int cluster_merge, int fused, const float* __restrict__ inv_freq,
-                        const int* __restrict__ slots, unsigned long long* timeline, int n_items, int per_head, int* status) {
+                        const int* __restrict__ slots, unsigned long long* timeline, const int4* __restrict__ unit_list, int units_early,
+                        int* status) {
   using Cfg = DecodeCfg<D, KP, RING>;
   constexpr int kDecKeys = Cfg::kKeys;
   constexpr int kDecKP = KP;
@@ -160,21 +159,30 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap map_kv, __nv_bfloat1
   // predecessor writes q and the slot of position p).  So it runs under the predecessor's tail.
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, c = lane & 3;
-  int split = blockIdx.x % splits;
-  int kvh = (blockIdx.x / splits) % nkv;
-  int ti = blockIdx.x / (splits * nkv);
-  if (per_head) {
-    const DecodeUnit unit = decode_unit<kDecKeys>(items, tok_req, positions, n_items, nkv, window, per_head, Cfg::kMaxSums / (nq / nkv), blockIdx.x);
-    if (unit.item < 0) return;                                // (no cluster in this form: nobody waits for this block)
-    split = unit.split;
-    splits = unit.splits;
-    kvh = unit.kvh;
-    ti = unit.item;
-  }
-  const int t = items ? __ldcg(items + ti) : ti;
   const int G = nq / nkv;
-  const int r = __ldcg(tok_req + t);
-  const int p = __ldcg(positions + t);
+  int split, kvh, t, r, p, pad = -1, pad_kvh = 0;
+  const bool dealt = RING && unit_list != nullptr;
+  auto store_padding = [&]() {
+    for (int e = tid; e < G * D; e += kDecWarps * 32) out[(size_t)pad * out_stride + (size_t)pad_kvh * G * D + e] = __float2bfloat16_rn(0.f);
+  };
+  if (dealt) {
+    if (!units_early) pdl_wait();                             // (the step's first layer: the units come from the kernel before)
+    const int4 a = __ldcg(unit_list + 2 * blockIdx.x), b = __ldcg(unit_list + 2 * blockIdx.x + 1);
+    t = a.x; r = a.y; p = a.z; kvh = a.w;
+    split = b.x; splits = b.y; pad = b.z; pad_kvh = b.w;
+    if (t < 0) {                                              // (no cluster in this form: nobody waits for this block)
+      pdl_wait();
+      if (pad >= 0) store_padding();
+      return;
+    }
+  } else {
+    split = blockIdx.x % splits;
+    kvh = (blockIdx.x / splits) % nkv;
+    const int ti = blockIdx.x / (splits * nkv);
+    t = items ? __ldcg(items + ti) : ti;
+    r = __ldcg(tok_req + t);
+    p = __ldcg(positions + t);
+  }
   const int lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
   const int nkeys = r < 0 ? 0 : p - lo + 1;
   int chunk_keys = (nkeys + splits - 1) / splits;
@@ -304,6 +312,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap map_kv, __nv_bfloat1
   }
   pdl_wait();
   pdl_launch_dependents();
+  if (dealt && pad >= 0) store_padding();
   if (tid == 0) timeline_stamp(timeline, 1);
   // With `fused`, the block whose key range ends at position p owns the token's new key and
   // value: it rotates the key, sends both to the cache (for later steps; nothing in this step waits
@@ -602,7 +611,7 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap map_kv, __nv_bfloat1
     if (splits == 1) {
       out[(size_t)t * out_stride + (size_t)h * D + col] = __float2bfloat16_rn(L > 0.f ? acc / L : 0.f);
     } else {
-      const size_t idx = per_head ? (size_t)blockIdx.x * G + row : ((size_t)t * nq + h) * splits + split;
+      const size_t idx = dealt ? (size_t)blockIdx.x * G + row : ((size_t)t * nq + h) * splits + split;
       part_acc[idx * D + col] = acc;
       if (col == 0) {
         part_ml[idx * 2] = M == -INFINITY ? -INFINITY : M * 0.6931471805599453f;   // natural-log units for the merge
@@ -627,8 +636,8 @@ decode_attention_kernel(const __grid_constant__ CUtensorMap map_kv, __nv_bfloat1
   __threadfence();
   // partial results of the group's heads are contiguous: [G][splits][D] and [G][splits][2], or, dealt out in units,
   // [splits][G][D] from the first unit of this (token, kv head) on
-  const size_t idx0 = per_head ? (size_t)(blockIdx.x - split) * G : ((size_t)t * nq + (size_t)kvh * G) * splits;
-  const size_t of_head = per_head ? 1 : splits, of_split = per_head ? G : 1;
+  const size_t idx0 = dealt ? (size_t)(blockIdx.x - split) * G : ((size_t)t * nq + (size_t)kvh * G) * splits;
+  const size_t of_head = dealt ? 1 : splits, of_split = dealt ? G : 1;
   float* w = reinterpret_cast<float*>(smem);                   // [G][splits] maxima m, then weights e^{m - M}
   float* lz = w + G * splits;                                  // [G][splits] sums l
   float* inv_l = lz + G * splits;                              // [G]
@@ -720,7 +729,7 @@ int launch_decode(const CUtensorMap& map_kv, int* status, void* out, float* part
                   const int* block_table, const int* items, const int* tok_req, const int* positions, int n_items,
                   int q_stride, int out_stride, int bt_stride, int nq, int nkv, int page_size, float scale,
                   int window, int splits, int num_pages, int* counters, void* stream, int fused,
-                  const float* inv_freq, const int* slots, int per_head) {
+                  const float* inv_freq, const int* slots, int per_head, const int* units, int units_early) {
   using Cfg = DecodeCfg<D, KP, RING>;
   constexpr int kSmem = Cfg::kSmem + Cfg::kAlign;
   static SmemRaised raised = {};                         // level 1: the ring; 2: the ring and the rows a cluster exchanges
@@ -741,7 +750,8 @@ int launch_decode(const CUtensorMap& map_kv, int* status, void* out, float* part
                                  (__nv_bfloat16*)out, part_acc, part_ml, (const __nv_bfloat16*)q,
                                  (const __nv_bfloat16*)cache, block_table, items, tok_req, positions, q_stride, out_stride, bt_stride,
                                  nq, nkv, page_size, scale * 1.4426950408889634f, window, splits, num_pages, page_shift, counters,
-                                 cluster ? 1 : 0, fused, inv_freq, slots, timeline_slot(), n_items, per_head, status);
+                                 cluster ? 1 : 0, fused, inv_freq, slots, timeline_slot(),
+                                 per_head ? (const int4*)units : nullptr, units_early, status);
   if (rc) return rc;
   if (cluster || per_head) return 0;
   if (splits > 1 && counters == nullptr)
@@ -758,7 +768,7 @@ static int decode_attention_entry(void* out, float* part_acc, float* part_ml, co
                                   int n_items, int q_stride, int out_stride, int bt_stride, int nq, int nkv, int d,
                                   int page_size, float scale, int window, int splits, int num_pages, int* counters,
                                   void* stream, int fused, const float* inv_freq, const int* slots, int per_head = 0,
-                                  int* status = nullptr) {
+                                  const int* units = nullptr, int units_early = 0, int* status = nullptr) {
   PTL_REQUIRE(n_items >= 0 && nq > 0 && nkv > 0 && page_size > 0 && num_pages > 0, "decode_attention: bad sizes");
   PTL_REQUIRE(nq % nkv == 0, "decode_attention: %d query heads are no multiple of %d kv heads", nq, nkv);
   if ((d != 64 && d != 128) || nq / nkv > 16) return -2;
@@ -766,14 +776,14 @@ static int decode_attention_entry(void* out, float* part_acc, float* part_ml, co
   PTL_REQUIRE(counters == nullptr || splits <= 512, "decode_attention: at most 512 splits with in-kernel merging");
   PTL_REQUIRE(aligned16(q) && aligned16(cache) && q_stride % 8 == 0, "decode_attention: q and cache must be 16-byte aligned");
   PTL_REQUIRE(!fused || q_stride >= (nq + 2 * nkv) * d, "decode_attention: the fused form needs the whole q|k|v row, %d < %d", q_stride, (nq + 2 * nkv) * d);
-  PTL_REQUIRE(per_head == 0 || (per_head >= n_items && counters && part_acc && part_ml && splits == 1),
-              "decode_attention: units of equal length need scratch buffers and counters");
+  PTL_REQUIRE(per_head == 0 || (per_head >= n_items && counters && part_acc && part_ml && splits == 1 && units && aligned16(units)),
+              "decode_attention: units of equal length need their list, scratch buffers and counters");
   if (n_items == 0) return 0;
   // the in-kernel merge keeps a maximum and a sum per (head of the group, split) in shared memory
   if ((long long)(nq / nkv) * splits > 4096) counters = nullptr;
 #define PTL_DECODE_ARGS map, status, out, part_acc, part_ml, q, cache, block_table, items, tok_req, positions, n_items, q_stride, \
                         out_stride, bt_stride, nq, nkv, page_size, scale, window, splits, num_pages, counters, stream, \
-                        fused, inv_freq, slots, per_head
+                        fused, inv_freq, slots, per_head, units, units_early
   CUtensorMap map{};
   if (status) {
     if (page_size % 16 || num_pages > 0x3ffffff0 || (long long)nkv * page_size > 0x7ffffff0LL) return -2;
@@ -831,17 +841,32 @@ PTL_EXPORT int ptl_decode_attention_rope_bf16(void* out, float* part_acc, float*
                                      num_pages, counters, stream, 1, inv_freq, slots);
 }
 
+// The units that a step's single tokens are dealt out in, for ptl_decode_attention_pages_bf16 with the same sizes: 8 ints for
+// each of nkv * per_head blocks.  -2: more tokens than one block lays out.
+PTL_EXPORT int ptl_decode_units(int* units, const int* items, const int* tok_req, const int* positions, int n_items, int nq, int nkv, int d,
+                                int window, int per_head, void* stream) {
+  using namespace ptl;
+  if (n_items > kDecPlanItems || (d != 64 && d != 128)) return -2;
+  PTL_REQUIRE(n_items > 0 && nkv > 0 && nq % nkv == 0 && nq / nkv <= 16 && per_head >= n_items && (long long)nkv * per_head <= (1 << 24) &&
+                  units && aligned16(units), "decode_units: bad sizes");
+  static_assert(DecodeCfg<64, 1, 3>::kKeys == DecodeCfg<128, 1, 2>::kKeys, "the forms that take units have tiles of one size");
+  const int max_splits = (d == 64 ? DecodeCfg<64, 1, 3>::kMaxSums : DecodeCfg<128, 1, 2>::kMaxSums) / (nq / nkv);
+  return launch_kernel("decode_units", decode_units_kernel, dim3(1), dim3(kDecPlanItems), 0, as_stream(stream), (int4*)units, items, tok_req,
+                       positions, n_items, nkv, window, per_head, (int)DecodeCfg<64, 1, 3>::kKeys, max_splits);
+}
+
 // Either form (fused != 0: as ptl_decode_attention_rope_bf16) for pages of whole sixteens of positions, fetched by TMA; -2 for
-// others.  per_head > 0, at least n_items: the step's keys dealt out in at most that many units per kv head (splits is 1,
-// part_acc [nkv * per_head][nq / nkv][d], part_ml [...][2]).  *status: raised when a wait for a copy gave up.
+// others.  per_head > 0, at least n_items: the step's keys dealt out in at most that many units per kv head, which `units` lists
+// (ptl_decode_units; splits is 1, part_acc [nkv * per_head][nq / nkv][d], part_ml [...][2]).  `units_early`: the list was written before a
+// kernel ran that the one ahead of this waited for.  *status: raised when a wait for a copy gave up.
 PTL_EXPORT int ptl_decode_attention_pages_bf16(void* out, float* part_acc, float* part_ml, const void* q, void* cache,
                                                const int* block_table, const int* items, const int* tok_req,
                                                const int* positions, int n_items, int q_stride, int out_stride, int bt_stride,
                                                int nq, int nkv, int d, int page_size, float scale, int window, int splits, int per_head,
-                                               int num_pages, int* counters, int fused, const float* inv_freq, const int* slots,
+                                               const int* units, int units_early, int num_pages, int* counters, int fused, const float* inv_freq, const int* slots,
                                                int* status, void* stream) {
   PTL_REQUIRE(status != nullptr, "decode_attention: needs a status word");
   return ptl::decode_attention_entry(out, part_acc, part_ml, q, cache, block_table, items, tok_req, positions, n_items,
                                      q_stride, out_stride, bt_stride, nq, nkv, d, page_size, scale, window, splits, num_pages, counters,
-                                     stream, fused, inv_freq, slots, per_head, status);
+                                     stream, fused, inv_freq, slots, per_head, units, units_early, status);
 }

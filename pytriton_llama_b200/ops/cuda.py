@@ -157,8 +157,10 @@ def load_library() -> ctypes.CDLL:
                                                    _ptr, _ptr, _ptr]
     lib.ptl_decode_attention_rope_bf16.restype = _c_int
     lib.ptl_decode_attention_pages_bf16.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int,
-                                                    _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_int, _c_int, _c_int, _ptr, _c_int,
-                                                    _ptr, _ptr, _ptr, _ptr]
+                                                    _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_int, _c_int, _ptr, _c_int, _c_int, _ptr,
+                                                    _c_int, _ptr, _ptr, _ptr, _ptr]
+    lib.ptl_decode_units.argtypes = [_ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _ptr]
+    lib.ptl_decode_units.restype = _c_int
     lib.ptl_decode_attention_pages_bf16.restype = _c_int
     lib.ptl_prefill_attention_bf16.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int,
                                                _c_int, _c_int, _c_f, _c_int, _c_int, _ptr]
@@ -869,6 +871,7 @@ class CudaOps:
         step's positions (the table of rotary angles) is forgotten."""
         self._rope_memo = None
         self._pair_memo = {}
+        self._units_memo = {}
 
     def _pair_angles(self, positions: torch.Tensor, freq: torch.Tensor, dims: int, amplitude: float) -> torch.Tensor:
         """(cos, sin) [tokens, dims/2, 2] of position * freq, worked out once per forward pass for every table of
@@ -983,6 +986,31 @@ class CudaOps:
             self._decode_counters = torch.zeros(self._DECODE_COUNTERS, dtype=torch.int32, device=self.device)
         return self._decode_counters
 
+    def _decode_unit_list(self, dec, tok_req, positions, nq: int, nkv: int, d: int, window: int, per_head: int):
+        """(units of equal length of the step's single tokens, whether a kernel has run since that waited for their list): worked out
+        once per forward pass and stream for every kind of attention, used by every layer of that kind.  (None, False): more tokens
+        than one block lays out."""
+        memo = getattr(self, "_units_memo", None)
+        if memo is None:
+            memo = self._units_memo = {}
+        stream = self._stream()
+        key = (stream, dec.items, dec.in_order, *(x for t in (dec.tensor, tok_req, positions) for x in (t.data_ptr(), t._version)), nq, nkv,
+               d, int(window), per_head)
+        have = memo.get(key)
+        if have is not None:
+            self.launches += have[-1]
+            have[-1] = 0
+            return have[0], True
+        units = self.empty((nkv * per_head, 8), torch.int32)
+        rc = self.lib.ptl_decode_units(_p(units), None if dec.in_order else _p(dec.tensor), _p(tok_req), _p(positions), dec.items, nq, nkv,
+                                       d, int(window), per_head, stream)
+        if rc == -2:
+            return None, False
+        self._check(rc, kernels=0)
+        # (the integers are held, so that their addresses are not given out again; the launch is counted where its list serves a second layer)
+        memo[key] = [units, dec.tensor, tok_req, positions, 1]
+        return units, False
+
     def _attention_tensor_cores(self, out, q, cache, block_table, tok_req, positions, nq, nkv, d, page_size, scale,
                                 window, hints, rope=None) -> None:
         """bfloat16 attention on the tensor cores: single tokens through the split-key decode kernel,
@@ -1014,8 +1042,10 @@ class CudaOps:
             tickets = q.shape[0] * nkv <= self._DECODE_COUNTERS and getattr(hints, "decode_counters", True)
             # Pages of whole sixteens are fetched by TMA.  Up to 148 pairs go in clusters where those fill three quarters of their 296
             # blocks or the contexts are short; more pairs in units of equal length, as many as fit at once (a batch of unequal
-            # contexts otherwise ends with the long ones' blocks alone: a step of 64 requests of 256 to 2,560 tokens, heads of 64,
-            # 1,742 us whole by cp.async, 1,625 in units; all of 1,408: 1,516 and 1,550); pairs beyond 7/8 of what fits at once go
+            # contexts otherwise ends with the long ones' blocks alone).  Steps of the 1B shape (heads of 64), by cp.async in equal splits
+            # and in units: 64 requests of 256 to 2,560 tokens 1,733 and 1,586 us, 33 (captured for 64) 1,641 and 1,333, 24 of 100 to
+            # 3,000 1,373 and 1,140, 32 of 1,000 1,139 and 1,132; only 64 equal contexts of 1,408, which cp.async
+            # shares out as well, 1,481 and 1,510.  Pairs beyond 7/8 of what fits at once go
             # whole with heads of 128 (200 requests of 64 to 1,024: 72 us, 98 by cp.async).  Few pairs of long contexts go in units
             # too with heads of 128 (one of 131,072 tokens: 92 us, 104 by splits).  With heads of 64 these two keep the
             # cp.async form (a step of 100 requests of 500: 2,855 us and 2,881; one context of 131,072: 51 us and 55).
@@ -1028,7 +1058,11 @@ class CudaOps:
                     parts = 1
                     if not whole:
                         per_head = max(self.DECODE_UNITS[d] // nkv, n_decode)
-                part_acc = part_ml = None
+                part_acc = part_ml = units = None
+                early = False
+                if per_head:
+                    units, early = self._decode_unit_list(dec, tok_req, positions, nq, nkv, d, window, per_head)
+                    per_head = per_head if units is not None else 0
                 if per_head:
                     part_acc = self.empty((nkv * per_head, group, d), torch.float32)
                     part_ml = self.empty((nkv * per_head, group, 2), torch.float32)
@@ -1038,7 +1072,7 @@ class CudaOps:
                 rc = self.lib.ptl_decode_attention_pages_bf16(
                     _p(out), _p(part_acc), _p(part_ml), _p(q), _p(cache), _p(block_table), None if dec.in_order else _p(dec.tensor),
                     _p(tok_req), _p(positions), n_decode, q.shape[1], nq * d, block_table.shape[1], nq, nkv, d, page_size, float(scale),
-                    int(window), parts, per_head, num_pages, _p(self._decode_tickets()), int(rope is not None),
+                    int(window), parts, per_head, _p(units), int(early), num_pages, _p(self._decode_tickets()), int(rope is not None),
                     _p(rope[0]) if rope is not None else None, _p(rope[1]) if rope is not None else None, _p(self._tc_status_word()),
                     stream)
                 if rc != -2:
