@@ -1045,14 +1045,15 @@ class CudaOps:
             # contexts otherwise ends with the long ones' blocks alone).  Steps of the 1B shape (heads of 64), by cp.async in equal splits
             # and in units: 64 requests of 256 to 2,560 tokens 1,733 and 1,586 us, 33 (captured for 64) 1,641 and 1,333, 24 of 100 to
             # 3,000 1,373 and 1,140, 32 of 1,000 1,139 and 1,132; only 64 equal contexts of 1,408, which cp.async
-            # shares out as well, 1,481 and 1,510.  Pairs beyond 7/8 of what fits at once go
-            # whole with heads of 128 (200 requests of 64 to 1,024: 72 us, 98 by cp.async).  Few pairs of long contexts go in units
-            # too with heads of 128 (one of 131,072 tokens: 92 us, 104 by splits).  With heads of 64 these two keep the
-            # cp.async form (a step of 100 requests of 500: 2,855 us and 2,881; one context of 131,072: 51 us and 55).
+            # shares out as well, 1,481 and 1,510.  Pairs beyond 7/8 of what fits at once go whole (heads of 64, by cp.async and so: 128
+            # requests of 64 to 1,024 1,668 and 1,622 us a step, of 900 to 1,000 1,886 and 1,815, 256 of 300 2,243 and 2,251; heads of
+            # 128, alone: 200 of 64 to 1,024 98 and 72 us).  Few pairs of long contexts go in units with heads of 128 (one of 131,072
+            # tokens alone: 104 us by splits and 92) and keep the cp.async form with heads of 64 (one of 30,000: 1,083 us a
+            # step and 1,092, of 100,000 1,397 and 1,411).
             parts = max(1, min(8, 296 // pairs, -(-longest // 128)))
             few_and_long = longest > self.DECODE_KEYS_PER_WIDE_BLOCK * parts and pairs * parts < 222 and pairs <= 148
             whole = pairs > 148 and pairs > self.DECODE_UNITS[d] * 7 // 8
-            if not forced and tickets and page_size % 16 == 0 and not (d == 64 and (few_and_long or whole)):
+            if not forced and tickets and page_size % 16 == 0 and not (d == 64 and few_and_long):
                 per_head = 0
                 if pairs > 148 or few_and_long:
                     parts = 1
