@@ -370,7 +370,7 @@ int gemm_simt(void* out, const void* A, const void* W, int M, int N, int K, int 
   const int vec_ok = sizeof(TI) == 4 && K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && aligned16(A) && aligned16(W) &&
                      batch_a % 4 == 0 && batch_w % 4 == 0;
   if constexpr (sizeof(TI) == 4 && sizeof(TO) == 4) {
-    if (vec_ok && N >= 16) {
+    if (vec_ok) {
       const auto few = [&](auto kernel, int mt, int rows, int warps, SmemRaised& raised) {
         const size_t smem = few_smem_bytes(mt, rows, warps);
         if (int rc = raise_shared_memory("gemm_simt_few", kernel, (int)smem, raised)) return rc;
