@@ -165,6 +165,18 @@ __device__ __forceinline__ void rope_rotate(float x1, float x2, float c, float s
   o2 = __fadd_rn(__fmul_rn(x2, c), __fmul_rn(x1, s));
 }
 
+// SMs of the current device (148, a B200's, where there is none to ask).
+inline int sm_count_of_device() {
+  static int sm_count = 0;
+  if (!sm_count) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+    if (sm_count <= 0) sm_count = 148;
+  }
+  return sm_count;
+}
+
 // ---------------------------------------------------------------- thread-block clusters
 // Arrive and wait of the cluster barrier (every thread of every block takes part), the address of
 // a peer block's shared memory, and stores into it.

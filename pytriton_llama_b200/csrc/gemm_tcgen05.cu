@@ -4,17 +4,6 @@
 
 namespace ptl {
 
-static int sm_count_of_device() {
-  static int sm_count = 0;
-  if (!sm_count) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-    if (sm_count <= 0) sm_count = 148;
-  }
-  return sm_count;
-}
-
 // The plan for a product with many tokens: features per tile (256, 192 where N is a multiple of
 // it, or 128) and, where the caller can add partial sums up, into how many parts the K range is cut.
 // The cost of a candidate is the number of rounds its work units (tiles x parts) take on the SMs times
