@@ -395,20 +395,22 @@ int gemm_simt(void* out, const void* A, const void* W, int M, int N, int K, int 
       if (M <= 16) PTL_FEW(16, 16, 4)
       if (M <= 32 && narrow) PTL_FEW(32, 8, 2)
 #undef PTL_FEW
+      // (weight rows are the grid's second dimension: more of them go to the tiles below, where they are its first)
+      const bool tiles = N <= 16 * 4 * 65535;
       const auto tiled = [&](auto kernel, int tm, int tn, SmemRaised& raised) {
         const int smem = kTileStages * (8 * tm + 16 * tn) * kTileLd * (int)sizeof(float);
         if (int rc = raise_shared_memory("gemm_simt_tile", kernel, smem, raised)) return rc;
         const dim3 grid((M + 8 * tm - 1) / (8 * tm), (N + 16 * tn - 1) / (16 * tn), batch);
-        PTL_REQUIRE(grid.y <= 65535, "gemm_simt: N=%d too large", N);
         return launch_kernel("gemm_simt_tile", kernel, grid, dim3(kTileThreads), smem, as_stream(stream), (float*)out, (const float*)A,
                              (const float*)W, M, N, K, lda, ldw, ldo, accumulate, batch_a, batch_w, batch_o, (const float*)gate_v, gate_ld);
       };
       static SmemRaised r88, r84, r54, r44;
-      switch (simt_tile(M, N, batch)) {
+      switch (tiles ? simt_tile(M, N, batch) : 0) {
         case 88: return tiled(gemm_simt_tile_kernel<8, 8>, 8, 8, r88);
         case 84: return tiled(gemm_simt_tile_kernel<8, 4>, 8, 4, r84);
         case 54: return tiled(gemm_simt_tile_kernel<5, 4>, 5, 4, r54);
-        default: return tiled(gemm_simt_tile_kernel<4, 4>, 4, 4, r44);
+        case 44: return tiled(gemm_simt_tile_kernel<4, 4>, 4, 4, r44);
+        default: break;
       }
     }
   }

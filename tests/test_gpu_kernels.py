@@ -707,6 +707,67 @@ def test_kernels_refuse_sizes_they_cannot_take(ops):
         ops.add_rmsnorm(torch.zeros(1, 60000, device="cuda"), None, torch.ones(60000, device="cuda"), 1e-5)
 
 
+@pytest.mark.parametrize("n, nkv, G, d, window, per_head", [(1, 8, 4, 64, 0, 74), (33, 8, 4, 64, 0, 74), (64, 8, 3, 128, 0, 64), (40, 8, 4, 64, 700, 74),
+                                                            (300, 1, 16, 128, 0, 444), (1024, 1, 1, 64, 0, 1024), (5, 2, 2, 64, 64, 9)])
+def test_units_of_a_step_of_single_tokens(ops, n, nkv, G, d, window, per_head):
+    """The list that the decode attention's blocks go by, against its definition: every real token in the fewest units that the
+    smallest fitting length makes, numbered token by token and kv head by kv head; padding rows take none of the units, and
+    every (padding row, kv head) has one block that stores its zeros."""
+    g = torch.Generator().manual_seed(n + per_head)
+    for padding in (0, n // 2, n):
+        ctx = torch.randint(1, 3000, (n,), generator=g)
+        rows = torch.randperm(n + 7, generator=g)[:n].int()
+        req, pos = torch.full((n + 7,), -1, dtype=torch.int32), torch.zeros(n + 7, dtype=torch.int32)
+        req[rows.long()], pos[rows.long()] = torch.arange(n, dtype=torch.int32), (ctx - 1).int()
+        gone = set(torch.randperm(n, generator=g)[:padding].tolist())
+        req[rows[sorted(gone)].long()] = -1
+        units = torch.full((nkv * per_head, 8), -7, dtype=torch.int32, device="cuda")
+        items, req_dev, pos_dev = rows.cuda(), req.cuda(), pos.cuda()
+        assert ops.lib.ptl_decode_units(units.data_ptr(), items.data_ptr(), req_dev.data_ptr(), pos_dev.data_ptr(), n, nkv * G, nkv, d, window,
+                                        per_head, torch.cuda.current_stream().cuda_stream) == 0
+        got, number = units.cpu().tolist(), {int(t): i for i, t in enumerate(rows)}
+        tiles = [0 if i in gone else -(-(min(int(c), window) if window else int(c)) // 64) for i, c in enumerate(ctx)]
+        splits = {}
+        for u, (t, r, p, head, split, of, _, _) in enumerate(got):
+            if t >= 0:
+                i = number[t]
+                assert (r, p) == (i, int(ctx[i]) - 1) and 0 <= split < of
+                splits.setdefault((i, head), []).append((u, split, of))
+        assert sorted(splits) == sorted((i, k) for i in range(n) if tiles[i] for k in range(nkv))
+        order = [e for key in sorted(splits) for e in splits[key]]
+        assert [u for u, _, _ in order] == list(range(len(order)))
+        assert all([s for _, s, _ in v] == list(range(v[0][2])) for v in splits.values())
+        if any(tiles):
+            length = next(c for c in range(1, 100) if sum(-(-k // c) for k in tiles) <= per_head)
+            assert all(len(v) == -(-tiles[i] // length) for (i, _), v in splits.items())
+        assert sorted((t, k) for *_, t, k in got if t >= 0) == sorted((int(rows[i]), k) for i in gone for k in range(nkv))
+
+
+@pytest.mark.parametrize("page, window", [(16, 0), (32, 300)])
+def test_decode_attention_of_more_pairs_than_fit_at_once(ops, page, window):
+    """Heads of 64, 70 requests of 8 kv heads: whole pairs, by TMA."""
+    test_decode_attention_by_pages_of_sixteen(ops, 32, 8, 64, page, window, 70, [1, 64, 65, 700, 63, 128, 2, 333])
+
+
+@pytest.mark.parametrize("N, K", [(1, 4), (3, 36), (8, 1024), (15, 2052)])
+def test_linear_float32_of_few_features(ops, N, K):
+    """Head gates and small routers: the kernels that read rows in packets of 16 bytes, at fewer features than their tiles have, give
+    the bits of wide weights' rows."""
+    test_linear_float32_gives_a_row_the_same_bits_whatever_its_company(ops, N, K)
+    x, w = rnd((200, K), torch.float32, 7).cuda(), rnd((64, K), torch.float32, 8).cuda()
+    for rows in (1, 8, 16, 30, 200):
+        assert torch.equal(ops.linear(x[:rows].contiguous(), w[:N].contiguous()), ops.linear(x[:rows].contiguous(), w)[:, :N])
+
+
+def test_linear_float32_of_more_features_than_a_grid_has_rows(ops):
+    """4.2 million weight rows: the tiles of many rows would need a second grid dimension above 65,535."""
+    N, K = 64 * 65535 + 70, 4
+    x, w = rnd((33, K), torch.float32, 7).cuda(), torch.randn(N, K, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    got = ops.linear(x, w)
+    at = torch.cat([torch.arange(100), torch.arange(N - 300, N)]).cuda()
+    assert torch.equal(got[:, at], ops.linear(x, w[at].contiguous()))
+
+
 @pytest.mark.parametrize("nq, nkv, d, page, window, rotate", [(32, 8, 64, 16, 0, True), (8, 2, 128, 32, 0, True),
                                                               (6, 3, 64, 8, 40, True), (4, 4, 64, 16, 0, False)])
 def test_decode_attention_with_rope_and_cache_write_folded_in(ops, nq, nkv, d, page, window, rotate):
