@@ -41,12 +41,11 @@ __device__ __forceinline__ void two_scale(float& hi, float& lo, float c) {
   hi = h;
 }
 
-// (Sums in one order; what is fetched ahead of them is not part of it: packets_ahead packets of a key, the
+// (Sums in one order; what is fetched ahead of them is not part of it: kPacketsAhead packets of a key, the
 // values of values_ahead keys.
 // Fetched one by one, every value waited for L2: 103 us a launch for four tokens of 32 heads at contexts of 33 to 143,
 // 39 us so.)
-// packets of a key (of up to 32 * dpl entries) per lane: the whole key, up to 16
-__host__ __device__ constexpr int packets_ahead(int dpl, int per_packet) { return 32 * dpl / per_packet < 16 ? 32 * dpl / per_packet : 16; }
+constexpr int kPacketsAhead = 16;     // packets of a key per lane: the whole key up to 64 floats
 __host__ __device__ constexpr int values_ahead(int dpl) { return dpl <= 2 ? 16 : dpl <= 4 ? 8 : 4; }
 
 template <typename T, int DPL>
@@ -82,7 +81,7 @@ paged_attention_simt_kernel(T* __restrict__ out, float* __restrict__ part_acc, f
   const int kvh = h / (nq / nkv);
   const size_t plane = (size_t)nkv * page_size * d;
   const int* bt = block_table + (size_t)(r < 0 ? 0 : r) * bt_stride;
-  constexpr int VN = Vec16<T>::N, kPacketsAhead = packets_ahead(DPL, VN);
+  constexpr int VN = Vec16<T>::N;
 
   float m = -INFINITY, l = 0.f, l_lo = 0.f;
   float acc[DPL], acc_lo[DPL];
