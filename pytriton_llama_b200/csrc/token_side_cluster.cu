@@ -52,21 +52,18 @@ token_side_cluster_kernel(float* __restrict__ residual, const __nv_bfloat16* __r
   const int rank = blockIdx.x % kTsBlocks, t0 = blockIdx.x / kTsBlocks * kTsTokens, c0 = rank * SL;
   const int nt = min(kTsTokens, n_tokens - t0);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c2 = (lane & 3) * 2;
-  // the weights, and this thread's table entries: written by no kernel of the step
+  // the weights: written by no kernel of the step
   for (int i = tid; i < dim * (SL / 8); i += kTsThreads)
     cp_async_16(smem_u32(wg + (i / (SL / 8)) * LB + i % (SL / 8) * 8), w_gate + (size_t)(i / (SL / 8)) * width + c0 + i % (SL / 8) * 8, true);
   for (int i = tid; i < SL * (dim / 8); i += kTsThreads)
     cp_async_16(smem_u32(wp + (i / (dim / 8)) * LD + i % (dim / 8) * 8), w_proj + (size_t)(c0 + i / (dim / 8)) * dim + i % (dim / 8) * 8, true);
   cp_async_commit();
   const bool own = tid < kTsTokens * per;
-  float entry = 0.f;
-  if (own && tid / per < nt) {
-    int tok = tokens[t0 + tid / per];
-    if (tok < 0 || tok >= vocab) tok = 0;
-    entry = __bfloat162float(table[(size_t)tok * table_ld + column + rank * per + tid % per]);
-  }
   pdl_wait();
   pdl_launch_dependents();
+  // this thread's table entry: a kernel of the step may have written the token; nothing needs the entry before the second barrier
+  const bool live = own && tid / per < nt;
+  int tok = live ? tokens[t0 + tid / per] : 0;
   for (int i = tid; i < kTsTokens * (SL / 4); i += kTsThreads) {
     const int r = i / (SL / 4), c = i % (SL / 4) * 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -86,6 +83,8 @@ token_side_cluster_kernel(float* __restrict__ residual, const __nv_bfloat16* __r
 #pragma unroll
     for (int e = 0; e < 4; ++e) ts_split((&v.x)[e], s16 + r * LB + c + e, kTsTokens * LB);
   }
+  if (tok < 0 || tok >= vocab) tok = 0;
+  const __nv_bfloat16 entry = live ? table[(size_t)tok * table_ld + column + rank * per + tid % per] : __float2bfloat16_rn(0.f);
   cp_async_wait<0>();
   __syncthreads();
   const int lm_row = lane & 15, lm_half = lane >> 4;
@@ -119,7 +118,7 @@ token_side_cluster_kernel(float* __restrict__ residual, const __nv_bfloat16* __r
     float z = 0.f;
 #pragma unroll
     for (int b = 0; b < kTsBlocks; ++b) z += zrecv[(b * kTsTokens + row) * per + d];
-    const float v = ts_gelu_tanh(z) * entry;
+    const float v = ts_gelu_tanh(z) * __bfloat162float(entry);
 #pragma unroll
     for (int b = 0; b < kTsBlocks; ++b) st_peer_f32(map_to_peer(smem_u32(g32 + row * dim + rank * per + d), b), v);
   }

@@ -32,6 +32,17 @@ def test_peers_run_before_their_shared_memory_is_touched(source, name, body):
     assert waits and waits[0] < PEER_ACCESS.search(body).start(), f"{source}: {name}"
 
 
+@pytest.mark.parametrize("name,inputs", [("token_side_cluster_kernel", ["tokens", "table", "residual"]), ("sample_cluster_kernel", ["logits"]),
+                                         ("decode_units_kernel", ["items", "tok_req", "positions"])])
+def test_what_a_kernel_of_the_step_may_have_written_is_read_after_the_wait(name, inputs):
+    """Reads above the wait on the predecessor are for what no kernel of the step writes; the step's tokens are not (a device kernel
+    puts the sampled ones in), nor is what is read by them."""
+    body = next(b for _, n, b in KERNELS if n == name)
+    for array in inputs:
+        read = re.search(rf"\b{array}\s*(?:\[|\+)", body)
+        assert read and body.index("pdl_wait()") < read.start(), (name, array)
+
+
 def test_the_kernels_with_clusters_are_found():
     found = {name for _, name, body in KERNELS if PEER_ACCESS.search(body)}
     assert {"decode_attention_kernel", "gemm_tc_kernel", "sample_cluster_kernel", "token_side_cluster_kernel"} <= found
