@@ -221,13 +221,13 @@ selective_scan_kernel(T* __restrict__ out, const T* __restrict__ xc, const float
   pdl_wait();
   pdl_launch_dependents();
   const int r = blockIdx.y;
-  const int lo = q_start[r], hi = q_start[r + 1];
-  if (hi <= lo || hi - lo > walk_max || state_slot[r] < 0) return;      // (longer portions: the segments below)
+  const int lo = q_start[r], hi = q_start[r + 1], slot = state_slot[r];      // (three loads side by side)
+  if (hi <= lo || hi - lo > walk_max || slot < 0) return;                    // (longer portions: the segments below)
   const int sub = threadIdx.x & 7, grp = threadIdx.x >> 3;
   const int c0 = blockIdx.x * 16;
   const bool live = c0 + grp < inner;
   const int c = live ? c0 + grp : inner - 1;          // lanes past the end shadow the last channel and store nothing
-  float* st = state + ((size_t)state_slot[r] * inner + c) * n_state;
+  float* st = state + ((size_t)slot * inner + c) * n_state;
   const bool from_zero = positions[lo] == 0;
   float S[NPL], a[NPL];
 #pragma unroll
@@ -435,8 +435,8 @@ gated_delta_rule_kernel(float* __restrict__ out, const T* __restrict__ qkv, cons
   pdl_wait();
   pdl_launch_dependents();
   const int r = blockIdx.z, h = blockIdx.y;
-  const int lo = q_start[r], hi = q_start[r + 1];
-  if (hi <= lo || hi - lo > walk_max || state_slot[r] < 0) return;      // (longer portions: delta_chunks.cu)
+  const int lo = q_start[r], hi = q_start[r + 1], slot = state_slot[r];      // (three loads side by side)
+  if (hi <= lo || hi - lo > walk_max || slot < 0) return;                    // (longer portions: delta_chunks.cu)
   const int sub = threadIdx.x & 7, grp = threadIdx.x >> 3;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int j0 = blockIdx.x * 16;
@@ -444,7 +444,7 @@ gated_delta_rule_kernel(float* __restrict__ out, const T* __restrict__ qkv, cons
   const int j = live ? j0 + grp : dv - 1;
   const int c = h / (heads / kv_heads);
   const int ld = 2 * kv_heads * d + heads * dv;
-  float* st = state + (((size_t)state_slot[r] * heads + h) * d) * dv + j;
+  float* st = state + (((size_t)slot * heads + h) * d) * dv + j;
   const bool from_zero = positions[lo] == 0;
   float2 S[HP];
 #pragma unroll
