@@ -121,7 +121,7 @@ __device__ __forceinline__ void store_result(float* __restrict__ out, size_t at,
 // a chunk's sum is the same chain of FMAs as anywhere else; the chunk sums of a round of turns meet in shared memory, where a
 // warp of its own adds them in order while the others are at the next round.  Weights and tokens come by cp.async into rows of 36 floats per chunk (a
 // quarter warp reads 8 chunks' packets from 32 different banks); the first turn's weights are asked for before the wait
-// on the predecessor, and a warp asks for its next turn as soon as it has multiplied the last.  What a warp cannot do is
+// on the predecessor (weights that a kernel of the step has written need an ordinary launch), and a warp asks for its next turn as soon as it has multiplied the last.  What a warp cannot do is
 // multiply one turn while it waits for the next, so the blocks are small and many warps share an SM: 8 rows and four warps (three blocks an
 // SM) against 16 rows and two warps 35 us and 47 (4 rows of 2,048 to 16,384 features), 16 rows and four warps from 9 rows on, where
 // the tokens' share of the copies counts (16 rows: 87 us against 101).  The tile kernel with 32 x 16 tiles that stood here

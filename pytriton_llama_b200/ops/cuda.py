@@ -487,9 +487,9 @@ class CudaOps:
         """x[T, K] @ w[N, K]^T.  float32: the library's own FFMA kernel (true 32-bit);
         bfloat16: the tensor-core product of this library (a cuBLAS product for sizes it leaves out).
         ``x`` may be a ``NormedActivation``.  ``fresh_weights``: ``w`` was written by an earlier kernel of the same
-        step (keys gathered for a product of queries against them).  The tensor-core kernel asks for its first weight
-        tiles before it waits for the kernel ahead of it, which is right for a model's weights only; such a product
-        is therefore launched as an ordinary successor of what runs before it."""
+        step (keys gathered for a product of queries against them).  The tensor-core kernels and, in float32, the kernel for
+        few rows ask for their first weights before they wait for the kernel ahead of them, which is right for a model's weights
+        only; such a product is therefore launched as an ordinary successor of what runs before it, in either type."""
         if fresh_weights and self.lib.ptl_get_dependent_launch():
             self.lib.ptl_set_dependent_launch(0)
             try:

@@ -759,6 +759,19 @@ def test_linear_float32_of_few_features(ops, N, K):
         assert torch.equal(ops.linear(x[:rows].contiguous(), w[:N].contiguous()), ops.linear(x[:rows].contiguous(), w)[:, :N])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_linear_with_weights_that_the_kernel_ahead_has_written(ops, dtype):
+    """``fresh_weights``, in both types: the product waits for the kernel that wrote its weights, which lets its successors start early."""
+    g = torch.Generator().manual_seed(3)
+    a, b = (torch.randn(n, 256, generator=g).to(dtype).cuda() for n in (4096, 512))
+    x = torch.randn(4, 512, generator=g).to(dtype).cuda()
+    w = ops.linear(a, b)
+    torch.cuda.synchronize()
+    want = ops.linear(x, w)
+    for _ in range(20):
+        assert torch.equal(ops.linear(x, ops.linear(a, b), fresh_weights=True), want)
+
+
 def test_linear_float32_of_more_features_than_a_grid_has_rows(ops):
     """4.2 million weight rows: the tiles of many rows would need a second grid dimension above 65,535."""
     N, K = 64 * 65535 + 70, 4
