@@ -2328,10 +2328,11 @@ class CudaOps:
     def sample_tokens(self, logits: torch.Tensor, temperature: Optional[torch.Tensor], top_p: Optional[torch.Tensor],
                       u: Optional[torch.Tensor], out: Optional[torch.Tensor] = None, logprobs: bool = False):
         """(``sample``'s tokens, with ``logprobs`` their ``token_logprobs``, else None) in one launch, for vocabularies of up to
-        131,072 tokens; larger ones by those two.  Greedy rows without log-probabilities have ``sample``'s two short launches."""
+        131,072 tokens and for not too many rows; others by those two, with the same tokens.  Greedy rows without log-probabilities
+        have ``sample``'s two short launches."""
         self._want(logits, "logits", torch.float32)
         rows, vocab = logits.shape
-        if vocab > self.SAMPLE_CLUSTER_VOCAB or (temperature is None and not logprobs):
+        if vocab > self.SAMPLE_CLUSTER_VOCAB or (temperature is None and not logprobs) or not self.samples_in_one_launch(rows, vocab):
             tokens = self.sample(logits, temperature, top_p, u, out=out)
             return tokens, self.token_logprobs(logits, tokens) if logprobs else None
         if out is None:
@@ -2349,6 +2350,13 @@ class CudaOps:
         return out, lp
 
     SAMPLE_CLUSTER_VOCAB = 131072
+
+    @staticmethod
+    def samples_in_one_launch(rows: int, vocab: int) -> bool:
+        """The one launch keeps eight blocks of 1,024 threads on a row, 18 rows at a time; the several launches spread their rows over
+        all SMs.  With the host's part of the call (numbers per row, a copy), several and one, for 128,256 tokens: 8 rows 83 and 47
+        us, 64 169 and 154, 128 266 and 286, 512 884 and 1,056; up to 32,768 the host's part decides (512 rows of 32,000: 835 and 790)."""
+        return rows <= 64 or vocab <= 32768
 
     def sample(self, logits: torch.Tensor, temperature: Optional[torch.Tensor], top_p: Optional[torch.Tensor],
                u: Optional[torch.Tensor], out: Optional[torch.Tensor] = None) -> torch.Tensor:

@@ -658,6 +658,18 @@ def test_sampling_in_one_launch_gives_the_tokens_of_the_several(ops, rows, vocab
     assert torch.equal(ops.sample_tokens(logits, None, None, None, logprobs=True)[0], ops.sample(logits, None, None, None))
 
 
+@pytest.mark.parametrize("rows, vocab, launches", [(64, 40000, 1), (65, 40000, 8), (70, 32768, 1)])
+def test_sampling_of_many_rows_by_the_several_launches(ops, rows, vocab, launches):
+    """Above 64 rows of a large vocabulary the several launches are the faster ones; the tokens are the same."""
+    g = torch.Generator().manual_seed(rows)
+    logits = torch.randn(rows, vocab, generator=g).cuda() * 2
+    t, p, u = (x.cuda() for x in (torch.full((rows,), 0.8), torch.linspace(0.3, 1.0, rows), torch.rand(rows, generator=g)))
+    want, before = ops.sample(logits, t, p, u), ops.launches
+    got, lp = ops.sample_tokens(logits, t, p, u, logprobs=True)
+    assert ops.launches - before == launches
+    assert torch.equal(got, want) and (lp - ops.token_logprobs(logits, want)).abs().max() <= 2e-5
+
+
 @pytest.mark.parametrize("vocab", [37, 32769, 131073])
 def test_sampling_gives_no_mass_to_logits_that_are_no_numbers(ops, vocab):
     """Rows with several NaNs, far apart and side by side, and rows with infinities: one token, the same from both kernels, and
