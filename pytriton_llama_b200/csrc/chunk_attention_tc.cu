@@ -292,10 +292,10 @@ PTL_EXPORT int ptl_chunk_attention_tc_bf16(void* out, int out_ld, int column, co
                                            int tile_tokens, int H, int G, int d, int page_size, float scale, int chunk, const float* r1,
                                            const float* r2, const float* talk, int num_pages, float out_scale, void* stream) {
   if ((d != 64 && d != 128) || H < 1 || H > ptl::kCtHeads || G < 1 || G > 2 || H % G || chunk < ptl::kCtRows || chunk % ptl::kCtRows ||
-      chunk > ptl::kCtMaxBlock || q_ld % 2 || out_ld % 2 || column % 2 || !ptl::aligned16(cache) ||
+      chunk > ptl::kCtMaxBlock || n_tiles > 65535 || q_ld % 2 || out_ld % 2 || column % 2 || !ptl::aligned16(cache) ||
       (reinterpret_cast<uintptr_t>(qkv) & 3u) || (reinterpret_cast<uintptr_t>(out) & 3u))
     return -2;
-  PTL_REQUIRE((r1 == nullptr) == (r2 == nullptr) && page_size > 0 && num_pages > 0 && n_tiles >= 0 && n_tiles <= 65535 && tile_tokens > 0 &&
+  PTL_REQUIRE((r1 == nullptr) == (r2 == nullptr) && page_size > 0 && num_pages > 0 && n_tiles >= 0 && tile_tokens > 0 &&
                   column >= 0 && column + H * d <= out_ld && q_ld >= H * d, "chunk_attention_tc: bad sizes");
   const dim3 grid((tile_tokens + ptl::kCtRows - 1) / ptl::kCtRows + 1, n_tiles);
   if (n_tiles == 0) return 0;

@@ -418,7 +418,7 @@ latent_merge_kernel(__nv_bfloat16* __restrict__ out, const float* __restrict__ p
   *reinterpret_cast<uint2*>(out + ((size_t)token * H + h) * R + 4 * threadIdx.x) = packed;
 }
 
-// What both kernels ask of sizes and addresses; -2: take another path.
+// What both kernels ask of sizes and addresses (and a grid's 65,535 tiles or single tokens); -2: take another path.
 inline bool latent_tc_fits(const void* out, const void* q, const void* cache, int H, int R, int n) {
   return (R == 128 || R == 256 || R == 512) && n >= 0 && n % 16 == 0 && n <= 64 && H > 0 && H <= 512 && aligned16(out) && aligned16(q) &&
          aligned16(cache);
@@ -458,8 +458,8 @@ int latent_decode(void* out, float* part, float* ml, const void* q, const void* 
 PTL_EXPORT int ptl_latent_prefill_bf16(void* out, const void* q, const void* cache, const int* block_table, const int* tiles, int n_tiles,
                                        int bt_stride, int H, int R, int n, int page_size, int num_pages, float scale, int tile_tokens,
                                        void* stream) {
-  if (!ptl::latent_tc_fits(out, q, cache, H, R, n)) return -2;
-  PTL_REQUIRE(n_tiles >= 0 && n_tiles <= 65535 && bt_stride > 0 && page_size > 0 && num_pages > 0 && tile_tokens > 0,
+  if (!ptl::latent_tc_fits(out, q, cache, H, R, n) || n_tiles > 65535) return -2;
+  PTL_REQUIRE(n_tiles >= 0 && bt_stride > 0 && page_size > 0 && num_pages > 0 && tile_tokens > 0,
               "latent_prefill: bad sizes");
   if (n_tiles == 0) return 0;
   const auto fn = R == 128 ? ptl::latent_prefill<128> : R == 256 ? ptl::latent_prefill<256> : ptl::latent_prefill<512>;
@@ -469,8 +469,8 @@ PTL_EXPORT int ptl_latent_prefill_bf16(void* out, const void* q, const void* cac
 PTL_EXPORT int ptl_latent_decode_bf16(void* out, float* part, float* ml, const void* q, const void* cache, const int* block_table,
                                       const int* tok_req, const int* positions, const int* items, int n_items, int bt_stride, int H, int R,
                                       int n, int page_size, int num_pages, int splits, float scale, void* stream) {
-  if (!ptl::latent_tc_fits(out, q, cache, H, R, n)) return -2;
-  PTL_REQUIRE(n_items >= 0 && n_items <= 65535 && bt_stride > 0 && page_size > 0 && num_pages > 0 && splits >= 1 && splits <= ptl::kLmShares &&
+  if (!ptl::latent_tc_fits(out, q, cache, H, R, n) || n_items > 65535) return -2;
+  PTL_REQUIRE(n_items >= 0 && bt_stride > 0 && page_size > 0 && num_pages > 0 && splits >= 1 && splits <= ptl::kLmShares &&
                   (splits == 1 || (part && ml)), "latent_decode: bad sizes");
   if (n_items == 0) return 0;
   const auto fn = R == 128 ? ptl::latent_decode<128> : R == 256 ? ptl::latent_decode<256> : ptl::latent_decode<512>;

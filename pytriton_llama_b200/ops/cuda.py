@@ -1865,7 +1865,8 @@ class CudaOps:
         """None where sizes, types or the lack of the step's work lists leave it to the other paths.  A single token's keys
         are shared out so that all shares together fill the SMs once, 64 keys at least."""
         dec, tiles = self._work(ctx, "decode_items"), self._work(ctx, "prefill_tiles")
-        if q.dtype != torch.bfloat16 or dec is None or tiles is None or H > 512 or not self.latent_on_tensor_cores(R, n):
+        if (q.dtype != torch.bfloat16 or dec is None or tiles is None or max(dec.items, tiles.items) > 65535 or H > 512
+                or not self.latent_on_tensor_cores(R, n)):
             return None
         self._want(q, "q")
         self._want(cache, "cache", q.dtype)

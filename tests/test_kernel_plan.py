@@ -62,3 +62,14 @@ def test_tiles_of_the_float32_product(lib):
                 (700, 2048): {88: 257, 84: 203, 54: 180, 44: 196}, (33, 512): {88: 156, 84: 83, 54: 61, 44: 55}}
     for (M, N), us in measured.items():
         assert us[lib.ptl_gemm_simt_tile(M, N, 1)] <= 1.05 * min(us.values()), (M, N)
+
+
+def test_steps_of_more_tiles_than_a_grid_holds_are_left_to_the_other_kernels(lib):
+    """-2 (take another path), not an error: the kernels that these entries replaced took steps of any size."""
+    p, f, i = ctypes.c_void_p(4096), ctypes.c_float(1.0), ctypes.c_int
+    size = lambda *v: [i(x) for x in v]
+    for n in (65536, 1 << 20):
+        assert lib.ptl_chunk_attention_tc_bf16(p, *size(1024, 0), p, i(1024), None, p, p, i(4), p, *size(n, 128, 8, 2, 128, 16), f, i(256), None,
+                                               None, None, i(10), f, None) == -2
+        assert lib.ptl_latent_prefill_bf16(p, p, p, p, p, *size(n, 4, 8, 512, 64, 16, 10), f, i(128), None) == -2
+        assert lib.ptl_latent_decode_bf16(p, None, None, p, p, p, p, p, None, *size(n, 4, 8, 512, 64, 16, 10, 1), f, None) == -2
