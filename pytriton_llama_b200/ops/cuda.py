@@ -994,9 +994,10 @@ class CudaOps:
         if memo is None:
             memo = self._units_memo = {}
         stream = self._stream()
-        key = (stream, dec.items, dec.in_order, *(x for t in (dec.tensor, tok_req, positions) for x in (t.data_ptr(), t._version)), nq, nkv,
-               d, int(window), per_head)
-        have = memo.get(key)
+        integers, key, have = (dec.tensor, tok_req, positions), None, None
+        if not any(t.is_inference() for t in integers):           # (those do not say whether they have been written since)
+            key = (stream, dec.items, dec.in_order, *(x for t in integers for x in (t.data_ptr(), t._version)), nq, nkv, d, int(window), per_head)
+            have = memo.get(key)
         if have is not None:
             self.launches += have[-1]
             have[-1] = 0
@@ -1008,7 +1009,8 @@ class CudaOps:
             return None, False
         self._check(rc, kernels=0)
         # (the integers are held, so that their addresses are not given out again; the launch is counted where its list serves a second layer)
-        memo[key] = [units, dec.tensor, tok_req, positions, 1]
+        if key is not None:
+            memo[key] = [units, *integers, 1]
         return units, False
 
     def _attention_tensor_cores(self, out, q, cache, block_table, tok_req, positions, nq, nkv, d, page_size, scale,

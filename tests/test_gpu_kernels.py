@@ -755,6 +755,32 @@ def test_units_of_a_step_of_single_tokens(ops, n, nkv, G, d, window, per_head):
         assert sorted((t, k) for *_, t, k in got if t >= 0) == sorted((int(rows[i]), k) for i in gone for k in range(nkv))
 
 
+def test_units_are_listed_again_when_the_step_changes(ops):
+    """The list is kept for the layers of one step only: not over a change of the step's integers in place, not over the start of a
+    forward pass, and not for tensors of inference mode, which do not count their changes."""
+    nq, nkv, d, page, n = 32, 8, 64, 16, 30
+    bt = torch.arange(n * 8, dtype=torch.int32).view(n, 8).cuda()
+    cache, q = rnd((n * 8, 2, nkv, page, d), torch.bfloat16, 1).cuda(), rnd((n, nq * d), torch.bfloat16, 2).cuda()
+
+    def both(positions, req, hints, scale=0.2):
+        got = ops.paged_attention(q, cache, bt, req, positions, nq, nkv, d, page, scale, hints=hints)
+        ops.begin_forward()
+        want = ops.paged_attention(q, cache, bt, req.clone(), positions.clone(), nq, nkv, d, page, scale, hints=_hints([1] * n, [128] * n))
+        assert torch.equal(got, want)
+
+    for inference in (False, True):
+        with torch.inference_mode(inference):
+            positions, req = torch.full((n,), 127, dtype=torch.int32).cuda(), torch.arange(n, dtype=torch.int32).cuda()
+            hints = _hints([1] * n, [128] * n)
+            both(positions, req, hints)
+            ops.paged_attention(q, cache, bt, req, positions, nq, nkv, d, page, 0.2, hints=hints)
+            positions[3:] = 5
+            both(positions, req, hints)
+            ops.paged_attention(q, cache, bt, req, positions, nq, nkv, d, page, 0.2, hints=hints)
+            req[4:9] = -1
+            both(positions, req, hints)
+
+
 @pytest.mark.parametrize("page, window", [(16, 0), (32, 300)])
 def test_decode_attention_of_more_pairs_than_fit_at_once(ops, page, window):
     """Heads of 64, 70 requests of 8 kv heads: whole pairs, by TMA."""
