@@ -10,8 +10,8 @@
 // squared is none) is walked token by token instead: in the products it would reach its chunk's earlier tokens, as 0 times it.
 //
 // The token-by-token walk is bound by the latency of its chain, 0.36 us a token at heads of 128 x 128: 738 us for
-// 2,048 tokens, whatever the number of SMs.  Here 16 heads of that size take 88 us (prepare: the chains of the 64 x 64 systems,
-// two blocks an SM) and 118 us (walk: 32 dependent chunks of three products).  The error against 64 bits is the walk's or less.
+// 2,048 tokens, whatever the number of SMs.  Here 8 heads of that size take 88 us (prepare: the chains of the 64 x 64 systems,
+// two blocks an SM) and 118 us (walk: 32 dependent chunks of three products, 128 blocks, one an SM).  The error against 64 bits is the walk's or less.
 #include "long_portions.cuh"
 #include "mma_utils.cuh"
 

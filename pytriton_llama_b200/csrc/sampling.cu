@@ -15,8 +15,9 @@
 // bucket's tokens narrows it again, a third one ends it.  Masses are added as 64-bit fixed-point
 // numbers (p * 2^40): integer sums do not depend on their order, so the histograms can be built
 // with atomics by 32 blocks per row and the choice is still the same in every run.
-// Six launches per call (row maxima by slices; three histogram levels; the kept mass by slices;
-// the draw), 32 blocks per row in the first five, so that a few rows still use many SMs.
+// One launch with a cluster of blocks per row does it for most calls (sample_cluster_kernel); very large vocabularies, and many
+// rows of large ones, take six (row maxima by slices; three histogram levels; the kept mass by slices; the draw), 32 blocks per
+// row in the first five.
 // `probs` is scratch memory of [rows, vocab] floats; `work` of kSampleWorkPerRow 64-bit words per
 // row, zero before the first call and left zero again by every call.
 #include "common.cuh"

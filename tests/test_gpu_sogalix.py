@@ -178,7 +178,7 @@ def test_delta_walk_and_its_state(ops, dtype, H, d):
 
 @pytest.mark.parametrize("H,d", [(1, 17), (2, 31), (2, 33), (1, 48), (1, 49), (2, 63)])
 def test_delta_walk_at_the_edges_of_a_group_of_columns(ops, H, d):
-    """Eight lanes walk two or four columns of the state, sixteen apart: heads that end inside such a group, to the same bounds."""
+    """Eight lanes walk two columns of the state, sixteen apart: heads that end inside such a group, to the same bounds."""
     for dtype in DTYPES:
         test_delta_walk_and_its_state(ops, dtype, H, d)
 
