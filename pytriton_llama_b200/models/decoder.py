@@ -106,9 +106,16 @@ class DecoderModel:
         """token_ids int32 [T]; ``cache_views(entry, write)`` gives the LayerCacheView of a run;
         returns float32 logits [len(logit_rows), vocab] (None when no row is wanted)."""
         ops = self.rt.ops
-        begin = getattr(ops, "begin_forward", None)
+        begin, end = getattr(ops, "begin_forward", None), getattr(ops, "end_forward", None)
         if begin is not None:
             begin()             # (what an operator set keeps per step, such as rotary angles, starts afresh)
+        try:
+            return self._forward(ops, token_ids, ctx, cache_views, logit_rows)
+        finally:
+            if end is not None:
+                end()
+
+    def _forward(self, ops, token_ids: torch.Tensor, ctx, cache_views, logit_rows: Optional[torch.Tensor]):
         ctx.tokens = token_ids
         if self.embedding_part is not None:
             if self.spec.position_vector is not None or self.embedding_norm is not None:

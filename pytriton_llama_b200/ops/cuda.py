@@ -873,6 +873,11 @@ class CudaOps:
         self._pair_memo = {}
         self._units_memo = {}
 
+    def end_forward(self) -> None:
+        """Called at the end of every forward pass: calls outside of one list their units themselves.  A list kept from one such
+        call to the next would be missing from a graph that captures the second of them."""
+        self._units_memo = None
+
     def _pair_angles(self, positions: torch.Tensor, freq: torch.Tensor, dims: int, amplitude: float) -> torch.Tensor:
         """(cos, sin) [tokens, dims/2, 2] of position * freq, worked out once per forward pass for every table of
         frequencies (float64) and used by every layer that has it."""
@@ -988,14 +993,12 @@ class CudaOps:
 
     def _decode_unit_list(self, dec, tok_req, positions, nq: int, nkv: int, d: int, window: int, per_head: int):
         """(units of equal length of the step's single tokens, whether a kernel has run since that waited for their list): worked out
-        once per forward pass and stream for every kind of attention, used by every layer of that kind.  (None, False): more tokens
-        than one block lays out."""
+        once per forward pass and stream for every kind of attention, used by every layer of that kind; outside of a forward pass for
+        every call.  (None, False): more tokens than one block lays out."""
         memo = getattr(self, "_units_memo", None)
-        if memo is None:
-            memo = self._units_memo = {}
         stream = self._stream()
         integers, key, have = (dec.tensor, tok_req, positions), None, None
-        if not any(t.is_inference() for t in integers):           # (those do not say whether they have been written since)
+        if memo is not None and not any(t.is_inference() for t in integers):      # (those do not say whether they have been written since)
             key = (stream, dec.items, dec.in_order, *(x for t in integers for x in (t.data_ptr(), t._version)), nq, nkv, d, int(window), per_head)
             have = memo.get(key)
         if have is not None:

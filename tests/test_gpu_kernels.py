@@ -781,6 +781,32 @@ def test_units_are_listed_again_when_the_step_changes(ops):
             both(positions, req, hints)
 
 
+def test_a_captured_call_lists_its_units_itself():
+    """... also when the same call ran just before the capture, outside of a forward pass: the replay goes by its own step's integers."""
+    from pytriton_llama_b200.ops.cuda import CudaOps
+    nq, nkv, d, page, n = 32, 8, 64, 16, 30
+    own = CudaOps(torch.device("cuda:0"))
+    bt, req = torch.arange(n * 8, dtype=torch.int32).view(n, 8).cuda(), torch.arange(n, dtype=torch.int32).cuda()
+    cache, q = rnd((n * 8, 2, nkv, page, d), torch.bfloat16, 1).cuda(), rnd((n, nq * d), torch.bfloat16, 2).cuda()
+    positions, hints = torch.full((n,), 127, dtype=torch.int32).cuda(), _hints([1] * n, [128] * n)
+
+    def call():
+        return own.paged_attention(q, cache, bt, req, positions, nq, nkv, d, page, 0.2, hints=hints)
+
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        call()
+    stream.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        got = call()
+    positions[2:] = 40
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, call())
+    own.check_status()
+
+
 @pytest.mark.parametrize("page, window", [(16, 0), (32, 300)])
 def test_decode_attention_of_more_pairs_than_fit_at_once(ops, page, window):
     """Heads of 64, 70 requests of 8 kv heads: whole pairs, by TMA."""
