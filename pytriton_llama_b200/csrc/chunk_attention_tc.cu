@@ -8,9 +8,10 @@
 // column of weights per thread, and the mixed float32 weights go to the tensor cores as three bfloat16 terms each (24 bits).
 // Nothing is rounded to 16 bits but the result.  The products also meet the zero weights of a row's later keys, and 0 times a value
 // that is no finite number is none: a head whose sums are not all finite is added up again, key by key and row by row.
-// Bound by the warp-level tensor instructions of a block's keys (one block per SM).  Replaces, for the portions of such sizes, a block per token on the CUDA cores that reads a block's keys and values from
-// L2 once per query: 2,048 tokens of 8 heads of 128 in blocks of 256 took 221 us.  Here: 66 us, bound by the chain of
-// products, exponentials and products of one block of eight warps per SM (12 % of the warp slots).
+// Bound by the warp-level tensor instructions of a block's keys (one block per SM).  Replaces, for the portions of such sizes, a
+// block per token on the CUDA cores that reads a block's keys and values from L2 once per query: 2,048 tokens of 8 heads of 128
+// in blocks of 256 took 221 us.  Here: 66 us, bound by the chain of products, exponentials and products of one block of eight
+// warps per SM (12 % of the warp slots).
 #include "mma_utils.cuh"
 
 namespace ptl {

@@ -868,30 +868,27 @@ class CudaOps:
 
     def begin_forward(self) -> None:
         """Called by the model at the start of every forward pass: what was worked out for the last
-        step's positions (the table of rotary angles) is forgotten."""
-        self._rope_memo = None
-        self._pair_memo = {}
-        self._units_memo = {}
+        step's positions (the tables of rotary angles, the units of single tokens) is forgotten."""
+        self._rope_memo, self._pair_memo, self._units_memo = {}, {}, {}
 
     def end_forward(self) -> None:
-        """Called at the end of every forward pass: calls outside of one list their units themselves.  A list kept from one such
-        call to the next would be missing from a graph that captures the second of them."""
-        self._units_memo = None
+        """Called at the end of every forward pass: calls outside of one work their tables and units out themselves.  One kept from
+        such a call to the next would be missing from a graph that captures the second of them."""
+        self._rope_memo = self._pair_memo = self._units_memo = None
 
     def _pair_angles(self, positions: torch.Tensor, freq: torch.Tensor, dims: int, amplitude: float) -> torch.Tensor:
-        """(cos, sin) [tokens, dims/2, 2] of position * freq, worked out once per forward pass for every table of
+        """(cos, sin) [tokens, dims/2, 2] of position * freq, worked out once per forward pass and stream for every table of
         frequencies (float64) and used by every layer that has it."""
-        memo = getattr(self, "_pair_memo", None)
-        if memo is None:
-            memo = self._pair_memo = {}
-        key = (positions.data_ptr(), positions.shape[0], freq.data_ptr(), dims, float(amplitude))
-        have = memo.get(key)
-        if have is not None and have[0] == positions._version:
-            return have[1]
+        memo, key = getattr(self, "_pair_memo", None), None
+        if memo is not None:
+            key = (self._stream(), positions.data_ptr(), positions._version, positions.shape[0], freq.data_ptr(), dims, float(amplitude))
+            if key in memo:
+                return memo[key][0]
         table = self.empty((positions.shape[0], dims // 2, 2), torch.float32)
         self._check(self.lib.ptl_pair_angles(_p(table), _p(positions), _p(freq), positions.shape[0], dims // 2, float(amplitude),
                                              self._stream()))
-        memo[key] = (positions._version, table, positions, freq)      # (held, so that their addresses are not given out again)
+        if memo is not None:
+            memo[key] = (table, positions, freq)                      # (held, so that their addresses are not given out again)
         return table
 
     def pair_rotate_store(self, proj: torch.Tensor, H: int, G: int, d: int, dv: int, bias: Optional[torch.Tensor],
@@ -927,14 +924,16 @@ class CudaOps:
                        num_slots, self._stream()))
 
     def _rope_table(self, positions: torch.Tensor, inv_freq: torch.Tensor, half: int) -> torch.Tensor:
-        """(cos, sin) [tokens, half] of this step's angles, worked out once per forward pass and used by every layer."""
-        key = (positions.data_ptr(), positions._version, inv_freq.data_ptr(), positions.shape[0], half)
-        memo = getattr(self, "_rope_memo", None)
-        if memo is not None and memo[0] == key:
-            return memo[1]
+        """(cos, sin) [tokens, half] of this step's angles, worked out once per forward pass and stream and used by every layer."""
+        memo, key = getattr(self, "_rope_memo", None), None
+        if memo is not None:
+            key = (self._stream(), positions.data_ptr(), positions._version, inv_freq.data_ptr(), positions.shape[0], half)
+            if key in memo:
+                return memo[key][0]
         table = self.empty((positions.shape[0], half, 2), torch.float32)
         self._check(self.lib.ptl_rope_table(_p(table), _p(positions), _p(inv_freq), positions.shape[0], half, self._stream()))
-        self._rope_memo = (key, table)
+        if memo is not None:
+            memo[key] = (table, positions, inv_freq)                  # (held, as above)
         return table
 
     def projected_rope_attention(self, x, w_qkv: torch.Tensor, positions: torch.Tensor, inv_freq: Optional[torch.Tensor],

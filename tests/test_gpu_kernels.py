@@ -807,6 +807,32 @@ def test_a_captured_call_lists_its_units_itself():
     own.check_status()
 
 
+@pytest.mark.parametrize("table", ["_rope_table", "_pair_angles"])
+def test_a_captured_call_works_its_angles_out_itself(table):
+    """The same for the tables of rotary angles, whose frequencies are given by address as well."""
+    from pytriton_llama_b200.ops.cuda import CudaOps
+    own, positions = CudaOps(torch.device("cuda:0")), torch.arange(70, dtype=torch.int32).cuda()
+    freq = 100.0 ** -torch.linspace(0, 1, 16, dtype=torch.float64)
+    more, freq = ((16,), freq.float().cuda()) if table == "_rope_table" else ((32, 1.0), freq.cuda())
+    call = lambda: getattr(own, table)(positions, freq, *more)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        call()
+    stream.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        got = call()
+    positions += 9
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(got, call())
+    own.begin_forward()
+    assert call() is call()
+    freq *= 0.5
+    own.end_forward()
+    assert not torch.equal(got, call())
+
+
 @pytest.mark.parametrize("page, window", [(16, 0), (32, 300)])
 def test_decode_attention_of_more_pairs_than_fit_at_once(ops, page, window):
     """Heads of 64, 70 requests of 8 kv heads: whole pairs, by TMA."""
