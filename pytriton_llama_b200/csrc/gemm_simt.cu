@@ -341,21 +341,21 @@ gemm_simt_tile_kernel(float* __restrict__ out, const float* __restrict__ A, cons
   }
 }
 
-// Results per thread (10 TM + TN) of a product: the shape whose blocks the busiest SM is soonest done with.  Blocks count in sets
-// of `held`, which take `us` (2,048 k values on a B200): fitted to products of the sizes below, not what fits on an SM (four of
-// 5 x 4 do).  64, 320 and 1,024 rows against weights of 2,048 to 16,384 rows: 320 rows 152 / 108 / 595 /
-// 425 us (q|k|v, output, gate and up, down projection of the 1B shape), 163 / 161 / 726 / 635 with 8 x 8 everywhere.  A rule by
-// the times of one, two and more blocks side by side took other shapes in between: two short generations of the 1B shape 32.7 ms
-// and 25.3 with this one, 31.3 and 28.2 with that.
+// Results per thread (10 TM + TN) of a product: the shape whose blocks the busiest SM is soonest done with, by what 1, 2, ...
+// blocks of a shape take side by side on an SM, up to as many as it holds (`us`, for 2,048 k values on a B200; blocks share its
+// FMA units, but one alone leaves them idle for its latencies).  Three of 5 x 4 stand for any number above two: the scheduler
+// spreads fewer than four per SM unevenly, 416 blocks take 173 us, 444 138.  Against the best of the four for
+// 33 to 2,048 rows, odd numbers of tiles among them, 512 to 16,384 features and 1,024 to 8,192 k values: 0.2 % slower on average, 10 % at most.
 inline int simt_tile(int M, int N, int batch) {
-  constexpr struct { int tm, tn, held; float us; } shapes[] = {{8, 8, 2, 246.f}, {8, 4, 3, 201.f}, {5, 4, 2, 105.f}, {4, 4, 4, 152.f}};
+  constexpr struct { int tm, tn, held; float us[4]; } shapes[] = {
+      {8, 8, 2, {164.f, 261.f}}, {8, 4, 3, {88.f, 193.f, 203.f}}, {5, 4, 4, {64.f, 109.f, 170.f, 181.f}}, {4, 4, 4, {56.f, 98.f, 116.f, 152.f}}};
   const int sms = sm_count_of_device();
   int best = 88;
   float least = 0.f;
   for (const auto& s : shapes) {
     const long long blocks = (long long)batch * ((M + 8 * s.tm - 1) / (8 * s.tm)) * ((N + 16 * s.tn - 1) / (16 * s.tn));
     const long long busiest = (blocks + sms - 1) / sms;
-    const float cost = s.tn == 8 && busiest == 1 ? 163.f : (float)((busiest + s.held - 1) / s.held) * s.us;   // (one of 8 x 8 alone: 163)
+    const float cost = (float)(busiest / s.held) * s.us[s.held - 1] + (busiest % s.held ? s.us[busiest % s.held - 1] : 0.f);
     if (least == 0.f || cost < least) { least = cost; best = 10 * s.tm + s.tn; }
   }
   return best;
@@ -512,6 +512,9 @@ int head_linear_few(void* out, const void* A, const void* W, int M, int N, int K
 }
 
 }  // namespace ptl
+
+// The tile shape that a float32 product of many rows takes, as 10 * rows + columns of a thread.
+PTL_EXPORT int ptl_gemm_simt_tile(int M, int N, int batch) { return ptl::simt_tile(M, N, batch); }
 
 PTL_EXPORT int ptl_gemm_simt_f32(void* out, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldo, int accumulate, void* stream) {
   return ptl::gemm_simt<float, float>(out, A, W, M, N, K, lda, ldw, ldo, accumulate, stream);
