@@ -73,6 +73,31 @@ template <typename T> __device__ __forceinline__ void store16(T* p, const Vec16<
 // exp(x), x <= 0, rounded once near 1: a decay of almost 1 acts a thousand times over, and any lean of its last bit with it.
 __device__ __forceinline__ float decay_exp(float x) { return x > -0.5f ? 1.0f + expm1f(x) : expf(x); }
 
+// ---------------------------------------------------------------- two float32 operations an instruction
+// Each half is rounded like the scalar operation.  The FMA units take both halves in two turns, so only issue slots are saved.
+__device__ __forceinline__ unsigned long long pair_bits(float2 v) { return *reinterpret_cast<unsigned long long*>(&v); }
+__device__ __forceinline__ float2 pair_of_bits(unsigned long long v) { return *reinterpret_cast<float2*>(&v); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(pair_bits(a)), "l"(pair_bits(b)), "l"(pair_bits(c)));
+  return pair_of_bits(d);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+  return pair_of_bits(d);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+  return pair_of_bits(d);
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+  unsigned long long d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(pair_bits(a)), "l"(pair_bits(b)));
+  return pair_of_bits(d);
+}
+
 // ---------------------------------------------------------------- reductions
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
