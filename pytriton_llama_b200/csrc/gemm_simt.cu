@@ -7,9 +7,9 @@
 //
 // Summation order, the same for every tile shape, so that a row's result does not depend on how
 // many rows the call has (a prompt portion and a single decoded token give the same bits):
-// the K range is cut into chunks of 32; inside a chunk the products are added one by one with
-// fused multiply-adds, k ascending, into a fresh accumulator; the chunk sums are added to the
-// running total with a compensated (Kahan) addition.  A plain running sum over K = 8,192 terms is
+// the K range is cut into chunks of 32; inside a chunk the products of even and of odd k are added one by one with
+// fused multiply-adds, k ascending, into two fresh accumulators (the two halves of a packed instruction), whose sum is the
+// chunk's; the chunk sums are added to the running total with a compensated (Kahan) addition.  A plain running sum over K = 8,192 terms is
 // wrong by about K/4 ulp of a term, which over 16 layers of a 2,048-wide model reaches 3e-4 in the
 // logits; with chunks the error of a product is that of one chunk, a few ulp.
 #include "common.cuh"
@@ -45,7 +45,7 @@ gemm_simt_kernel(TO* __restrict__ out, const TI* __restrict__ A, const TI* __res
   const int tx = tid % (BN / TN);  // along N
   const int ty = tid / (BN / TN);  // along M
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[TM][TN], sum[TM][TN], comp[TM][TN];
+  float acc[2][TM][TN], sum[TM][TN], comp[TM][TN];        // acc: even and odd k
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
@@ -67,7 +67,7 @@ gemm_simt_kernel(TO* __restrict__ out, const TI* __restrict__ A, const TI* __res
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+      for (int j = 0; j < TN; ++j) acc[0][i][j] = acc[1][i][j] = 0.f;
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
       float a[TM], b[TN];
@@ -78,12 +78,12 @@ gemm_simt_kernel(TO* __restrict__ out, const TI* __restrict__ A, const TI* __res
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        for (int j = 0; j < TN; ++j) acc[kk & 1][i][j] = fmaf(a[i], b[j], acc[kk & 1][i][j]);
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int j = 0; j < TN; ++j) kahan_add(sum[i][j], comp[i][j], acc[i][j]);
+      for (int j = 0; j < TN; ++j) kahan_add(sum[i][j], comp[i][j], __fadd_rn(acc[0][i][j], acc[1][i][j]));
     __syncthreads();
   }
 #pragma unroll
@@ -184,11 +184,11 @@ gemm_simt_few_kernel(float* __restrict__ out, const float* __restrict__ A, const
     if (works && turn < turns) {
       copy_wait<0>();
       __syncwarp();
-      float acc[RL][MT];
+      float2 acc[RL][MT];
 #pragma unroll
       for (int r = 0; r < RL; ++r)
 #pragma unroll
-        for (int m = 0; m < MT; ++m) acc[r][m] = 0.f;
+        for (int m = 0; m < MT; ++m) acc[r][m] = make_float2(0.f, 0.f);
       const float* wp = ws + group * RL * kFewLd + chunk * 36;
       const float* xp = xs + chunk * 36;
 #pragma unroll 2
@@ -196,18 +196,20 @@ gemm_simt_few_kernel(float* __restrict__ out, const float* __restrict__ A, const
         float4 w[RL];
 #pragma unroll
         for (int r = 0; r < RL; ++r) w[r] = *reinterpret_cast<const float4*>(wp + r * kFewLd + k);
+        constexpr int MS = MT < 4 ? MT : 4;                              // token rows at a time: their FMAs lie between two of one sum
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-          const float4 x = *reinterpret_cast<const float4*>(xp + m * kFewLd + k);
+        for (int m0 = 0; m0 < MT; m0 += MS) {
+          float4 x[MS];
 #pragma unroll
-          for (int r = 0; r < RL; ++r) {
-            float a = acc[r][m];
-            a = fmaf(x.x, w[r].x, a);
-            a = fmaf(x.y, w[r].y, a);
-            a = fmaf(x.z, w[r].z, a);
-            a = fmaf(x.w, w[r].w, a);
-            acc[r][m] = a;
-          }
+          for (int m = 0; m < MS; ++m) x[m] = *reinterpret_cast<const float4*>(xp + (m0 + m) * kFewLd + k);
+#pragma unroll
+          for (int m = 0; m < MS; ++m)
+#pragma unroll
+            for (int r = 0; r < RL; ++r) acc[r][m0 + m] = fma2(make_float2(x[m].x, x[m].y), make_float2(w[r].x, w[r].y), acc[r][m0 + m]);
+#pragma unroll
+          for (int m = 0; m < MS; ++m)
+#pragma unroll
+            for (int r = 0; r < RL; ++r) acc[r][m0 + m] = fma2(make_float2(x[m].z, x[m].w), make_float2(w[r].z, w[r].w), acc[r][m0 + m]);
         }
       }
       __syncwarp();
@@ -220,7 +222,7 @@ gemm_simt_few_kernel(float* __restrict__ out, const float* __restrict__ A, const
 #pragma unroll
       for (int r = 0; r < RL; ++r)
 #pragma unroll
-        for (int m = 0; m < MT; ++m) dst[r * MT + m] = acc[r][m];
+        for (int m = 0; m < MT; ++m) dst[r * MT + m] = __fadd_rn(acc[r][m].x, acc[r][m].y);
     }
     if (!works && round > 0) {                                           // the round before, while this one is multiplied
       const float* done = sums + (size_t)((round - 1) & 1) * WARPS * 8 * SUMS_LD;
@@ -249,13 +251,15 @@ gemm_simt_few_kernel(float* __restrict__ out, const float* __restrict__ A, const
 // More rows (prompts): bound by the FMAs.  128 threads, TM x TN results each (rows 8 apart, columns 16 apart) with sum, compensation
 // and chunk accumulator in registers; a chunk of 32 k values per stage, rows kept along K as they come (cp.async, a ring of
 // three stages) with 36 floats a row: a thread reads four k values of a row in one packet, and the eight rows of a quarter
-// warp's packets start in different banks.  8 x 8 results read a packet per 16 FMAs; smaller ones are for weights of few rows,
-// whose 64 x 128 tiles leave SMs without work (simt_tile below).  320 rows to 16,384 features of 2,048: 596 us, 36 TFLOP/s, three
-// quarters of what shared memory's bandwidth allows at a packet per 16 FMAs; the 32 x 16 tiles that were here: 12.5 TFLOP/s.
+// warp's packets start in different banks.  The products of two neighbouring k values are one packed instruction
+// (pairs lie side by side in the packets as they are read), which leaves issue slots for the rest; 8 x 4 results, or fewer for weights
+// of few rows, whose tiles leave SMs without work (simt_tile below).  320 rows to 16,384 features of 2,048: 551 us, 39 TFLOP/s, 596
+// with scalar FMAs and 8 x 8 results; to 2,048 features 94 and 108.  Packed FMAs with three different operands, and
+// nothing else, reach 59 TFLOP/s with 8 x 4 results.  Two halves of a block at neighbouring chunks: 635 us, though 46 in place of 57 where a tile per SM is all there is.
 constexpr int kTileLd = kSimtChunk + 4, kTileStages = 3, kTileThreads = 128;
 
 template <int TM, int TN>
-__global__ void __launch_bounds__(kTileThreads, TM * TN >= 64 ? 2 : TM * TN >= 32 ? 3 : 4)
+__global__ void __launch_bounds__(kTileThreads, TM * TN >= 32 ? 3 : 4)
 gemm_simt_tile_kernel(float* __restrict__ out, const float* __restrict__ A, const float* __restrict__ W, int M, int N, int K, int lda,
                       int ldw, int ldo, int accumulate, long long batch_a, long long batch_w, long long batch_o,
                       const float* __restrict__ gate, int gate_ld) {
@@ -283,11 +287,11 @@ gemm_simt_tile_kernel(float* __restrict__ out, const float* __restrict__ A, cons
       copy16_async(stage + r * kTileLd + 4 * p, ok ? src : A, ok);
     }
   };
-  float sum[TM][TN], comp[TM][TN];
+  float2 sum[TM][TN / 2], comp[TM][TN / 2];             // of two columns each
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) { sum[i][j] = 0.f; comp[i][j] = 0.f; }
+    for (int j = 0; j < TN / 2; ++j) sum[i][j] = comp[i][j] = make_float2(0.f, 0.f);
 #pragma unroll
   for (int c = 0; c < kTileStages - 1; ++c) {
     if (c < chunks) fetch(c);
@@ -300,11 +304,11 @@ gemm_simt_tile_kernel(float* __restrict__ out, const float* __restrict__ A, cons
     copy_commit();
     const float* xs = tile_smem + (size_t)(c % kTileStages) * ROWS * kTileLd + ty * kTileLd;
     const float* ws = tile_smem + ((size_t)(c % kTileStages) * ROWS + BM + tx) * kTileLd;
-    float acc[TM][TN];
+    float2 acc[TM][TN];                                                    // sums of even and of odd k
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int j = 0; j < TN; ++j) acc[i][j] = 0.f;
+      for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
 #pragma unroll 2
     for (int k = 0; k < kSimtChunk; k += 4) {
       float4 w[TN];
@@ -314,19 +318,21 @@ gemm_simt_tile_kernel(float* __restrict__ out, const float* __restrict__ A, cons
       for (int i = 0; i < TM; ++i) {
         const float4 x = *reinterpret_cast<const float4*>(xs + 8 * i * kTileLd + k);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(x.x, w[j].x, acc[i][j]);
+        for (int j = 0; j < TN; ++j) acc[i][j] = fma2(make_float2(x.x, x.y), make_float2(w[j].x, w[j].y), acc[i][j]);
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(x.y, w[j].y, acc[i][j]);
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(x.z, w[j].z, acc[i][j]);
-#pragma unroll
-        for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(x.w, w[j].w, acc[i][j]);
+        for (int j = 0; j < TN; ++j) acc[i][j] = fma2(make_float2(x.z, x.w), make_float2(w[j].z, w[j].w), acc[i][j]);
       }
     }
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int j = 0; j < TN; ++j) kahan_add(sum[i][j], comp[i][j], acc[i][j]);
+      for (int j = 0; j < TN / 2; ++j) {                                   // kahan_add of two columns
+        const float2 chunk = make_float2(__fadd_rn(acc[i][2 * j].x, acc[i][2 * j].y), __fadd_rn(acc[i][2 * j + 1].x, acc[i][2 * j + 1].y));
+        const float2 y = sub2(chunk, comp[i][j]);
+        const float2 t = add2(sum[i][j], y);
+        comp[i][j] = sub2(sub2(t, sum[i][j]), y);
+        sum[i][j] = t;
+      }
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -336,7 +342,7 @@ gemm_simt_tile_kernel(float* __restrict__ out, const float* __restrict__ A, cons
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int n = n0 + tx + 16 * j;
-      if (n < N) store_result(out, (size_t)m * ldo + n, sum[i][j] * row_gate, accumulate);
+      if (n < N) store_result(out, (size_t)m * ldo + n, (j & 1 ? sum[i][j / 2].y : sum[i][j / 2].x) * row_gate, accumulate);
     }
   }
 }
@@ -348,9 +354,9 @@ gemm_simt_tile_kernel(float* __restrict__ out, const float* __restrict__ A, cons
 // 33 to 2,048 rows, odd numbers of tiles among them, 512 to 16,384 features and 1,024 to 8,192 k values: 0.2 % slower on average, 10 % at most.
 inline int simt_tile(int M, int N, int batch) {
   constexpr struct { int tm, tn, held; float us[4]; } shapes[] = {
-      {8, 8, 2, {164.f, 261.f}}, {8, 4, 3, {88.f, 193.f, 203.f}}, {5, 4, 4, {64.f, 109.f, 170.f, 181.f}}, {4, 4, 4, {56.f, 98.f, 116.f, 152.f}}};
+      {8, 4, 3, {88.f, 193.f, 203.f}}, {5, 4, 4, {64.f, 109.f, 170.f, 181.f}}, {4, 4, 4, {56.f, 98.f, 116.f, 152.f}}};
   const int sms = sm_count_of_device();
-  int best = 88;
+  int best = 84;
   float least = 0.f;
   for (const auto& s : shapes) {
     const long long blocks = (long long)batch * ((M + 8 * s.tm - 1) / (8 * s.tm)) * ((N + 16 * s.tn - 1) / (16 * s.tn));
@@ -404,9 +410,8 @@ int gemm_simt(void* out, const void* A, const void* W, int M, int N, int K, int 
         return launch_kernel("gemm_simt_tile", kernel, grid, dim3(kTileThreads), smem, as_stream(stream), (float*)out, (const float*)A,
                              (const float*)W, M, N, K, lda, ldw, ldo, accumulate, batch_a, batch_w, batch_o, (const float*)gate_v, gate_ld);
       };
-      static SmemRaised r88, r84, r54, r44;
+      static SmemRaised r84, r54, r44;
       switch (tiles ? simt_tile(M, N, batch) : 0) {
-        case 88: return tiled(gemm_simt_tile_kernel<8, 8>, 8, 8, r88);
         case 84: return tiled(gemm_simt_tile_kernel<8, 4>, 8, 4, r84);
         case 54: return tiled(gemm_simt_tile_kernel<5, 4>, 5, 4, r54);
         case 44: return tiled(gemm_simt_tile_kernel<4, 4>, 4, 4, r44);
