@@ -149,6 +149,8 @@ def load_library() -> ctypes.CDLL:
         fn = getattr(lib, name)
         fn.argtypes = _GEMM_SIG
         fn.restype = _c_int
+    lib.ptl_gemm_simt_stream_f32.argtypes = [_ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _ptr, _ptr]
+    lib.ptl_gemm_simt_stream_f32.restype = _c_int
     lib.ptl_decode_attention_bf16.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int,
                                               _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_int, _c_int, _ptr, _ptr]
     lib.ptl_decode_attention_bf16.restype = _c_int
@@ -510,6 +512,11 @@ class CudaOps:
             raise KernelError(f"linear: x is [{M},{K}] but w is {list(w.shape)}")
         if x.dtype == torch.float32:
             out = self.empty((M, N), torch.float32)
+            if 0 < M <= 32:
+                rc = self.lib.ptl_gemm_simt_stream_f32(_p(out), _p(x), _p(w), M, N, K, K, K, N, 0, _p(self._tc_status_word()), self._stream())
+                if rc != -2:
+                    self._check(rc)
+                    return out
             self._check(self.lib.ptl_gemm_simt_f32(_p(out), _p(x), _p(w), M, N, K, K, K, N, 0, self._stream()))
             return out
         if not (out_dtype == torch.bfloat16 and self.library_product(M, N, K, self.EPI_BF16)):

@@ -849,6 +849,13 @@ def test_linear_float32_of_few_features(ops, N, K):
         assert torch.equal(ops.linear(x[:rows].contiguous(), w[:N].contiguous()), ops.linear(x[:rows].contiguous(), w)[:, :N])
 
 
+@pytest.mark.parametrize("N, K", [(8, 32), (9, 288), (300, 2080), (4801, 1056)])
+def test_linear_float32_of_whole_chunks(ops, N, K):
+    """K a multiple of 32: up to 32 rows (16 against wide weights) go through the kernel that fetches by TMA, the others do not; less than a
+    turn of 256, a turn and a chunk, several rounds of turns, the last block with fewer weight rows."""
+    test_linear_float32_gives_a_row_the_same_bits_whatever_its_company(ops, N, K)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_linear_with_weights_that_the_kernel_ahead_has_written(ops, dtype):
     """``fresh_weights``, in both types: the product waits for the kernel that wrote its weights, which lets its successors start early."""
