@@ -6,7 +6,7 @@
 // the cluster through distributed shared memory.  Both products run on the tensor cores; s and g are float32 and go there as three
 // bfloat16 terms each (24 bits).  The weights' parts (32 KB a block at 1,024 x 64) are fetched before the wait on the
 // predecessor.  Bound by the latency of three cluster barriers at a few tokens.  2,048 tokens of width 1,024: 91 us
-// as one block per token, 36 here; 8 tokens: 22.4 and 7.7.
+// as one block per token, 32 here; 8 tokens: 22.4 and 7.7.
 #include "mma_utils.cuh"
 
 namespace ptl {
@@ -195,6 +195,180 @@ int token_side_cluster(float* residual, const void* x, const float* bias, const 
                                (const __nv_bfloat16*)w_proj, norm_w, eps, n_tokens);
 }
 
+// Many tokens: a block owns sixteen whole rows, and nothing crosses blocks.  Each of its sixteen warps takes a sixteenth of the width as
+// its share of the sum over W_gate (all dims), then a sixteenth of W_proj's rows; a lane reads the weights in packets of eight
+// values straight from L2 as the MMAs' operand (the eight stand for two steps' places of K, in both operands alike), the
+// ones of W_gate before the wait on the predecessor.  What bounds it: 256 KB of weights a block out of L2, and the reads of the rows before anything can begin.
+// 2,048 tokens of width 1,024, 64 dims: 14.4 us, 32.2 by clusters, whose three barriers a tile cost more than their shares save.
+// The line: at 500 tokens 10.6 us by clusters and 14.0 so, at 1,000 20.6 and 14.1, and neither moves before the next wave of blocks.
+constexpr int kRowsFrom = 768;
+constexpr int kTrThreads = 512, kTrWarps = kTrThreads / 32;
+__host__ __device__ constexpr int tr_ld(int n) { return n + 32; }       // rows of 16-bit terms: two neighbouring rows' four packets in eight bank groups
+__host__ __device__ constexpr size_t tr_smem(int width, int dim) {
+  const size_t terms = (size_t)6 * kTsTokens * tr_ld(width), sums = (size_t)4 * kTrWarps * kTsTokens * dim;
+  return (size_t)4 * kTsTokens * (width + 4) + (terms > sums ? terms : sums) + (size_t)6 * kTsTokens * tr_ld(dim);
+}
+
+template <int WIDTH, int DIM>
+__global__ void __launch_bounds__(kTrThreads, 1)
+token_side_rows_kernel(float* __restrict__ residual, const __nv_bfloat16* __restrict__ x, const float* __restrict__ bias,
+                       const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ table, int table_ld, int column,
+                       int vocab, const __nv_bfloat16* __restrict__ w_gate, const __nv_bfloat16* __restrict__ w_proj,
+                       const float* __restrict__ norm_w, float eps, int n_tokens) {
+  constexpr int LS = WIDTH + 4, LT = tr_ld(WIDTH), LG = tr_ld(DIM), SLICE = WIDTH / kTrWarps, KB = SLICE / 32, NZ = DIM / 8, NY = SLICE / 8;
+  extern __shared__ __align__(16) unsigned char tr_raw[];
+  float* s32 = reinterpret_cast<float*>(tr_raw);                                     // [16][LS]
+  __nv_bfloat16* s16 = reinterpret_cast<__nv_bfloat16*>(s32 + kTsTokens * LS);       // [3][16][LT]; then the warps' sums of z [16 warps][16][DIM]
+  float* zpart = reinterpret_cast<float*>(s16);
+  constexpr size_t terms = (size_t)3 * kTsTokens * LT, sums = (size_t)2 * kTrWarps * kTsTokens * DIM;
+  __nv_bfloat16* g16 = s16 + (terms > sums ? terms : sums);                          // [3][16][LG]
+  __shared__ float s_ss[kTrWarps][kTsTokens];
+  const int t0 = blockIdx.x * kTsTokens, nt = min(kTsTokens, n_tokens - t0);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q8 = (lane & 3) * 8, c2 = (lane & 3) * 2;
+  uint4 wg[KB][NZ];                                     // (written by no kernel of the step)
+#pragma unroll
+  for (int k = 0; k < KB; ++k)
+#pragma unroll
+    for (int n = 0; n < NZ; ++n) wg[k][n] = __ldg(reinterpret_cast<const uint4*>(w_gate + (size_t)(8 * n + g) * WIDTH + warp * SLICE + 32 * k + q8));
+  pdl_wait();
+  pdl_launch_dependents();
+  constexpr int PER = DIM * kTsTokens / kTrThreads;     // elements of z that a thread finishes
+  int tok[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int row = (tid + i * kTrThreads) / DIM;
+    tok[i] = row < nt ? tokens[t0 + row] : 0;
+    if (tok[i] < 0 || tok[i] >= vocab) tok[i] = 0;
+  }
+#pragma unroll 4
+  for (int i = tid; i < kTsTokens * (WIDTH / 4); i += kTrThreads) {
+    const int r = i / (WIDTH / 4), c = i % (WIDTH / 4) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < nt) {
+      v = *reinterpret_cast<const float4*>(residual + (size_t)(t0 + r) * WIDTH + c);
+      if (x) {
+        const uint2 raw = *reinterpret_cast<const uint2*>(x + (size_t)(t0 + r) * WIDTH + c);
+        const float2 lo = unpack_bf16(raw.x), hi = unpack_bf16(raw.y);
+        v.x += lo.x; v.y += lo.y; v.z += hi.x; v.w += hi.y;
+      }
+      if (bias) {
+        const float4 b = *reinterpret_cast<const float4*>(bias + c);
+        v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+      }
+    }
+    *reinterpret_cast<float4*>(s32 + r * LS + c) = v;
+#pragma unroll
+    for (int w = 0; w < 3; ++w) {                       // (the terms of ts_split)
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+      *reinterpret_cast<uint2*>(s16 + (w * kTsTokens + r) * LT + c) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+      const float2 a = __bfloat1622float2(lo), b = __bfloat1622float2(hi);
+      v.x -= a.x; v.y -= a.y; v.z -= b.x; v.w -= b.y;
+    }
+  }
+  __nv_bfloat16 entry[PER];
+#pragma unroll
+  for (int i = 0; i < PER; ++i) entry[i] = table[(size_t)tok[i] * table_ld + column + (tid + i * kTrThreads) % DIM];
+  __syncthreads();
+  // this warp's share of z
+  float acc[NZ][4];
+#pragma unroll
+  for (int n = 0; n < NZ; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
+#pragma unroll
+  for (int k = 0; k < KB; ++k)
+#pragma unroll
+    for (int w = 2; w >= 0; --w) {
+      const __nv_bfloat16* at = s16 + (w * kTsTokens + g) * LT + warp * SLICE + 32 * k + q8;
+      const uint4 up = *reinterpret_cast<const uint4*>(at), low = *reinterpret_cast<const uint4*>(at + 8 * LT);
+      const uint32_t a0[4] = {up.x, low.x, up.y, low.y}, a1[4] = {up.z, low.z, up.w, low.w};
+#pragma unroll
+      for (int n = 0; n < NZ; ++n) {
+        mma_bf16_16816(acc[n], a0, wg[k][n].x, wg[k][n].y);
+        mma_bf16_16816(acc[n], a1, wg[k][n].z, wg[k][n].w);
+      }
+    }
+  // this warp's rows of W_proj, while the shares are added up
+  uint4 wp[NY][DIM / 32];
+#pragma unroll
+  for (int j = 0; j < NY; ++j)
+#pragma unroll
+    for (int k = 0; k < DIM / 32; ++k) wp[j][k] = __ldg(reinterpret_cast<const uint4*>(w_proj + (size_t)(warp * SLICE + 8 * j + g) * DIM + 32 * k + q8));
+  __syncthreads();                                      // the terms have been read
+#pragma unroll
+  for (int n = 0; n < NZ; ++n)
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      *reinterpret_cast<float2*>(zpart + (warp * kTsTokens + g + 8 * i) * DIM + 8 * n + c2) = make_float2(acc[n][2 * i], acc[n][2 * i + 1]);
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const int at = tid + i * kTrThreads;
+    float z = 0.f;
+#pragma unroll
+    for (int w = 0; w < kTrWarps; ++w) z += zpart[w * kTsTokens * DIM + at];
+    const float v = at / DIM < nt ? ts_gelu_tanh(z) * __bfloat162float(entry[i]) : 0.f;
+    ts_split(v, g16 + at / DIM * LG + at % DIM, kTsTokens * LG);
+  }
+  __syncthreads();
+  float y[NY][4];
+#pragma unroll
+  for (int j = 0; j < NY; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) y[j][e] = 0.f;
+#pragma unroll
+  for (int k = 0; k < DIM / 32; ++k)
+#pragma unroll
+    for (int w = 2; w >= 0; --w) {
+      const __nv_bfloat16* at = g16 + (w * kTsTokens + g) * LG + 32 * k + q8;
+      const uint4 up = *reinterpret_cast<const uint4*>(at), low = *reinterpret_cast<const uint4*>(at + 8 * LG);
+      const uint32_t a0[4] = {up.x, low.x, up.y, low.y}, a1[4] = {up.z, low.z, up.w, low.w};
+#pragma unroll
+      for (int j = 0; j < NY; ++j) {
+        mma_bf16_16816(y[j], a0, wp[j][k].x, wp[j][k].y);
+        mma_bf16_16816(y[j], a1, wp[j][k].z, wp[j][k].w);
+      }
+    }
+  float ss[2] = {0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < NY; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) ss[e >> 1] = fmaf(y[j][e], y[j][e], ss[e >> 1]);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 1);
+    ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 2);
+    if ((lane & 3) == 0) s_ss[warp][g + 8 * i] = ss[i];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int row = g + 8 * i;
+    if (row >= nt) continue;
+    float total = 0.f;
+#pragma unroll
+    for (int w = 0; w < kTrWarps; ++w) total += s_ss[w][row];
+    const float rrms = 1.0f / sqrtf(total / (float)WIDTH + eps);
+#pragma unroll
+    for (int j = 0; j < NY; ++j) {
+      const int c = warp * SLICE + 8 * j + c2;
+      const float2 w = *reinterpret_cast<const float2*>(norm_w + c), s = *reinterpret_cast<const float2*>(s32 + row * LS + c);
+      *reinterpret_cast<float2*>(residual + (size_t)(t0 + row) * WIDTH + c) = make_float2(s.x + y[j][2 * i] * rrms * w.x, s.y + y[j][2 * i + 1] * rrms * w.y);
+    }
+  }
+}
+
+template <int WIDTH, int DIM>
+int token_side_rows(float* residual, const void* x, const float* bias, const int* tokens, const void* table, int table_ld, int column, int vocab,
+                    const void* w_gate, const void* w_proj, const float* norm_w, int n_tokens, float eps, void* stream) {
+  static SmemRaised raised;
+  auto kernel = token_side_rows_kernel<WIDTH, DIM>;
+  if (int rc = raise_shared_memory("token_side", kernel, (int)tr_smem(WIDTH, DIM), raised)) return rc;
+  return launch_kernel("token_side", kernel, dim3((n_tokens + kTsTokens - 1) / kTsTokens), dim3(kTrThreads), tr_smem(WIDTH, DIM),
+                       as_stream(stream), residual, (const __nv_bfloat16*)x, bias, tokens, (const __nv_bfloat16*)table, table_ld, column, vocab,
+                       (const __nv_bfloat16*)w_gate, (const __nv_bfloat16*)w_proj, norm_w, eps, n_tokens);
+}
+
 }  // namespace ptl
 
 // -2: widths other than 512, 1,024 and 2,048, dims that are no whole sixteens up to 128, or rows off their boundaries.
@@ -208,6 +382,11 @@ PTL_EXPORT int ptl_token_side_cluster_bf16(float* residual, const void* x, const
   PTL_REQUIRE(n_tokens >= 0 && n_tokens <= (1 << 27) && column >= 0 && column + dim <= table_ld && eps > 0.f && vocab > 0,
               "token_side: bad sizes width=%d dim=%d column=%d of %d", width, dim, column, table_ld);
   if (n_tokens == 0) return 0;
+  if (n_tokens >= kRowsFrom && width <= 1024 && (dim == 32 || dim == 64)) {
+    const auto rows = width == 512 ? dim == 32 ? token_side_rows<512, 32> : token_side_rows<512, 64>
+                                   : dim == 32 ? token_side_rows<1024, 32> : token_side_rows<1024, 64>;
+    return rows(residual, x, bias, tokens, table, table_ld, column, vocab, w_gate, w_proj, norm_w, n_tokens, eps, stream);
+  }
   const auto fn = width == 512 ? token_side_cluster<64> : width == 1024 ? token_side_cluster<128> : token_side_cluster<256>;
   return fn(residual, x, bias, tokens, table, table_ld, column, dim, vocab, w_gate, w_proj, norm_w, n_tokens, eps, stream);
 }

@@ -272,6 +272,12 @@ def test_side_term_in_a_cluster(ops, T, W, dim):
         assert (got.double().cpu() - want).abs().max() <= 2e-5 * float(want.abs().max())
 
 
+@pytest.mark.parametrize("T,W,dim", [(768, 1024, 64), (781, 512, 32), (900, 512, 64), (769, 1024, 32)])
+def test_side_term_of_many_tokens(ops, T, W, dim):
+    """From 768 tokens on a block owns whole rows: whole sixteens and remainders, both widths and dims it takes."""
+    test_side_term_in_a_cluster(ops, T, W, dim)
+
+
 @pytest.mark.parametrize("H,G,d,page,chunk,options", [(8, 2, 128, 16, 256, True), (4, 2, 64, 8, 48, True), (1, 1, 128, 4, 16, False),
                                                       (6, 2, 64, 16, 240, True)])
 def test_chunk_attention_on_the_tensor_cores(ops, H, G, d, page, chunk, options):
