@@ -86,8 +86,10 @@ __global__ void causal_conv_kernel(T* __restrict__ out, const T* __restrict__ x,
 }
 
 // The same for steps with portions, TAPS taps and rows of whole pairs: a thread takes two neighbouring channels of kConvTokens
-// tokens and keeps the last inputs in registers; eight rows are requested together.
-constexpr int kConvTokens = 32;
+// tokens and keeps the last inputs in registers.  Its rows, and those before the first, are requested together, before it is known
+// whose they are.  Bound by that one trip to L2 and by what is in flight: 200 tokens of 3,072 channels 5.6 us with the
+// state's launch, 2,048 16.5 (there the SiLU's instructions count); with 32 tokens a thread, eight at a time, 11.0 and 17.7.
+constexpr int kConvTokens = 8;
 template <typename T> struct ConvPair;
 template <> struct ConvPair<float> {
   float2 raw;
@@ -124,15 +126,21 @@ causal_conv_rows_kernel(T* __restrict__ out, const T* __restrict__ x, int ld, in
   };
   float2 past[TAPS > 1 ? TAPS - 1 : 1];      // the inputs before the token, oldest first
   int req = -1;                              // whose inputs they are
-  for (int t0 = first; t0 < end; t0 += 8) {
-    ConvPair<T> raw[8];
+  ConvPair<T> raw[kConvTokens], before[TAPS > 1 ? TAPS - 1 : 1];
+  int reqs[kConvTokens];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) raw[k] = row(min(t0 + k, end - 1));
+  for (int k = 0; k < kConvTokens; ++k) reqs[k] = tok_req[min(first + k, end - 1)];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+  for (int j = 0; j < TAPS - 1; ++j) before[j] = row(max(first - (TAPS - 1 - j), 0));
+#pragma unroll
+  for (int k = 0; k < kConvTokens; ++k) raw[k] = row(min(first + k, end - 1));
+  {
+    const int t0 = first;
+#pragma unroll
+    for (int k = 0; k < kConvTokens; ++k) {
       const int t = t0 + k;
       if (t >= end) break;
-      const int r = tok_req[t];
+      const int r = reqs[k];
       if (r < 0) { req = -1; continue; }
       if (r != req) {                        // the thread's first token, or a request's: fetch what lies before it
         req = r;
@@ -143,7 +151,7 @@ causal_conv_rows_kernel(T* __restrict__ out, const T* __restrict__ x, int ld, in
           const int back = TAPS - 1 - j;
           past[j] = make_float2(0.f, 0.f);
           if (back <= in_step) {
-            past[j] = row(t - back).get();
+            past[j] = k == 0 ? before[j].get() : row(t - back).get();
             past[j].x += own.x; past[j].y += own.y;
           } else if (back <= pos) {
             const float* s = st + (size_t)(j + in_step) * channels;
