@@ -43,7 +43,7 @@ _SIGNATURES = {
     "ptl_gated_delta_rule": [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f,
                              _c_f, _c_int, _ptr],
     "ptl_gated_delta_chunks": [_ptr, _ptr, _c_int, _c_int, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
-                               _c_f, _c_f, _c_int, _ptr],
+                               _c_f, _c_f, _c_int, _ptr, _ptr],
     "ptl_gated_head_norm": [_ptr, _c_int, _c_int, _ptr, _ptr, _c_f, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f, _c_int, _c_int,
                             _ptr],
     "ptl_kv_write_normed": [_ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ll, _c_f, _ptr],
@@ -1303,8 +1303,9 @@ class CudaOps:
             work = self.empty((chunks * H, self.lib.ptl_delta_chunk_floats(d, dv)), torch.float32)
             fn = getattr(self.lib, "ptl_gated_delta_chunks" + _suffix(qkv.dtype))
             self._check(fn(_p(out), _p(work), chunks, long, _p(qkv), _p(ba), _p(rate), _p(dt_bias), _p(state), _p(ctx.q_start), _p(ctx.positions),
-                           _p(ctx.state_slot), ctx.num_requests, H, G, d, dv, float(unit_eps), float(q_scale), walk_max, self._stream()),
-                        kernels=2)
+                           _p(ctx.state_slot), ctx.num_requests, H, G, d, dv, float(unit_eps), float(q_scale), walk_max,
+                           _p(self._tc_status_word()), self._stream()),
+                        kernels=3)
         return out
 
     def gated_head_norm(self, o: torch.Tensor, weight: torch.Tensor, eps: float, gate: torch.Tensor, gate_column: int, H: int,
