@@ -194,6 +194,196 @@ chunk_attention_kernel(T* __restrict__ out, int out_ld, int column, const T* __r
   }
 }
 
+// Single tokens of a bfloat16 cache with up to eight query heads over up to two kv heads of 64 or 128 entries, blocks of up to 256
+// positions: the same sums, a block per token whose sixteen warps share the keys.  A lane owns an eighth (or a quarter) of eight entries of
+// every head: four keys' products with eight heads meet in one butterfly that leaves a (key, head) in every lane, and for the
+// values the warps' sums meet in shared memory.  What bounds it: the trips to memory of its five steps, one after the other, and from some
+// hundred keys on their 512 bytes each through one SM.  Eight tokens of 8 heads of 128 at the end of 256 positions: 16.2 us, the kernel above
+// (a thread per key) 44.0; at 24 positions 7.2 and 15.2.
+constexpr int kCsThreads = 512, kCsWarps = kCsThreads / 32, kCsHeads = 8, kCsMaxBlock = 256;
+
+template <int D, int G>
+__global__ void __launch_bounds__(kCsThreads)
+chunk_attention_single_kernel(__nv_bfloat16* __restrict__ out, int out_ld, int column, const __nv_bfloat16* __restrict__ qkv, int q_ld,
+                              const float* __restrict__ q_bias, const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table,
+                              int table_width, const int* __restrict__ tok_req, const int* __restrict__ positions, int H, int page_size,
+                              float scale, int chunk, const float* __restrict__ r1, const float* __restrict__ r2, const float* __restrict__ talk,
+                              int num_pages, float out_scale, const int* __restrict__ items) {
+  constexpr int HG = kCsHeads / G, E = D / 32;                // places for a kv head's query heads, entries of a lane
+  extern __shared__ __align__(16) float cs_smem[];
+  float* s_w = cs_smem;                                       // [256 keys][8 heads]: scores, weights, mixed weights
+  float* s_sum = s_w + kCsMaxBlock * kCsHeads;                // [16 warps][8 heads][D]
+  __shared__ long long s_at[kCsMaxBlock];
+  __shared__ float s_talk[kCsHeads * kCsHeads];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int t = items ? items[blockIdx.x] : blockIdx.x;
+  const int r = tok_req[t];
+  if (r < 0) return;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, group = H / G;
+  const int p = positions[t], lo = p - p % chunk, n = p - lo + 1;
+  const size_t page_stride = (size_t)G * page_size * 2 * D, plane = (size_t)page_size * D;
+  // the queries (with their bias) of this lane's entries; a place without a head holds zeros
+  float q[kCsHeads][E];
+#pragma unroll
+  for (int a = 0; a < kCsHeads; ++a) {
+    const int h = a / HG * group + a % HG;
+    const bool there = a % HG < group;
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      q[a][e] = there ? to_f32(qkv[(size_t)t * q_ld + h * D + lane * E + e]) + (q_bias ? q_bias[h * D + lane * E + e] : 0.f) : 0.f;
+  }
+  if (tid < n) {
+    const int pos = lo + tid, page = block_table[(size_t)r * table_width + pos / page_size];
+    s_at[tid] = page >= 0 && page < num_pages ? (long long)((size_t)page * page_stride + (size_t)(pos % page_size) * D) : -1;
+  }
+  if (talk && tid < H * H) s_talk[tid] = talk[tid];
+  __syncthreads();
+  // a lane's entries of a row of the cache
+  const auto entries = [&](long long at, float (&x)[E]) {
+    if (at < 0) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) x[e] = 0.f;
+      return;
+    }
+    const __nv_bfloat162* src = reinterpret_cast<const __nv_bfloat162*>(cache + at + lane * E);
+    __nv_bfloat162 raw[E / 2];
+    if constexpr (E == 4) *reinterpret_cast<uint2*>(raw) = *reinterpret_cast<const uint2*>(src);
+    else raw[0] = *src;
+#pragma unroll
+    for (int e = 0; e < E / 2; ++e) {
+      const float2 v = __bfloat1622float2(raw[e]);
+      x[2 * e] = v.x;
+      x[2 * e + 1] = v.y;
+    }
+  };
+  // scores, four keys at a time: lane 8 k + a ends up with key k's of head place a
+  const int a0 = lane & 7, my_head = a0 / HG * group + a0 % HG;
+  const bool my_there = a0 % HG < group;
+  const float f1 = r1 && my_there ? r1[my_head] : 0.f, f2 = r1 && my_there ? r2[my_head] : 0.f;
+#pragma unroll 2
+  for (int j0 = 4 * warp; j0 < n; j0 += 4 * kCsWarps) {
+    float x[4][G][E], v[32];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const long long at = j0 + k < n ? s_at[j0 + k] : -1;
+#pragma unroll
+      for (int c = 0; c < G; ++c) entries(at < 0 ? -1 : at + (long long)(c * plane), x[k][c]);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int a = 0; a < kCsHeads; ++a) {
+        float sum = 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) sum = fmaf(q[a][e], x[k][a / HG][e], sum);
+        v[8 * k + a] = sum;
+      }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int i = 0; i < o; ++i) {
+        const float send = up ? v[i] : v[i + o], keep = up ? v[i + o] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+    const int j = j0 + (lane >> 3);
+    if (j < n) {
+      float sc = -INFINITY;
+      if (my_there && s_at[j] >= 0) {
+        sc = v[0] * scale;
+        if (r1) sc -= f1 * log1pf(f2 * (float)(p - lo - j));
+      }
+      s_w[j * kCsHeads + a0] = sc;
+    }
+  }
+  __syncthreads();
+  if (warp < kCsHeads) {                                       // softmax, a warp per head place
+    float x[kCsMaxBlock / 32], m = -INFINITY, sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < kCsMaxBlock / 32; ++i) {
+      x[i] = lane + 32 * i < n ? s_w[(lane + 32 * i) * kCsHeads + warp] : -INFINITY;
+      m = fmaxf(m, x[i]);
+    }
+    m = warp_max(m);
+#pragma unroll
+    for (int i = 0; i < kCsMaxBlock / 32; ++i) {
+      x[i] = x[i] == -INFINITY ? 0.f : expf(x[i] - m);
+      sum += x[i];
+    }
+    sum = warp_sum(sum);
+    const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+#pragma unroll
+    for (int i = 0; i < kCsMaxBlock / 32; ++i)
+      if (lane + 32 * i < n) s_w[(lane + 32 * i) * kCsHeads + warp] = x[i] * inv;
+  }
+  __syncthreads();
+  if (talk) {                                                  // a key's column of weights per thread
+    if (tid < n) {
+      float x[kCsHeads], y[kCsHeads];
+#pragma unroll
+      for (int a = 0; a < kCsHeads; ++a) x[a] = s_w[tid * kCsHeads + a];
+#pragma unroll
+      for (int b = 0; b < kCsHeads; ++b) {
+        y[b] = 0.f;
+        if (b % HG >= group) continue;
+        const float* row = s_talk + (b / HG * group + b % HG) * H;
+#pragma unroll
+        for (int a = 0; a < kCsHeads; ++a)
+          if (a % HG < group) y[b] = fmaf(row[a / HG * group + a % HG], x[a], y[b]);
+      }
+#pragma unroll
+      for (int b = 0; b < kCsHeads; ++b) s_w[tid * kCsHeads + b] = y[b];
+    }
+    __syncthreads();
+  }
+  // outputs: a warp's keys, all heads
+  float acc[kCsHeads][E];
+#pragma unroll
+  for (int a = 0; a < kCsHeads; ++a)
+#pragma unroll
+    for (int e = 0; e < E; ++e) acc[a][e] = 0.f;
+#pragma unroll 4
+  for (int j = warp; j < n; j += kCsWarps) {
+    const long long at = s_at[j];
+    float x[G][E];
+#pragma unroll
+    for (int c = 0; c < G; ++c) entries(at < 0 ? -1 : at + (long long)((G + c) * plane), x[c]);
+    const float4 w0 = *reinterpret_cast<const float4*>(s_w + j * kCsHeads), w1 = *reinterpret_cast<const float4*>(s_w + j * kCsHeads + 4);
+    const float w[kCsHeads] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+    for (int a = 0; a < kCsHeads; ++a)
+#pragma unroll
+      for (int e = 0; e < E; ++e) acc[a][e] = fmaf(w[a], x[a / HG][e], acc[a][e]);
+  }
+#pragma unroll
+  for (int a = 0; a < kCsHeads; ++a)
+#pragma unroll
+    for (int e = 0; e < E; e += 2) *reinterpret_cast<float2*>(s_sum + (warp * kCsHeads + a) * D + lane * E + e) = make_float2(acc[a][e], acc[a][e + 1]);
+  __syncthreads();
+  for (int i = tid; i < kCsHeads * D; i += kCsThreads) {
+    const int a = i / D, e = i % D;
+    if (a % HG >= group) continue;
+    float sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < kCsWarps; ++w) sum += s_sum[w * kCsHeads * D + i];
+    out[(size_t)t * out_ld + column + (a / HG * group + a % HG) * D + e] = __float2bfloat16_rn(sum * out_scale);
+  }
+}
+
+template <int D, int G>
+int chunk_attention_single(void* out, int out_ld, int column, const void* qkv, int q_ld, const float* q_bias, const void* cache, const int* bt,
+                           int table_width, const int* tok_req, const int* positions, int rows, int H, int page_size, float scale, int chunk,
+                           const float* r1, const float* r2, const float* talk, int num_pages, float out_scale, const int* items, void* stream) {
+  static SmemRaised raised;
+  constexpr int smem = (kCsMaxBlock * kCsHeads + kCsWarps * kCsHeads * D) * (int)sizeof(float);
+  if (int rc = raise_shared_memory("chunk_attention_single", chunk_attention_single_kernel<D, G>, smem, raised)) return rc;
+  return launch_kernel("chunk_attention_single", chunk_attention_single_kernel<D, G>, dim3(rows), dim3(kCsThreads), smem, as_stream(stream),
+                       (__nv_bfloat16*)out, out_ld, column, (const __nv_bfloat16*)qkv, q_ld, q_bias, (const __nv_bfloat16*)cache, bt,
+                       table_width, tok_req, positions, H, page_size, scale, chunk, r1, r2, talk, num_pages, out_scale, items);
+}
+
 template <typename T>
 int kv_write_normed(void* cache, const void* qkv, const float* bias, const int* slots, int tokens, int H, int G, int d, int dv,
                     int page_size, long long num_slots, float eps, void* stream) {
@@ -247,3 +437,21 @@ int chunk_attention(void* out, int out_ld, int column, const void* qkv, int q_ld
   }
 PTL_CHUNK_ATTENTION(_f32, float)
 PTL_CHUNK_ATTENTION(_bf16, __nv_bfloat16)
+
+// Single tokens.  -2: sizes or addresses for the kernel above.
+PTL_EXPORT int ptl_chunk_attention_single_bf16(void* out, int out_ld, int column, const void* qkv, int q_ld, const float* q_bias, const void* cache,
+                                               const int* block_table, int table_width, const int* tok_req, const int* positions, int rows, int H,
+                                               int G, int d, int page_size, float scale, int chunk, const float* r1, const float* r2,
+                                               const float* talk, int num_pages, float out_scale, const int* items, void* stream) {
+  using namespace ptl;
+  if ((d != 64 && d != 128) || H < 1 || H > kCsHeads || G < 1 || G > 2 || H % G || H / G > kCsHeads / G || chunk < 1 || chunk > kCsMaxBlock ||
+      !aligned16(cache))
+    return -2;
+  PTL_REQUIRE((r1 == nullptr) == (r2 == nullptr) && page_size > 0 && num_pages > 0 && rows >= 0 && column >= 0 && column + H * d <= out_ld &&
+                  q_ld >= H * d, "chunk_attention_single: bad sizes");
+  if (rows == 0) return 0;
+  const auto fn = d == 64 ? G == 1 ? chunk_attention_single<64, 1> : chunk_attention_single<64, 2>
+                          : G == 1 ? chunk_attention_single<128, 1> : chunk_attention_single<128, 2>;
+  return fn(out, out_ld, column, qkv, q_ld, q_bias, cache, block_table, table_width, tok_req, positions, rows, H, page_size, scale, chunk, r1, r2,
+            talk, num_pages, out_scale, items, stream);
+}

@@ -210,6 +210,9 @@ def load_library() -> ctypes.CDLL:
     lib.ptl_chunk_attention_tc_bf16.argtypes = [_ptr, _c_int, _c_int, _ptr, _c_int, _ptr, _ptr, _ptr, _c_int, _ptr, _c_int, _c_int, _c_int,
                                                 _c_int, _c_int, _c_int, _c_f, _c_int, _ptr, _ptr, _ptr, _c_int, _c_f, _ptr]
     lib.ptl_chunk_attention_tc_bf16.restype = _c_int
+    lib.ptl_chunk_attention_single_bf16.argtypes = [_ptr, _c_int, _c_int, _ptr, _c_int, _ptr, _ptr, _ptr, _c_int, _ptr, _ptr, _c_int, _c_int, _c_int,
+                                                    _c_int, _c_int, _c_f, _c_int, _ptr, _ptr, _ptr, _c_int, _c_f, _ptr, _ptr]
+    lib.ptl_chunk_attention_single_bf16.restype = _c_int
     lib.ptl_gemm_tc_bf16_clamped_glu.argtypes = [_ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _ptr, _c_f, _c_f, _c_f, _ptr, _ptr]
     lib.ptl_gemm_tc_bf16_clamped_glu.restype = _c_int
     lib.ptl_token_side_cluster_bf16.argtypes = _SIGNATURES["ptl_token_side"]
@@ -1391,6 +1394,14 @@ class CudaOps:
                 if not dec.items:
                     return
                 rows = (None if dec.in_order else dec.tensor, dec.items)       # the single tokens, a block each
+            if rows is not None or (dec.items and not tiles.items):
+                rc = self.lib.ptl_chunk_attention_single_bf16(
+                    _p(out), out.shape[1], int(column), _p(qkv), qkv.shape[1], _p(bias), _p(cache), _p(block_table), block_table.shape[1],
+                    _p(ctx.tok_req), _p(ctx.positions), dec.items, H, G, d, page_size, float(scale), int(chunk), _p(r1), _p(r2), _p(talk),
+                    cache.shape[0], float(out_scale), None if dec.in_order else _p(dec.tensor), self._stream())
+                if rc != -2:
+                    self._check(rc)
+                    return
         self.chunk_attention(qkv, bias, cache, block_table, ctx.tok_req, ctx.positions, H, G, d, dv, page_size, scale, chunk, r1, r2, talk,
                              out, column, out_scale, rows=rows)
 
