@@ -19,6 +19,7 @@
 // being the product.
 // Sizes: M <= 8, K % 8 == 0, and as many blocks as are resident at once (the launcher says no
 // otherwise and the caller takes the tcgen05 product).
+#include <algorithm>
 #include "mma_utils.cuh"
 
 namespace ptl {
@@ -26,6 +27,8 @@ namespace ptl {
 constexpr int kSmallRows = 8;        // output features per block
 constexpr int kSmallTokens = 8;      // token columns of the MMA
 constexpr int kSmallWarps = 8;
+constexpr int kSmallResident = 5;    // blocks an SM holds by their registers
+constexpr size_t kSmallSmemPerSm = 228 * 1024;
 constexpr int kSmallPad = 8;         // bfloat16 of padding per shared-memory row: rows start in different banks
 
 struct SmallGemmParams {
@@ -177,14 +180,14 @@ gemm_small_kernel(const SmallGemmParams p_in) {
 template <int EPI>
 static int launch_small(const SmallGemmParams& p, int blocks, size_t smem, cudaStream_t stream, int products = 1) {
   static SmemRaised raised = {};
-  if (int rc = raise_shared_memory("gemm_small", gemm_small_kernel<EPI>, 100 * 1024, raised)) return rc;
+  if (int rc = raise_shared_memory("gemm_small", gemm_small_kernel<EPI>, (int)kSmallSmemPerSm - 1024, raised)) return rc;
   return launch_kernel("gemm_small", gemm_small_kernel<EPI>, dim3(blocks, products), dim3(kSmallWarps * 32), smem, stream, p);
 }
 
 }  // namespace ptl
 
 // Returns 0, -1 on an error, or -2 when the sizes are not this kernel's (more than 8 tokens, K no
-// multiple of 8, rows too long for three blocks per SM, or more blocks than are resident at once):
+// multiple of 8, or more blocks than are resident at once):
 // the caller then takes the tcgen05 product.  Arguments as ptl_gemm_tc_bf16_norm (epi 0, 1 or 2);
 // with `xs` a token gets one slot of `sumsq` per 8 features, *slots_out = ceil(N / 8).
 static int gemm_small_impl(void* out, const void* X, const void* W, int M, int N, int K, int ld_out, int epi, void* xs,
@@ -209,14 +212,11 @@ static int gemm_small_impl(void* out, const void* X, const void* W, int M, int N
   const int row_elems = kSmallWarps * p.k_per_warp + kSmallPad;
   const size_t smem = (size_t)(kSmallRows + kSmallTokens) * row_elems * 2 + (kSmallWarps * kSmallRows * kSmallTokens + kSmallTokens) * 4;
   const int blocks = (N + kSmallRows - 1) / kSmallRows;
-  static int resident = 0;                                // blocks of this kernel the device holds at once: three per SM
-  if (!resident) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    resident = 3 * (sms > 0 ? sms : 148);
-  }
-  if (smem > 74 * 1024 || blocks > resident) return -2;
+  // As many blocks as are resident at once, by shared memory (registers allow five per SM).  Rows of 1,024 fit five blocks an SM, rows of 4,096
+  // one: 4,096 features of 1,024 and 1,024 of 4,096, eight tokens, took 5 to 6 us a launch of a step by the tcgen05 product, and a step of
+  // 114 launches 501 us where three blocks an SM and 74 KB a block were the line, 439 so.
+  const int per_sm = std::min(kSmallResident, (int)(kSmallSmemPerSm / (smem + 1024)));
+  if (blocks > per_sm * sm_count_of_device()) return -2;
   if (xs) {
     if (epi != 2) return -2;
     PTL_REQUIRE(norm_w && sumsq && slots_out && sumsq_ld >= blocks, "gemm_small: the next norm's input needs its weight, the sums (a slot per 8 features) and a place for their count");

@@ -8,8 +8,9 @@
 // them from a tile of the step's list (128 tokens of one request) and walks the keys up to its last token's position in
 // tiles of 32, a ring of three; eight warps, four row groups by two: for the scores the two split the tile's keys, for the
 // weighted sums the latent's columns, the weights (rounded once to bfloat16, as the softmax over stored scores
-// did) pass through shared memory.  Bound by the warp-level tensor instructions and the fragments read for them, 434 KB per 64 x 32 scores; eight
-// prompts of 65 to 440 tokens (8 heads, R 512, n 64): 68 us a layer.
+// did) pass through shared memory.  The rows of keys and queries come by one bulk copy each, a warp's lanes a tile (as copies of 16 bytes
+// they held all warps up for 1,200 of a tile's 5,500 cycles).  Bound by the fragments read for the warp-level tensor instructions, 434 KB per 64 x 32 scores; eight
+// prompts of 65 to 440 tokens (8 heads, R 512, n 64): LP_NOW us alone, 55 before.
 //
 // latent_decode: single tokens, all heads of a token (up to 16 per block) against a share of its keys, 64 at a time, two
 // tiles in flight; the float32 weights go to the tensor cores as three bfloat16 terms each (24 bits), so that nothing of
@@ -21,6 +22,7 @@
 // four such layers 5.52 -> 2.61 ms), and for decoding the CUDA-core kernel with a warp per token, head and share (48 + 30 us
 // a layer with dependent launches; a step of eight 731 -> 536 us).
 #include "mma_utils.cuh"
+#include "tcgen05_utils.cuh"
 
 namespace ptl {
 
@@ -52,8 +54,10 @@ template <int R>
 __global__ void __launch_bounds__(kLpThreads, 1)
 latent_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
                       const int* __restrict__ block_table, const int* __restrict__ tiles, int bt_stride, int H, int d, int page_size,
-                      int num_pages, float scale_log2) {
+                      int num_pages, float scale_log2, int* status) {
   extern __shared__ __align__(128) unsigned char lp_smem[];
+  __shared__ uint64_t s_bars[kLpStages + 1];                      // a tile's rows are here; the queries are
+  __shared__ int s_abort;
   __shared__ float s_max[2][kLpRows];
   __shared__ float s_sum[2][kLpRows];
   const int* tile = tiles + 4 * blockIdx.y;                       // request row, first token row, tokens, first position (inputs of the step)
@@ -64,63 +68,126 @@ latent_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __re
   pdl_launch_dependents();
   if (req < 0 || row0 >= rows) return;
   const int ld = latent_row_bytes(d);
-  const uint32_t sq = smem_u32(lp_smem), sk = sq + kLpRows * ld, sp = sk + kLpStages * kLpKeys * ld;
+  const uint32_t sq = smem_u32(lp_smem), sk = sq + kLpRows * ld, sp = sk + kLpStages * kLpKeys * ld, sx = sp + kLpRows * kLpWeightBytes;
   const int* bt = block_table + (size_t)req * bt_stride;
   const int last_row = min(row0 + kLpRows, rows) - 1;
   const int keys = pos0 + last_row / H + 1;                       // keys that the block's last token sees
   const int n_tiles = (keys + kLpKeys - 1) / kLpKeys;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, c2 = (lane & 3) * 2;
-  const int wm = warp & 3, wn = warp >> 2;                        // row group of 16, half of the keys / of the columns
+  // scores: 32 rows (wr), 16 keys (wn), half of the dot product (wk), the halves added for 16 of the rows each (wm); weighted sums: 32 rows, a
+  // quarter of the columns (wc)
+  const int wr = warp & 1, wn = (warp >> 1) & 1, wk = warp >> 2, wm = 2 * wr + wk, wc = warp >> 1;
 
-  const __nv_bfloat16* q0 = q + ((size_t)token0 * H + row0) * d;
-  for (int idx = tid; idx < kLpRows * (d / 8); idx += kLpThreads) {
-    const int r = idx / (d / 8), c = idx % (d / 8);
-    const bool ok = row0 + r < rows;
-    cp_async_16(sq + r * ld + 16 * c, q0 + (ok ? (size_t)r * d + 8 * c : 0), ok);
-  }
-  cp_async_commit();
+  const uint32_t bars = smem_u32(s_bars);
+  volatile int* const abort_flag = &s_abort;
+  if (tid == 0) {
 #pragma unroll
-  for (int s = 0; s < kLpStages - 1; ++s) {
-    if (s < n_tiles) latent_fetch<kLpKeys>(sk + s * kLpKeys * ld, cache, bt, s * kLpKeys, keys, d, page_size, num_pages);
-    cp_async_commit();
+    for (int i = 0; i <= kLpStages; ++i) mbar_init(bars + 8 * i, kLpThreads / 32);
+    s_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // Every warp fetches four keys of a tile, a lane each (75 cycles a copy: one warp's 32 would take 2,400); the lane's page is looked up a tile ahead
+  constexpr int OWN = kLpKeys / (kLpThreads / 32), OWN_ROWS = kLpRows / (kLpThreads / 32);
+  static_assert(OWN <= 32 && OWN_ROWS <= 32, "a lane a row");
+  const int own = warp * OWN + lane;
+  int key = own, entry = own / page_size, offset = own % page_size, page = -1;
+  const int step_entries = kLpKeys / page_size, step_offset = kLpKeys % page_size;
+  const auto look_up = [&] {
+    page = -1;
+    if (lane < OWN && key < keys) asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(page) : "l"(bt + entry));
+  };
+  look_up();
+  __syncthreads();
+  const auto copy_row = [&](uint32_t dst, const __nv_bfloat16* src, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(dst), "l"(src), "r"(d * 2), "r"(bar) : "memory");
+  };
+  const auto fetch = [&](int t) {                                 // this warp's keys of tile t; zeros for keys without a page
+    const uint32_t stage = sk + (t % kLpStages) * kLpKeys * ld, bar = bars + 8 * (t % kLpStages);
+    const bool ok = page >= 0 && page < num_pages;
+    const unsigned held = __ballot_sync(0xffffffffu, ok), missing = ((1u << OWN) - 1) & ~held;
+    for (unsigned miss = missing; miss; miss &= miss - 1)
+      for (int c = lane; c < d / 8; c += 32) st_shared_16(stage + (warp * OWN + __ffs(miss) - 1) * ld + 16 * c, make_uint4(0u, 0u, 0u, 0u));
+    if (missing) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // (a later tile's copies come after these)
+    __syncwarp();
+    if (lane == 0) mbar_expect_tx(bar, __popc(held) * d * 2);
+    __syncwarp();
+    if (ok) copy_row(stage + own * ld, cache + ((size_t)page * page_size + offset) * d, bar);
+    key += kLpKeys;
+    entry += step_entries;
+    offset += step_offset;
+    if (offset >= page_size) { offset -= page_size; ++entry; }
+    look_up();
+  };
+  if (lane == 0) mbar_expect_tx(bars + 8 * kLpStages, OWN_ROWS * d * 2);
+  __syncwarp();
+  if (lane < OWN_ROWS) {                                          // (rows past the last one hold it again)
+    const int r = warp * OWN_ROWS + lane;
+    copy_row(sq + r * ld, q + ((size_t)token0 * H + min(row0 + r, rows - 1)) * d, bars + 8 * kLpStages);
+  }
+  for (int t = 0; t < min(n_tiles, kLpStages - 1); ++t) fetch(t);
   // rows of this thread: wm * 16 + g and + 8; a row past the end sees what the last one sees and is not stored
   int pos[2];
 #pragma unroll
   for (int i = 0; i < 2; ++i) pos[i] = pos0 + min(row0 + wm * 16 + g + 8 * i, rows - 1) / H;
-  constexpr int NT = R / 16;                                      // 8-column blocks of a warp's half of the latent
-  float o[NT][4];
+  constexpr int NT = R / 32;                                      // 8-column blocks of a warp's quarter of the latent
+  float o[2][NT][4];
 #pragma unroll
-  for (int j = 0; j < NT; ++j)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int e = 0; e < 4; ++e) o[j][e] = 0.f;
-  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o[i][j][e] = 0.f;
+  float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, l[2] = {0.f, 0.f};      // rows wr * 32 + g + 8 i; of the warp's own 16
   const int lm_row = lane & 15, lm_half = lane >> 4;              // rows and packet of an ldmatrix.x4 of 16 x 16
 
+  mbar_wait(bars + 8 * kLpStages, 0, abort_flag, status, 41);     // (a wait that gives up sets the status; the block goes on to its end)
   for (int t = 0; t < n_tiles; ++t) {
-    cp_async_wait<kLpStages - 2>();
+    mbar_wait(bars + 8 * (t % kLpStages), (t / kLpStages) & 1, abort_flag, status, 42);
     __syncthreads();
-    if (t + kLpStages - 1 < n_tiles)
-      latent_fetch<kLpKeys>(sk + ((t + kLpStages - 1) % kLpStages) * kLpKeys * ld, cache, bt, (t + kLpStages - 1) * kLpKeys, keys, d,
-                            page_size, num_pages);
-    cp_async_commit();
+    if (t + kLpStages - 1 < n_tiles) fetch(t + kLpStages - 1);
     const uint32_t kt = sk + (t % kLpStages) * kLpKeys * ld;
-    // scores of 16 rows and 16 keys
+    // scores of 32 rows and 16 keys over half of the columns; the other half's come through shared memory
+    float part[2][2][4];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) part[i][j][e] = 0.f;
+    const uint32_t qa = sq + (wr * 32 + lm_row) * ld + 16 * lm_half;
+    const uint32_t ka = kt + (wn * 16 + (lane & 7) + 8 * lm_half) * ld + 16 * ((lane >> 3) & 1);
+    const int k_mid = (d / 16 + 1) / 2, k_end = wk ? d / 16 : k_mid;
+#pragma unroll 2
+    for (int k = wk ? k_mid : 0; k < k_end; ++k) {
+      uint32_t a[2][4], b[4];
+      ldmatrix_x4(a[0], qa + 32 * k);
+      ldmatrix_x4(a[1], qa + 16 * ld + 32 * k);
+      ldmatrix_x4(b, ka + 32 * k);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        mma_bf16_16816(part[i][0], a[i], b[0], b[1]);
+        mma_bf16_16816(part[i][1], a[i], b[2], b[3]);
+      }
+    }
     float s[2][4];
 #pragma unroll
     for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) s[j][e] = 0.f;
-    const uint32_t qa = sq + (wm * 16 + lm_row) * ld + 16 * lm_half;
-    const uint32_t ka = kt + (wn * 16 + (lane & 7) + 8 * lm_half) * ld + 16 * ((lane >> 3) & 1);
-#pragma unroll 4
-    for (int k = 0; k < d / 16; ++k) {
-      uint32_t a[4], b[4];
-      ldmatrix_x4(a, qa + 32 * k);
-      ldmatrix_x4(b, ka + 32 * k);
-      mma_bf16_16816(s[0], a, b[0], b[1]);
-      mma_bf16_16816(s[1], a, b[2], b[3]);
-    }
+      for (int e = 0; e < 4; e += 2) {
+        const float give0 = wk ? part[0][j][e] : part[1][j][e], give1 = wk ? part[0][j][e + 1] : part[1][j][e + 1];
+        asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(sx + (((warp * 4 + 2 * j + e / 2) * 32 + lane) << 3)), "f"(give0), "f"(give1) : "memory");
+      }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; e += 2) {
+        float got0, got1;
+        asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(got0), "=f"(got1) : "r"(sx + ((((warp ^ 4) * 4 + 2 * j + e / 2) * 32 + lane) << 3)) : "memory");
+        s[j][e] = (wk ? part[1][j][e] : part[0][j][e]) + got0;
+        s[j][e + 1] = (wk ? part[1][j][e + 1] : part[0][j][e + 1]) + got1;
+      }
     // to base 2, the causal bound, the rows' maxima over both halves of the keys
     float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
@@ -141,45 +208,54 @@ latent_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __re
       s_max[wn][wm * 16 + g + 8] = mx[1];
     }
     __syncthreads();
-    float alpha[2];
+    float alpha[4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const float now = fmaxf(m[i], fmaxf(mx[i], s_max[wn ^ 1][wm * 16 + g + 8 * i]));      // (key 0 is in the first tile: finite)
+    for (int i = 0; i < 4; ++i) {
+      const int row = wr * 32 + g + 8 * i;
+      const float now = fmaxf(m[i], fmaxf(s_max[0][row], s_max[1][row]));      // (key 0 is in the first tile: finite)
       alpha[i] = exp2f(m[i] - now);
       m[i] = now;
-      l[i] *= alpha[i];
     }
+    const float own_m[2] = {wk ? m[2] : m[0], wk ? m[3] : m[1]};
+    l[0] *= wk ? alpha[2] : alpha[0];
+    l[1] *= wk ? alpha[3] : alpha[1];
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       float p[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        p[e] = exp2f(s[j][e] - m[e >> 1]);
+        p[e] = exp2f(s[j][e] - own_m[e >> 1]);
         l[e >> 1] += p[e];
       }
       const uint32_t at = sp + (wm * 16 + g) * kLpWeightBytes + (wn * 16 + j * 8 + c2) * 2;
       asm volatile("st.shared.b32 [%0], %1;" ::"r"(at), "r"(pack_bf16(p[0], p[1])) : "memory");
       asm volatile("st.shared.b32 [%0], %1;" ::"r"(at + 8 * kLpWeightBytes), "r"(pack_bf16(p[2], p[3])) : "memory");
     }
-    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f)) {
+    if (__any_sync(0xffffffffu, alpha[0] != 1.f || alpha[1] != 1.f || alpha[2] != 1.f || alpha[3] != 1.f)) {
 #pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        o[j][0] *= alpha[0]; o[j][1] *= alpha[0];
-        o[j][2] *= alpha[1]; o[j][3] *= alpha[1];
-      }
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) {
+          o[i][j][0] *= alpha[2 * i]; o[i][j][1] *= alpha[2 * i];
+          o[i][j][2] *= alpha[2 * i + 1]; o[i][j][3] *= alpha[2 * i + 1];
+        }
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < kLpKeys / 16; ++k) {
-      uint32_t a[4];
-      ldmatrix_x4(a, sp + (wm * 16 + lm_row) * kLpWeightBytes + 32 * k + 16 * lm_half);
-      const uint32_t va = kt + (16 * k + lm_row) * ld + wn * R + 16 * lm_half;       // (R bytes: half of the latent's columns)
+      uint32_t a[2][4];
+      ldmatrix_x4(a[0], sp + (wr * 32 + lm_row) * kLpWeightBytes + 32 * k + 16 * lm_half);
+      ldmatrix_x4(a[1], sp + (wr * 32 + 16 + lm_row) * kLpWeightBytes + 32 * k + 16 * lm_half);
+      const uint32_t va = kt + (16 * k + lm_row) * ld + wc * (R / 2) + 16 * lm_half;       // (R / 2 bytes: a quarter of the latent's columns)
 #pragma unroll
       for (int j = 0; j < NT; j += 2) {
         uint32_t b[4];
         ldmatrix_x4_trans(b, va + 16 * j);
-        mma_bf16_16816(o[j], a, b[0], b[1]);
-        mma_bf16_16816(o[j + 1], a, b[2], b[3]);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          mma_bf16_16816(o[i][j], a[i], b[0], b[1]);
+          mma_bf16_16816(o[i][j + 1], a[i], b[2], b[3]);
+        }
       }
     }
   }
@@ -194,14 +270,14 @@ latent_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __re
   }
   __syncthreads();
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int row = wm * 16 + g + 8 * i;
+  for (int i = 0; i < 4; ++i) {
+    const int row = wr * 32 + g + 8 * i;
     if (row0 + row >= rows) continue;
     const float inv = 1.0f / (s_sum[0][row] + s_sum[1][row]);
-    __nv_bfloat16* dst = out + ((size_t)token0 * H + row0 + row) * R + wn * (R / 2) + c2;
+    __nv_bfloat16* dst = out + ((size_t)token0 * H + row0 + row) * R + wc * (R / 4) + c2;
 #pragma unroll
     for (int j = 0; j < NT; ++j)
-      *reinterpret_cast<uint32_t*>(dst + 8 * j) = pack_bf16(o[j][2 * i] * inv, o[j][2 * i + 1] * inv);
+      *reinterpret_cast<uint32_t*>(dst + 8 * j) = pack_bf16(o[i >> 1][j][2 * (i & 1)] * inv, o[i >> 1][j][2 * (i & 1) + 1] * inv);
   }
 }
 
@@ -426,14 +502,14 @@ inline bool latent_tc_fits(const void* out, const void* q, const void* cache, in
 
 template <int R>
 int latent_prefill(void* out, const void* q, const void* cache, const int* bt, const int* tiles, int n_tiles, int bt_stride, int H, int d,
-                   int page_size, int num_pages, float scale, int tile_tokens, void* stream) {
-  const int smem = (kLpRows + kLpStages * kLpKeys) * latent_row_bytes(d) + kLpRows * kLpWeightBytes;
+                   int page_size, int num_pages, float scale, int tile_tokens, int* status, void* stream) {
+  const int smem = (kLpRows + kLpStages * kLpKeys) * latent_row_bytes(d) + kLpRows * kLpWeightBytes + kLpThreads * 32;
   static SmemRaised raised;
   if (int rc = raise_shared_memory("latent_prefill", latent_prefill_kernel<R>, 200 * 1024, raised)) return rc;
   const dim3 grid((tile_tokens * H + kLpRows - 1) / kLpRows, n_tiles);
   return launch_kernel("latent_prefill", latent_prefill_kernel<R>, grid, dim3(kLpThreads), smem, as_stream(stream), (__nv_bfloat16*)out,
                        (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, tiles, bt_stride, H, d, page_size, num_pages,
-                       scale * 1.4426950408889634f);
+                       scale * 1.4426950408889634f, status);
 }
 
 template <int R>
@@ -455,15 +531,22 @@ int latent_decode(void* out, float* part, float* ml, const void* q, const void* 
 
 }  // namespace ptl
 
-PTL_EXPORT int ptl_latent_prefill_bf16(void* out, const void* q, const void* cache, const int* block_table, const int* tiles, int n_tiles,
-                                       int bt_stride, int H, int R, int n, int page_size, int num_pages, float scale, int tile_tokens,
-                                       void* stream) {
+// `status`: set where a wait inside the kernel gave up (null: nowhere).
+PTL_EXPORT int ptl_latent_prefill_status_bf16(void* out, const void* q, const void* cache, const int* block_table, const int* tiles, int n_tiles,
+                                              int bt_stride, int H, int R, int n, int page_size, int num_pages, float scale, int tile_tokens,
+                                              void* status, void* stream) {
   if (!ptl::latent_tc_fits(out, q, cache, H, R, n) || n_tiles > 65535) return -2;
   PTL_REQUIRE(n_tiles >= 0 && bt_stride > 0 && page_size > 0 && num_pages > 0 && tile_tokens > 0,
               "latent_prefill: bad sizes");
   if (n_tiles == 0) return 0;
   const auto fn = R == 128 ? ptl::latent_prefill<128> : R == 256 ? ptl::latent_prefill<256> : ptl::latent_prefill<512>;
-  return fn(out, q, cache, block_table, tiles, n_tiles, bt_stride, H, R + n, page_size, num_pages, scale, tile_tokens, stream);
+  return fn(out, q, cache, block_table, tiles, n_tiles, bt_stride, H, R + n, page_size, num_pages, scale, tile_tokens, (int*)status, stream);
+}
+PTL_EXPORT int ptl_latent_prefill_bf16(void* out, const void* q, const void* cache, const int* block_table, const int* tiles, int n_tiles,
+                                       int bt_stride, int H, int R, int n, int page_size, int num_pages, float scale, int tile_tokens,
+                                       void* stream) {
+  return ptl_latent_prefill_status_bf16(out, q, cache, block_table, tiles, n_tiles, bt_stride, H, R, n, page_size, num_pages, scale, tile_tokens,
+                                        nullptr, stream);
 }
 
 PTL_EXPORT int ptl_latent_decode_bf16(void* out, float* part, float* ml, const void* q, const void* cache, const int* block_table,

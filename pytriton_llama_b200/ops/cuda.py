@@ -247,6 +247,8 @@ def load_library() -> ctypes.CDLL:
     lib.ptl_latent_prefill_bf16.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_f,
                                             _c_int, _ptr]
     lib.ptl_latent_prefill_bf16.restype = _c_int
+    lib.ptl_latent_prefill_status_bf16.argtypes = lib.ptl_latent_prefill_bf16.argtypes[:-1] + [_ptr, _ptr]
+    lib.ptl_latent_prefill_status_bf16.restype = _c_int
     lib.ptl_latent_decode_bf16.argtypes = [_ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _ptr, _c_int, _c_int, _c_int, _c_int, _c_int,
                                            _c_int, _c_int, _c_int, _c_f, _ptr]
     lib.ptl_latent_decode_bf16.restype = _c_int
@@ -1901,9 +1903,9 @@ class CudaOps:
             return None
         out = self.empty((q.shape[0], H * R), q.dtype)
         if tiles.items:
-            self._check(self.lib.ptl_latent_prefill_bf16(
+            self._check(self.lib.ptl_latent_prefill_status_bf16(
                 _p(out), _p(q), _p(cache), _p(block_table), _p(tiles.tensor), tiles.items, block_table.shape[1], H, R, n, page_size,
-                cache.shape[0], float(scale), self.QUERY_TILE, self._stream()))
+                cache.shape[0], float(scale), self.QUERY_TILE, _p(self._tc_status_word()), self._stream()))
         if dec.items:
             longest = getattr(ctx, "max_ctx_len", 0) or block_table.shape[1] * page_size
             splits = max(1, min(-(-longest // 64), self._sm_count // (dec.items * -(-H // 16))))

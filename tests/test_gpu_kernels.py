@@ -1050,3 +1050,9 @@ def test_product_for_a_few_tokens_and_small_weights(_ops, M, N, K):
     alone = ops.gemm_tc(x[:1].contiguous().cuda(), w.cuda(), ops.EPI_F32)
     assert torch.equal(alone.cpu()[0], results[True][0][0])
     assert ops.gemm_tc_status() == 0
+
+
+@pytest.mark.parametrize("M, N, K", [(8, 4096, 1024), (3, 5920, 1000), (8, 1184, 4096), (5, 36, 7168)])
+def test_product_for_a_few_tokens_up_to_the_blocks_an_sm_holds(_ops, M, N, K):
+    """The most blocks of 148 SMs: five an SM (by registers) of short rows, one of long ones, the longest row that fits."""
+    test_product_for_a_few_tokens_and_small_weights(_ops, M, N, K)
