@@ -147,7 +147,8 @@ __device__ __forceinline__ float block_max(float v, float* scratch) {
 // not depend on earlier kernels (set-up, fetching weights), then `pdl_wait()` holds each thread
 // until every earlier kernel has finished and its writes are visible.  `pdl_launch_dependents()`
 // lets the successor start likewise.  Rule: no access to memory that another kernel of the step
-// writes, and no global write at all, before `pdl_wait()`.
+// writes, and no global write at all, before `pdl_wait()`; and no `pdl_launch_dependents()` before it either, so that what runs
+// beside a kernel's first part is the one kernel before it (decode attention reads what kernels further back have written).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -85,6 +85,7 @@ gemm_simt_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_
     }
     return;
   }
+  pdl_wait();                                                  // (nothing is lost: a turn needs the tokens too)
   pdl_launch_dependents();
   const auto meet = [] { asm volatile("bar.sync 1, %0;" ::"n"((WARPS + 1) * 32) : "memory"); };
   const int chunk = lane & 7, group = lane >> 3;
@@ -94,7 +95,6 @@ gemm_simt_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_
 #pragma unroll
   for (int i = 0; i < PER; ++i) { sum[i] = 0.f; comp[i] = 0.f; }
   const bool works = warp < WARPS;
-  if (!works) pdl_wait();
   const int rounds = (turns + WARPS - 1) / WARPS;
   int in_tile = 0, done_round = 0, done_tile = blockIdx.x;      // round of the tile: being multiplied, being added
   int first = 0, buffer = 0;                                                         // this tile's turns before, parity of the rounds

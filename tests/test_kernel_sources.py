@@ -46,3 +46,24 @@ def test_what_a_kernel_of_the_step_may_have_written_is_read_after_the_wait(name,
 def test_the_kernels_with_clusters_are_found():
     found = {name for _, name, body in KERNELS if PEER_ACCESS.search(body)}
     assert {"decode_attention_kernel", "gemm_tc_kernel", "sample_cluster_kernel", "token_side_cluster_kernel"} <= found
+
+
+def _blocks_around(body, at):
+    """Where the blocks that hold a place of a kernel's body open, outermost first."""
+    opened = []
+    for i, c in enumerate(body[:at]):
+        if c == "{":
+            opened.append(i)
+        elif c == "}":
+            opened.pop()
+    return opened
+
+
+@pytest.mark.parametrize("source,name,body", [k for k in KERNELS if "pdl_launch_dependents()" in k[2]], ids=lambda v: v if len(v) < 60 else "")
+def test_dependents_start_behind_the_wait_on_the_predecessor(source, name, body):
+    """A kernel that let its successor start before it has waited itself would have three kernels run side by side, and the successor's
+    reads ahead of its wait are right beside its predecessor only: on every path a wait of the same or an enclosing block comes first."""
+    for launch in re.finditer(r"pdl_launch_dependents\(\)", body):
+        around = _blocks_around(body, launch.start())
+        waits = [_blocks_around(body, w.start()) for w in re.finditer(r"(?<=[;{}])\s*pdl_wait\(\);", body[:launch.start()])]
+        assert any(w == around[:len(w)] for w in waits), f"{source}: {name}"
