@@ -32,7 +32,7 @@ __device__ __forceinline__ void stream_kahan(float& sum, float& comp, float chun
 template <int MT, int ROWS, int WARPS, int STAGES>
 __global__ void __launch_bounds__((WARPS + 2) * 32)
 gemm_simt_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map, float* __restrict__ out,
-                        int M, int N, int K, int ldo, int accumulate, int* __restrict__ status) {
+                        int M, int N, int K, int ldo, int accumulate, int* __restrict__ status, CopyWaits waits) {
   static_assert(STAGES >= WARPS, "a stage's next filling is waited for a round after its last at the earliest");
   constexpr int kStage = (ROWS + MT) * 1024, SUMS_LD = stream_sums_ld(MT, ROWS);
   extern __shared__ __align__(1024) unsigned char stream_smem[];
@@ -53,6 +53,7 @@ gemm_simt_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_
   }
   __syncthreads();
   if (base & 1023u) {                                          // never expected (the same in every block)
+    pdl_wait();
     if (threadIdx.x == 0 && status) atomicExch(status, 99);
     return;
   }
@@ -60,28 +61,29 @@ gemm_simt_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_
     if (lane == 0) {
       const int ahead = min(all, STAGES);
       int turn = 0, n0 = blockIdx.x * ROWS, turn_x = 0;
-      const auto weights = [&](int s) {
-        mbar_expect_tx(full(s), kStage);
-        tma_load_3d(base + s * kStage, &w_map, full(s), 0, turn * 8, n0);
+      const auto weights = [&](int s, int t) {
+        if (t != waits.withheld) {
+          mbar_expect_tx(full(s), kStage);
+          tma_load_3d(base + s * kStage, &w_map, full(s), 0, turn * 8, n0);
+        }
         if (++turn == turns) { turn = 0; n0 += gridDim.x * ROWS; }
       };
-      const auto tokens = [&](int s) {
-        tma_load_3d(base + s * kStage + ROWS * 1024, &x_map, full(s), 0, turn_x * 8, 0);
+      const auto tokens = [&](int s, int t) {
+        if (t != waits.withheld) tma_load_3d(base + s * kStage + ROWS * 1024, &x_map, full(s), 0, turn_x * 8, 0);
         if (++turn_x == turns) turn_x = 0;
       };
-      for (int t = 0; t < ahead; ++t) weights(t);
+      for (int t = 0; t < ahead; ++t) weights(t, t);
       pdl_wait();
-      for (int t = 0; t < ahead; ++t) tokens(t);
+      for (int t = 0; t < ahead; ++t) tokens(t, t);
       int s = 0, round = 0, t = ahead;
       for (; t < all; ++t) {
-        if (!mbar_wait(empty(s), round, abort_flag, status, 21)) break;
-        weights(s);
-        tokens(s);
+        if (!mbar_wait(empty(s), round, abort_flag, status, 21, waits.polls)) break;
+        weights(s, t);
+        tokens(s, t);
         if (++s == STAGES) { s = 0; round ^= 1; }
       }
-      if (*abort_flag)                                         // leave no copy in flight behind
-        for (int i = max(0, t - STAGES); i < t; ++i)
-          for (uint32_t n = 0; n < (1u << 16) && !mbar_try_wait(full(i % STAGES), (i / STAGES) & 1); ++n) __nanosleep(100);
+      // leave no copy in flight behind, also where a warp gives up after the last one was asked for (else they are here by the time the warps are done)
+      for (int i = max(0, t - STAGES); i < t; ++i) mbar_drain(full(i % STAGES), (i / STAGES) & 1);
     }
     return;
   }
@@ -102,7 +104,7 @@ gemm_simt_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_
     const int turn = in_tile * WARPS + warp;
     if (works && n > 0 && turn < turns) {
       const int g = first + turn, s = g % STAGES;
-      mbar_wait(full(s), (g / STAGES) & 1, abort_flag, status, 22);      // (given up: the flag is set, and the warps go on to their meetings)
+      mbar_wait(full(s), (g / STAGES) & 1, abort_flag, status, 22, waits.polls);      // (given up: the flag is set, and the warps go on to their meetings)
       float2 acc[RL][MT];                                               // sums of even and of odd k
 #pragma unroll
       for (int r = 0; r < RL; ++r)
@@ -133,7 +135,7 @@ gemm_simt_stream_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_
         }
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(empty(s));
+      if (lane == 0 && !*abort_flag) mbar_arrive(empty(s));              // (a stage that did not come must not be asked for again)
       float* dst = sums + (size_t)buffer * WARPS * 8 * SUMS_LD + (warp * 8 + chunk) * SUMS_LD + group * (RL * MT + 8);
 #pragma unroll
       for (int r = 0; r < RL; ++r)
@@ -201,7 +203,7 @@ static int stream_map(CUtensorMap* map, const void* base, int rows, int K, int l
 
 template <int MT, int ROWS, int WARPS, int STAGES, int HELD>
 static int launch_stream(float* out, const float* A, const float* W, int M, int N, int K, int lda, int ldw, int ldo, int accumulate, int* status,
-                         cudaStream_t stream) {
+                         cudaStream_t stream, CopyWaits waits) {
   static SmemRaised raised;
   auto kernel = gemm_simt_stream_kernel<MT, ROWS, WARPS, STAGES>;
   constexpr int smem = stream_smem_bytes(MT, ROWS, WARPS, STAGES);
@@ -211,14 +213,13 @@ static int launch_stream(float* out, const float* A, const float* W, int M, int 
   if (!rc) rc = stream_map(&x_map, A, M, K, lda, MT);
   if (rc) return rc;
   return launch_kernel("gemm_simt_stream", kernel, dim3(std::min((N + ROWS - 1) / ROWS, HELD * sm_count_of_device())), dim3((WARPS + 2) * 32), smem, stream, w_map, x_map, out, M, N,
-                       K, ldo, accumulate, status);
+                       K, ldo, accumulate, status, waits);
 }
 
 }  // namespace ptl
 
-// -2: sizes that gemm_simt takes.
-PTL_EXPORT int ptl_gemm_simt_stream_f32(void* out, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldo, int accumulate,
-                                        void* status, void* stream) {
+static int stream_product(void* out, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldo, int accumulate, void* status,
+                          void* stream, ptl::CopyWaits waits = {}) {
   using namespace ptl;
   const bool narrow = N < 4736;       // fewer than four blocks of eight rows per SM
   if (M < 1 || M > 32 || (M > 16 && !narrow) || N < 1 || K < 32 || K % 32 || lda < K || ldw < K || ldo < N || lda % 4 || ldw % 4 || !aligned16(A) ||
@@ -226,7 +227,7 @@ PTL_EXPORT int ptl_gemm_simt_stream_f32(void* out, const void* A, const void* W,
     return -2;
 #define PTL_STREAM(MT, ROWS, WARPS, STAGES, HELD)                                                                               \
   return launch_stream<MT, ROWS, WARPS, STAGES, HELD>((float*)out, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldo, accumulate, \
-                                                (int*)status, as_stream(stream))
+                                                (int*)status, as_stream(stream), waits)
   if (M <= 1) PTL_STREAM(1, 8, 4, 5, 4);
   if (M <= 2) PTL_STREAM(2, 8, 4, 4, 4);
   if (M <= 4) PTL_STREAM(4, 8, 4, 4, 3);
@@ -234,4 +235,17 @@ PTL_EXPORT int ptl_gemm_simt_stream_f32(void* out, const void* A, const void* W,
   if (M <= 16) PTL_STREAM(16, 16, 4, 4, 1);
   PTL_STREAM(32, 8, 2, 3, 1);
 #undef PTL_STREAM
+}
+
+// -2: sizes that gemm_simt takes.
+PTL_EXPORT int ptl_gemm_simt_stream_f32(void* out, const void* A, const void* W, int M, int N, int K, int lda, int ldw, int ldo, int accumulate,
+                                        void* status, void* stream) {
+  return stream_product(out, A, W, M, N, K, lda, ldw, ldo, accumulate, status, stream);
+}
+// Self-test of the bounded waits: they give up after `polls` polls, and no block asks for its turn `no_turn` (counted over its tiles).  The
+// kernel must then write *status (21 or 22) and return; `out` holds nothing of value.
+PTL_EXPORT int ptl_gemm_simt_stream_wait_selftest(void* out, const void* A, const void* W, int M, int N, int K, void* status, void* stream,
+                                                  unsigned polls, int no_turn) {
+  PTL_REQUIRE(status && polls >= 1 && polls <= (1u << 16), "gemm_simt_stream_wait_selftest: a status word, and between 1 and 65536 polls");
+  return stream_product(out, A, W, M, N, K, K, K, N, 0, status, stream, {polls, no_turn});
 }

@@ -49,6 +49,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   if (status) atomicExch(status, code);
   return false;
 }
+// What a kernel that fetches by bulk copies does once a wait for one of them has given up: before the block ends, wait (bounded too) for
+// what it has asked for, because a copy still in flight would land in shared memory that another block holds by then.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity, uint32_t limit = 1u << 16) {
+  for (uint32_t i = 0; i < limit && !mbar_try_wait(bar, parity); ++i) __nanosleep(100);
+}
+// Bounds of a kernel's waits for its copies, and the one of its fetches (counted from 0) that a self-test leaves out (-1: none).
+struct CopyWaits {
+  uint32_t polls = kPollLimit;
+  int withheld = -1;
+};
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y) : "memory");

@@ -1,6 +1,7 @@
 """Each CUDA kernel alone against its plain PyTorch statement (tests/torch_ops.py), at sizes other
 than the engine's tests use: widths that are no power of two, rows that are not 16-byte
 multiples, head sizes from 16 to 256, odd head counts and groups (GPU)."""
+import ctypes
 import math
 
 import pytest
@@ -1056,3 +1057,18 @@ def test_product_for_a_few_tokens_and_small_weights(_ops, M, N, K):
 def test_product_for_a_few_tokens_up_to_the_blocks_an_sm_holds(_ops, M, N, K):
     """The most blocks of 148 SMs: five an SM (by registers) of short rows, one of long ones, the longest row that fits."""
     test_product_for_a_few_tokens_and_small_weights(_ops, M, N, K)
+@pytest.mark.parametrize("no_turn", [0, 3, 5])
+def test_float32_product_of_few_rows_gives_up_a_turn_that_does_not_come(_ops, no_turn):
+    """No block asks for one of its turns (of the ring's first filling, and of a later one): the waits run out, the status is set, and the
+    block ends once the copies it did ask for are there."""
+    lib, status = _ops.lib, _ops._tc_status_word()
+    lib.ptl_gemm_simt_stream_wait_selftest.argtypes = [ctypes.c_void_p] * 3 + [ctypes.c_int] * 3 + [ctypes.c_void_p] * 2 + [ctypes.c_uint, ctypes.c_int]
+    assert _ops.gemm_tc_status() == 0
+    x, w, out = rnd((4, 2048), torch.float32, 97).cuda(), rnd((40, 2048), torch.float32, 98).cuda(), torch.zeros((4, 40), device="cuda")
+    args = [t.data_ptr() for t in (out, x, w)] + [4, 40, 2048, status.data_ptr(), torch.cuda.current_stream().cuda_stream]
+    assert lib.ptl_gemm_simt_stream_wait_selftest(*args, 300, no_turn) == 0, lib.ptl_last_error().decode()
+    torch.cuda.synchronize()
+    assert _ops.gemm_tc_status() in (21, 22)
+    want = _ops.linear(x, w)
+    assert lib.ptl_gemm_simt_stream_wait_selftest(*args, 65536, -1) == 0
+    assert torch.equal(out, want) and _ops.gemm_tc_status() == 0
