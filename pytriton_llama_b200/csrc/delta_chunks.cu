@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(kDcThreads, 1)
 delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, float* work, const T* __restrict__ qkv,
                         const float* __restrict__ ba, const float* __restrict__ rate, const float* __restrict__ dt_bias, int kv_heads,
                         float unit_eps, float q_scale, const int* __restrict__ q_start, const int* __restrict__ positions,
-                        const int* __restrict__ state_slot, int requests, int heads, int dv, int walk_max, int* status) {
+                        const int* __restrict__ state_slot, int requests, int heads, int dv, int walk_max, int* status, CopyWaits waits) {
   constexpr int LD = D + 4, RB = D / 32;
   extern __shared__ __align__(16) float dw_smem[];
   constexpr int kChunk = (int)dc_walk_floats(D);
@@ -352,7 +352,7 @@ delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, floa
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   auto fetch = [&](int chunk) {
-    if (tid != 0) return;
+    if (tid != 0 || chunk == waits.withheld) return;
     const uint32_t bar = full + 8 * (chunk & 1);
     mbar_expect_tx(bar, kChunk * 4);
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -372,9 +372,13 @@ delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, floa
     const float* wv = base + chunk * stride + dc_values_at(D);
     float* columns = base + chunk * stride + dc_columns_at(D, dv) + (size_t)j0 * (D + kDcTokens);
     const float v0 = wv[(size_t)rg * dv + j0 + s], v1 = wv[(size_t)(rg + 32) * dv + j0 + s], decay = wv[(size_t)kDcTokens * dv];
-    // this chunk is here (one that did not come sets the status and is worked as it is); the chunk before has been read and its state written
-    mbar_wait(full + 8 * (chunk & 1), chunk >> 1 & 1, abort_flag, status, 31);
-    __syncthreads();
+    // this chunk is here; the chunk before has been read and its state written.  A chunk that does not come ends the walk with the
+    // status set: nothing else is in flight then, and the state in memory stays what it was
+    const bool came = mbar_wait(full + 8 * (chunk & 1), chunk >> 1 & 1, abort_flag, status, 31, waits.polls);
+    if (__syncthreads_or(!came)) {
+      if (tid == 0) mbar_drain(full + 8 * (chunk & 1), chunk >> 1 & 1);
+      return;
+    }
     if (chunk + 1 < chunks) fetch(chunk + 1);
     float first[2];
     dc_product<2, D, LD, LD>(s_c + (chunk & 1) * kChunk + rg * LD, s_s, s, first);
@@ -409,7 +413,7 @@ delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, floa
 template <int D>
 __global__ void __launch_bounds__(kDcThreads, 2)
 delta_chunk_outputs_kernel(float* __restrict__ out, const float* __restrict__ work, const int* __restrict__ q_start, const int* __restrict__ state_slot,
-                           int requests, int heads, int dv, int walk_max, int* status) {
+                           int requests, int heads, int dv, int walk_max, int* status, CopyWaits waits) {
   constexpr int K = D + kDcTokens, LA = K + 4;
   extern __shared__ __align__(16) float do_smem[];
   float* s_a = do_smem;                                  // [64 tokens][queries D | weights 64]
@@ -435,7 +439,7 @@ delta_chunk_outputs_kernel(float* __restrict__ out, const float* __restrict__ wo
     mbar_expect_tx(full, (kDcTokens + cols) * K * 4);
   }
   __syncthreads();
-  if (tid < kDcTokens + cols) {
+  if (tid < kDcTokens + cols && tid != waits.withheld) {
     const bool is_a = tid < kDcTokens;
     const int r = is_a ? tid : tid - kDcTokens;
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -443,8 +447,11 @@ delta_chunk_outputs_kernel(float* __restrict__ out, const float* __restrict__ wo
   }
   if (tid >= kDcTokens + cols && tid < kDcTokens + kDcOutCols)          // columns that there are not
     for (int k = 0; k < K; ++k) s_b[(tid - kDcTokens) * LA + k] = 0.f;
-  mbar_wait(full, 0, abort_flag, status, 32);
-  __syncthreads();
+  const bool came = mbar_wait(full, 0, abort_flag, status, 32, waits.polls);
+  if (__syncthreads_or(!came)) {                         // (nothing is written; the status says so)
+    if (tid == 0) mbar_drain(full, 0);
+    return;
+  }
   float sum[4][4];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
@@ -488,7 +495,7 @@ delta_chunk_outputs_kernel(float* __restrict__ out, const float* __restrict__ wo
 template <typename T, int D>
 int delta_chunks(float* out, float* work, int chunks, int portions, const void* qkv, const float* ba, const float* rate, const float* dt_bias, float* state,
                  const int* q_start, const int* positions, const int* state_slot, int requests, int heads, int kv_heads, int dv,
-                 float unit_eps, float q_scale, int walk_max, int* status, void* stream) {
+                 float unit_eps, float q_scale, int walk_max, int* status, void* stream, CopyWaits walk_waits, CopyWaits output_waits) {
   static SmemRaised raised_p, raised_w, raised_o;
   if (int rc = raise_shared_memory("delta_chunk_prepare", delta_chunk_prepare_kernel<T, D>, (int)dc_prepare_smem(D), raised_p)) return rc;
   if (int rc = raise_shared_memory("delta_chunk_walk", delta_chunk_walk_kernel<T, D>, (int)dc_walk_smem(D), raised_w)) return rc;
@@ -499,24 +506,25 @@ int delta_chunks(float* out, float* work, int chunks, int portions, const void* 
   if (int rc = raise_shared_memory("delta_chunk_outputs", delta_chunk_outputs_kernel<D>, (int)dc_outputs_smem(D), raised_o)) return rc;
   if (int rc = launch_kernel("delta_chunk_walk", delta_chunk_walk_kernel<T, D>, dim3(dv / kDcCols, heads, portions), dim3(kDcThreads), dc_walk_smem(D),
                              as_stream(stream), out, state, work, (const T*)qkv, ba, rate, dt_bias, kv_heads, unit_eps, q_scale, q_start,
-                             positions, state_slot, requests, heads, dv, walk_max, status))
+                             positions, state_slot, requests, heads, dv, walk_max, status, walk_waits))
     return rc;
   return launch_kernel("delta_chunk_outputs", delta_chunk_outputs_kernel<D>, dim3(chunks, heads, (dv + kDcOutCols - 1) / kDcOutCols),
                        dim3(kDcThreads), dc_outputs_smem(D), as_stream(stream), out, (const float*)work, q_start, state_slot, requests, heads, dv,
-                       walk_max, status);
+                       walk_max, status, output_waits);
 }
 
 template <typename T>
 int delta_chunks_any(float* out, float* work, int chunks, int portions, const void* qkv, const float* ba, const float* rate, const float* dt_bias,
                      float* state, const int* q_start, const int* positions, const int* state_slot, int requests, int heads, int kv_heads,
-                     int d, int dv, float unit_eps, float q_scale, int walk_max, int* status, void* stream) {
+                     int d, int dv, float unit_eps, float q_scale, int walk_max, int* status, void* stream, CopyWaits walk_waits = {},
+                     CopyWaits output_waits = {}) {
   PTL_REQUIRE(requests >= 0 && requests <= 65535 && portions >= 0 && portions <= requests && heads > 0 && heads <= 65535 && kv_heads > 0 && heads % kv_heads == 0 && chunks >= 0 && walk_max >= 0 &&
                   (d == 64 || d == 128) && dv > 0 && dv % kDcCols == 0 && aligned16(work),
               "gated_delta_rule in chunks: bad sizes heads=%d kv_heads=%d d=%d (64 or 128) dv=%d", heads, kv_heads, d, dv);
   if (requests == 0 || chunks == 0 || portions == 0) return 0;
   const auto fn = d == 64 ? delta_chunks<T, 64> : delta_chunks<T, 128>;
   return fn(out, work, chunks, portions, qkv, ba, rate, dt_bias, state, q_start, positions, state_slot, requests, heads, kv_heads, dv, unit_eps,
-            q_scale, walk_max, status, stream);
+            q_scale, walk_max, status, stream, walk_waits, output_waits);
 }
 
 }  // namespace ptl
@@ -533,3 +541,16 @@ PTL_EXPORT long long ptl_delta_chunk_floats(int d, int dv) { return (long long)p
   }
 PTL_DELTA_CHUNKS(_f32, float)
 PTL_DELTA_CHUNKS(_bf16, __nv_bfloat16)
+
+// Self-test of the bounded waits: the float32 form whose waits give up after `polls` polls and in which every walk leaves out the copy of
+// chunk `no_chunk`, or every block of the outputs that of row `no_row` (-1: none).  The kernel must then write *status (31: the walk, 32: the
+// outputs) and return; a walk that gives up leaves the state as it was, and `out` holds nothing of value.
+PTL_EXPORT int ptl_gated_delta_chunks_wait_selftest(float* out, float* work, int chunks, int portions, const void* qkv, const float* ba,
+                                                    const float* rate, const float* dt_bias, float* state, const int* q_start,
+                                                    const int* positions, const int* state_slot, int requests, int heads, int kv_heads, int d,
+                                                    int dv, float unit_eps, float q_scale, int walk_max, void* status, void* stream,
+                                                    unsigned polls, int no_chunk, int no_row) {
+  PTL_REQUIRE(status && polls >= 1 && polls <= (1u << 16), "gated_delta_chunks_wait_selftest: a status word, and between 1 and 65536 polls");
+  return ptl::delta_chunks_any<float>(out, work, chunks, portions, qkv, ba, rate, dt_bias, state, q_start, positions, state_slot, requests, heads,
+                                      kv_heads, d, dv, unit_eps, q_scale, walk_max, (int*)status, stream, {polls, no_chunk}, {polls, no_row});
+}

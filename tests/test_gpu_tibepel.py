@@ -1,6 +1,7 @@
 """The Tibepel decoder on the GPU: every new kernel against the plain PyTorch statement of its operator
 (tests/torch_ops.py), attention inputs made so that one key stands out at the edges of blocks and pages, and the
 engine -- whole prompts, decoding, portions, mixed batches, generation -- against tests/plain_tibepel.py."""
+import ctypes
 import json
 import math
 import random
@@ -332,6 +333,35 @@ def test_chunk_attention_keeps_a_bad_value_from_earlier_tokens(ops, G, d, talk, 
     assert torch.equal(got.isfinite(), want.isfinite()) and got[:at].isfinite().all() and not got[at:at + 3].isfinite().all()
     fine = want.isfinite()
     assert ((got - want)[fine].abs() <= 2 ** -7 * want[fine].abs() + 2e-5 * float(want[fine].abs().max())).all()
+
+
+@pytest.mark.parametrize("no_chunk,no_row,code", [(0, -1, 31), (2, -1, 31), (-1, 5, 32), (-1, 70, 32)])
+def test_delta_chunks_give_up_copies_that_do_not_come(ops, no_chunk, no_row, code):
+    """A chunk of the walk, or a row of the outputs' operands, is never asked for: the waits run out, the status is set, the kernels end by
+    themselves, a walk leaves the states as they were; the next call on the same device is right."""
+    H, d, dv, T = 2, 64, 16, 300
+    g = torch.Generator().manual_seed(9)
+    qkv, ba, rate, dtb, S = (torch.randn(T, 2 * H * d + H * dv, generator=g), torch.randn(T, 2 * H, generator=g), torch.rand(H, generator=g),
+                             torch.randn(H, generator=g), torch.randn(1, H, d, dv, generator=g))
+    ctx = _ctx([T], [7], [0], "cuda:0")
+    dev = [t.cuda() for t in (qkv, ba, rate, dtb)]
+    right_state = S.cuda()
+    right = ops.gated_delta_rule(*dev, right_state, ctx, H, H, d, dv, 1e-6, d ** -0.5)
+    lib, status, state, out = ops.lib, ops._tc_status_word(), S.cuda(), torch.zeros(T, H * dv, device="cuda")
+    chunks = T // 64 + 1
+    work = torch.zeros(chunks * H, lib.ptl_delta_chunk_floats(d, dv), device="cuda")
+    ptr = lambda *ts: [ctypes.c_void_p(t.data_ptr()) for t in ts]
+    call = lambda polls, chunk, row: lib.ptl_gated_delta_chunks_wait_selftest(
+        *ptr(out, work), chunks, 1, *ptr(*dev, state, ctx.q_start, ctx.positions, ctx.state_slot), 1, H, H, d, dv, ctypes.c_float(1e-6),
+        ctypes.c_float(d ** -0.5), 128, *ptr(status), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), polls, chunk, row)
+    assert ops.gemm_tc_status() == 0
+    assert call(300, no_chunk, no_row) == 0, lib.ptl_last_error().decode()
+    torch.cuda.synchronize()
+    assert ops.gemm_tc_status() == code
+    assert torch.equal(state, S.cuda()) == (code == 31)
+    state.copy_(S)
+    assert call(65536, -1, -1) == 0
+    assert torch.equal(out, right) and torch.equal(state, right_state) and ops.gemm_tc_status() == 0
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
