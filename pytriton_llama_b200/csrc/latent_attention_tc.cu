@@ -6,11 +6,13 @@
 //
 // latent_prefill: portions of prompts.  The rows of q, (token, head) after (token, head), are one matrix: a block takes 64 of
 // them from a tile of the step's list (128 tokens of one request) and walks the keys up to its last token's position in
-// tiles of 32, a ring of three; eight warps, four row groups by two: for the scores the two split the tile's keys, for the
-// weighted sums the latent's columns, the weights (rounded once to bfloat16, as the softmax over stored scores
-// did) pass through shared memory.  The rows of keys and queries come by one bulk copy each, a warp's lanes a tile (as copies of 16 bytes
-// they held all warps up for 1,200 of a tile's 5,500 cycles).  Bound by the fragments read for the warp-level tensor instructions, 434 KB per 64 x 32 scores; eight
-// prompts of 65 to 440 tokens (8 heads, R 512, n 64): LP_NOW us alone, 55 before.
+// tiles of 32, a ring of three.  Of the scores each of the eight warps works 32 rows by 16 keys over half of the columns (the halves meet through
+// shared memory), of the weighted sums 32 rows by a quarter of the latent's columns; the weights (rounded once to bfloat16, as the
+// softmax over stored scores did) pass through shared memory.  The rows of keys and queries come by one bulk copy each, a warp's lanes a
+// tile (as copies of 16 bytes they held all warps up for 1,200 of a tile's 5,500 cycles).  Bound by the fragments read for the warp-level tensor
+// instructions, 303 KB per 64 x 32 scores (16 rows a warp: 434).  8 heads, R 512, n 64, us against copies of 16 bytes and 16 rows a warp: eight
+// prompts of 65 to 440 tokens 60 and 71, one of 2,048 242 and 294, of 33 7.8 and 9.3, 128 tokens after 4,000 339 and 414; 16 heads, R 128: 202 and 207,
+// of 33 5.1 and 4.8.
 //
 // latent_decode: single tokens, all heads of a token (up to 16 per block) against a share of its keys, 64 at a time, two
 // tiles in flight; the float32 weights go to the tensor cores as three bfloat16 terms each (24 bits), so that nothing of
@@ -54,7 +56,7 @@ template <int R>
 __global__ void __launch_bounds__(kLpThreads, 1)
 latent_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
                       const int* __restrict__ block_table, const int* __restrict__ tiles, int bt_stride, int H, int d, int page_size,
-                      int num_pages, float scale_log2, int* status) {
+                      int num_pages, float scale_log2, int* status, CopyWaits waits) {
   extern __shared__ __align__(128) unsigned char lp_smem[];
   __shared__ uint64_t s_bars[kLpStages + 1];                      // a tile's rows are here; the queries are
   __shared__ int s_abort;
@@ -103,6 +105,7 @@ latent_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __re
                  ::"r"(dst), "l"(src), "r"(d * 2), "r"(bar) : "memory");
   };
   const auto fetch = [&](int t) {                                 // this warp's keys of tile t; zeros for keys without a page
+    if (t == waits.withheld) return;
     const uint32_t stage = sk + (t % kLpStages) * kLpKeys * ld, bar = bars + 8 * (t % kLpStages);
     const bool ok = page >= 0 && page < num_pages;
     const unsigned held = __ballot_sync(0xffffffffu, ok), missing = ((1u << OWN) - 1) & ~held;
@@ -141,10 +144,16 @@ latent_prefill_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __re
   float m[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY}, l[2] = {0.f, 0.f};      // rows wr * 32 + g + 8 i; of the warp's own 16
   const int lm_row = lane & 15, lm_half = lane >> 4;              // rows and packet of an ldmatrix.x4 of 16 x 16
 
-  mbar_wait(bars + 8 * kLpStages, 0, abort_flag, status, 41);     // (a wait that gives up sets the status; the block goes on to its end)
+  bool came = mbar_wait(bars + 8 * kLpStages, 0, abort_flag, status, 41, waits.polls);
   for (int t = 0; t < n_tiles; ++t) {
-    mbar_wait(bars + 8 * (t % kLpStages), (t / kLpStages) & 1, abort_flag, status, 42);
-    __syncthreads();
+    came = mbar_wait(bars + 8 * (t % kLpStages), (t / kLpStages) & 1, abort_flag, status, 42, waits.polls) && came;
+    if (__syncthreads_or(!came)) {                                // (the status says so; nothing is stored)
+      if (tid == 0) {
+        mbar_drain(bars + 8 * kLpStages, 0);
+        for (int i = t; i < min(n_tiles, t + kLpStages - 1); ++i) mbar_drain(bars + 8 * (i % kLpStages), (i / kLpStages) & 1);
+      }
+      return;
+    }
     if (t + kLpStages - 1 < n_tiles) fetch(t + kLpStages - 1);
     const uint32_t kt = sk + (t % kLpStages) * kLpKeys * ld;
     // scores of 32 rows and 16 keys over half of the columns; the other half's come through shared memory
@@ -502,14 +511,14 @@ inline bool latent_tc_fits(const void* out, const void* q, const void* cache, in
 
 template <int R>
 int latent_prefill(void* out, const void* q, const void* cache, const int* bt, const int* tiles, int n_tiles, int bt_stride, int H, int d,
-                   int page_size, int num_pages, float scale, int tile_tokens, int* status, void* stream) {
+                   int page_size, int num_pages, float scale, int tile_tokens, int* status, void* stream, CopyWaits waits) {
   const int smem = (kLpRows + kLpStages * kLpKeys) * latent_row_bytes(d) + kLpRows * kLpWeightBytes + kLpThreads * 32;
   static SmemRaised raised;
   if (int rc = raise_shared_memory("latent_prefill", latent_prefill_kernel<R>, 200 * 1024, raised)) return rc;
   const dim3 grid((tile_tokens * H + kLpRows - 1) / kLpRows, n_tiles);
   return launch_kernel("latent_prefill", latent_prefill_kernel<R>, grid, dim3(kLpThreads), smem, as_stream(stream), (__nv_bfloat16*)out,
                        (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, tiles, bt_stride, H, d, page_size, num_pages,
-                       scale * 1.4426950408889634f, status);
+                       scale * 1.4426950408889634f, status, waits);
 }
 
 template <int R>
@@ -531,22 +540,36 @@ int latent_decode(void* out, float* part, float* ml, const void* q, const void* 
 
 }  // namespace ptl
 
-// `status`: set where a wait inside the kernel gave up (null: nowhere).
-PTL_EXPORT int ptl_latent_prefill_status_bf16(void* out, const void* q, const void* cache, const int* block_table, const int* tiles, int n_tiles,
-                                              int bt_stride, int H, int R, int n, int page_size, int num_pages, float scale, int tile_tokens,
-                                              void* status, void* stream) {
+static int latent_prefill_any(void* out, const void* q, const void* cache, const int* block_table, const int* tiles, int n_tiles, int bt_stride,
+                              int H, int R, int n, int page_size, int num_pages, float scale, int tile_tokens, void* status, void* stream,
+                              ptl::CopyWaits waits = {}) {
   if (!ptl::latent_tc_fits(out, q, cache, H, R, n) || n_tiles > 65535) return -2;
   PTL_REQUIRE(n_tiles >= 0 && bt_stride > 0 && page_size > 0 && num_pages > 0 && tile_tokens > 0,
               "latent_prefill: bad sizes");
   if (n_tiles == 0) return 0;
   const auto fn = R == 128 ? ptl::latent_prefill<128> : R == 256 ? ptl::latent_prefill<256> : ptl::latent_prefill<512>;
-  return fn(out, q, cache, block_table, tiles, n_tiles, bt_stride, H, R + n, page_size, num_pages, scale, tile_tokens, (int*)status, stream);
+  return fn(out, q, cache, block_table, tiles, n_tiles, bt_stride, H, R + n, page_size, num_pages, scale, tile_tokens, (int*)status, stream, waits);
 }
+// For callers without a status word: a wait that gives up is not reported.
 PTL_EXPORT int ptl_latent_prefill_bf16(void* out, const void* q, const void* cache, const int* block_table, const int* tiles, int n_tiles,
                                        int bt_stride, int H, int R, int n, int page_size, int num_pages, float scale, int tile_tokens,
                                        void* stream) {
-  return ptl_latent_prefill_status_bf16(out, q, cache, block_table, tiles, n_tiles, bt_stride, H, R, n, page_size, num_pages, scale, tile_tokens,
-                                        nullptr, stream);
+  return latent_prefill_any(out, q, cache, block_table, tiles, n_tiles, bt_stride, H, R, n, page_size, num_pages, scale, tile_tokens, nullptr, stream);
+}
+// `status`: set where a wait inside the kernel gave up.
+PTL_EXPORT int ptl_latent_prefill_status_bf16(void* out, const void* q, const void* cache, const int* block_table, const int* tiles, int n_tiles,
+                                              int bt_stride, int H, int R, int n, int page_size, int num_pages, float scale, int tile_tokens,
+                                              void* status, void* stream) {
+  return latent_prefill_any(out, q, cache, block_table, tiles, n_tiles, bt_stride, H, R, n, page_size, num_pages, scale, tile_tokens, status, stream);
+}
+// Self-test of the bounded waits: they give up after `polls` polls, and no block fetches its tile `no_tile` of keys.  The kernel must then
+// write *status (42) and return; `out` holds nothing of value.
+PTL_EXPORT int ptl_latent_prefill_wait_selftest(void* out, const void* q, const void* cache, const int* block_table, const int* tiles, int n_tiles,
+                                                int bt_stride, int H, int R, int n, int page_size, int num_pages, float scale, int tile_tokens,
+                                                void* status, void* stream, unsigned polls, int no_tile) {
+  PTL_REQUIRE(status && polls >= 1 && polls <= (1u << 16), "latent_prefill_wait_selftest: a status word, and between 1 and 65536 polls");
+  return latent_prefill_any(out, q, cache, block_table, tiles, n_tiles, bt_stride, H, R, n, page_size, num_pages, scale, tile_tokens, status, stream,
+                            {polls, no_tile});
 }
 
 PTL_EXPORT int ptl_latent_decode_bf16(void* out, float* part, float* ml, const void* q, const void* cache, const int* block_table,

@@ -1,6 +1,7 @@
 """The Sogalix decoder on the GPU: every new kernel against the plain PyTorch statement of its operator
 (tests/torch_ops.py), inputs made so that one key, the sink term or a far token shows, and the engine -- whole
 prompts, decoding, portions, mixed batches, captured steps, generation -- against tests/plain_sogalix.py."""
+import ctypes
 import json
 import math
 import random
@@ -393,6 +394,55 @@ def test_latents_on_the_tensor_cores_at_the_edges_of_tiles(ops, H, R, n, page):
         assert ((got - want).abs()[single] <= 2 ** -7 * want.abs()[single] + 1e-4).all()
         rest = [t for t in range(len(want)) if t != 4 and t not in single]
         assert (got - want).abs()[rest].max() <= 2 ** -7 * float(cache.abs().max())
+
+
+@pytest.mark.parametrize("H,R,n,page", [(4, 128, 16, 24), (8, 512, 64, 48), (3, 256, 0, 64), (5, 128, 64, 33)])
+def test_latents_of_prompts_over_pages_of_other_lengths(ops, H, R, n, page):
+    """Pages that a tile of 32 keys does not divide, or that hold several: prompts and portions of long contexts.  A page that is not
+    held counts as zeros."""
+    g = torch.Generator().manual_seed(page)
+    d, q_lens, starts = R + n, [150, 70, 300, 2], [0, 131, 411, 700]
+    ctx = [s + k for s, k in zip(starts, q_lens)]
+    pages = sum(-(-c // page) for c in ctx) + 3
+    bt, _ = _paged(g, q_lens, starts, page, pages, width=-(-712 // page) + 2)
+    q, cache = _rand(g, sum(q_lens), H * d, scale=1.5).bfloat16(), _rand(g, pages, page * d, scale=0.7).bfloat16()
+    hints = ops.hints_for(q_lens, ctx)
+    cd, cc = _ctx(q_lens, starts, [0] * 4, "cuda:0"), _ctx(q_lens, starts, [0] * 4, "cpu")
+    hints.positions, hints.tok_req = cd.positions, cd.tok_req
+    run = lambda c, t: ops.latent_attention(q.cuda(), c.cuda(), t.cuda(), hints, H, R, n, page, d ** -0.5)
+    got = run(cache, bt)
+    want = TorchOps().latent_attention(q, cache, bt, cc, H, R, n, page, d ** -0.5).double()
+    assert (got.double().cpu() - want).abs().max() <= 2 ** -7 * float(cache.abs().max())
+    holes, at = bt.clone(), [(0, 1), (2, 0), (2, 5), (2, 6)]
+    for r, k in at:
+        holes[r, k] = -1
+    zeros, over = torch.cat([cache, torch.zeros(1, page * d).bfloat16()]), bt.clone()
+    for r, k in at:
+        over[r, k] = pages
+    assert torch.equal(run(cache, holes), run(zeros, over))
+
+
+@pytest.mark.parametrize("no_tile", [0, 1, 4])
+def test_latents_of_prompts_give_up_a_tile_that_does_not_come(ops, no_tile):
+    """No block fetches one of its tiles of keys: the waits run out, the status is set, and the blocks end by themselves without a result."""
+    H, R, n, page, T = 4, 128, 16, 16, 200
+    g = torch.Generator().manual_seed(1)
+    q, cache = _rand(g, T, H * (R + n)).bfloat16().cuda(), _rand(g, 13, page * (R + n)).bfloat16().cuda()
+    bt, hints = torch.arange(13, dtype=torch.int32, device="cuda")[None], ops.hints_for([T], [T])
+    tiles, out, lib, status = hints.work["prefill_tiles"], torch.zeros(T, H * R, device="cuda").bfloat16(), ops.lib, ops._tc_status_word()
+    ptr = lambda *ts: [ctypes.c_void_p(t.data_ptr()) for t in ts]
+    call = lambda polls, tile: lib.ptl_latent_prefill_wait_selftest(
+        *ptr(out, q, cache, bt, tiles.tensor), tiles.items, 13, H, R, n, page, 13, ctypes.c_float(0.1), ops.QUERY_TILE, *ptr(status),
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), polls, tile)
+    assert ops.gemm_tc_status() == 0
+    assert call(300, no_tile) == 0, lib.ptl_last_error().decode()
+    torch.cuda.synchronize()
+    assert ops.gemm_tc_status() == 42
+    assert not out[32 * no_tile:].any() and (no_tile == 0 or out[:32 * no_tile].any())       # tokens that see no key of the tile are there
+    hints.positions, hints.tok_req = torch.arange(T, dtype=torch.int32, device="cuda"), torch.zeros(T, dtype=torch.int32, device="cuda")
+    want = ops.latent_attention(q, cache, bt, hints, H, R, n, page, 0.1)
+    assert call(65536, -1) == 0
+    assert torch.equal(out, want) and ops.gemm_tc_status() == 0
 
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
