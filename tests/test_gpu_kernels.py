@@ -1057,6 +1057,42 @@ def test_product_for_a_few_tokens_and_small_weights(_ops, M, N, K):
 def test_product_for_a_few_tokens_up_to_the_blocks_an_sm_holds(_ops, M, N, K):
     """The most blocks of 148 SMs: five an SM (by registers) of short rows, one of long ones, the longest row that fits."""
     test_product_for_a_few_tokens_and_small_weights(_ops, M, N, K)
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+@pytest.mark.parametrize("d, page, window, splits", [(64, 16, 0, 1), (128, 16, 0, 1), (256, 8, 0, 1), (48, 16, 700, 1), (16, 4, 0, 1), (64, 16, 0, 3)])
+def test_cuda_core_attention_gives_a_token_the_same_bits_whatever_its_company(ops, dtype, d, page, window, splits):
+    """Tokens of contexts around a group of 32 keys and the 512 whose weights are worked out together, alone (four warps a head) and among so
+    many that a warp takes a head; the keys grow along the context, so that the maximum does in every group, and a page is missing."""
+    ctx, nq, nkv = [1, 32, 33, 512, 513, 1025, 1500], 8, 2
+    pages = [-(-c // page) for c in ctx]
+    table, at = torch.full((len(ctx), max(pages)), -1, dtype=torch.int32), 0
+    for r, n in enumerate(pages):
+        table[r, :n] = torch.arange(at, at + n, dtype=torch.int32)
+        at += n
+    table[5, 3] = -1
+    cache = rnd((at, 2, nkv, page, d), DT[dtype], 91, 0.5)
+    growth = torch.cat([torch.arange(n * page) / 400.0 + 0.2 for n in pages]).view(at, 1, page, 1)
+    cache[:, 0] = (cache[:, 0].float() * growth).to(DT[dtype])
+    q = rnd((len(ctx), nq * d), DT[dtype], 92)
+    positions = torch.tensor([c - 1 for c in ctx], dtype=torch.int32)
+    dev = [t.cuda() for t in (cache, table)]
+    call = lambda rows: ops.paged_attention(q[rows].cuda(), dev[0], dev[1], rows.int().cuda(), positions[rows].cuda(), nq, nkv, d, page, d ** -0.5,
+                                            window=window, splits=splits)
+    many = torch.arange(len(ctx)).repeat(23)                          # 161 tokens of 8 heads: more than eight heads an SM
+    assert len(many) * nq >= 8 * ops._sm_count
+    together = call(many)
+    for r in range(len(ctx)):
+        alone = call(torch.tensor([r]))
+        assert all(torch.equal(alone[0], together[i]) for i in range(r, len(many), len(ctx))), r
+    want = torch.zeros(len(ctx), nq * d, dtype=torch.float64)
+    for r, c in enumerate(ctx):
+        keys = [n for n in range(max(0, c - window) if window else 0, c) if int(table[r, n // page]) >= 0]
+        kv = torch.stack([cache[int(table[r, n // page]), :, :, n % page] for n in keys]).double()          # [keys, 2, nkv, d]
+        for h in range(nq):
+            p = torch.softmax(kv[:, 0, h // (nq // nkv)] @ q[r, h * d:(h + 1) * d].double() * d ** -0.5, 0)
+            want[r, h * d:(h + 1) * d] = p @ kv[:, 1, h // (nq // nkv)]
+    close(together[:len(ctx)], want, dtype, "against 64 bits")
+
+
 @pytest.mark.parametrize("no_turn", [0, 3, 5])
 def test_float32_product_of_few_rows_gives_up_a_turn_that_does_not_come(_ops, no_turn):
     """No block asks for one of its turns (of the ring's first filling, and of a later one): the waits run out, the status is set, and the
