@@ -195,18 +195,26 @@ int token_side_cluster(float* residual, const void* x, const float* bias, const 
                                (const __nv_bfloat16*)w_proj, norm_w, eps, n_tokens);
 }
 
-// Many tokens: a block owns sixteen whole rows, and nothing crosses blocks.  Each of its sixteen warps takes a sixteenth of the width as
-// its share of the sum over W_gate (all dims), then a sixteenth of W_proj's rows; a lane reads the weights in packets of eight
-// values straight from L2 as the MMAs' operand (the eight stand for two steps' places of K, in both operands alike), the
-// ones of W_gate before the wait on the predecessor.  What bounds it: 256 KB of weights a block out of L2, and the reads of the rows before anything can begin.
-// 2,048 tokens of width 1,024, 64 dims: 14.4 us, 32.2 by clusters, whose three barriers a tile cost more than their shares save.
-// The line: at 500 tokens 10.6 us by clusters and 14.0 so, at 1,000 20.6 and 14.1, and neither moves before the next wave of blocks.
-constexpr int kRowsFrom = 768;
+// Many tokens: a block owns sixteen whole rows, and nothing crosses blocks.  Its sixteen warps take, for z, an eighth of the width and half of
+// the dims each, then a sixteenth of W_proj's rows; a lane reads the weights in packets of eight values straight from L2 (those of W_gate
+// before the wait on the predecessor), and the four lanes of a row trade words until each holds its own of the MMAs' operands.  All
+// sums in the cluster form's order (a rank's eighth of z in one chain, the ranks in order; the squares by the cluster's warps), so that a
+// token has the same bits in either.  What bounds it: 256 KB of weights a block out of L2, and the reads of the rows before anything can begin.
 constexpr int kTrThreads = 512, kTrWarps = kTrThreads / 32;
-__host__ __device__ constexpr int tr_ld(int n) { return n + 32; }       // rows of 16-bit terms: two neighbouring rows' four packets in eight bank groups
+__host__ __device__ constexpr int tr_ld(int n) { return n + 8; }        // rows of 16-bit terms: eight rows' packets in different banks
 __host__ __device__ constexpr size_t tr_smem(int width, int dim) {
-  const size_t terms = (size_t)6 * kTsTokens * tr_ld(width), sums = (size_t)4 * kTrWarps * kTsTokens * dim;
+  const size_t terms = (size_t)6 * kTsTokens * tr_ld(width), sums = (size_t)4 * kTsBlocks * kTsTokens * dim;
   return (size_t)4 * kTsTokens * (width + 4) + (terms > sums ? terms : sums) + (size_t)6 * kTsTokens * tr_ld(dim);
+}
+// Words 4 q .. 4 q + 3 of a row's sixteen in lane q of four -> words q, q + 4, q + 8, q + 12.
+__device__ __forceinline__ void tr_trade(uint4& v) {
+  const bool odd = threadIdx.x & 1, high = threadIdx.x & 2;
+  const uint32_t a = __shfl_xor_sync(0xffffffffu, odd ? v.x : v.y, 1), b = __shfl_xor_sync(0xffffffffu, odd ? v.z : v.w, 1);
+  (odd ? v.x : v.y) = a;
+  (odd ? v.z : v.w) = b;
+  const uint32_t c = __shfl_xor_sync(0xffffffffu, high ? v.x : v.z, 2), d = __shfl_xor_sync(0xffffffffu, high ? v.y : v.w, 2);
+  (high ? v.x : v.z) = c;
+  (high ? v.y : v.w) = d;
 }
 
 template <int WIDTH, int DIM>
@@ -215,21 +223,24 @@ token_side_rows_kernel(float* __restrict__ residual, const __nv_bfloat16* __rest
                        const int* __restrict__ tokens, const __nv_bfloat16* __restrict__ table, int table_ld, int column,
                        int vocab, const __nv_bfloat16* __restrict__ w_gate, const __nv_bfloat16* __restrict__ w_proj,
                        const float* __restrict__ norm_w, float eps, int n_tokens) {
-  constexpr int LS = WIDTH + 4, LT = tr_ld(WIDTH), LG = tr_ld(DIM), SLICE = WIDTH / kTrWarps, KB = SLICE / 32, NZ = DIM / 8, NY = SLICE / 8;
+  constexpr int LS = WIDTH + 4, LT = tr_ld(WIDTH), LG = tr_ld(DIM), SL = WIDTH / kTsBlocks, SLICE = WIDTH / kTrWarps, KB = SL / 32, NZ = DIM / 16, NY = SLICE / 8;
+  constexpr int NT = SL / 64, CW = kTsBlocks * (kTsThreads / 32);       // of the cluster form: blocks of eight columns per warp, warps
   extern __shared__ __align__(16) unsigned char tr_raw[];
   float* s32 = reinterpret_cast<float*>(tr_raw);                                     // [16][LS]
-  __nv_bfloat16* s16 = reinterpret_cast<__nv_bfloat16*>(s32 + kTsTokens * LS);       // [3][16][LT]; then the warps' sums of z [16 warps][16][DIM]
+  __nv_bfloat16* s16 = reinterpret_cast<__nv_bfloat16*>(s32 + kTsTokens * LS);       // [3][16][LT]; then the ranks' sums of z [8][16][DIM]
   float* zpart = reinterpret_cast<float*>(s16);
-  constexpr size_t terms = (size_t)3 * kTsTokens * LT, sums = (size_t)2 * kTrWarps * kTsTokens * DIM;
+  constexpr size_t terms = (size_t)3 * kTsTokens * LT, sums = (size_t)2 * kTsBlocks * kTsTokens * DIM;
   __nv_bfloat16* g16 = s16 + (terms > sums ? terms : sums);                          // [3][16][LG]
-  __shared__ float s_ss[kTrWarps][kTsTokens];
+  __shared__ float s_ss[CW][kTsTokens];
+  __shared__ float s_rank[kTsBlocks][kTsTokens];
   const int t0 = blockIdx.x * kTsTokens, nt = min(kTsTokens, n_tokens - t0);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, q8 = (lane & 3) * 8, c2 = (lane & 3) * 2;
+  const int rank = warp >> 1, half = warp & 1, lm_row = lane & 15, lm_half = lane >> 4;
   uint4 wg[KB][NZ];                                     // (written by no kernel of the step)
 #pragma unroll
   for (int k = 0; k < KB; ++k)
 #pragma unroll
-    for (int n = 0; n < NZ; ++n) wg[k][n] = __ldg(reinterpret_cast<const uint4*>(w_gate + (size_t)(8 * n + g) * WIDTH + warp * SLICE + 32 * k + q8));
+    for (int n = 0; n < NZ; ++n) wg[k][n] = __ldg(reinterpret_cast<const uint4*>(w_gate + (size_t)(8 * (half * NZ + n) + g) * WIDTH + rank * SL + 32 * k + q8));
   pdl_wait();
   pdl_launch_dependents();
   constexpr int PER = DIM * kTsTokens / kTrThreads;     // elements of z that a thread finishes
@@ -276,18 +287,22 @@ token_side_rows_kernel(float* __restrict__ residual, const __nv_bfloat16* __rest
 #pragma unroll
     for (int e = 0; e < 4; ++e) acc[n][e] = 0.f;
 #pragma unroll
-  for (int k = 0; k < KB; ++k)
+  for (int k = 0; k < KB; ++k) {
+#pragma unroll
+    for (int n = 0; n < NZ; ++n) tr_trade(wg[k][n]);
 #pragma unroll
     for (int w = 2; w >= 0; --w) {
-      const __nv_bfloat16* at = s16 + (w * kTsTokens + g) * LT + warp * SLICE + 32 * k + q8;
-      const uint4 up = *reinterpret_cast<const uint4*>(at), low = *reinterpret_cast<const uint4*>(at + 8 * LT);
-      const uint32_t a0[4] = {up.x, low.x, up.y, low.y}, a1[4] = {up.z, low.z, up.w, low.w};
+      uint32_t a0[4], a1[4];
+      const uint32_t at = smem_u32(s16 + (w * kTsTokens + lm_row) * LT + rank * SL + 32 * k + 8 * lm_half);
+      ldmatrix_x4(a0, at);
+      ldmatrix_x4(a1, at + 32);
 #pragma unroll
       for (int n = 0; n < NZ; ++n) {
         mma_bf16_16816(acc[n], a0, wg[k][n].x, wg[k][n].y);
         mma_bf16_16816(acc[n], a1, wg[k][n].z, wg[k][n].w);
       }
     }
+  }
   // this warp's rows of W_proj, while the shares are added up
   uint4 wp[NY][DIM / 32];
 #pragma unroll
@@ -299,14 +314,14 @@ token_side_rows_kernel(float* __restrict__ residual, const __nv_bfloat16* __rest
   for (int n = 0; n < NZ; ++n)
 #pragma unroll
     for (int i = 0; i < 2; ++i)
-      *reinterpret_cast<float2*>(zpart + (warp * kTsTokens + g + 8 * i) * DIM + 8 * n + c2) = make_float2(acc[n][2 * i], acc[n][2 * i + 1]);
+      *reinterpret_cast<float2*>(zpart + (rank * kTsTokens + g + 8 * i) * DIM + 8 * (half * NZ + n) + c2) = make_float2(acc[n][2 * i], acc[n][2 * i + 1]);
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
     const int at = tid + i * kTrThreads;
     float z = 0.f;
 #pragma unroll
-    for (int w = 0; w < kTrWarps; ++w) z += zpart[w * kTsTokens * DIM + at];
+    for (int b = 0; b < kTsBlocks; ++b) z += zpart[b * kTsTokens * DIM + at];
     const float v = at / DIM < nt ? ts_gelu_tanh(z) * __bfloat162float(entry[i]) : 0.f;
     ts_split(v, g16 + at / DIM * LG + at % DIM, kTsTokens * LG);
   }
@@ -317,28 +332,40 @@ token_side_rows_kernel(float* __restrict__ residual, const __nv_bfloat16* __rest
 #pragma unroll
     for (int e = 0; e < 4; ++e) y[j][e] = 0.f;
 #pragma unroll
-  for (int k = 0; k < DIM / 32; ++k)
+  for (int k = 0; k < DIM / 32; ++k) {
 #pragma unroll
-    for (int w = 2; w >= 0; --w) {
-      const __nv_bfloat16* at = g16 + (w * kTsTokens + g) * LG + 32 * k + q8;
-      const uint4 up = *reinterpret_cast<const uint4*>(at), low = *reinterpret_cast<const uint4*>(at + 8 * LG);
-      const uint32_t a0[4] = {up.x, low.x, up.y, low.y}, a1[4] = {up.z, low.z, up.w, low.w};
+    for (int j = 0; j < NY; ++j) tr_trade(wp[j][k]);
 #pragma unroll
-      for (int j = 0; j < NY; ++j) {
-        mma_bf16_16816(y[j], a0, wp[j][k].x, wp[j][k].y);
-        mma_bf16_16816(y[j], a1, wp[j][k].z, wp[j][k].w);
+    for (int step = 0; step < 2; ++step)
+#pragma unroll
+      for (int w = 2; w >= 0; --w) {
+        uint32_t a[4];
+        ldmatrix_x4(a, smem_u32(g16 + (w * kTsTokens + lm_row) * LG + 32 * k + 16 * step + 8 * lm_half));
+#pragma unroll
+        for (int j = 0; j < NY; ++j) mma_bf16_16816(y[j], a, step ? wp[j][k].z : wp[j][k].x, step ? wp[j][k].w : wp[j][k].y);
       }
+  }
+#pragma unroll
+  for (int j0 = 0; j0 < NY; j0 += NT) {
+    float ss[2] = {0.f, 0.f};
+#pragma unroll
+    for (int j = j0; j < j0 + NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) ss[e >> 1] = fmaf(y[j][e], y[j][e], ss[e >> 1]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 1);
+      ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 2);
+      if ((lane & 3) == 0) s_ss[(warp * NY + j0) / NT][g + 8 * i] = ss[i];
     }
-  float ss[2] = {0.f, 0.f};
+  }
+  __syncthreads();
+  if (tid < kTsTokens * kTsBlocks) {
+    const int row = tid % kTsTokens, peer = tid / kTsTokens;
+    float v = 0.f;
 #pragma unroll
-  for (int j = 0; j < NY; ++j)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) ss[e >> 1] = fmaf(y[j][e], y[j][e], ss[e >> 1]);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 1);
-    ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], 2);
-    if ((lane & 3) == 0) s_ss[warp][g + 8 * i] = ss[i];
+    for (int w = 0; w < kTsThreads / 32; ++w) v += s_ss[peer * (kTsThreads / 32) + w][row];
+    s_rank[peer][row] = v;
   }
   __syncthreads();
 #pragma unroll
@@ -347,7 +374,7 @@ token_side_rows_kernel(float* __restrict__ residual, const __nv_bfloat16* __rest
     if (row >= nt) continue;
     float total = 0.f;
 #pragma unroll
-    for (int w = 0; w < kTrWarps; ++w) total += s_ss[w][row];
+    for (int b = 0; b < kTsBlocks; ++b) total += s_rank[b][row];
     const float rrms = 1.0f / sqrtf(total / (float)WIDTH + eps);
 #pragma unroll
     for (int j = 0; j < NY; ++j) {
@@ -382,7 +409,10 @@ PTL_EXPORT int ptl_token_side_cluster_bf16(float* residual, const void* x, const
   PTL_REQUIRE(n_tokens >= 0 && n_tokens <= (1 << 27) && column >= 0 && column + dim <= table_ld && eps > 0.f && vocab > 0,
               "token_side: bad sizes width=%d dim=%d column=%d of %d", width, dim, column, table_ld);
   if (n_tokens == 0) return 0;
-  if (n_tokens >= kRowsFrom && width <= 1024 && (dim == 32 || dim == 64)) {
+  // The rows' form from where the cluster form needs another turn of clusters; its own time is that of one block an SM up to 2,368 tokens.  Width
+  // 1,024: 64 dims 11.8 us by clusters and 14.6 by rows at 768 tokens, 15.9 and 14.5 at 784; 32 dims 10.9 and 11.3 at 1,072, 11.8 and 11.2 at
+  // 1,088; 2,048 tokens of 64 dims 32.3 and 14.9.  Width 512: 64 dims 9.0 and 9.2 at 560, 10.2 and 9.2 at 576; 32 dims 6.8 both from 560 to 576, 7.0 and 6.8 at 592.
+  if (n_tokens > (width == 512 ? 560 : dim == 64 ? 768 : 1072) && width <= 1024 && (dim == 32 || dim == 64)) {
     const auto rows = width == 512 ? dim == 32 ? token_side_rows<512, 32> : token_side_rows<512, 64>
                                    : dim == 32 ? token_side_rows<1024, 32> : token_side_rows<1024, 64>;
     return rows(residual, x, bias, tokens, table, table_ld, column, vocab, w_gate, w_proj, norm_w, n_tokens, eps, stream);

@@ -279,6 +279,24 @@ def test_side_term_of_many_tokens(ops, T, W, dim):
     test_side_term_in_a_cluster(ops, T, W, dim)
 
 
+@pytest.mark.parametrize("T,W,dim", [(800, 1024, 64), (1100, 1024, 32), (600, 512, 64), (600, 512, 32)])
+def test_side_term_of_a_token_does_not_depend_on_the_step(ops, T, W, dim):
+    """A token's bits are the same among few tokens (a cluster's blocks share a row) and among so many that a block owns whole rows."""
+    g = torch.Generator().manual_seed(T * W + dim)
+    V = 50
+    ids = torch.randint(0, V, (T,), generator=g, dtype=torch.int32).cuda()
+    side, wg, wp = (t.bfloat16().cuda() for t in (torch.randn(V, 3 * dim, generator=g), torch.randn(dim, W, generator=g) / W ** 0.5,
+                                                  torch.randn(W, dim, generator=g) / dim ** 0.5))
+    res, nw, bias = (t.cuda() for t in (torch.randn(T, W, generator=g), torch.randn(W, generator=g), torch.randn(W, generator=g)))
+    x = torch.randn(T, W, generator=g).bfloat16().cuda()
+    whole = res.clone()
+    ops.token_side(whole, x, bias, ids, side, dim, dim, wg, wp, nw, 1e-5)
+    for a, b in ((0, 100), (100, 117), (T - 33, T)):
+        part = res[a:b].clone()
+        ops.token_side(part, x[a:b].clone(), bias, ids[a:b].clone(), side, dim, dim, wg, wp, nw, 1e-5)
+        assert torch.equal(part, whole[a:b]), (a, b)
+
+
 @pytest.mark.parametrize("H,G,d,page,chunk,options", [(8, 2, 128, 16, 256, True), (4, 2, 64, 8, 48, True), (1, 1, 128, 4, 16, False),
                                                       (6, 2, 64, 16, 240, True)])
 def test_chunk_attention_on_the_tensor_cores(ops, H, G, d, page, chunk, options):
