@@ -5,7 +5,7 @@
 // page * page_stride + (g * page_size + offset) * d + e, of the values at
 // page * page_stride + G * page_size * d + (g * page_size + offset) * dv + e, page_stride = G * page_size * (d + dv).
 // Scores, weights and all sums are float32; T is the element type of q, of the cache and of the result.
-#include "common.cuh"
+#include "mma_utils.cuh"
 
 namespace ptl {
 
@@ -221,17 +221,37 @@ chunk_attention_single_kernel(__nv_bfloat16* __restrict__ out, int out_ld, int c
   const int r = tok_req[t];
   if (r < 0) return;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, group = H / G;
-  const int p = positions[t], lo = p - p % chunk, n = p - lo + 1;
+  const int p = positions[t], lo = p - p % chunk, n = min(p - lo + 1, table_width * page_size);      // (no more keys than the table can name)
   const size_t page_stride = (size_t)G * page_size * 2 * D, plane = (size_t)page_size * D;
-  // the queries (with their bias) of this lane's entries; a place without a head holds zeros
+  // the queries (with their bias) of this lane's entries, for the warps that have keys to score; a place without a head holds zeros
   float q[kCsHeads][E];
 #pragma unroll
-  for (int a = 0; a < kCsHeads; ++a) {
-    const int h = a / HG * group + a % HG;
-    const bool there = a % HG < group;
+  for (int a = 0; a < kCsHeads; ++a)
 #pragma unroll
-    for (int e = 0; e < E; ++e)
-      q[a][e] = there ? to_f32(qkv[(size_t)t * q_ld + h * D + lane * E + e]) + (q_bias ? q_bias[h * D + lane * E + e] : 0.f) : 0.f;
+    for (int e = 0; e < E; ++e) q[a][e] = 0.f;
+  if (4 * warp < n) {
+#pragma unroll
+    for (int a = 0; a < kCsHeads; ++a) {
+      if (a % HG >= group) continue;
+      const int at = (a / HG * group + a % HG) * D + lane * E;
+      uint32_t raw[E / 2];
+      if constexpr (E == 4) *reinterpret_cast<uint2*>(raw) = *reinterpret_cast<const uint2*>(qkv + (size_t)t * q_ld + at);
+      else raw[0] = *reinterpret_cast<const uint32_t*>(qkv + (size_t)t * q_ld + at);
+#pragma unroll
+      for (int e = 0; e < E; e += 2) {
+        const float2 v = unpack_bf16(raw[e / 2]);
+        q[a][e] = v.x;
+        q[a][e + 1] = v.y;
+      }
+      if (q_bias) {
+#pragma unroll
+        for (int e = 0; e < E; e += 2) {
+          const float2 b = *reinterpret_cast<const float2*>(q_bias + at + e);
+          q[a][e] += b.x;
+          q[a][e + 1] += b.y;
+        }
+      }
+    }
   }
   if (tid < n) {
     const int pos = lo + tid, page = block_table[(size_t)r * table_width + pos / page_size];
@@ -445,10 +465,14 @@ PTL_EXPORT int ptl_chunk_attention_single_bf16(void* out, int out_ld, int column
                                                const float* talk, int num_pages, float out_scale, const int* items, void* stream) {
   using namespace ptl;
   if ((d != 64 && d != 128) || H < 1 || H > kCsHeads || G < 1 || G > 2 || H % G || H / G > kCsHeads / G || chunk < 1 || chunk > kCsMaxBlock ||
-      !aligned16(cache))
+      !aligned16(cache) || !aligned16(qkv) || q_ld % 8 || (reinterpret_cast<uintptr_t>(q_bias) & 7u))
     return -2;
   PTL_REQUIRE((r1 == nullptr) == (r2 == nullptr) && page_size > 0 && num_pages > 0 && rows >= 0 && column >= 0 && column + H * d <= out_ld &&
                   q_ld >= H * d, "chunk_attention_single: bad sizes");
+  // A block holds an SM (by its registers), and few heads in short blocks of positions have little for sixteen warps: beyond two turns of SMs
+  // they are left to the kernel above.  4 heads of 64 in blocks of 64, positions spread over them: 296 tokens 14.7 us there and 11.9 here, 600 17.8 and
+  // 22.4, 4 heads in blocks of 128 28.2 and 28.7; 8 heads of 128 in blocks of 256: 600 tokens 104 and 64 (all at the 17th position 20 and 31, all at the last 137 and 115).
+  if (rows > 2 * sm_count_of_device() && H * chunk < 512) return -2;
   if (rows == 0) return 0;
   const auto fn = d == 64 ? G == 1 ? chunk_attention_single<64, 1> : chunk_attention_single<64, 2>
                           : G == 1 ? chunk_attention_single<128, 1> : chunk_attention_single<128, 2>;

@@ -298,7 +298,8 @@ def test_side_term_of_a_token_does_not_depend_on_the_step(ops, T, W, dim):
 
 
 @pytest.mark.parametrize("H,G,d,page,chunk,options", [(8, 2, 128, 16, 256, True), (4, 2, 64, 8, 48, True), (1, 1, 128, 4, 16, False),
-                                                      (6, 2, 64, 16, 240, True)])
+                                                      (6, 2, 64, 16, 240, True), (8, 1, 128, 16, 256, True), (6, 1, 64, 8, 48, True),
+                                                      (5, 1, 64, 16, 64, True)])
 def test_chunk_attention_on_the_tensor_cores(ops, H, G, d, page, chunk, options):
     """Against the general kernel on the same inputs: scores, weights and sums are float32 in both, so that only the result's
     rounding (2^-8 of it) and float32 sums differ.  Portions begin and end inside sixteens and cross blocks of positions."""
@@ -351,6 +352,56 @@ def test_chunk_attention_keeps_a_bad_value_from_earlier_tokens(ops, G, d, talk, 
     assert torch.equal(got.isfinite(), want.isfinite()) and got[:at].isfinite().all() and not got[at:at + 3].isfinite().all()
     fine = want.isfinite()
     assert ((got - want)[fine].abs() <= 2 ** -7 * want[fine].abs() + 2e-5 * float(want[fine].abs().max())).all()
+
+
+def _single_tokens(ops, positions, H, G, d, page, chunk, change=lambda cache, table: None, width=0):
+    """Single tokens at these positions of requests of their own, by the step's operator and by the general kernel."""
+    g = torch.Generator().manual_seed(len(positions) + H * d)
+    R, per = len(positions), width or max(positions) // page + 1
+    table = torch.randperm(R * per, generator=g).int().view(R, per)
+    cache = torch.randn(R * per, G * page * 2 * d, generator=g).bfloat16()
+    change(cache, table)
+    cache, table, qkv = cache.cuda(), table.cuda(), torch.randn(R, H * d + 2 * G * d, generator=g).bfloat16().cuda()
+    opt = [t.cuda() for t in (torch.randn(H * d + 2 * G * d, generator=g) * 0.3, torch.rand(H, generator=g), torch.rand(H, generator=g) + 0.1,
+                              torch.randn(H, H, generator=g))]
+    c = _ctx([1] * R, positions, list(range(R)), "cuda:0")
+    c.work = ops.hints_for([1] * R, [p + 1 for p in positions]).work
+    got, want = (torch.zeros(R, H * d, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    ops.chunk_attention_of_step(c, qkv, opt[0], cache, table, H, G, d, d, page, 0.2, chunk, *opt[1:], got, 0, 0.7)
+    ops.chunk_attention(qkv, opt[0], cache, table, c.tok_req, c.positions, H, G, d, d, page, 0.2, chunk, *opt[1:], want, 0, 0.7)
+    got, want = got.double().cpu(), want.double().cpu()
+    assert torch.equal(got.isfinite(), want.isfinite())
+    fine = want.isfinite()
+    assert ((got - want)[fine].abs() <= 2 ** -7 * want[fine].abs() + 2e-5 * float(want[fine].abs().max())).all()
+    return got
+
+
+@pytest.mark.parametrize("H,G,d,page,chunk", [(8, 1, 128, 16, 256), (8, 2, 64, 8, 256), (5, 1, 64, 16, 64), (6, 2, 128, 16, 48)])
+@pytest.mark.parametrize("rows", [7, 300])
+def test_chunk_attention_of_single_tokens(ops, H, G, d, page, chunk, rows):
+    """As many heads as the kernel takes and fewer, few tokens and more than two turns of SMs (which few heads in short blocks leave to the
+    general kernel), at the beginning, inside and at the end of their blocks; a page that is not held."""
+    places = [0, 1, 15, 16, chunk // 2, chunk - 2, chunk - 1]
+    positions = [chunk * (r % 2) + places[r % 7] for r in range(rows)]
+
+    def missing(cache, table):
+        table[5, positions[5] // page - 1] = -1
+    _single_tokens(ops, positions, H, G, d, page, chunk, missing)
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_chunk_attention_of_single_tokens_with_a_bad_value(ops, bad):
+    """A value and a key that are no finite numbers: the results, finite or not, are those of the general kernel."""
+    def spoil(cache, table):
+        cache[table[2, 3], 2 * 16 * 64 + 5 * 64 + 9] = bad          # value of kv head 0 at position 53 of the third request
+        cache[table[4, 0], 3 * 64 + 7] = bad                        # key of kv head 0 at position 3 of the fifth
+    got = _single_tokens(ops, [60, 61, 62, 52, 30], 4, 2, 64, 16, 64, spoil)
+    assert got[[0, 1, 3]].isfinite().all() and not got[2].isfinite().all() and not got[4].isfinite().all()
+
+
+def test_chunk_attention_of_single_tokens_reads_no_further_than_its_table(ops):
+    """A position beyond what the block table can name sees the keys that it names."""
+    _single_tokens(ops, [70, 40, 63], 4, 2, 64, 16, 128, width=4)
 
 
 @pytest.mark.parametrize("no_chunk,no_row,code", [(0, -1, 31), (2, -1, 31), (-1, 5, 32), (-1, 70, 32)])
