@@ -25,15 +25,23 @@ __device__ __forceinline__ void kahan_add(float& sum, float& comp, float chunk) 
   comp = __fsub_rn(__fsub_rn(t, sum), y);
   sum = t;
 }
+__device__ __forceinline__ void kahan_add_pair(float2& sum, float2& comp, float2 chunk) {
+  const float2 y = sub2(chunk, comp);
+  const float2 t = add2(sum, y);
+  comp = sub2(sub2(t, sum), y);
+  sum = t;
+}
 
-template <typename TI, typename TO, int BM, int BN, int TM, int TN>
+// What the kernels below cannot read in packets of 16 bytes, and 16-bit operands: any type and alignment.  CHAINS of FMAs a chunk: two
+// where another kernel may take other rows of the same product (float32, K a multiple of 4), else one.
+template <typename TI, typename TO, int BM, int BN, int TM, int TN, int CHAINS>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_simt_kernel(TO* __restrict__ out, const TI* __restrict__ A, const TI* __restrict__ W,
                  int M, int N, int K, int lda, int ldw, int ldo, int accumulate,
                  long long batch_a, long long batch_w, long long batch_o, const TI* __restrict__ gate, int gate_ld) {
   constexpr int BK = kSimtChunk;
   constexpr int THREADS = (BM / TM) * (BN / TN);
-  static_assert(TM % 4 == 0 || TM == 2 || TM == 1, "rows per thread");
+  static_assert(TM % 4 == 0, "rows per thread, two an instruction");
   pdl_wait();
   pdl_launch_dependents();
   A += (size_t)blockIdx.z * batch_a;
@@ -45,11 +53,11 @@ gemm_simt_kernel(TO* __restrict__ out, const TI* __restrict__ A, const TI* __res
   const int tx = tid % (BN / TN);  // along N
   const int ty = tid / (BN / TN);  // along M
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[2][TM][TN], sum[TM][TN], comp[TM][TN];        // acc: even and odd k
+  float2 acc[CHAINS][TM / 2][TN], sum[TM / 2][TN], comp[TM / 2][TN];      // of two rows each
 #pragma unroll
-  for (int i = 0; i < TM; ++i)
+  for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) { sum[i][j] = 0.f; comp[i][j] = 0.f; }
+    for (int j = 0; j < TN; ++j) sum[i][j] = comp[i][j] = make_float2(0.f, 0.f);
 
   for (int k0 = 0; k0 < K; k0 += BK) {
     // any element type and alignment: consecutive threads walk along K so that global reads coalesce
@@ -65,25 +73,26 @@ gemm_simt_kernel(TO* __restrict__ out, const TI* __restrict__ A, const TI* __res
     }
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+    for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-      for (int j = 0; j < TN; ++j) acc[0][i][j] = acc[1][i][j] = 0.f;
+      for (int j = 0; j < TN; ++j) acc[0][i][j] = acc[CHAINS - 1][i][j] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int kk = 0; kk < BK; ++kk) {
-      float a[TM], b[TN];
+      float2 a[TM / 2];
+      float b[TN];
 #pragma unroll
-      for (int i = 0; i < TM; ++i) a[i] = As[kk][ty * TM + i];
+      for (int i = 0; i < TM / 2; ++i) a[i] = *reinterpret_cast<const float2*>(&As[kk][ty * TM + 2 * i]);
 #pragma unroll
       for (int j = 0; j < TN; ++j) b[j] = Ws[kk][tx * TN + j];
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
+      for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-        for (int j = 0; j < TN; ++j) acc[kk & 1][i][j] = fmaf(a[i], b[j], acc[kk & 1][i][j]);
+        for (int j = 0; j < TN; ++j) acc[kk % CHAINS][i][j] = fma2(a[i], make_float2(b[j], b[j]), acc[kk % CHAINS][i][j]);
     }
 #pragma unroll
-    for (int i = 0; i < TM; ++i)
+    for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
-      for (int j = 0; j < TN; ++j) kahan_add(sum[i][j], comp[i][j], __fadd_rn(acc[0][i][j], acc[1][i][j]));
+      for (int j = 0; j < TN; ++j) kahan_add_pair(sum[i][j], comp[i][j], CHAINS == 2 ? add2(acc[0][i][j], acc[1][i][j]) : acc[0][i][j]);
     __syncthreads();
   }
 #pragma unroll
@@ -96,7 +105,7 @@ gemm_simt_kernel(TO* __restrict__ out, const TI* __restrict__ A, const TI* __res
       const int gn = n0 + tx * TN + j;
       if (gn >= N) continue;
       TO* o = out + (size_t)gm * ldo + gn;
-      float v = sum[i][j] * row_gate;
+      float v = (i & 1 ? sum[i / 2][j].y : sum[i / 2][j].x) * row_gate;
       if (accumulate) v += to_f32(*o);
       *o = from_f32<TO>(v);
     }
@@ -309,7 +318,7 @@ gemm_simt_tile_kernel(float* __restrict__ out, const float* __restrict__ A, cons
     for (int i = 0; i < TM; ++i)
 #pragma unroll
       for (int j = 0; j < TN; ++j) acc[i][j] = make_float2(0.f, 0.f);
-#pragma unroll 2
+#pragma unroll (TM * TN <= 16 ? 4 : 2)
     for (int k = 0; k < kSimtChunk; k += 4) {
       float4 w[TN];
 #pragma unroll
@@ -326,13 +335,9 @@ gemm_simt_tile_kernel(float* __restrict__ out, const float* __restrict__ A, cons
 #pragma unroll
     for (int i = 0; i < TM; ++i)
 #pragma unroll
-      for (int j = 0; j < TN / 2; ++j) {                                   // kahan_add of two columns
-        const float2 chunk = make_float2(__fadd_rn(acc[i][2 * j].x, acc[i][2 * j].y), __fadd_rn(acc[i][2 * j + 1].x, acc[i][2 * j + 1].y));
-        const float2 y = sub2(chunk, comp[i][j]);
-        const float2 t = add2(sum[i][j], y);
-        comp[i][j] = sub2(sub2(t, sum[i][j]), y);
-        sum[i][j] = t;
-      }
+      for (int j = 0; j < TN / 2; ++j)
+        kahan_add_pair(sum[i][j], comp[i][j],
+                       make_float2(__fadd_rn(acc[i][2 * j].x, acc[i][2 * j].y), __fadd_rn(acc[i][2 * j + 1].x, acc[i][2 * j + 1].y)));
   }
 #pragma unroll
   for (int i = 0; i < TM; ++i) {
@@ -421,20 +426,15 @@ int gemm_simt(void* out, const void* A, const void* W, int M, int N, int K, int 
   }
   // narrow tiles: the rows the kernels above cannot read in packets of 16 bytes, and the library-free check of the
   // bfloat16 products
-  if (M > 32) {
-    constexpr int BM = 128, BN = 64, TM = 8, TN = 4;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
+  const auto narrow_tiles = [&](auto kernel, int bm, int bn, int threads) {
+    const dim3 grid((N + bn - 1) / bn, (M + bm - 1) / bm, batch);
     PTL_REQUIRE(grid.y <= 65535, "gemm_simt: M=%d too large", M);
-    return launch_kernel("gemm_simt", gemm_simt_kernel<TI, TO, BM, BN, TM, TN>, grid, dim3((BM / TM) * (BN / TN)), 0,
-                         as_stream(stream), (TO*)out, (const TI*)A, (const TI*)W, M, N, K, lda, ldw, ldo, accumulate,
-                         batch_a, batch_w, batch_o, gate, gate_ld);
-  } else {
-    constexpr int BM = 32, BN = 16, TM = 4, TN = 1;
-    dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, batch);
-    return launch_kernel("gemm_simt", gemm_simt_kernel<TI, TO, BM, BN, TM, TN>, grid, dim3((BM / TM) * (BN / TN)), 0,
-                         as_stream(stream), (TO*)out, (const TI*)A, (const TI*)W, M, N, K, lda, ldw, ldo, accumulate,
-                         batch_a, batch_w, batch_o, gate, gate_ld);
-  }
+    return launch_kernel("gemm_simt", kernel, grid, dim3(threads), 0, as_stream(stream), (TO*)out, (const TI*)A, (const TI*)W, M, N, K, lda, ldw,
+                         ldo, accumulate, batch_a, batch_w, batch_o, gate, gate_ld);
+  };
+  if (sizeof(TI) == 4 && K % 4 == 0)
+    return M > 32 ? narrow_tiles(gemm_simt_kernel<TI, TO, 64, 64, 4, 4, 2>, 64, 64, 256) : narrow_tiles(gemm_simt_kernel<TI, TO, 32, 16, 4, 1, 2>, 32, 16, 128);
+  return M > 32 ? narrow_tiles(gemm_simt_kernel<TI, TO, 128, 64, 8, 4, 1>, 128, 64, 256) : narrow_tiles(gemm_simt_kernel<TI, TO, 32, 16, 4, 1, 1>, 32, 16, 128);
 }
 
 // The heads' products of a step with few tokens, 16-bit operands: a warp per output feature o of a head reads the weight

@@ -1093,6 +1093,17 @@ def test_cuda_core_attention_gives_a_token_the_same_bits_whatever_its_company(op
     close(together[:len(ctx)], want, dtype, "against 64 bits")
 
 
+@pytest.mark.parametrize("M, N, K", [(40, 70, 36), (100, 130, 2052), (33, 17, 4), (70, 300, 1028)])
+def test_linear_float32_off_the_boundaries_gives_the_same_bits(ops, M, N, K):
+    """Rows that do not start at 16 bytes go to narrow tiles of any alignment: K a multiple of 4 is summed there as the other kernels do."""
+    x, w = rnd((M, K), torch.float32, 95).cuda(), rnd((N, K), torch.float32, 96).cuda()
+    off = torch.empty(M * K + 1, device="cuda")[1:].view(M, K).copy_(x)
+    assert off.data_ptr() % 16
+    want = ops.linear(x, w)
+    for rows in (M, 32, 1):
+        assert torch.equal(ops.linear(off[:rows], w), want[:rows]), rows
+
+
 @pytest.mark.parametrize("no_turn", [0, 3, 5])
 def test_float32_product_of_few_rows_gives_up_a_turn_that_does_not_come(_ops, no_turn):
     """No block asks for one of its turns (of the ring's first filling, and of a later one): the waits run out, the status is set, and the
