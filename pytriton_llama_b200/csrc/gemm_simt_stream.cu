@@ -225,6 +225,9 @@ static int stream_product(void* out, const void* A, const void* W, int M, int N,
   if (M < 1 || M > 32 || (M > 16 && !narrow) || N < 1 || K < 32 || K % 32 || lda < K || ldw < K || ldo < N || lda % 4 || ldw % 4 || !aligned16(A) ||
       !aligned16(W))
     return -2;
+  // Weights of a few hundred KB are there after one trip, and the kernel that copies them without a ring has less to set up: a row to 8 features
+  // of 32 1.5 us there and 1.9 here, to 256 of 1,024 2.0 and 2.3, to 2,048 of 256 2.4 and 2.1, to 512 of 2,048 3.5 both; two rows to 256 of 1,024 2.25 and 2.30.
+  if (M <= 2 && N <= (M == 1 ? 1024 : 256) && (long long)N * K <= 1 << 19) return -2;
 #define PTL_STREAM(MT, ROWS, WARPS, STAGES, HELD)                                                                               \
   return launch_stream<MT, ROWS, WARPS, STAGES, HELD>((float*)out, (const float*)A, (const float*)W, M, N, K, lda, ldw, ldo, accumulate, \
                                                 (int*)status, as_stream(stream), waits)
