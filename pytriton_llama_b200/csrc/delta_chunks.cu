@@ -327,21 +327,16 @@ delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, floa
   float* s_c = dw_smem;                                  // [2][WK 64 rows of LD | keys D rows of 68]
   float* s_s = s_c + 2 * kChunk;                         // [8][LD]: the state's columns
   float* s_u = s_s + kDcCols * LD;                       // [8][68]
-  pdl_wait();
-  pdl_launch_dependents();
+  // before the wait only the step's own integers, which the kernel before this one reads too; no block leaves before it
   const LongPortion at = locate_portion<true, kDcTokens>(q_start, requests, walk_max, blockIdx.z);
-  if (at.r < 0 || state_slot[at.r] < 0) return;
-  const int r = at.r, lo = at.lo, n = at.n, chunk0 = at.piece0, h = blockIdx.y, j0 = blockIdx.x * kDcCols;
+  const int slot = at.r < 0 ? -1 : state_slot[at.r];
+  const int lo = at.lo, n = at.n, chunk0 = at.piece0, h = blockIdx.y, j0 = blockIdx.x * kDcCols;
   const int chunks = (n + kDcTokens - 1) / kDcTokens;
   const int tid = threadIdx.x, lane = tid & 31, s = lane & 7, rg = (tid >> 5) * 4 + (lane >> 3);
   const size_t stride = (size_t)heads * dc_floats(D, dv);
   float* base = work + ((size_t)chunk0 * heads + h) * dc_floats(D, dv);
-  float* st = state + (((size_t)state_slot[r] * heads + h) * D) * dv + j0;
-  const bool from_zero = positions[lo] == 0;
-  for (int i = tid; i < D * kDcCols; i += kDcThreads) {
-    const int e = i / kDcCols, c = i % kDcCols;
-    s_s[c * LD + e] = from_zero ? 0.f : st[(size_t)e * dv + c];
-  }
+  float* st = state + (((size_t)slot * heads + h) * D) * dv + j0;
+  const bool from_zero = slot >= 0 && positions[lo] == 0;
   // one bulk copy a chunk (as copies of 16 bytes, 17 a thread, issuing them took 1,140 of a chunk's 4,400 cycles)
   const uint32_t full = smem_u32(s_u + kDcCols * kDcSysLd);
   volatile int* const abort_flag = reinterpret_cast<volatile int*>(s_u + kDcCols * kDcSysLd + 4);
@@ -351,6 +346,9 @@ delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, floa
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_wait();
+  pdl_launch_dependents();
+  if (slot < 0) return;
   auto fetch = [&](int chunk) {
     if (tid != 0 || chunk == waits.withheld) return;
     const uint32_t bar = full + 8 * (chunk & 1);
@@ -358,27 +356,35 @@ delta_chunk_walk_kernel(float* __restrict__ out, float* __restrict__ state, floa
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  ::"r"(smem_u32(s_c + (chunk & 1) * kChunk)), "l"(base + chunk * stride), "r"(kChunk * 4), "r"(bar) : "memory");
   };
+  // Waits for a chunk, the whole block.  One that does not come ends the walk with the status set: nothing else is in flight then, and the
+  // state in memory stays what it was.
+  auto here = [&](int chunk) {
+    const uint32_t bar = full + 8 * (chunk & 1), parity = chunk >> 1 & 1;
+    const bool came = mbar_wait(bar, parity, abort_flag, status, 31, waits.polls);
+    const bool lost = __syncthreads_or(!came);
+    if (lost && tid == 0) mbar_drain(bar, parity);
+    return !lost;
+  };
+  fetch(0);
+  for (int i = tid; i < D * kDcCols; i += kDcThreads) {
+    const int e = i / kDcCols, c = i % kDcCols;
+    s_s[c * LD + e] = from_zero ? 0.f : st[(size_t)e * dv + c];
+  }
   bool bad = false;
   for (int i = tid; i < chunks; i += kDcThreads) bad = bad || base[i * stride + dc_flags_at(D, dv) + 1] != 0.f;
   const bool walk = __syncthreads_or(bad);
   if (blockIdx.x == 0)
     for (int i = tid; i < chunks; i += kDcThreads) base[i * stride + dc_flags_at(D, dv) + 2] = walk ? 1.f : 0.f;
-  if (walk)
+  if (walk) {
+    if (!here(0)) return;                  // (the tokens' walk takes the chunk's place)
     dc_walk_tokens<T, D>(out + (size_t)lo * heads * dv, qkv + (size_t)lo * (2 * kv_heads * D + heads * dv), ba + (size_t)lo * 2 * heads, n,
                          rate[h], dt_bias[h], heads, kv_heads, dv, h, j0, unit_eps, q_scale, s_s, s_c);
-  else
-    fetch(0);
+  }
   for (int chunk = walk ? chunks : 0; chunk < chunks; ++chunk) {
     const float* wv = base + chunk * stride + dc_values_at(D);
     float* columns = base + chunk * stride + dc_columns_at(D, dv) + (size_t)j0 * (D + kDcTokens);
     const float v0 = wv[(size_t)rg * dv + j0 + s], v1 = wv[(size_t)(rg + 32) * dv + j0 + s], decay = wv[(size_t)kDcTokens * dv];
-    // this chunk is here; the chunk before has been read and its state written.  A chunk that does not come ends the walk with the
-    // status set: nothing else is in flight then, and the state in memory stays what it was
-    const bool came = mbar_wait(full + 8 * (chunk & 1), chunk >> 1 & 1, abort_flag, status, 31, waits.polls);
-    if (__syncthreads_or(!came)) {
-      if (tid == 0) mbar_drain(full + 8 * (chunk & 1), chunk >> 1 & 1);
-      return;
-    }
+    if (!here(chunk)) return;              // this chunk is here; the chunk before has been read and its state written
     if (chunk + 1 < chunks) fetch(chunk + 1);
     float first[2];
     dc_product<2, D, LD, LD>(s_c + (chunk & 1) * kChunk + rg * LD, s_s, s, first);
@@ -418,16 +424,14 @@ delta_chunk_outputs_kernel(float* __restrict__ out, const float* __restrict__ wo
   extern __shared__ __align__(16) float do_smem[];
   float* s_a = do_smem;                                  // [64 tokens][queries D | weights 64]
   float* s_b = s_a + kDcTokens * LA;                     // [64 columns][state D | U 64]
-  pdl_wait();
-  pdl_launch_dependents();
+  // (before the wait as in the walk)
   const LongPortion at = locate_portion<false, kDcTokens>(q_start, requests, walk_max, blockIdx.x);
-  if (at.r < 0 || state_slot[at.r] < 0) return;
+  const bool there = at.r >= 0 && state_slot[at.r] >= 0;
   const int first = ((int)blockIdx.x - at.piece0) * kDcTokens, h = blockIdx.y, n = min(kDcTokens, at.n - first), j0 = blockIdx.z * kDcOutCols;
   const int cols = min(kDcOutCols, dv - j0), tid = threadIdx.x;
   // (a warp is four rows by eight columns: a packet of either operand takes two turns of the shared memory, of sixteen columns four)
   const int tx = (tid >> 7) * 8 + (tid & 7), ty = (tid >> 5 & 3) * 4 + (tid >> 3 & 3);
   const float* base = work + ((size_t)blockIdx.x * heads + h) * dc_floats(D, dv);
-  if (base[dc_flags_at(D, dv) + 2] != 0.f) return;       // walked token by token
   const float *queries = base + dc_walk_floats(D), *columns = base + dc_columns_at(D, dv) + (size_t)j0 * K;
   // a bulk copy per row, all of them counted on one barrier
   const uint32_t full = smem_u32(s_b + kDcOutCols * LA);
@@ -439,6 +443,10 @@ delta_chunk_outputs_kernel(float* __restrict__ out, const float* __restrict__ wo
     mbar_expect_tx(full, (kDcTokens + cols) * K * 4);
   }
   __syncthreads();
+  pdl_wait();
+  pdl_launch_dependents();
+  if (!there) return;
+  const float walked = base[dc_flags_at(D, dv) + 2];     // (on its way while the copies are)
   if (tid < kDcTokens + cols && tid != waits.withheld) {
     const bool is_a = tid < kDcTokens;
     const int r = is_a ? tid : tid - kDcTokens;
@@ -452,6 +460,7 @@ delta_chunk_outputs_kernel(float* __restrict__ out, const float* __restrict__ wo
     if (tid == 0) mbar_drain(full, 0);
     return;
   }
+  if (walked != 0.f) return;                             // token by token, the outputs with it
   float sum[4][4];
 #pragma unroll
   for (int a = 0; a < 4; ++a)

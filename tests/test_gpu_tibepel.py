@@ -404,6 +404,12 @@ def test_chunk_attention_of_single_tokens_reads_no_further_than_its_table(ops):
     _single_tokens(ops, [70, 40, 63], 4, 2, 64, 16, 128, width=4)
 
 
+@pytest.mark.parametrize("H,G,d,dv", [(2, 1, 64, 72), (1, 1, 128, 120)])
+def test_gated_delta_rule_in_chunks_with_a_part_of_the_last_columns(ops, H, G, d, dv):
+    """Value widths whose second block of 64 columns is not whole."""
+    test_gated_delta_rule_in_chunks_of_64_tokens(ops, "float32", H, G, d, dv)
+
+
 @pytest.mark.parametrize("no_chunk,no_row,code", [(0, -1, 31), (2, -1, 31), (-1, 5, 32), (-1, 70, 32)])
 def test_delta_chunks_give_up_copies_that_do_not_come(ops, no_chunk, no_row, code):
     """A chunk of the walk, or a row of the outputs' operands, is never asked for: the waits run out, the status is set, the kernels end by
