@@ -58,7 +58,7 @@ struct SmallGemmParams {
 
 // EPI: 0 bfloat16 store, 1 float32 store, 2 add into the float32 residual
 template <int EPI>
-__global__ void __launch_bounds__(kSmallWarps * 32, 3)
+__global__ void __launch_bounds__(kSmallWarps * 32, kSmallResident)
 gemm_small_kernel(const SmallGemmParams p_in) {
   SmallGemmParams p = p_in;
   if (EPI == 0) {
@@ -212,10 +212,13 @@ static int gemm_small_impl(void* out, const void* X, const void* W, int M, int N
   const int row_elems = kSmallWarps * p.k_per_warp + kSmallPad;
   const size_t smem = (size_t)(kSmallRows + kSmallTokens) * row_elems * 2 + (kSmallWarps * kSmallRows * kSmallTokens + kSmallTokens) * 4;
   const int blocks = (N + kSmallRows - 1) / kSmallRows;
-  // As many blocks as are resident at once, by shared memory (registers allow five per SM).  Rows of 1,024 fit five blocks an SM, rows of 4,096
-  // one: 4,096 features of 1,024 and 1,024 of 4,096, eight tokens, took 5 to 6 us a launch of a step by the tcgen05 product, and a step of
-  // 114 launches 501 us where three blocks an SM and 74 KB a block were the line, 439 so.
-  const int per_sm = std::min(kSmallResident, (int)(kSmallSmemPerSm / (smem + 1024)));
+  // As many blocks as are resident at once, by shared memory and registers: rows of 1,024 fit five blocks an SM, rows of 4,096 one.  4,096 features
+  // of 1,024 and 1,024 of 4,096, eight tokens: a step of 114 launches 501 us by the tcgen05 product, 439 so.  From four tokens on the rows of
+  // tokens that every block fetches count as well, and many blocks of short rows lose: a product and the one back, eight tokens, us by the
+  // tcgen05 product and so: 4,736 features of 1,024 13.1 and 11.1 (four blocks an SM), 5,920 of 1,024 11.2 and 12.5, 4,736 of 768 9.0 and 11.1, 4,096
+  // of 512 7.5 and 7.7; two tokens 12.7 and 9.3, 11.0 both, 8.7 and 8.8, 7.2 and 6.5.
+  const int by_tokens = M <= 3 ? kSmallResident : K >= 1024 ? 4 : 3;
+  const int per_sm = std::min(by_tokens, (int)(kSmallSmemPerSm / (smem + 1024)));
   if (blocks > per_sm * sm_count_of_device()) return -2;
   if (xs) {
     if (epi != 2) return -2;

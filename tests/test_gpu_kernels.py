@@ -1057,6 +1057,8 @@ def test_product_for_a_few_tokens_and_small_weights(_ops, M, N, K):
 def test_product_for_a_few_tokens_up_to_the_blocks_an_sm_holds(_ops, M, N, K):
     """The most blocks of 148 SMs: five an SM (by registers) of short rows, one of long ones, the longest row that fits."""
     test_product_for_a_few_tokens_and_small_weights(_ops, M, N, K)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("d, page, window, splits", [(64, 16, 0, 1), (128, 16, 0, 1), (256, 8, 0, 1), (48, 16, 700, 1), (16, 4, 0, 1), (64, 16, 0, 3)])
 def test_cuda_core_attention_gives_a_token_the_same_bits_whatever_its_company(ops, dtype, d, page, window, splits):

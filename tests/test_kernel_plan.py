@@ -73,3 +73,10 @@ def test_steps_of_more_tiles_than_a_grid_holds_are_left_to_the_other_kernels(lib
                                                None, None, i(10), f, None) == -2
         assert lib.ptl_latent_prefill_bf16(p, p, p, p, p, *size(n, 4, 8, 512, 64, 16, 10), f, i(128), None) == -2
         assert lib.ptl_latent_decode_bf16(p, None, None, p, p, p, p, p, None, *size(n, 4, 8, 512, 64, 16, 10, 1), f, None) == -2
+
+
+def test_products_of_a_few_tokens_with_many_blocks_of_short_rows_are_left_to_the_other_product(lib):
+    """From four tokens on: beyond four blocks of eight features an SM, three where the rows have fewer than 1,024 values; and wherever shared memory holds fewer."""
+    p, i = ctypes.c_void_p(4096), ctypes.c_int
+    for M, N, K in [(4, 4744, 1024), (8, 5920, 1024), (4, 3560, 768), (8, 4096, 512), (1, 5928, 512), (3, 2376, 2560)]:
+        assert lib.ptl_gemm_small_bf16(p, p, p, i(M), i(N), i(K), i(N), i(0), None, None, None, i(0), None, None, i(0), i(0), ctypes.c_float(0.0), None) == -2
