@@ -195,11 +195,11 @@ chunk_attention_kernel(T* __restrict__ out, int out_ld, int column, const T* __r
 }
 
 // Single tokens of a bfloat16 cache with up to eight query heads over up to two kv heads of 64 or 128 entries, blocks of up to 256
-// positions: the same sums, a block per token whose sixteen warps share the keys.  A lane owns an eighth (or a quarter) of eight entries of
+// positions: the same sums, a block per token whose sixteen warps share the keys.  A lane owns four (heads of 64: two) neighbouring entries of
 // every head: four keys' products with eight heads meet in one butterfly that leaves a (key, head) in every lane, and for the
 // values the warps' sums meet in shared memory.  What bounds it: the trips to memory of its five steps, one after the other, and from some
-// hundred keys on their 512 bytes each through one SM.  Eight tokens of 8 heads of 128 at the end of 256 positions: 16.2 us, the kernel above
-// (a thread per key) 44.0; at 24 positions 7.2 and 15.2.
+// hundred keys on their 512 bytes each through one SM.  Eight tokens of 8 heads of 128 at the end of 256 positions: 15.8 us, the kernel above
+// (a thread per key) 43.8; at the 17th 6.3 and 14.6.
 constexpr int kCsThreads = 512, kCsWarps = kCsThreads / 32, kCsHeads = 8, kCsMaxBlock = 256;
 
 template <int D, int G>
@@ -223,40 +223,39 @@ chunk_attention_single_kernel(__nv_bfloat16* __restrict__ out, int out_ld, int c
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, group = H / G;
   const int p = positions[t], lo = p - p % chunk, n = min(p - lo + 1, table_width * page_size);      // (no more keys than the table can name)
   const size_t page_stride = (size_t)G * page_size * 2 * D, plane = (size_t)page_size * D;
-  // the queries (with their bias) of this lane's entries, for the warps that have keys to score; a place without a head holds zeros
+  // asked for together: the key's page, and the queries (with their bias) of this lane's entries, for the warps that have keys to score; a place
+  // without a head holds zeros
+  const int pos = lo + tid, page = tid < n ? block_table[(size_t)r * table_width + pos / page_size] : -1;
+  uint32_t raw[kCsHeads][E / 2];
+  float2 bias[kCsHeads][E / 2];
+#pragma unroll
+  for (int a = 0; a < kCsHeads; ++a) {
+    const bool there = 4 * warp < n && a % HG < group;
+    const int at = (a / HG * group + a % HG) * D + lane * E;
+#pragma unroll
+    for (int e = 0; e < E / 2; ++e) {
+      raw[a][e] = 0u;
+      bias[a][e] = make_float2(0.f, 0.f);
+    }
+    if (there) {
+      if constexpr (E == 4) *reinterpret_cast<uint2*>(raw[a]) = *reinterpret_cast<const uint2*>(qkv + (size_t)t * q_ld + at);
+      else raw[a][0] = *reinterpret_cast<const uint32_t*>(qkv + (size_t)t * q_ld + at);
+      if (q_bias) {
+#pragma unroll
+        for (int e = 0; e < E / 2; ++e) bias[a][e] = *reinterpret_cast<const float2*>(q_bias + at + 2 * e);
+      }
+    }
+  }
+  if (tid < n) s_at[tid] = page >= 0 && page < num_pages ? (long long)((size_t)page * page_stride + (size_t)(pos % page_size) * D) : -1;
   float q[kCsHeads][E];
 #pragma unroll
   for (int a = 0; a < kCsHeads; ++a)
 #pragma unroll
-    for (int e = 0; e < E; ++e) q[a][e] = 0.f;
-  if (4 * warp < n) {
-#pragma unroll
-    for (int a = 0; a < kCsHeads; ++a) {
-      if (a % HG >= group) continue;
-      const int at = (a / HG * group + a % HG) * D + lane * E;
-      uint32_t raw[E / 2];
-      if constexpr (E == 4) *reinterpret_cast<uint2*>(raw) = *reinterpret_cast<const uint2*>(qkv + (size_t)t * q_ld + at);
-      else raw[0] = *reinterpret_cast<const uint32_t*>(qkv + (size_t)t * q_ld + at);
-#pragma unroll
-      for (int e = 0; e < E; e += 2) {
-        const float2 v = unpack_bf16(raw[e / 2]);
-        q[a][e] = v.x;
-        q[a][e + 1] = v.y;
-      }
-      if (q_bias) {
-#pragma unroll
-        for (int e = 0; e < E; e += 2) {
-          const float2 b = *reinterpret_cast<const float2*>(q_bias + at + e);
-          q[a][e] += b.x;
-          q[a][e + 1] += b.y;
-        }
-      }
+    for (int e = 0; e < E; e += 2) {
+      const float2 v = unpack_bf16(raw[a][e / 2]);
+      q[a][e] = v.x + bias[a][e / 2].x;
+      q[a][e + 1] = v.y + bias[a][e / 2].y;
     }
-  }
-  if (tid < n) {
-    const int pos = lo + tid, page = block_table[(size_t)r * table_width + pos / page_size];
-    s_at[tid] = page >= 0 && page < num_pages ? (long long)((size_t)page * page_stride + (size_t)(pos % page_size) * D) : -1;
-  }
   if (talk && tid < H * H) s_talk[tid] = talk[tid];
   __syncthreads();
   // a lane's entries of a row of the cache
@@ -470,8 +469,9 @@ PTL_EXPORT int ptl_chunk_attention_single_bf16(void* out, int out_ld, int column
   PTL_REQUIRE((r1 == nullptr) == (r2 == nullptr) && page_size > 0 && num_pages > 0 && rows >= 0 && column >= 0 && column + H * d <= out_ld &&
                   q_ld >= H * d, "chunk_attention_single: bad sizes");
   // A block holds an SM (by its registers), and few heads in short blocks of positions have little for sixteen warps: beyond two turns of SMs
-  // they are left to the kernel above.  4 heads of 64 in blocks of 64, positions spread over them: 296 tokens 14.7 us there and 11.9 here, 600 17.8 and
-  // 22.4, 4 heads in blocks of 128 28.2 and 28.7; 8 heads of 128 in blocks of 256: 600 tokens 104 and 64 (all at the 17th position 20 and 31, all at the last 137 and 115).
+  // they are left to the kernel above.  Positions spread over the blocks, us there and here: 4 heads of 64 in blocks of 64, 296 tokens 14.7 and
+  // 11.5, 600 17.9 and 22.4; in blocks of 128 28.2 and 28.9; 8 heads of 128 in blocks of 256, 600 tokens 104 and 56 (all at the 17th position 20 and
+  // 26, all at the last 137 and 101).
   if (rows > 2 * sm_count_of_device() && H * chunk < 512) return -2;
   if (rows == 0) return 0;
   const auto fn = d == 64 ? G == 1 ? chunk_attention_single<64, 1> : chunk_attention_single<64, 2>
