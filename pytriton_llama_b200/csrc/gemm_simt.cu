@@ -355,8 +355,10 @@ gemm_simt_tile_kernel(float* __restrict__ out, const float* __restrict__ A, cons
 // Results per thread (10 TM + TN) of a product: the shape whose blocks the busiest SM is soonest done with, by what 1, 2, ...
 // blocks of a shape take side by side on an SM, up to as many as it holds (`us`, for 2,048 k values on a B200; blocks share its
 // FMA units, but one alone leaves them idle for its latencies).  Three of 5 x 4 stand for any number above two: the scheduler
-// spreads fewer than four per SM unevenly, 416 blocks take 173 us, 444 138.  Against the best of the four for
-// 33 to 2,048 rows, odd numbers of tiles among them, 512 to 16,384 features and 1,024 to 8,192 k values: 0.2 % slower on average, 10 % at most.
+// spreads fewer than four per SM unevenly, 416 blocks took 173 us, 444 138.  The times are those of scalar FMAs.  With packed ones even numbers of blocks take 85, 138 and
+// 195 us (8 x 4), 60, 94, 133 and 171 (5 x 4), 51, 78, 109 and 141 (4 x 4): the same order but for two of 4 x 4, which a
+// single one of 8 x 4 is still preferred to, 8 % slower.  Against the best of the three for 153 sizes of 33 to 2,048 rows, 512 to 16,384
+// features and 1,024 to 8,192 k values: 0.9 % slower on average, 8.8 % at most.
 inline int simt_tile(int M, int N, int batch) {
   constexpr struct { int tm, tn, held; float us[4]; } shapes[] = {
       {8, 4, 3, {88.f, 193.f, 203.f}}, {5, 4, 4, {64.f, 109.f, 170.f, 181.f}}, {4, 4, 4, {56.f, 98.f, 116.f, 152.f}}};

@@ -8,8 +8,8 @@
 // one chunk for a quarter of the weight rows and all token rows.  A chunk is a 128-byte row of the TMA tile: with the 128-byte swizzle the
 // eight chunks of a quarter warp lie in different banks.
 // The form by cp.async (gemm_simt_few, which keeps what is no multiple of 32) has a warp copy its own turns, 24 instructions a lane and
-// turn, and wait for them with nothing else in flight: 4 rows to 16,384 features of 2,048 35.5 us there and 25.6 here, to 128,256 features
-// 236 and 162 (6.5 TB/s), 2,048 features of 8,192 24.7 and 18.9; 16 rows to 16,384 features 88 and 49.
+// turn, and wait for them with nothing else in flight, us there and here: 4 rows to 16,384 features of 2,048 34 and 24, to 32,000 of 1,024 40 and
+// 22, 2,048 features of 8,192 24 and 18; 16 rows to 16,384 features 85 and 48; a row to 16,384 27 and 21.
 #include <algorithm>
 #include "tcgen05_utils.cuh"
 

@@ -1283,8 +1283,9 @@ class CudaOps:
         return out
 
     # The longest portion that the gated delta rule walks token by token; every request goes by its own length.  The walk costs
-    # 0.35 us a token and runs beside others' walks (8 heads of 128: 128 tokens 49 us walked, 49 in chunks; four of them 57 and 77, 16 of
-    # them 220 and 178; one of 160 tokens 60 and 53; of 2,048: 718 and 166).
+    # 0.36 us a token and runs beside others' walks (8 heads of 128: 128 tokens 50 us walked, 47 in chunks; four of them 58 and 75, 16 of
+    # them 224 and 162; 112 tokens 44 and 47; 160 62 and 49, four of them 71 and 83; 2,048: 738 and 136.  4 heads of 64: 96 tokens 32 and
+    # 31, 16 of 128 tokens 51 and 50).
     DELTA_WALK_MAX_TOKENS = 128
 
     def gated_delta_rule(self, qkv: torch.Tensor, ba: torch.Tensor, rate: torch.Tensor, dt_bias: torch.Tensor, state: torch.Tensor,
